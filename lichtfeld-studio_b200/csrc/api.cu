@@ -391,7 +391,7 @@ int lfs_rasterize_to_pixels_from_world_3dgs_bwd(int N, int64_t n_isects, int cha
                  nullptr, W, H, (W + 15) / 16, (H + 15) / 16, eff_model, channels, 0, masks, nullptr, rolling};
     rc = launch_raster_bwd(a, render_alphas, last_ids, nullptr, v_render_colors, v_render_alphas, accum, accum_extra, S(stream));
     if (rc != LFS_OK) return rc;
-    return launch_grad_epilogue_op(N, cam, accum, means, quats, scales, channels, accum_extra, v_means, v_quats, v_scales,
+    return launch_grad_epilogue_op(N, cam, accum, records, means, quats, scales, channels, accum_extra, v_means, v_quats, v_scales,
                                    v_colors, v_opacities, S(stream));
 }
 

@@ -81,11 +81,14 @@ inline int effective_model(int model, const float* radial, const float* tangenti
     return (model == LFS_PINHOLE && (radial || tangential || thin_prism)) ? LFS_PINHOLE_OPENCV : model;
 }
 
-// One packed 64-byte record per Gaussian for the rasterizer:
-//   r0 = (M00, M01, M02, gro.x)   M = diag(1/scale) * R^T
-//   r1 = (M10, M11, M12, gro.y)   gro = M * (ray_origin - mean)
-//   r2 = (M20, M21, M22, gro.z)
+// One packed 64-byte record per Gaussian for the rasterizer. Cameras with one ray origin (global shutter), d = the pixel's
+// camera-space direction, (e1, e2, w) = (p1, p2, p3) . d, phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) (RayFrame in gsmath.cuh):
+//   r0 = (p1, c)              c = -|g|^2 log2(e) / 2: the response is exp2(c phi)
+//   r1 = (p2, phi_max)        p2.x = 0 for the planar models (pinhole, OpenCV); alpha < 1/255 for certain when phi > phi_max
+//   r2 = (p3, 0)
 //   r3 = (red, green, blue, opacity)
+// Rolling shutter, where the ray origin differs from pixel to pixel:
+//   r0 .. r2 = rows of M = diag(1/scale) R^T, each followed by its element of gro = M (start-pose origin - mean); r3 as above
 constexpr int kRecordFloats = 16;
 
 // Host-side launchers shared between translation units (all asynchronous on `st`).

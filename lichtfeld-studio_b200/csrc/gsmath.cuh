@@ -247,6 +247,18 @@ __device__ __forceinline__ bool image_to_cam_ray(const CamDev& c, float px, floa
     }
 }
 
+// Camera-space direction of a pixel centre, not normalised: (x, y, 1) for the planar models.
+template <int MODEL>
+__device__ __forceinline__ bool pixel_cam_dir(const CamDev& c, float px, float py, f3& d) {
+    if (MODEL == LFS_PINHOLE) {
+        d = {(px - c.cx) / c.fx, (py - c.cy) / c.fy, 1.f};
+        return true;
+    }
+    const bool valid = image_to_cam_ray<MODEL>(c, px, py, d);
+    if (MODEL == LFS_PINHOLE_OPENCV) d = {d.x / d.z, d.y / d.z, 1.f};
+    return valid;
+}
+
 // World-space ray direction of a pixel centre.
 template <int MODEL>
 __device__ __forceinline__ bool pixel_world_dir(const CamDev& c, float px, float py, f3& d) {
@@ -383,6 +395,72 @@ __device__ __forceinline__ void sh_basis(int degree, float dx, float dy, float d
     B[17] = fTmp2B * fS2;
     B[24] = 0.6258357354491763f * fC3;
     B[16] = 0.6258357354491763f * fS3;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Ray frame of a Gaussian, for cameras whose rays share one origin (global shutter).
+//
+// With M = S^-1 R^T, g = M (o - mu) and u = M d the squared distance of the ray (o, d) from the centre in whitened space is
+// P = |u x g|^2 / |u|^2 = |g|^2 sin^2(u, g). In an orthonormal whitened frame O whose third row is -g/|g| this is
+// P = |g|^2 (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) with (e1, e2, w) = O M d: three linear forms of the pixel direction instead of
+// a matrix product, a cross product and two norms. O is free to turn about g; row 2 is taken along M (axis x g) so that
+// the form of e2 in camera space has the closed form v / sqrt(v^T Sigma v), v = e_x x mu_c, whose x coefficient is 0.
+// P does not change when the three forms are scaled together; callers scale them by |mu_c| / |g| (w near 1 at the centre).
+// ---------------------------------------------------------------------------------------------
+struct RayFrame {
+    float O[9];     // rows: directions of e1, e2, w in whitened space
+    float gamma;    // |g|; g = -gamma * (row 3)
+    float V[9];     // camera-space axes of the Gaussian: column i of Rc R
+    float m[3];     // camera-space mean
+    float v[3];     // numerator of the form of e2
+    float inv_nv;   // 1 / sqrt(v^T Sigma v)
+};
+__device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 om, f3 scale, const float* is, RayFrame& f) {
+    // Rinv m = mu - o. Rinv is a rotation only up to rounding, so its transpose misses the solution by about 1e-7 rad, the
+    // same way for every Gaussian: one step of refinement
+#pragma unroll
+    for (int a = 0; a < 3; ++a) f.m[a] = -(cam.Rinv[a] * om.x + cam.Rinv[3 + a] * om.y + cam.Rinv[6 + a] * om.z);
+    float res[3];
+    const float o3[3] = {om.x, om.y, om.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        res[a] = fmaf(cam.Rinv[a * 3 + 2], f.m[2], fmaf(cam.Rinv[a * 3 + 1], f.m[1], fmaf(cam.Rinv[a * 3], f.m[0], o3[a])));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        f.m[a] -= cam.Rinv[a] * res[0] + cam.Rinv[3 + a] * res[1] + cam.Rinv[6 + a] * res[2];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            f.V[a * 3 + i] = cam.Rinv[a] * R[i] + cam.Rinv[3 + a] * R[3 + i] + cam.Rinv[6 + a] * R[6 + i];
+    }
+    f.v[0] = 0.f; f.v[1] = -f.m[2]; f.v[2] = f.m[1];
+    const bool planar = cam.model == LFS_PINHOLE || cam.model == LFS_PINHOLE_OPENCV;
+    const float yz = f.m[1] * f.m[1] + f.m[2] * f.m[2];
+    // a wide camera can have the centre along its own x axis: the y axis serves there
+    if (!planar && yz < 1e-6f * (f.m[0] * f.m[0] + yz)) { f.v[0] = f.m[2]; f.v[1] = 0.f; f.v[2] = -f.m[0]; }
+    float r2[3], r3[3];
+    const float sc[3] = {scale.x, scale.y, scale.z};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        r2[i] = sc[i] * (f.V[i] * f.v[0] + f.V[3 + i] * f.v[1] + f.V[6 + i] * f.v[2]);
+        r3[i] = -is[i] * (R[i] * om.x + R[3 + i] * om.y + R[6 + i] * om.z);
+    }
+    const float n2 = r2[0] * r2[0] + r2[1] * r2[1] + r2[2] * r2[2];
+    f.gamma = sqrtf(r3[0] * r3[0] + r3[1] * r3[1] + r3[2] * r3[2]);
+    if (f.m[0] == 0.f && f.m[1] == 0.f && f.m[2] == 0.f) {   // the camera sits on the centre: P = 0 along every ray
+#pragma unroll
+        for (int k = 0; k < 9; ++k) f.O[k] = 0.f;
+        f.O[8] = 1.f;
+        f.gamma = 0.f;
+        f.inv_nv = 0.f;
+        return;
+    }
+    f.inv_nv = 1.0f / sqrtf(n2);
+    const float i3 = 1.0f / f.gamma;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) { f.O[3 + i] = r2[i] * f.inv_nv; f.O[6 + i] = r3[i] * i3; }
+    f.O[0] = f.O[4] * f.O[8] - f.O[5] * f.O[7];
+    f.O[1] = f.O[5] * f.O[6] - f.O[3] * f.O[8];
+    f.O[2] = f.O[3] * f.O[7] - f.O[4] * f.O[6];
 }
 
 // Tile rectangle covered by a projected Gaussian: [x0,x1) x [y0,y1) in tile units. The float ->

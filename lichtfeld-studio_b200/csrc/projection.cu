@@ -320,8 +320,7 @@ int launch_projection_ut(int C, int N, const float* means, const float* quats, c
 }
 
 // ---------------------------------------------------------------------------------------------
-// Rasterizer record from activated parameters: M = diag(1/s) R^T with the quaternion
-// re-normalised, gro = M (ray_origin - mean).
+// Rasterizer record from activated parameters (layout in common.cuh) with the quaternion re-normalised.
 // ---------------------------------------------------------------------------------------------
 // Also computes the exact screen-space bounding box (in whole pixels, inclusive, clamped to 16 bits) of the
 // pixels whose ray can reach alpha >= 1/255: alpha = opacity * exp(-d^2/2) with d the distance from the ray to
@@ -376,18 +375,41 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         }
     }
     const float is[3] = {1.0f / scale.x, 1.0f / scale.y, 1.0f / scale.z};
-    float M[9];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) M[a * 3 + c] = is[a] * R[c * 3 + a];
     const f3 om{cam.ro[0] - mean.x, cam.ro[1] - mean.y, cam.ro[2] - mean.z};
-    const float g0 = M[0] * om.x + M[1] * om.y + M[2] * om.z;
-    const float g1 = M[3] * om.x + M[4] * om.y + M[5] * om.z;
-    const float g2 = M[6] * om.x + M[7] * om.y + M[8] * om.z;
-    rec[0] = make_float4(M[0], M[1], M[2], g0);
-    rec[1] = make_float4(M[3], M[4], M[5], g1);
-    rec[2] = make_float4(M[6], M[7], M[8], g2);
+    if (cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {
+        RayFrame f;
+        ray_frame(cam, R, om, scale, is, f);
+        const float m2 = f.m[0] * f.m[0] + f.m[1] * f.m[1] + f.m[2] * f.m[2];
+        const float lambda = m2 > 0.f ? sqrtf(m2) / f.gamma : 1.0f;
+        float p1[3], p3[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            p1[k] = lambda * (f.O[0] * is[0] * f.V[k * 3] + f.O[1] * is[1] * f.V[k * 3 + 1] + f.O[2] * is[2] * f.V[k * 3 + 2]);
+            p3[k] = lambda * (f.O[6] * is[0] * f.V[k * 3] + f.O[7] * is[1] * f.V[k * 3 + 1] + f.O[8] * is[2] * f.V[k * 3 + 2]);
+        }
+        // e1 vanishes along the ray through the centre: what rounding left of p1 . mu_c is taken out again
+        const float t = fmaf(p1[2], f.m[2], fmaf(p1[1], f.m[1], p1[0] * f.m[0])) / fmaxf(m2, 1e-30f);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p1[k] = fmaf(-t, f.m[k], p1[k]);
+        const float n2 = lambda * f.inv_nv;
+        const float G = f.gamma * f.gamma;
+        rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
+        rec[1] = make_float4(f.v[0] * n2, f.v[1] * n2, f.v[2] * n2, -2.0f * __uint_as_float(thr_bits) / fmaxf(G, 1e-30f));
+        // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
+        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], 0.f) : make_float4(0.6101f, 0.5303f, 0.5887f, 0.f);
+    } else {
+        float M[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) M[a * 3 + c] = is[a] * R[c * 3 + a];
+        const float g0 = M[0] * om.x + M[1] * om.y + M[2] * om.z;
+        const float g1 = M[3] * om.x + M[4] * om.y + M[5] * om.z;
+        const float g2 = M[6] * om.x + M[7] * om.y + M[8] * om.z;
+        rec[0] = make_float4(M[0], M[1], M[2], g0);
+        rec[1] = make_float4(M[3], M[4], M[5], g1);
+        rec[2] = make_float4(M[6], M[7], M[8], g2);
+    }
     rec[3] = make_float4(r, g, b, opacity);
 }
 

@@ -8,16 +8,16 @@
 // Design (instruction-issue bound, no tensor cores: the largest contraction is 3x3):
 //  * one CTA per 16x16 tile, one thread per pixel, warps cover 8x4 pixel patches;
 //  * the tile's depth-sorted Gaussians are staged in shared memory in batches (192 records forward, 64 backward) of
-//    packed 64-byte records (M = S^-1 R^T, gro = M (o - mu), colour, opacity) built once per Gaussian,
-//    so no quaternion -> matrix work is repeated per tile or per pixel;
+//    packed 64-byte records built once per Gaussian, so no per-Gaussian work is repeated per tile or per pixel;
 //  * per warp, a ballot over the batch keeps the records whose screen-space box overlaps the warp's 8x4 patch;
-//  * per pair the response is -0.5 |u x gro|^2 / |u|^2 with u = M d (same value as the normalised
-//    cross-product form), preceded by an exp-free conservative rejection test;
-//  * backward: every (warp, Gaussian) contribution is 16 numbers that are LINEAR in the per-pixel
-//    terms (sum v_u (x) d, sum v_gro, v_rgb, v_opacity). They are summed over the warp by a transpose through
-//    padded shared-memory rows (warp_reduce16), combined across the 8 warps by shared-memory atomics, and leave the
-//    CTA as four float4 reductions per (tile, Gaussian). The nonlinear quaternion / scale VJP runs once per Gaussian
-//    in the epilogue instead of once per pixel pair.
+//  * per pair the response is exp(-|g|^2 phi / 2), phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) with three linear forms of the
+//    pixel direction (RayFrame, gsmath.cuh): 10 instructions up to the exp-free rejection test for the planar camera models
+//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840: forward 624 -> 430 us, backward 1441 -> 1065);
+//  * backward: every (warp, Gaussian) contribution is 12 numbers that are LINEAR in the per-pixel terms (kSums). They
+//    are summed over the warp by a transpose through padded shared-memory rows (warp_reduce), combined across the 8 warps
+//    by shared-memory atomics, and leave the CTA as 16-byte reductions per (tile, Gaussian). The nonlinear quaternion / scale
+//    VJP runs once per Gaussian in the epilogue instead of once per pixel pair;
+//  * a rolling shutter gives every pixel its own ray origin: the RS instantiations keep u = M d and 16 sums.
 #include "gsmath.cuh"
 #include "raster.cuh"
 
@@ -47,6 +47,30 @@ __device__ __forceinline__ void warp_patch(int tile, int tw, uint32_t& px, uint3
 __device__ __forceinline__ bool box_overlaps(uint2 box, uint32_t px, uint32_t py) {
     return (box.x & 0xFFFFu) <= (px >> 16) && (box.x >> 16) >= (px & 0xFFFFu) &&
            (box.y & 0xFFFFu) <= (py >> 16) && (box.y >> 16) >= (py & 0xFFFFu);
+}
+
+// The three linear forms of a record (common.cuh) at a pixel direction. For the planar models d = (x, y, 1), p2.x = 0.
+struct RayForms { float e1, e2, w, E, den; };
+template <int MODEL>
+__device__ __forceinline__ RayForms ray_forms(const float4& r0, const float4& r1, const float4& r2, const f3& d) {
+    RayForms f;
+    if (MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV) {
+        f.e1 = r0.x * d.x + (r0.y * d.y + r0.z);
+        f.e2 = r1.y * d.y + r1.z;
+        f.w = r2.x * d.x + (r2.y * d.y + r2.z);
+    } else {
+        f.e1 = r0.x * d.x + (r0.y * d.y + r0.z * d.z);
+        f.e2 = r1.x * d.x + (r1.y * d.y + r1.z * d.z);
+        f.w = r2.x * d.x + (r2.y * d.y + r2.z * d.z);
+    }
+    f.E = f.e1 * f.e1 + f.e2 * f.e2;
+    f.den = f.w * f.w + f.E;
+    return f;
+}
+__device__ __forceinline__ float exp2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 __device__ __forceinline__ int32_t load_count(const int32_t* n_dev, int64_t n_host) {
@@ -149,7 +173,7 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
     const CamDev& cam = cams[0];
     f3 d, oo{0.f, 0.f, 0.f};
     const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
-                           : pixel_world_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
+                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
     bool done = !inside || !ray_ok;
     uint32_t patch_x, patch_y;
     warp_patch(tile, tw, patch_x, patch_y);
@@ -202,25 +226,29 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                     const int t = w * 32 + __ffs(bits) - 1;
                     bits &= bits - 1;
                     const float4 r0 = st.rec[t * 4 + 0], r1 = st.rec[t * 4 + 1], r2 = st.rec[t * 4 + 2];
-                    const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
-                    const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
-                    const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
-                    float gx = r0.w, gy = r1.w, gz = r2.w;
-                    if (RS) {
-                        gx += r0.x * oo.x + r0.y * oo.y + r0.z * oo.z;
-                        gy += r1.x * oo.x + r1.y * oo.y + r1.z * oo.z;
-                        gz += r2.x * oo.x + r2.y * oo.y + r2.z * oo.z;
+                    float alpha;
+                    if (!RS) {
+                        const RayForms f = ray_forms<MODEL>(r0, r1, r2, d);
+                        if (f.E > r1.w * f.den) continue;
+                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * exp2_approx(r0.w * __fdividef(f.E, f.den)));
+                    } else {
+                        const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
+                        const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
+                        const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
+                        const float gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
+                        const float gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
+                        const float gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
+                        const float cx = uy * gz - gy * uz;
+                        const float cy = uz * gx - gz * ux;
+                        const float cz = ux * gy - gx * uy;
+                        const float cc = cx * cx + cy * cy + cz * cz;
+                        const float uu = ux * ux + uy * uy + uz * uz;
+                        // power = -0.5 cc / uu ; reject when power < thr  <=>  cc > -2 thr uu
+                        if (cc > -2.0f * __uint_as_float(st.box[t].z) * uu) continue;
+                        const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
+                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * __expf(power));
                     }
-                    const float cx = uy * gz - gy * uz;
-                    const float cy = uz * gx - gz * ux;
-                    const float cz = ux * gy - gx * uy;
-                    const float cc = cx * cx + cy * cy + cz * cz;
-                    const float uu = ux * ux + uy * uy + uz * uz;
-                    // power = -0.5 cc / uu ; reject when power < thr  <=>  cc > -2 thr uu
-                    if (cc > -2.0f * __uint_as_float(st.box[t].z) * uu) continue;
                     const float4 r3 = st.rec[t * 4 + 3];
-                    const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
-                    const float alpha = fminf(0.999f, r3.w * __expf(power));
                     if (alpha < kAlphaMin) continue;
                     const float next_T = T * (1.0f - alpha);
                     if (next_T <= 1e-4f) { done = true; break; }
@@ -259,18 +287,19 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
 }
 
 // ---------------------------------------------------------------------------------------------
-// 16 values per lane -> per-value sums over the warp, value k left in lanes 2k and 2k+1.
-// The transpose goes through shared memory owned by the warp instead of a shuffle butterfly (about 40 issue slots
-// against 90): row k (36 floats, 32 used) holds value k of the 32 lanes. The row stride of 36 floats puts the 16-byte
+// NS values per lane -> per-value sums over the warp, value k left in lanes 2k and 2k+1 (lanes from 2 NS on repeat the last).
+// The transpose goes through shared memory owned by the warp instead of a shuffle butterfly (for 16 values about 40 issue
+// slots against 90): row k (36 floats, 32 used) holds value k of the 32 lanes. The row stride of 36 floats puts the 16-byte
 // loads of one quarter-warp (lane = 2 k + h reads the 16 lanes of half h of row k) on eight different bank groups, and
 // the scalar stores of one row are contiguous. The closing shuffle needs every lane's sum, hence every lane's loads,
 // before any lane returns, so the next call may overwrite the rows.
 constexpr int kRedStride = 36;
-__device__ __forceinline__ float warp_reduce16(const float (&v)[16], float* __restrict__ red, int lane) {
+template <int NS>
+__device__ __forceinline__ float warp_reduce(const float (&v)[NS], float* __restrict__ red, int lane) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) red[k * kRedStride + lane] = v[k];
+    for (int k = 0; k < NS; ++k) red[k * kRedStride + lane] = v[k];
     __syncwarp();
-    const float4* half = reinterpret_cast<const float4*>(red + (lane >> 1) * kRedStride + 16 * (lane & 1));
+    const float4* half = reinterpret_cast<const float4*>(red + min(lane >> 1, NS - 1) * kRedStride + 16 * (lane & 1));
     float s = 0.f;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -286,14 +315,19 @@ __device__ __forceinline__ float __reduce_add_sync_f32(float x) {
     return x;
 }
 
-template <int BATCH>
+// Sums per (warp, Gaussian). One ray origin: 12 = sums over the pixels of, with q = vis dL/dalpha (the opacity term),
+// omega = w / den and phi = E / den,
+//   q omega e1, q omega e2 | the same two times phi | q omega^2 e1^2, q omega^2 e1 e2, q omega^2 e2^2 | q phi | rgb | q
+// Rolling shutter: 16 = sum v_u (x) d, sum v_gro, rgb, opacity.
+constexpr int kSums = 12, kSumsRs = 16;
+template <int BATCH, int NS>
 struct BwdShared {
     Stage<BATCH> stage[3];       // batch b is walked while b+1 and b+2 are in flight
     uint32_t sid[4][BATCH];      // Gaussian index per slot; four deep: batch b+2 is staged while batch b-1 is flushed
-    float sacc[2][BATCH * 16];   // per-slot sums of the batch being walked / the batch being flushed
+    float sacc[2][BATCH * NS];   // per-slot sums of the batch being walked / the batch being flushed
     float sextra[2][BATCH];
     int stouched[2][BATCH];
-    float red[kBlock / 32][16 * kRedStride];  // per-warp transpose rows of warp_reduce16
+    float red[kBlock / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
 };
 
 // EXTRA: the output has 1 or 4 channels and its last one blends bounds.w (see the forward). XGRAD: also return
@@ -310,7 +344,8 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
     const float* __restrict__ v_render, const float* __restrict__ v_alphas, float* __restrict__ accum,
     float* __restrict__ accum_extra) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BwdShared<BATCH>& sm = *reinterpret_cast<BwdShared<BATCH>*>(smem_raw);
+    constexpr int NS = RS ? kSumsRs : kSums;
+    BwdShared<BATCH, NS>& sm = *reinterpret_cast<BwdShared<BATCH, NS>*>(smem_raw);
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
@@ -321,7 +356,7 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
     const CamDev& cam = cams[0];
     f3 d, oo{0.f, 0.f, 0.f};
     const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
-                           : pixel_world_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
+                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
     const bool active = inside && ray_ok;
     const int pid = min(i * W + j, W * H - 1);
     uint32_t patch_x, patch_y;
@@ -334,7 +369,6 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
 
     const float T_final = 1.0f - render_alphas[pid];
     float T = T_final;
-    float bufr = 0.f, bufg = 0.f, bufb = 0.f, bufx = 0.f;
     const int32_t bin_final = active ? last_ids[pid] : 0;
     float vcr, vcg, vcb, vcx = 0.f;
     float v_a = v_alphas ? v_alphas[pid] : 0.f;
@@ -356,18 +390,20 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
         if (!EXTRA || channels == 4) bg_dot = background[0] * vcr + background[1] * vcg + background[2] * vcb;
         if (EXTRA) bg_dot += background[channels - 1] * vcx;
     }
-    const float tail_c = T_final * (v_a - bg_dot);
+    // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
+    // (colour . v_colour) alpha T of every entry behind
+    float behind = T_final * (v_a - bg_dot);
     const int32_t warp_bin_final = __reduce_max_sync(0xffffffffu, bin_final);
     const int lane = threadIdx.x & 31;
     float* red = sm.red[threadIdx.x >> 5];
 
     for (int e = threadIdx.x; e < 2 * BATCH; e += kBlock) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) (&sm.sacc[0][0])[e * 16 + k] = 0.f;
+        for (int k = 0; k < NS; ++k) (&sm.sacc[0][0])[e * NS + k] = 0.f;
         (&sm.sextra[0][0])[e] = 0.f;
         (&sm.stouched[0][0])[e] = 0;
     }
-    // flush the sums of batch k (four 16-byte reductions per touched Gaussian) and leave its buffers zeroed
+    // flush the sums of batch k (16-byte reductions per touched Gaussian) and leave its buffers zeroed
     auto flush = [&](int k) {
         const int size_k = min(BATCH, range_end - k * BATCH - range_start);
         float* acc_k = sm.sacc[k & 1];
@@ -375,9 +411,9 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
             if (sm.stouched[k & 1][e]) {
                 const uint32_t g = sm.sid[k & 3][e];
                 float4* dst = reinterpret_cast<float4*>(accum) + (size_t)g * 4;
-                float4* src = reinterpret_cast<float4*>(acc_k) + e * 4;
+                float4* src = reinterpret_cast<float4*>(acc_k) + e * (NS / 4);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < NS / 4; ++q) {
                     atomicAdd(dst + q, src[q]);
                     src[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
@@ -435,74 +471,90 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
                 // the image, beyond their last contributor or below the alpha threshold continue with alpha = vis = 0,
                 // which makes every term they add exactly zero, so no per-lane branching is needed below.
                 const float4 r0 = st.rec[t * 4 + 0], r1 = st.rec[t * 4 + 1], r2 = st.rec[t * 4 + 2];
-                const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
-                const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
-                const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
-                float gx = r0.w, gy = r1.w, gz = r2.w;
-                if (RS) {
-                    gx += r0.x * oo.x + r0.y * oo.y + r0.z * oo.z;
-                    gy += r1.x * oo.x + r1.y * oo.y + r1.z * oo.z;
-                    gz += r2.x * oo.x + r2.y * oo.y + r2.z * oo.z;
+                bool valid = active && (batch_end - t <= bin_final);
+                float vis;
+                RayForms f;
+                float ux, uy, uz, gx, gy, gz, inv;
+                if (!RS) {
+                    f = ray_forms<MODEL>(r0, r1, r2, d);
+                    valid = valid && !(f.E > r1.w * f.den);
+                } else {
+                    ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
+                    uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
+                    uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
+                    gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
+                    gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
+                    gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
+                    const float cx = uy * gz - gy * uz;
+                    const float cy = uz * gx - gz * ux;
+                    const float cz = ux * gy - gx * uy;
+                    const float cc = cx * cx + cy * cy + cz * cz;
+                    const float uu = ux * ux + uy * uy + uz * uz;
+                    valid = valid && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
+                    inv = rsqrtf(fmaxf(uu, 1e-37f));
+                    vis = -0.5f * (cc * (inv * inv));
                 }
-                float cx = uy * gz - gy * uz;
-                float cy = uz * gx - gz * ux;
-                float cz = ux * gy - gx * uy;
-                const float cc = cx * cx + cy * cy + cz * cz;
-                const float uu = ux * ux + uy * uy + uz * uz;
-                bool valid = active && (batch_end - t <= bin_final) && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
                 if (!__any_sync(0xffffffffu, valid)) continue;
                 const float4 r3 = st.rec[t * 4 + 3];
-                const float inv = rsqrtf(fmaxf(uu, 1e-37f));
-                cx *= inv; cy *= inv; cz *= inv;  // cross(normalised u, gro)
-                const float power = -0.5f * (cx * cx + cy * cy + cz * cz);
-                float vis = __expf(power);
+                float rden = 0.f, phi = 0.f;
+                if (!RS) {
+                    rden = __fdividef(1.0f, f.den);
+                    phi = f.E * rden;
+                    vis = exp2_approx(r0.w * phi);
+                } else {
+                    vis = __expf(vis);
+                }
                 float alpha = fminf(0.999f, r3.w * vis);
                 valid = valid && !(alpha < kAlphaMin);
                 if (!__any_sync(0xffffffffu, valid)) continue;
                 if (!valid) { vis = 0.f; alpha = 0.f; }
-                float v[16];
+                float v[NS];
                 {
                     const float ra = __frcp_rn(1.0f - alpha);
                     T *= ra;
                     const float fac = alpha * T;
-                    v[12] = fac * vcr; v[13] = fac * vcg; v[14] = fac * vcb;
-                    float v_alpha = (r3.x * T - bufr * ra) * vcr + (r3.y * T - bufg * ra) * vcg + (r3.z * T - bufb * ra) * vcb;
-                    float xval = 0.f;
-                    if (EXTRA) {
-                        xval = __uint_as_float(st.box[t].w);
-                        v_alpha += (xval * T - bufx * ra) * vcx;
-                    }
-                    v_alpha += ra * tail_c;  // T_final * ra * (v_alpha_out - background . v_colour_out)
+                    // colour . v_colour of this entry: the colours only ever meet the output gradient in this product
+                    float cv = r3.x * vcr + r3.y * vcg + r3.z * vcb;
+                    if (EXTRA) cv += __uint_as_float(st.box[t].w) * vcx;
+                    const float v_alpha = cv * T + ra * behind;
+                    behind -= cv * fac;
                     // geometry and opacity only while alpha is not clamped at 0.999
                     const float gate = (r3.w * vis <= 0.999f) ? vis : 0.f;
-                    const float s = -gate * (r3.w * v_alpha);  // v_c = s * c with c = n x g
-                    // with n = u / |u|, gn = g . n and w = gn n - g (minus the part of g orthogonal to n):
-                    //   v_g = v_c x n = -s w,   v_u = (v_n - (v_n . n) n) / |u| = (s gn / |u|) w
-                    const float nx = ux * inv, ny = uy * inv, nz = uz * inv;
-                    const float gn = gx * nx + gy * ny + gz * nz;
-                    const float wx = gn * nx - gx, wy = gn * ny - gy, wz = gn * nz - gz;
-                    const float ku = s * gn * inv;
-                    const float vux = ku * wx, vuy = ku * wy, vuz = ku * wz;
-                    v[0] = vux * d.x; v[1] = vux * d.y; v[2] = vux * d.z;
-                    v[3] = vuy * d.x; v[4] = vuy * d.y; v[5] = vuy * d.z;
-                    v[6] = vuz * d.x; v[7] = vuz * d.y; v[8] = vuz * d.z;
-                    v[9] = -s * wx; v[10] = -s * wy; v[11] = -s * wz;
-                    if (RS) {
+                    const float q = gate * v_alpha;
+                    if (!RS) {
+                        const float omega = f.w * rden, qo = q * omega;
+                        v[0] = qo * f.e1; v[1] = qo * f.e2;
+                        v[2] = v[0] * phi; v[3] = v[1] * phi;
+                        const float t1 = v[0] * omega, t2 = v[1] * omega;
+                        v[4] = t1 * f.e1; v[5] = t1 * f.e2; v[6] = t2 * f.e2;
+                        v[7] = q * phi;
+                        v[8] = fac * vcr; v[9] = fac * vcg; v[10] = fac * vcb;
+                        v[11] = q;
+                    } else {
+                        const float s = -(r3.w * q);  // v_c = s * c with c = n x g
+                        // with n = u / |u|, gn = g . n and w = gn n - g (minus the part of g orthogonal to n):
+                        //   v_g = v_c x n = -s w,   v_u = (v_n - (v_n . n) n) / |u| = (s gn / |u|) w
+                        const float nx = ux * inv, ny = uy * inv, nz = uz * inv;
+                        const float gn = gx * nx + gy * ny + gz * nz;
+                        const float wx = gn * nx - gx, wy = gn * ny - gy, wz = gn * nz - gz;
+                        const float ku = s * gn * inv;
+                        const float vux = ku * wx, vuy = ku * wy, vuz = ku * wz;
+                        const float vgx = -s * wx, vgy = -s * wy, vgz = -s * wz;
                         // g = M (o_start - mu) + M (o_pixel - o_start): the second term adds v_g (x) (o_pixel - o_start) to v_M
-                        v[0] += v[9] * oo.x;  v[1] += v[9] * oo.y;  v[2] += v[9] * oo.z;
-                        v[3] += v[10] * oo.x; v[4] += v[10] * oo.y; v[5] += v[10] * oo.z;
-                        v[6] += v[11] * oo.x; v[7] += v[11] * oo.y; v[8] += v[11] * oo.z;
+                        const float rs_sums[16] = {vux * d.x + vgx * oo.x, vux * d.y + vgx * oo.y, vux * d.z + vgx * oo.z,
+                                                   vuy * d.x + vgy * oo.x, vuy * d.y + vgy * oo.y, vuy * d.z + vgy * oo.z,
+                                                   vuz * d.x + vgz * oo.x, vuz * d.y + vgz * oo.y, vuz * d.z + vgz * oo.z,
+                                                   vgx, vgy, vgz, fac * vcr, fac * vcg, fac * vcb, q};
+#pragma unroll
+                        for (int k = 0; k < NS; ++k) v[k] = rs_sums[k];
                     }
-                    v[15] = gate * v_alpha;
-                    bufr += r3.x * fac; bufg += r3.y * fac; bufb += r3.z * fac;
-                    if (EXTRA) bufx += xval * fac;
                     if (XGRAD) {
                         const float xs = __reduce_add_sync_f32(fac * vcx);
                         if (lane == 0) atomicAdd(&sm.sextra[b & 1][t], xs);
                     }
                 }
-                const float total = warp_reduce16(v, red, lane);
-                if ((lane & 1) == 0) atomicAdd(&sacc[t * 16 + (lane >> 1)], total);
+                const float total = warp_reduce<NS>(v, red, lane);
+                if ((lane & 1) == 0 && lane < 2 * NS) atomicAdd(&sacc[t * NS + (lane >> 1)], total);
                 if (lane == 0) sm.stouched[b & 1][t] = 1;
             }
         }
@@ -513,26 +565,68 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------
-// Per-Gaussian gradient from the 16 accumulated numbers. Outputs gradients w.r.t. the ACTIVATED
-// mean / quaternion / scale / opacity and the colour.
+// Per-Gaussian gradient from the accumulated sums. Outputs gradients w.r.t. the ACTIVATED mean / quaternion / scale /
+// opacity and the colour. `opacity` is the blended opacity of the record.
+//
+// One ray origin. With u' = O u (RayFrame) the loss reaches M and g through phi(u', g') and |g|^2 only, and
+// v_M = sum v_u (x) d + v_g (x) (o - mu) collapses to O^T Y O S R^T with the symmetric Y below: the part of the two terms that
+// grows with the distance cancels in the algebra instead of in float32. Then v_scale_j = -(O^T Y O)_jj / s_j and
+// v_mean = -M^T v_g.
 // ---------------------------------------------------------------------------------------------
 struct GaussGrad {
     float v_mean[3], v_quat[4], v_scale[3], v_opac, v_rgb[3];
 };
 
 __device__ __forceinline__ void gaussian_vjp(const CamDev& cam, const float* acc /*16*/, f3 mean, float qw, float qx,
-                                             float qy, float qz, f3 scale, GaussGrad& o) {
+                                             float qy, float qz, f3 scale, float opacity, GaussGrad& o) {
     float R[9], inv_norm, qn[4];
     quat_to_rotmat_renorm(qw, qx, qy, qz, R, inv_norm, qn);
     const float is[3] = {1.0f / scale.x, 1.0f / scale.y, 1.0f / scale.z};
-    const float omu[3] = {cam.ro[0] - mean.x, cam.ro[1] - mean.y, cam.ro[2] - mean.z};
-    const float G[3] = {acc[9], acc[10], acc[11]};
-    // v_Mt = A + G (x) (o - mu)
-    float vMt[9];
+    const f3 om{cam.ro[0] - mean.x, cam.ro[1] - mean.y, cam.ro[2] - mean.z};
+    float G[3], vMt[9];
+    if (cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {
+        RayFrame f;
+        ray_frame(cam, R, om, scale, is, f);
+        const float og = opacity * f.gamma, y = -og * f.gamma;
+        const float Y00 = y * acc[4], Y01 = y * acc[5], Y11 = y * acc[6], Y02 = -y * acc[2], Y12 = -y * acc[3];
+        const float Y22 = y * (acc[7] - acc[4] - acc[6]);
+        const float g0 = -og * acc[0], g1 = -og * acc[1], g2 = og * acc[7];
+        const float sc[3] = {scale.x, scale.y, scale.z};
+        float YO[9], Z[9];
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 3; ++k) {
+            YO[k] = Y00 * f.O[k] + Y01 * f.O[3 + k] + Y02 * f.O[6 + k];
+            YO[3 + k] = Y01 * f.O[k] + Y11 * f.O[3 + k] + Y12 * f.O[6 + k];
+            YO[6 + k] = Y02 * f.O[k] + Y12 * f.O[3 + k] + Y22 * f.O[6 + k];
+            G[k] = f.O[k] * g0 + f.O[3 + k] * g1 + f.O[6 + k] * g2;
+        }
 #pragma unroll
-        for (int b = 0; b < 3; ++b) vMt[a * 3 + b] = acc[a * 3 + b] + G[a] * omu[b];
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) Z[j * 3 + k] = (f.O[j] * YO[k] + f.O[3 + j] * YO[3 + k] + f.O[6 + j] * YO[6 + k]) * sc[k];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) vMt[j * 3 + a] = Z[j * 3] * R[a * 3] + Z[j * 3 + 1] * R[a * 3 + 1] + Z[j * 3 + 2] * R[a * 3 + 2];
+            o.v_scale[j] = -is[j] * is[j] * Z[j * 3 + j];
+        }
+        o.v_rgb[0] = acc[8]; o.v_rgb[1] = acc[9]; o.v_rgb[2] = acc[10];
+        o.v_opac = acc[11];
+    } else {
+        const float omu[3] = {om.x, om.y, om.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            G[a] = acc[9 + a];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) vMt[a * 3 + b] = acc[a * 3 + b] + G[a] * omu[b];   // A + G (x) (o - mu)
+        }
+        // v_scale[j] = -is[j]^2 sum_a R[a][j] v_M[a][j] = -is[j]^2 sum_a R[a][j] vMt[j][a]
+#pragma unroll
+        for (int jx = 0; jx < 3; ++jx)
+            o.v_scale[jx] = -is[jx] * is[jx] * (R[0 * 3 + jx] * vMt[jx * 3 + 0] + R[1 * 3 + jx] * vMt[jx * 3 + 1] + R[2 * 3 + jx] * vMt[jx * 3 + 2]);
+        o.v_rgb[0] = acc[12]; o.v_rgb[1] = acc[13]; o.v_rgb[2] = acc[14];
+        o.v_opac = acc[15];
+    }
     // v_(o-mu) = Mt^T G with Mt[a][b] = is[a] R[b][a]  ->  sum_a is[a] R[b][a] G[a]
 #pragma unroll
     for (int b = 0; b < 3; ++b)
@@ -552,17 +646,11 @@ __device__ __forceinline__ void gaussian_vjp(const CamDev& cam, const float* acc
     const float dq = vqn[0] * qn[0] + vqn[1] * qn[1] + vqn[2] * qn[2] + vqn[3] * qn[3];
 #pragma unroll
     for (int k = 0; k < 4; ++k) o.v_quat[k] = (vqn[k] - dq * qn[k]) * inv_norm;
-    // v_scale[j] = -is[j]^2 sum_a R[a][j] v_M[a][j] = -is[j]^2 sum_a R[a][j] vMt[j][a]
-#pragma unroll
-    for (int jx = 0; jx < 3; ++jx)
-        o.v_scale[jx] = -is[jx] * is[jx] * (R[0 * 3 + jx] * vMt[jx * 3 + 0] + R[1 * 3 + jx] * vMt[jx * 3 + 1] + R[2 * 3 + jx] * vMt[jx * 3 + 2]);
-    o.v_rgb[0] = acc[12]; o.v_rgb[1] = acc[13]; o.v_rgb[2] = acc[14];
-    o.v_opac = acc[15];
 }
 
 __global__ void __launch_bounds__(256) grad_epilogue_op_kernel(
-    int N, const CamDev* __restrict__ cams, const float* __restrict__ accum, const float* __restrict__ means,
-    const float* __restrict__ quats, const float* __restrict__ scales, int channels, const float* __restrict__ accum_extra,
+    int N, const CamDev* __restrict__ cams, const float* __restrict__ accum, const float4* __restrict__ records,
+    const float* __restrict__ means, const float* __restrict__ quats, const float* __restrict__ scales, int channels, const float* __restrict__ accum_extra,
     float* __restrict__ v_means, float* __restrict__ v_quats, float* __restrict__ v_scales, float* __restrict__ v_colors,
     float* __restrict__ v_opacities) {
     const CamDev& cam = cams[0];
@@ -574,7 +662,7 @@ __global__ void __launch_bounds__(256) grad_epilogue_op_kernel(
         const float4 q = reinterpret_cast<const float4*>(quats)[g];
         GaussGrad o;
         gaussian_vjp(cam, acc, f3{means[g * 3], means[g * 3 + 1], means[g * 3 + 2]}, q.x, q.y, q.z, q.w,
-                     f3{scales[g * 3], scales[g * 3 + 1], scales[g * 3 + 2]}, o);
+                     f3{scales[g * 3], scales[g * 3 + 1], scales[g * 3 + 2]}, records[(size_t)g * 4 + 3].w, o);
 #pragma unroll
         for (int k = 0; k < 3; ++k) { v_means[g * 3 + k] = o.v_mean[k]; v_scales[g * 3 + k] = o.v_scale[k]; }
         if (channels >= 3) {
@@ -675,7 +763,7 @@ __global__ void __launch_bounds__(256, 4) grad_epilogue_fused_kernel(
             const float nrm = fmaxf(sqrtf(n2), 1e-12f);
             const float q[4] = {qr.x / nrm, qr.y / nrm, qr.z / nrm, qr.w / nrm};
             GaussGrad o;
-            gaussian_vjp(cam, acc, mean, q[0], q[1], q[2], q[3], scale, o);
+            gaussian_vjp(cam, acc, mean, q[0], q[1], q[2], q[3], scale, r3.w, o);
             // activation backward: sigmoid, exp, x / max(|x|, eps)
             go = o.v_opac * (opacity * (1.0f - opacity));
             gs[0] = o.v_scale[0] * scale.x; gs[1] = o.v_scale[1] * scale.y; gs[2] = o.v_scale[2] * scale.z;
@@ -1011,13 +1099,13 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
 #define LFS_BWD_BATCH 64
 #endif
     constexpr int kBwdBatch = LFS_BWD_BATCH;
-    const size_t smem = sizeof(BwdShared<kBwdBatch>);
+    constexpr size_t smem = sizeof(BwdShared<kBwdBatch, kSums>), smem_rs = sizeof(BwdShared<kBwdBatch, kSumsRs>);
     static bool attr_set = false;
 #define LFS_BWD_ATTR(MODEL, EXTRA, XGRAD)                                                                                     \
     cudaFuncSetAttribute(raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                          (int)smem);                                                                                           \
     cudaFuncSetAttribute(raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                         (int)smem)
+                         (int)smem_rs)
     if (!attr_set) {
         LFS_BWD_ATTR(LFS_PINHOLE, false, false); LFS_BWD_ATTR(LFS_PINHOLE, true, false); LFS_BWD_ATTR(LFS_PINHOLE, true, true);
         LFS_BWD_ATTR(LFS_FISHEYE, false, false); LFS_BWD_ATTR(LFS_FISHEYE, true, false); LFS_BWD_ATTR(LFS_FISHEYE, true, true);
@@ -1028,7 +1116,7 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     }
 #undef LFS_BWD_ATTR
 #define LFS_BWD4(MODEL, EXTRA, XGRAD, RS)                                                                                     \
-    raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, RS><<<n_tiles, kBlock, smem, st>>>(                                      \
+    raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, RS><<<n_tiles, kBlock, RS ? smem_rs : smem, st>>>(                       \
         a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
         a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
         v_alphas, accum, accum_extra)
@@ -1050,12 +1138,12 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     return check_launch("raster_bwd");
 }
 
-int launch_grad_epilogue_op(int N, const CamDev* cam, const float* accum, const float* means, const float* quats,
-                            const float* scales, int channels, const float* accum_extra, float* v_means, float* v_quats,
+int launch_grad_epilogue_op(int N, const CamDev* cam, const float* accum, const float4* records, const float* means,
+                            const float* quats, const float* scales, int channels, const float* accum_extra, float* v_means, float* v_quats,
                             float* v_scales, float* v_colors, float* v_opacities, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     LFS_TIMED("grad_epilogue", st);
-    grad_epilogue_op_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, cam, accum, means, quats, scales, channels, accum_extra,
+    grad_epilogue_op_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, cam, accum, records, means, quats, scales, channels, accum_extra,
                                                               v_means, v_quats, v_scales, v_colors, v_opacities);
     return check_launch("grad_epilogue_op");
 }

@@ -30,8 +30,8 @@ int launch_raster_fwd(const RasterArgs& a, float* render, float* alphas, int32_t
 // accum_extra [N] (zeroed by the caller) receives the gradient of the per-Gaussian extra value; null drops it.
 int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int32_t* last_ids, const float* extra_sum,
                       const float* v_render, const float* v_alphas, float* accum, float* accum_extra, cudaStream_t st);
-int launch_grad_epilogue_op(int N, const CamDev* cam, const float* accum, const float* means, const float* quats,
-                            const float* scales, int channels, const float* accum_extra, float* v_means, float* v_quats,
+int launch_grad_epilogue_op(int N, const CamDev* cam, const float* accum, const float4* records, const float* means,
+                            const float* quats, const float* scales, int channels, const float* accum_extra, float* v_means, float* v_quats,
                             float* v_scales, float* v_colors, float* v_opacities, cudaStream_t st);
 // In-place Adam of the five small groups inside the gradient stage: index 0..4 = means, sh0, scaling_raw, rotation_raw,
 // opacity_raw. step_size = lr * bias_correction1_rcp.
