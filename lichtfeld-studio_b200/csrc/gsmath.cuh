@@ -247,18 +247,6 @@ __device__ __forceinline__ bool image_to_cam_ray(const CamDev& c, float px, floa
     }
 }
 
-// Camera-space direction of a pixel centre, not normalised: (x, y, 1) for the planar models.
-template <int MODEL>
-__device__ __forceinline__ bool pixel_cam_dir(const CamDev& c, float px, float py, f3& d) {
-    if (MODEL == LFS_PINHOLE) {
-        d = {(px - c.cx) / c.fx, (py - c.cy) / c.fy, 1.f};
-        return true;
-    }
-    const bool valid = image_to_cam_ray<MODEL>(c, px, py, d);
-    if (MODEL == LFS_PINHOLE_OPENCV) d = {d.x / d.z, d.y / d.z, 1.f};
-    return valid;
-}
-
 // World-space ray direction of a pixel centre.
 template <int MODEL>
 __device__ __forceinline__ bool pixel_world_dir(const CamDev& c, float px, float py, f3& d) {
@@ -267,6 +255,28 @@ __device__ __forceinline__ bool pixel_world_dir(const CamDev& c, float px, float
     d.x = c.Rinv[0] * cr.x + c.Rinv[1] * cr.y + c.Rinv[2] * cr.z;
     d.y = c.Rinv[3] * cr.x + c.Rinv[4] * cr.y + c.Rinv[5] * cr.z;
     d.z = c.Rinv[6] * cr.x + c.Rinv[7] * cr.y + c.Rinv[8] * cr.z;
+    return valid;
+}
+
+// Camera-space direction of a pixel centre, not normalised: (x, y, 1) for the planar models. It is the float32 world-space
+// unit ray, the one on which a pair's alpha falls on either side of its cut, taken back through Rinv in double (once per
+// pixel): the ray itself stays the one every other use of the camera sees.
+template <int MODEL>
+__device__ __forceinline__ bool pixel_cam_dir(const CamDev& c, float px, float py, f3& d) {
+    f3 wd;
+    const bool valid = pixel_world_dir<MODEL>(c, px, py, wd);
+    const double w[3] = {wd.x, wd.y, wd.z};
+    double v[3], r[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = c.Rinv[a] * w[0] + c.Rinv[3 + a] * w[1] + c.Rinv[6 + a] * w[2];
+    // Rinv is a rotation up to float32 rounding: one refinement step
+#pragma unroll
+    for (int a = 0; a < 3; ++a) r[a] = w[a] - (c.Rinv[a * 3] * v[0] + c.Rinv[a * 3 + 1] * v[1] + c.Rinv[a * 3 + 2] * v[2]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] += c.Rinv[a] * r[0] + c.Rinv[3 + a] * r[1] + c.Rinv[6 + a] * r[2];
+    const bool planar = MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV;
+    const double iz = planar ? 1.0 / v[2] : 1.0;
+    d = {(float)(v[0] * iz), (float)(v[1] * iz), planar ? 1.f : (float)v[2]};
     return valid;
 }
 

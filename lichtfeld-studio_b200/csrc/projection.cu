@@ -387,14 +387,24 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
             p1[k] = lambda * (f.O[0] * is[0] * f.V[k * 3] + f.O[1] * is[1] * f.V[k * 3 + 1] + f.O[2] * is[2] * f.V[k * 3 + 2]);
             p3[k] = lambda * (f.O[6] * is[0] * f.V[k * 3] + f.O[7] * is[1] * f.V[k * 3 + 1] + f.O[8] * is[2] * f.V[k * 3 + 2]);
         }
-        // e1 vanishes along the ray through the centre: what rounding left of p1 . mu_c is taken out again
-        const float t = fmaf(p1[2], f.m[2], fmaf(p1[1], f.m[1], p1[0] * f.m[0])) / fmaxf(m2, 1e-30f);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) p1[k] = fmaf(-t, f.m[k], p1[k]);
         const float n2 = lambda * f.inv_nv;
+        float p2[3] = {f.v[0] * n2, f.v[1] * n2, f.v[2] * n2};
+        // e1 and e2 vanish along the ray through the centre: what rounding left of p . mu_c is taken out of the coefficient that
+        // mu_c weighs most (z for the planar models)
+        const int km = (cam.model == LFS_PINHOLE || cam.model == LFS_PINHOLE_OPENCV) ? 2
+                       : fabsf(f.m[2]) >= fmaxf(fabsf(f.m[0]), fabsf(f.m[1]))       ? 2
+                       : fabsf(f.m[1]) >= fabsf(f.m[0])                             ? 1 : 0;
+        if (m2 > 0.f) {
+            const float im = 1.0f / (km == 2 ? f.m[2] : km == 1 ? f.m[1] : f.m[0]);
+            const float t1 = (float)((double)p1[0] * f.m[0] + (double)p1[1] * f.m[1] + (double)p1[2] * f.m[2]) * im;
+            const float t2 = (float)((double)p2[0] * f.m[0] + (double)p2[1] * f.m[1] + (double)p2[2] * f.m[2]) * im;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k == km) { p1[k] -= t1; p2[k] -= t2; }
+        }
         const float G = f.gamma * f.gamma;
         rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
-        rec[1] = make_float4(f.v[0] * n2, f.v[1] * n2, f.v[2] * n2, -2.0f * __uint_as_float(thr_bits) / fmaxf(G, 1e-30f));
+        rec[1] = make_float4(p2[0], p2[1], p2[2], -2.0f * __uint_as_float(thr_bits) / fmaxf(G, 1e-30f));
         // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
         rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], 0.f) : make_float4(0.6101f, 0.5303f, 0.5887f, 0.f);
     } else {
