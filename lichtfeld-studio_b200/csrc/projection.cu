@@ -322,14 +322,93 @@ int launch_projection_ut(int C, int N, const float* means, const float* quats, c
 // ---------------------------------------------------------------------------------------------
 // Rasterizer record from activated parameters (layout in common.cuh) with the quaternion re-normalised.
 // ---------------------------------------------------------------------------------------------
-// Also computes the exact screen-space bounding box (in whole pixels, inclusive, clamped to 16 bits) of the
-// pixels whose ray can reach alpha >= 1/255: alpha = opacity * exp(-d^2/2) with d the distance from the ray to
-// the centre in the whitened frame, so those rays are exactly the ones that hit the ellipsoid
-// (x-mu)^T M^T M (x-mu) <= rho^2, rho^2 = 2 ln(255 opacity). Under a pinhole camera its outline is a conic whose
-// axis-aligned tangents follow from the dual quadric B = mu_c mu_c^T - Sigma_c:
-// x_n = (B02 -+ sqrt(B02^2 - B00 B22)) / B22 (same with index 1 for y). A margin keeps the box conservative under
-// rounding; when the ellipsoid reaches the camera plane (B22 <= 0) or the camera is not a pinhole the box is the
-// whole image. The rasterizer uses it only to skip (warp patch, Gaussian) pairs that cannot contribute.
+// Also computes a screen-space bounding box (in whole pixels, inclusive, clamped to 16 bits) of the pixels whose ray can
+// reach alpha >= 1/255: alpha = opacity * exp(-d^2/2) with d the distance from the ray to the centre in the whitened frame,
+// so those rays are exactly the ones that hit the ellipsoid (x-mu)^T M^T M (x-mu) <= rho^2, rho^2 = 2 ln(255 opacity).
+// Under a pinhole camera its outline is a conic whose axis-aligned tangents follow from the dual quadric
+// B = mu_c mu_c^T - Sigma_c: x_n = (B02 -+ sqrt(B02^2 - B00 B22)) / B22 (same with index 1 for y). A distorted pinhole maps
+// that rectangle by interval arithmetic (opencv_box); a fisheye takes the cone around the ellipsoid to a ring sector
+// (fisheye_box). A margin keeps the box conservative under rounding; when the ellipsoid reaches the camera plane (B22 <= 0,
+// for a fisheye: the origin) or the camera is none of the three the box is the whole image. The rasterizer uses it only to
+// skip (warp patch, Gaussian) pairs that cannot contribute.
+// a . b for nearly orthogonal vectors, as if summed in twice the precision (products split by fma, sums by two-sum;
+// Ogita, Rump and Oishi's Dot2)
+__device__ __forceinline__ float residual3(const float* a, const float* b) {
+    float h = a[0] * b[0], c = fmaf(a[0], b[0], -h);
+#pragma unroll
+    for (int k = 1; k < 3; ++k) {
+        const float p = a[k] * b[k], e = fmaf(a[k], b[k], -p);
+        const float t = h + p, z = t - h;
+        c += ((h - (t - z)) + (p - z)) + e;
+        h = t;
+    }
+    return h + c;
+}
+
+struct Itv { float lo, hi; };
+__device__ __forceinline__ Itv operator+(Itv a, Itv b) { return {a.lo + b.lo, a.hi + b.hi}; }
+__device__ __forceinline__ Itv operator+(float a, Itv b) { return {a + b.lo, a + b.hi}; }
+__device__ __forceinline__ Itv operator*(float a, Itv b) { return a >= 0.f ? Itv{a * b.lo, a * b.hi} : Itv{a * b.hi, a * b.lo}; }
+__device__ __forceinline__ Itv operator*(Itv a, Itv b) {
+    const float p = a.lo * b.lo, q = a.lo * b.hi, r = a.hi * b.lo, t = a.hi * b.hi;
+    return {fminf(fminf(p, q), fminf(r, t)), fmaxf(fmaxf(p, q), fmaxf(r, t))};
+}
+__device__ __forceinline__ Itv square(Itv a) {
+    const float p = a.lo * a.lo, q = a.hi * a.hi;
+    return {a.lo <= 0.f && a.hi >= 0.f ? 0.f : fminf(p, q), fmaxf(p, q)};
+}
+
+// Rectangle of undistorted normalised coordinates -> rectangle of distorted ones (opencv_distortion of gsmath.cuh on intervals).
+__device__ __forceinline__ bool opencv_box(const CamDev& cam, float* lo, float* hi) {
+    const float* k = cam.dist;
+    const Itv u{lo[0], hi[0]}, v{lo[1], hi[1]};
+    const Itv u2 = square(u), v2 = square(v), r2 = u2 + v2, uv = 2.f * (u * v);
+    const Itv num = 1.f + r2 * (k[0] + r2 * (k[1] + k[2] * r2));
+    const Itv den = 1.f + r2 * (k[3] + r2 * (k[4] + k[5] * r2));
+    if (!(den.lo > 0.05f)) return false;
+    const Itv icd = num * Itv{1.0f / den.hi, 1.0f / den.lo};
+    const Itv x = icd * u + k[6] * uv + k[7] * (r2 + 2.f * u2) + r2 * (k[8] + k[9] * r2);
+    const Itv y = icd * v + k[6] * (r2 + 2.f * v2) + k[7] * uv + r2 * (k[10] + k[11] * r2);
+    lo[0] = x.lo; hi[0] = x.hi; lo[1] = y.lo; hi[1] = y.hi;
+    return x.hi - x.lo < 1e6f && y.hi - y.lo < 1e6f;   // false for NaN
+}
+
+// Fisheye: the rays lie in the cone of half angle beta around the centre, tan beta = the largest tangent-plane extent of the
+// dual quadric over all directions; the image of the cone lies in the ring sector theta0 +- beta, psi0 +- asin(sin beta /
+// sin theta0). The radius is monotone in theta up to max_angle, which bounds every valid ray (known for k4 = 0 only).
+__device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, float s00, float s01, float s02, float s11,
+                                            float s12, float s22, float* lo, float* hi) {
+    const float m2 = mc[0] * mc[0] + mc[1] * mc[1] + mc[2] * mc[2];
+    if (cam.k[3] != 0.f || !(m2 > 0.f)) return false;
+    const float im = 1.0f / sqrtf(m2);
+    const float e0 = mc[0] * im, e1 = mc[1] * im, e2 = mc[2] * im;
+    const float t0 = s00 * e0 + s01 * e1 + s02 * e2, t1 = s01 * e0 + s11 * e1 + s12 * e2, t2 = s02 * e0 + s12 * e1 + s22 * e2;
+    const float along = t0 * e0 + t1 * e1 + t2 * e2, tt = t0 * t0 + t1 * t1 + t2 * t2;
+    const float B22 = m2 - along;
+    if (!(B22 > 0.02f * m2)) return false;
+    const float cross2 = fmaxf(0.f, tt - along * along);             // |part of Sigma e across e|^2
+    const float tr = s00 + s11 + s22 - along;                        // trace and squared norm of Sigma across e
+    const float fro = s00 * s00 + s11 * s11 + s22 * s22 + 2.f * (s01 * s01 + s02 * s02 + s12 * s12) - 2.f * tt + along * along;
+    const float lmax = 0.5f * (tr + sqrtf(fmaxf(0.f, 2.f * fro - tr * tr))) * 1.001f;
+    const float ext = (sqrtf(cross2) + sqrtf(cross2 + lmax * B22)) / B22;
+    const float beta = atanf(ext) * 1.001f;
+    const float n = sqrtf(mc[0] * mc[0] + mc[1] * mc[1]), theta0 = atan2f(n, mc[2]);
+    const float th_lo = fmaxf(theta0 - beta, 0.f) * 0.9999f, th_hi = fminf(theta0 + beta, cam.max_angle) * 1.0001f;
+    if (!(th_hi >= th_lo)) return false;
+    const float r_lo = fisheye_poly_odd(cam.k, th_lo), r_hi = fmaxf(r_lo, fisheye_poly_odd(cam.k, th_hi));
+    const float sb = sinf(beta) * 1.001f, st = n * im;
+    float cmin = -1.f, cmax = 1.f, smin = -1.f, smax = 1.f;          // ranges of cos psi and sin psi
+    if (beta < 1.5f && sb < st) {
+        const float cp = mc[0] / n, sp = mc[1] / n, sd = sb / st, cd = sqrtf(fmaxf(0.f, 1.f - sd * sd));
+        const float ca = cp * cd - sp * sd, cb = cp * cd + sp * sd, sa = sp * cd + cp * sd, sc = sp * cd - cp * sd;
+        cmax = cp >= cd ? 1.f : fmaxf(ca, cb); cmin = -cp >= cd ? -1.f : fminf(ca, cb);
+        smax = sp >= cd ? 1.f : fmaxf(sa, sc); smin = -sp >= cd ? -1.f : fminf(sa, sc);
+    }
+    lo[0] = fminf(cmin * r_lo, cmin * r_hi); hi[0] = fmaxf(cmax * r_lo, cmax * r_hi);
+    lo[1] = fminf(smin * r_lo, smin * r_hi); hi[1] = fmaxf(smax * r_lo, smax * r_hi);
+    return true;
+}
+
 __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
                                             f3 scale, float r, float g, float b, float opacity, float extra, float4* rec,
                                             uint4& box) {
@@ -339,7 +418,7 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
     const uint32_t thr_bits = __float_as_uint(-logf(fmaxf(255.0f * opacity, 1e-30f)) - 0.02f);
     const uint32_t extra_bits = __float_as_uint(extra);  // blended into the last channel of 1- and 4-channel renders
     box = make_uint4(0xFFFF0000u, 0xFFFF0000u, thr_bits, extra_bits);  // (lo | hi << 16) per axis: everything
-    if (cam.model == LFS_PINHOLE && cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {   // one pose for every pixel
+    if (cam.model != LFS_EQUIRECTANGULAR && cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {   // one pose for every pixel
         const float rho2 = 2.0f * (logf(fmaxf(255.0f * opacity, 1.0f)) + 0.03f);
         // V = R_c R with R_c = Rinv^T ; Sigma_c = rho2 V S^2 V^T ; mu_c = R_c mean + t
         float V[9];
@@ -353,19 +432,31 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
                              cam.Rinv[1] * mean.x + cam.Rinv[4] * mean.y + cam.Rinv[7] * mean.z + cam.ty,
                              cam.Rinv[2] * mean.x + cam.Rinv[5] * mean.y + cam.Rinv[8] * mean.z + cam.tz};
         auto sig = [&](int a, int c) { return V[a * 3] * s2[0] * V[c * 3] + V[a * 3 + 1] * s2[1] * V[c * 3 + 1] + V[a * 3 + 2] * s2[2] * V[c * 3 + 2]; };
-        const float B22 = mc[2] * mc[2] - sig(2, 2);
-        if (mc[2] > 0.f && B22 > 0.02f * mc[2] * mc[2]) {
+        float lo[2], hi[2];   // in units of the focal length, before the principal point
+        bool bounded = false;
+        if (cam.model == LFS_FISHEYE) {
+            bounded = fisheye_box(cam, mc, sig(0, 0), sig(0, 1), sig(0, 2), sig(1, 1), sig(1, 2), sig(2, 2), lo, hi);
+        } else {
+            const float B22 = mc[2] * mc[2] - sig(2, 2);
+            if (mc[2] > 0.f && B22 > 0.02f * mc[2] * mc[2]) {
+#pragma unroll
+                for (int ax = 0; ax < 2; ++ax) {
+                    const float Ba2 = mc[ax] * mc[2] - sig(ax, 2);
+                    const float Baa = mc[ax] * mc[ax] - sig(ax, ax);
+                    const float disc = sqrtf(fmaxf(0.f, Ba2 * Ba2 - Baa * B22));
+                    lo[ax] = (Ba2 - disc) / B22; hi[ax] = (Ba2 + disc) / B22;
+                }
+                bounded = cam.model == LFS_PINHOLE || opencv_box(cam, lo, hi);
+            }
+        }
+        if (bounded) {
             uint32_t packed[2];
             const float f[2] = {cam.fx, cam.fy}, c0[2] = {cam.cx, cam.cy};
 #pragma unroll
             for (int ax = 0; ax < 2; ++ax) {
-                const float Ba2 = mc[ax] * mc[2] - sig(ax, 2);
-                const float Baa = mc[ax] * mc[ax] - sig(ax, ax);
-                const float disc = sqrtf(fmaxf(0.f, Ba2 * Ba2 - Baa * B22));
-                const float lo_n = (Ba2 - disc) / B22, hi_n = (Ba2 + disc) / B22;
                 const float fl = fabsf(f[ax]);
-                const float lo_px = fminf(f[ax] * lo_n, f[ax] * hi_n) + c0[ax], hi_px = fmaxf(f[ax] * lo_n, f[ax] * hi_n) + c0[ax];
-                const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * fl * (hi_n - lo_n);
+                const float lo_px = fminf(f[ax] * lo[ax], f[ax] * hi[ax]) + c0[ax], hi_px = fmaxf(f[ax] * lo[ax], f[ax] * hi[ax]) + c0[ax];
+                const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * fl * (hi[ax] - lo[ax]);
                 // pixel j has its centre at j + 0.5
                 const float lo_j = floorf(lo_px - 0.5f - margin), hi_j = ceilf(hi_px - 0.5f + margin);
                 const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo_j, 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi_j, 0.f), 65535.f);
@@ -396,8 +487,7 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
                        : fabsf(f.m[1]) >= fabsf(f.m[0])                             ? 1 : 0;
         if (m2 > 0.f) {
             const float im = 1.0f / (km == 2 ? f.m[2] : km == 1 ? f.m[1] : f.m[0]);
-            const float t1 = (float)((double)p1[0] * f.m[0] + (double)p1[1] * f.m[1] + (double)p1[2] * f.m[2]) * im;
-            const float t2 = (float)((double)p2[0] * f.m[0] + (double)p2[1] * f.m[1] + (double)p2[2] * f.m[2]) * im;
+            const float t1 = residual3(p1, f.m) * im, t2 = residual3(p2, f.m) * im;
 #pragma unroll
             for (int k = 0; k < 3; ++k)
                 if (k == km) { p1[k] -= t1; p2[k] -= t2; }

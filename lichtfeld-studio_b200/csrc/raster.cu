@@ -95,31 +95,31 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// Each thread owns kParts quarter-record slots q = k * kBlock + tid of a batch: entry q >> 2, part q & 3.
-template <int BATCH>
+// Each thread owns kParts quarter-record slots q = k * BLOCK + tid of a batch: entry q >> 2, part q & 3.
+template <int BATCH, int BLOCK>
 struct StageIds {
-    static constexpr int kParts = (BATCH * 4 + kBlock - 1) / kBlock;
+    static constexpr int kParts = (BATCH * 4 + BLOCK - 1) / BLOCK;
     uint32_t g[kParts];
 };
 
 // ids of the batch whose first list position is `first` and which runs forward (step +1) or backward (-1)
-template <int BATCH>
-__device__ __forceinline__ void load_ids(StageIds<BATCH>& ids, const uint32_t* __restrict__ flatten_ids, int32_t first,
+template <int BATCH, int BLOCK>
+__device__ __forceinline__ void load_ids(StageIds<BATCH, BLOCK>& ids, const uint32_t* __restrict__ flatten_ids, int32_t first,
                                          int step, int batch_size) {
 #pragma unroll
-    for (int k = 0; k < StageIds<BATCH>::kParts; ++k) {
-        const int e = (k * kBlock + threadIdx.x) >> 2;
+    for (int k = 0; k < StageIds<BATCH, BLOCK>::kParts; ++k) {
+        const int e = (k * BLOCK + threadIdx.x) >> 2;
         ids.g[k] = e < batch_size ? flatten_ids[first + step * e] : 0u;
     }
 }
 
-template <int BATCH>
-__device__ __forceinline__ void issue_stage(Stage<BATCH>& st, uint32_t* sid, const StageIds<BATCH>& ids,
+template <int BATCH, int BLOCK>
+__device__ __forceinline__ void issue_stage(Stage<BATCH>& st, uint32_t* sid, const StageIds<BATCH, BLOCK>& ids,
                                             const float4* __restrict__ records, const uint4* __restrict__ bounds,
                                             int batch_size) {
 #pragma unroll
-    for (int k = 0; k < StageIds<BATCH>::kParts; ++k) {
-        const int q = k * kBlock + threadIdx.x;
+    for (int k = 0; k < StageIds<BATCH, BLOCK>::kParts; ++k) {
+        const int q = k * BLOCK + threadIdx.x;
         const int e = q >> 2, part = q & 3;
         if (e < batch_size) {
             cp_async16(&st.rec[q], records + (size_t)ids.g[k] * 4 + part);
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
     uint32_t cur_idx = 0;
     float pr = 0.f, pg = 0.f, pb = 0.f, px = 0.f;
 
-    StageIds<BATCH> ids;
+    StageIds<BATCH, kBlock> ids;
     if (n_batches > 0) {
         load_ids(ids, flatten_ids, range_start, 1, min(BATCH, range_end - range_start));
         issue_stage(stage[0], nullptr, ids, records, bounds, min(BATCH, range_end - range_start));
@@ -320,21 +320,31 @@ __device__ __forceinline__ float __reduce_add_sync_f32(float x) {
 //   q omega e1, q omega e2 | the same two times phi | q omega^2 e1^2, q omega^2 e1 e2, q omega^2 e2^2 | q phi | rgb | q
 // Rolling shutter: 16 = sum v_u (x) d, sum v_gro, rgb, opacity.
 constexpr int kSums = 12, kSumsRs = 16;
+#ifndef LFS_BWD_PX
+#define LFS_BWD_PX 2
+#endif
+constexpr int kBwdPx = LFS_BWD_PX, kBwdBlock = 256 / kBwdPx;
 template <int BATCH, int NS>
 struct BwdShared {
     Stage<BATCH> stage[3];       // batch b is walked while b+1 and b+2 are in flight
-    uint32_t sid[4][BATCH];      // Gaussian index per slot; four deep: batch b+2 is staged while batch b-1 is flushed
-    float sacc[2][BATCH * NS];   // per-slot sums of the batch being walked / the batch being flushed
-    float sextra[2][BATCH];
-    int stouched[2][BATCH];
-    float red[kBlock / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
+    uint32_t sid[3][BATCH];      // Gaussian index per slot
+    float red[kBwdBlock / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
 };
+
+// 1 / x for x in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23).
+__device__ __forceinline__ float rcp_newton(float x) {
+    const float y = __fdividef(1.0f, x);
+    return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
 
 // EXTRA: the output has 1 or 4 channels and its last one blends bounds.w (see the forward). XGRAD: also return
 // the gradient of that per-Gaussian value in accum_extra [N] (operator-level colours with 1 or 4 channels;
 // the fused render modes drop it like gsplat/Rasterization.cpp:575-590 does).
+// One thread owns PX horizontally adjacent pixels, a warp a patch of 4 PX x 8: the two pixels' terms are added in registers,
+// so the warp reduction (12 stores, 4 wide loads, the reduction to memory), the record loads and the list walk are paid once
+// for two pixels.
 template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS>
-__global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
+__global__ void __launch_bounds__(kBwdBlock) raster_bwd_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds,
     const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
@@ -345,86 +355,71 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
     float* __restrict__ accum_extra) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int NS = RS ? kSumsRs : kSums;
+    constexpr int PX = kBwdPx;
     BwdShared<BATCH, NS>& sm = *reinterpret_cast<BwdShared<BATCH, NS>*>(smem_raw);
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
     if (masks && !masks[tile]) return;  // gsplat/RasterizeToPixelsFromWorld3DGSBwd.cu:84
-    int i, j;
-    pixel_of_thread(tile, tw, i, j);
-    const bool inside = (i < H && j < W);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // warps tile the 16x16 block as patches of 4 PX x 8 pixels
+    constexpr int kPatchesX = 16 / (4 * PX);
+    const int patch_x0 = (tile % tw) * 16 + (warp % kPatchesX) * 4 * PX, patch_y0 = (tile / tw) * 16 + (warp / kPatchesX) * 8;
+    const uint32_t patch_x = patch_x0 | ((patch_x0 + 4 * PX - 1) << 16), patch_y = patch_y0 | ((patch_y0 + 7) << 16);
+    const int i = patch_y0 + (lane >> 2), j0 = patch_x0 + PX * (lane & 3);
     const CamDev& cam = cams[0];
-    f3 d, oo{0.f, 0.f, 0.f};
-    const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
-                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
-    const bool active = inside && ray_ok;
-    const int pid = min(i * W + j, W * H - 1);
-    uint32_t patch_x, patch_y;
-    warp_patch(tile, tw, patch_x, patch_y);
+
+    f3 d[PX], oo[PX];
+    int32_t bin_final[PX];   // last list position that reached the pixel; below every position for pixels that take no part
+    float T[PX], vcr[PX], vcg[PX], vcb[PX], vcx[PX];
+    // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
+    // (colour . v_colour) alpha T of every entry behind
+    float behind[PX];
+    int32_t warp_bin_final = 0;
+#pragma unroll
+    for (int p = 0; p < PX; ++p) {
+        const int j = j0 + p;
+        oo[p] = f3{0.f, 0.f, 0.f};
+        const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], oo[p])
+                               : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p]);
+        const bool active = i < H && j < W && ray_ok;
+        const int pid = min(i * W + j, W * H - 1);
+        const float T_final = 1.0f - render_alphas[pid];
+        T[p] = T_final;
+        bin_final[p] = active ? last_ids[pid] : -1;
+        warp_bin_final = max(warp_bin_final, bin_final[p]);
+        float v_a = v_alphas ? v_alphas[pid] : 0.f;
+        vcx[p] = 0.f;
+        if (!EXTRA) {
+            vcr[p] = v_render[pid * 3 + 0]; vcg[p] = v_render[pid * 3 + 1]; vcb[p] = v_render[pid * 3 + 2];
+        } else {
+            vcr[p] = vcg[p] = vcb[p] = 0.f;
+            if (channels == 4) { vcr[p] = v_render[pid * 4 + 0]; vcg[p] = v_render[pid * 4 + 1]; vcb[p] = v_render[pid * 4 + 2]; }
+            vcx[p] = v_render[pid * channels + channels - 1];
+            if (normalize) {
+                // output = sum / max(alpha, 1e-10): chain rule of the division and of clamp_min
+                const float a = 1.0f - T_final, ac = fmaxf(a, 1e-10f);
+                if (a > 1e-10f) v_a -= extra_sum[pid] / (ac * ac) * vcx[p];
+                vcx[p] = vcx[p] / ac;
+            }
+        }
+        float bg_dot = 0.f;
+        if (background) {
+            if (!EXTRA || channels == 4) bg_dot = background[0] * vcr[p] + background[1] * vcg[p] + background[2] * vcb[p];
+            if (EXTRA) bg_dot += background[channels - 1] * vcx[p];
+        }
+        behind[p] = T_final * (v_a - bg_dot);
+    }
+    warp_bin_final = __reduce_max_sync(0xffffffffu, warp_bin_final);
 
     const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
     const int32_t range_start = tile_offsets[tile];
     const int32_t range_end = (tile == n_tiles - 1) ? n_isects : tile_offsets[tile + 1];
     const int n_batches = (range_end - range_start + BATCH - 1) / BATCH;
-
-    const float T_final = 1.0f - render_alphas[pid];
-    float T = T_final;
-    const int32_t bin_final = active ? last_ids[pid] : 0;
-    float vcr, vcg, vcb, vcx = 0.f;
-    float v_a = v_alphas ? v_alphas[pid] : 0.f;
-    if (!EXTRA) {
-        vcr = v_render[pid * 3 + 0]; vcg = v_render[pid * 3 + 1]; vcb = v_render[pid * 3 + 2];
-    } else {
-        vcr = vcg = vcb = 0.f;
-        if (channels == 4) { vcr = v_render[pid * 4 + 0]; vcg = v_render[pid * 4 + 1]; vcb = v_render[pid * 4 + 2]; }
-        vcx = v_render[pid * channels + channels - 1];
-        if (normalize) {
-            // output = sum / max(alpha, 1e-10): chain rule of the division and of clamp_min
-            const float a = 1.0f - T_final, ac = fmaxf(a, 1e-10f);
-            if (a > 1e-10f) v_a -= extra_sum[pid] / (ac * ac) * vcx;
-            vcx = vcx / ac;
-        }
-    }
-    float bg_dot = 0.f;
-    if (background) {
-        if (!EXTRA || channels == 4) bg_dot = background[0] * vcr + background[1] * vcg + background[2] * vcb;
-        if (EXTRA) bg_dot += background[channels - 1] * vcx;
-    }
-    // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
-    // (colour . v_colour) alpha T of every entry behind
-    float behind = T_final * (v_a - bg_dot);
-    const int32_t warp_bin_final = __reduce_max_sync(0xffffffffu, bin_final);
-    const int lane = threadIdx.x & 31;
-    float* red = sm.red[threadIdx.x >> 5];
-
-    for (int e = threadIdx.x; e < 2 * BATCH; e += kBlock) {
-#pragma unroll
-        for (int k = 0; k < NS; ++k) (&sm.sacc[0][0])[e * NS + k] = 0.f;
-        (&sm.sextra[0][0])[e] = 0.f;
-        (&sm.stouched[0][0])[e] = 0;
-    }
-    // flush the sums of batch k (16-byte reductions per touched Gaussian) and leave its buffers zeroed
-    auto flush = [&](int k) {
-        const int size_k = min(BATCH, range_end - k * BATCH - range_start);
-        float* acc_k = sm.sacc[k & 1];
-        for (int e = threadIdx.x; e < size_k; e += kBlock) {
-            if (sm.stouched[k & 1][e]) {
-                const uint32_t g = sm.sid[k & 3][e];
-                float4* dst = reinterpret_cast<float4*>(accum) + (size_t)g * 4;
-                float4* src = reinterpret_cast<float4*>(acc_k) + e * (NS / 4);
-#pragma unroll
-                for (int q = 0; q < NS / 4; ++q) {
-                    atomicAdd(dst + q, src[q]);
-                    src[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                if (XGRAD) { atomicAdd(accum_extra + g, sm.sextra[k & 1][e]); sm.sextra[k & 1][e] = 0.f; }
-                sm.stouched[k & 1][e] = 0;
-            }
-        }
-    };
+    float* red = sm.red[warp];
 
     // batches run back to front: slot e of batch b holds list position batch_end - e
-    StageIds<BATCH> ids;
+    StageIds<BATCH, kBwdBlock> ids;
     auto batch_count = [&](int k) { return min(BATCH, range_end - k * BATCH - range_start); };
     auto batch_top = [&](int k) { return range_end - 1 - k * BATCH; };
     if (n_batches > 0) {
@@ -437,21 +432,20 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
         }
     }
     // One barrier per batch: after it, batch b is in shared memory and every warp has finished walking batch b-1,
-    // so batch b+2 may be staged over b-1's records and b-1's sums may be flushed while batch b is walked.
+    // so batch b+2 may be staged over b-1's records.
     for (int b = 0; b < n_batches; ++b) {
         const int32_t batch_end = batch_top(b);
         const int32_t batch_size = batch_count(b);
         if (b + 1 < n_batches) cp_async_wait<1>(); else cp_async_wait<0>();
         __syncthreads();
         if (b + 2 < n_batches) {
-            issue_stage(sm.stage[(b + 2) % 3], sm.sid[(b + 2) & 3], ids, records, bounds, batch_count(b + 2));
+            issue_stage(sm.stage[(b + 2) % 3], sm.sid[(b + 2) % 3], ids, records, bounds, batch_count(b + 2));
             if (b + 3 < n_batches) load_ids(ids, flatten_ids, batch_top(b + 3), -1, batch_count(b + 3));
         }
-        if (b > 0) flush(b - 1);
-        float* sacc = sm.sacc[b & 1];
         const Stage<BATCH>& st = sm.stage[b % 3];
+        const uint32_t* sid = sm.sid[b % 3];
         // entries (back to front) that no pixel of this warp reaches (beyond its last contributor) or whose
-        // box misses this warp's 8x4 patch are dropped up front: one ballot word per 32 entries
+        // box misses this warp's patch are dropped up front: one ballot word per 32 entries
         const int t_begin = max(0, batch_end - warp_bin_final);
         uint32_t live[BATCH / 32];
 #pragma unroll
@@ -467,100 +461,119 @@ __global__ void __launch_bounds__(kBlock) raster_bwd_kernel(
             while (bits) {
                 const int t = w * 32 + __ffs(bits) - 1;
                 bits &= bits - 1;
-                // Every lane evaluates the pair (the record reads are warp-wide broadcasts); lanes that are outside
+                // Every lane evaluates the pair (the record reads are warp-wide broadcasts); pixels that are outside
                 // the image, beyond their last contributor or below the alpha threshold continue with alpha = vis = 0,
                 // which makes every term they add exactly zero, so no per-lane branching is needed below.
                 const float4 r0 = st.rec[t * 4 + 0], r1 = st.rec[t * 4 + 1], r2 = st.rec[t * 4 + 2];
-                bool valid = active && (batch_end - t <= bin_final);
-                float vis;
-                RayForms f;
-                float ux, uy, uz, gx, gy, gz, inv;
-                if (!RS) {
-                    f = ray_forms<MODEL>(r0, r1, r2, d);
-                    valid = valid && !(f.E > r1.w * f.den);
-                } else {
-                    ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
-                    uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
-                    uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
-                    gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
-                    gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
-                    gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
-                    const float cx = uy * gz - gy * uz;
-                    const float cy = uz * gx - gz * ux;
-                    const float cz = ux * gy - gx * uy;
-                    const float cc = cx * cx + cy * cy + cz * cz;
-                    const float uu = ux * ux + uy * uy + uz * uz;
-                    valid = valid && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
-                    inv = rsqrtf(fmaxf(uu, 1e-37f));
-                    vis = -0.5f * (cc * (inv * inv));
-                }
-                if (!__any_sync(0xffffffffu, valid)) continue;
-                const float4 r3 = st.rec[t * 4 + 3];
-                float rden = 0.f, phi = 0.f;
-                if (!RS) {
-                    rden = __fdividef(1.0f, f.den);
-                    phi = f.E * rden;
-                    vis = exp2_approx(r0.w * phi);
-                } else {
-                    vis = __expf(vis);
-                }
-                float alpha = fminf(0.999f, r3.w * vis);
-                valid = valid && !(alpha < kAlphaMin);
-                if (!__any_sync(0xffffffffu, valid)) continue;
-                if (!valid) { vis = 0.f; alpha = 0.f; }
-                float v[NS];
-                {
-                    const float ra = __frcp_rn(1.0f - alpha);
-                    T *= ra;
-                    const float fac = alpha * T;
-                    // colour . v_colour of this entry: the colours only ever meet the output gradient in this product
-                    float cv = r3.x * vcr + r3.y * vcg + r3.z * vcb;
-                    if (EXTRA) cv += __uint_as_float(st.box[t].w) * vcx;
-                    const float v_alpha = cv * T + ra * behind;
-                    behind -= cv * fac;
-                    // geometry and opacity only while alpha is not clamped at 0.999
-                    const float gate = (r3.w * vis <= 0.999f) ? vis : 0.f;
-                    const float q = gate * v_alpha;
+                bool valid[PX], any_valid = false;
+                float vis[PX];
+                RayForms f[PX];
+                float ux[PX], uy[PX], uz[PX], gx[PX], gy[PX], gz[PX], inv[PX];
+#pragma unroll
+                for (int p = 0; p < PX; ++p) {
                     if (!RS) {
-                        const float omega = f.w * rden, qo = q * omega;
-                        v[0] = qo * f.e1; v[1] = qo * f.e2;
-                        v[2] = v[0] * phi; v[3] = v[1] * phi;
-                        const float t1 = v[0] * omega, t2 = v[1] * omega;
-                        v[4] = t1 * f.e1; v[5] = t1 * f.e2; v[6] = t2 * f.e2;
-                        v[7] = q * phi;
-                        v[8] = fac * vcr; v[9] = fac * vcg; v[10] = fac * vcb;
-                        v[11] = q;
+                        f[p] = ray_forms<MODEL>(r0, r1, r2, d[p]);
+                        valid[p] = (batch_end - t <= bin_final[p]) && !(f[p].E > r1.w * f[p].den);
+                    } else {
+                        ux[p] = r0.x * d[p].x + r0.y * d[p].y + r0.z * d[p].z;
+                        uy[p] = r1.x * d[p].x + r1.y * d[p].y + r1.z * d[p].z;
+                        uz[p] = r2.x * d[p].x + r2.y * d[p].y + r2.z * d[p].z;
+                        gx[p] = r0.w + (r0.x * oo[p].x + r0.y * oo[p].y + r0.z * oo[p].z);
+                        gy[p] = r1.w + (r1.x * oo[p].x + r1.y * oo[p].y + r1.z * oo[p].z);
+                        gz[p] = r2.w + (r2.x * oo[p].x + r2.y * oo[p].y + r2.z * oo[p].z);
+                        const float cx = uy[p] * gz[p] - gy[p] * uz[p];
+                        const float cy = uz[p] * gx[p] - gz[p] * ux[p];
+                        const float cz = ux[p] * gy[p] - gx[p] * uy[p];
+                        const float cc = cx * cx + cy * cy + cz * cz;
+                        const float uu = ux[p] * ux[p] + uy[p] * uy[p] + uz[p] * uz[p];
+                        valid[p] = (batch_end - t <= bin_final[p]) && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
+                        inv[p] = rsqrtf(fmaxf(uu, 1e-37f));
+                        vis[p] = -0.5f * (cc * (inv[p] * inv[p]));
+                    }
+                    any_valid = any_valid || valid[p];
+                }
+                if (!__any_sync(0xffffffffu, any_valid)) continue;
+                const float4 r3 = st.rec[t * 4 + 3];
+                float rden[PX], phi[PX], alpha[PX];
+                any_valid = false;
+#pragma unroll
+                for (int p = 0; p < PX; ++p) {
+                    rden[p] = phi[p] = 0.f;
+                    if (!RS) {
+                        rden[p] = __fdividef(1.0f, f[p].den);
+                        phi[p] = f[p].E * rden[p];
+                        vis[p] = exp2_approx(r0.w * phi[p]);
+                    } else {
+                        vis[p] = __expf(vis[p]);
+                    }
+                    alpha[p] = fminf(0.999f, r3.w * vis[p]);
+                    valid[p] = valid[p] && !(alpha[p] < kAlphaMin);
+                    any_valid = any_valid || valid[p];
+                }
+                if (!__any_sync(0xffffffffu, any_valid)) continue;
+                float v[NS];
+                float xs = 0.f;
+#pragma unroll
+                for (int p = 0; p < PX; ++p) {
+                    if (!valid[p]) { vis[p] = 0.f; alpha[p] = 0.f; }
+                    const float ra = rcp_newton(1.0f - alpha[p]);
+                    T[p] *= ra;
+                    const float fac = alpha[p] * T[p];
+                    // colour . v_colour of this entry: the colours only ever meet the output gradient in this product
+                    float cv = r3.x * vcr[p] + r3.y * vcg[p] + r3.z * vcb[p];
+                    if (EXTRA) cv += __uint_as_float(st.box[t].w) * vcx[p];
+                    const float v_alpha = cv * T[p] + ra * behind[p];
+                    behind[p] -= cv * fac;
+                    // geometry and opacity only while alpha is not clamped at 0.999
+                    const float gate = (r3.w * vis[p] <= 0.999f) ? vis[p] : 0.f;
+                    const float q = gate * v_alpha;
+                    auto add = [&](int k, float a, float c) { v[k] = p == 0 ? a * c : fmaf(a, c, v[k]); };
+                    if (!RS) {
+                        const float omega = f[p].w * rden[p], qo = q * omega;
+                        const float th1 = qo * f[p].e1, th2 = qo * f[p].e2;
+                        const float t1 = th1 * omega, t2 = th2 * omega;
+                        if (p == 0) { v[0] = th1; v[1] = th2; v[11] = q; } else { v[0] += th1; v[1] += th2; v[11] += q; }
+                        add(2, th1, phi[p]); add(3, th2, phi[p]);
+                        add(4, t1, f[p].e1); add(5, t1, f[p].e2); add(6, t2, f[p].e2);
+                        add(7, q, phi[p]);
+                        add(8, fac, vcr[p]); add(9, fac, vcg[p]); add(10, fac, vcb[p]);
                     } else {
                         const float s = -(r3.w * q);  // v_c = s * c with c = n x g
                         // with n = u / |u|, gn = g . n and w = gn n - g (minus the part of g orthogonal to n):
                         //   v_g = v_c x n = -s w,   v_u = (v_n - (v_n . n) n) / |u| = (s gn / |u|) w
-                        const float nx = ux * inv, ny = uy * inv, nz = uz * inv;
-                        const float gn = gx * nx + gy * ny + gz * nz;
-                        const float wx = gn * nx - gx, wy = gn * ny - gy, wz = gn * nz - gz;
-                        const float ku = s * gn * inv;
-                        const float vux = ku * wx, vuy = ku * wy, vuz = ku * wz;
-                        const float vgx = -s * wx, vgy = -s * wy, vgz = -s * wz;
+                        const float nx = ux[p] * inv[p], ny = uy[p] * inv[p], nz = uz[p] * inv[p];
+                        const float gn = gx[p] * nx + gy[p] * ny + gz[p] * nz;
+                        const float wx = gn * nx - gx[p], wy = gn * ny - gy[p], wz = gn * nz - gz[p];
+                        const float ku = s * gn * inv[p];
+                        const float vu[3] = {ku * wx, ku * wy, ku * wz}, vg[3] = {-s * wx, -s * wy, -s * wz};
+                        const float dd[3] = {d[p].x, d[p].y, d[p].z}, od[3] = {oo[p].x, oo[p].y, oo[p].z};
                         // g = M (o_start - mu) + M (o_pixel - o_start): the second term adds v_g (x) (o_pixel - o_start) to v_M
-                        const float rs_sums[16] = {vux * d.x + vgx * oo.x, vux * d.y + vgx * oo.y, vux * d.z + vgx * oo.z,
-                                                   vuy * d.x + vgy * oo.x, vuy * d.y + vgy * oo.y, vuy * d.z + vgy * oo.z,
-                                                   vuz * d.x + vgz * oo.x, vuz * d.y + vgz * oo.y, vuz * d.z + vgz * oo.z,
-                                                   vgx, vgy, vgz, fac * vcr, fac * vcg, fac * vcb, q};
+                        const float rgbq[4] = {fac * vcr[p], fac * vcg[p], fac * vcb[p], q};
 #pragma unroll
-                        for (int k = 0; k < NS; ++k) v[k] = rs_sums[k];
+                        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                const float x = vu[r] * dd[c] + vg[r] * od[c];
+                                if (p == 0) v[r * 3 + c] = x; else v[r * 3 + c] += x;
+                            }
+                            if (p == 0) v[9 + r] = vg[r]; else v[9 + r] += vg[r];
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (p == 0) v[NS - 4 + k] = rgbq[k]; else v[NS - 4 + k] += rgbq[k];
                     }
-                    if (XGRAD) {
-                        const float xs = __reduce_add_sync_f32(fac * vcx);
-                        if (lane == 0) atomicAdd(&sm.sextra[b & 1][t], xs);
-                    }
+                    if (XGRAD) xs += fac * vcx[p];
+                }
+                const uint32_t g = sid[t];
+                if (XGRAD) {
+                    xs = __reduce_add_sync_f32(xs);
+                    if (lane == 0) atomicAdd(accum_extra + g, xs);
                 }
                 const float total = warp_reduce<NS>(v, red, lane);
-                if ((lane & 1) == 0 && lane < 2 * NS) atomicAdd(&sacc[t * NS + (lane >> 1)], total);
-                if (lane == 0) sm.stouched[b & 1][t] = 1;
+                if ((lane & 1) == 0 && lane < 2 * NS) atomicAdd(accum + (size_t)g * 16 + (lane >> 1), total);
             }
         }
     }
-    __syncthreads();
-    if (n_batches > 0) flush(n_batches - 1);
     cp_async_wait<0>();
 }
 
@@ -1116,7 +1129,7 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     }
 #undef LFS_BWD_ATTR
 #define LFS_BWD4(MODEL, EXTRA, XGRAD, RS)                                                                                     \
-    raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, RS><<<n_tiles, kBlock, RS ? smem_rs : smem, st>>>(                       \
+    raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, RS><<<n_tiles, kBwdBlock, RS ? smem_rs : smem, st>>>(                       \
         a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
         a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
         v_alphas, accum, accum_extra)
