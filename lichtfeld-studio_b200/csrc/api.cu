@@ -345,7 +345,8 @@ int lfs_rasterize_to_pixels_from_world_3dgs_fwd(int N, int64_t n_isects, int cha
     LFS_REQUIRE(camera_model != LFS_EQUIRECTANGULAR || (!rolling && !radial_coeffs),
                 "the equirectangular model has a global shutter and no distortion coefficients");
     if (rc != LFS_OK) return rc;
-    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, records, bounds, nullptr, nullptr, S(stream));
+    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, bounds, nullptr, nullptr,
+                             S(stream));
     if (rc != LFS_OK) return rc;
     RasterArgs a{cam, records, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,
                  nullptr, W, H, (W + 15) / 16, (H + 15) / 16, eff_model, channels, 0, masks, nullptr, rolling};
@@ -384,7 +385,7 @@ int lfs_rasterize_to_pixels_from_world_3dgs_bwd(int N, int64_t n_isects, int cha
     LFS_REQUIRE(camera_model != LFS_EQUIRECTANGULAR || (!rolling && !radial_coeffs),
                 "the equirectangular model has a global shutter and no distortion coefficients");
     if (rc != LFS_OK) return rc;
-    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, records, bounds,
+    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, bounds,
                              reinterpret_cast<float4*>(accum), accum_extra, S(stream));
     if (rc != LFS_OK) return rc;
     RasterArgs a{cam, records, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,

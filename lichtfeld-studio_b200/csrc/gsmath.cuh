@@ -417,6 +417,9 @@ __device__ __forceinline__ void sh_basis(int degree, float dx, float dy, float d
 // the form of e2 in camera space has the closed form v / sqrt(v^T Sigma v), v = e_x x mu_c, whose x coefficient is 0.
 // P does not change when the three forms are scaled together; callers scale them by |mu_c| / |g| (w near 1 at the centre).
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float fdot3(float a0, float b0, float a1, float b1, float a2, float b2) {
+    return fmaf(a2, b2, fmaf(a1, b1, a0 * b0));
+}
 struct RayFrame {
     float O[9];     // rows: directions of e1, e2, w in whitened space
     float gamma;    // |g|; g = -gamma * (row 3)
@@ -429,7 +432,7 @@ __device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 
     // Rinv m = mu - o. Rinv is a rotation only up to rounding, so its transpose misses the solution by about 1e-7 rad, the
     // same way for every Gaussian: one step of refinement
 #pragma unroll
-    for (int a = 0; a < 3; ++a) f.m[a] = -(cam.Rinv[a] * om.x + cam.Rinv[3 + a] * om.y + cam.Rinv[6 + a] * om.z);
+    for (int a = 0; a < 3; ++a) f.m[a] = -fdot3(cam.Rinv[a], om.x, cam.Rinv[3 + a], om.y, cam.Rinv[6 + a], om.z);
     float res[3];
     const float o3[3] = {om.x, om.y, om.z};
 #pragma unroll
@@ -437,10 +440,10 @@ __device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 
         res[a] = fmaf(cam.Rinv[a * 3 + 2], f.m[2], fmaf(cam.Rinv[a * 3 + 1], f.m[1], fmaf(cam.Rinv[a * 3], f.m[0], o3[a])));
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        f.m[a] -= cam.Rinv[a] * res[0] + cam.Rinv[3 + a] * res[1] + cam.Rinv[6 + a] * res[2];
+        f.m[a] -= fdot3(cam.Rinv[a], res[0], cam.Rinv[3 + a], res[1], cam.Rinv[6 + a], res[2]);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-            f.V[a * 3 + i] = cam.Rinv[a] * R[i] + cam.Rinv[3 + a] * R[3 + i] + cam.Rinv[6 + a] * R[6 + i];
+            f.V[a * 3 + i] = fdot3(cam.Rinv[a], R[i], cam.Rinv[3 + a], R[3 + i], cam.Rinv[6 + a], R[6 + i]);
     }
     f.v[0] = 0.f; f.v[1] = -f.m[2]; f.v[2] = f.m[1];
     const bool planar = cam.model == LFS_PINHOLE || cam.model == LFS_PINHOLE_OPENCV;
@@ -451,11 +454,11 @@ __device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 
     const float sc[3] = {scale.x, scale.y, scale.z};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        r2[i] = sc[i] * (f.V[i] * f.v[0] + f.V[3 + i] * f.v[1] + f.V[6 + i] * f.v[2]);
-        r3[i] = -is[i] * (R[i] * om.x + R[3 + i] * om.y + R[6 + i] * om.z);
+        r2[i] = sc[i] * fdot3(f.V[i], f.v[0], f.V[3 + i], f.v[1], f.V[6 + i], f.v[2]);
+        r3[i] = -is[i] * fdot3(R[i], om.x, R[3 + i], om.y, R[6 + i], om.z);
     }
-    const float n2 = r2[0] * r2[0] + r2[1] * r2[1] + r2[2] * r2[2];
-    f.gamma = sqrtf(r3[0] * r3[0] + r3[1] * r3[1] + r3[2] * r3[2]);
+    const float n2 = fdot3(r2[0], r2[0], r2[1], r2[1], r2[2], r2[2]);
+    f.gamma = sqrtf(fdot3(r3[0], r3[0], r3[1], r3[1], r3[2], r3[2]));
     if (f.m[0] == 0.f && f.m[1] == 0.f && f.m[2] == 0.f) {   // the camera sits on the centre: P = 0 along every ray
 #pragma unroll
         for (int k = 0; k < 9; ++k) f.O[k] = 0.f;
@@ -468,9 +471,9 @@ __device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 
     const float i3 = 1.0f / f.gamma;
 #pragma unroll
     for (int i = 0; i < 3; ++i) { f.O[3 + i] = r2[i] * f.inv_nv; f.O[6 + i] = r3[i] * i3; }
-    f.O[0] = f.O[4] * f.O[8] - f.O[5] * f.O[7];
-    f.O[1] = f.O[5] * f.O[6] - f.O[3] * f.O[8];
-    f.O[2] = f.O[3] * f.O[7] - f.O[4] * f.O[6];
+    f.O[0] = fmaf(f.O[4], f.O[8], -f.O[5] * f.O[7]);
+    f.O[1] = fmaf(f.O[5], f.O[6], -f.O[3] * f.O[8]);
+    f.O[2] = fmaf(f.O[3], f.O[7], -f.O[4] * f.O[6]);
 }
 
 // Tile rectangle covered by a projected Gaussian: [x0,x1) x [y0,y1) in tile units. The float ->

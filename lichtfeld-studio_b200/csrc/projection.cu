@@ -409,95 +409,22 @@ __device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, 
     return true;
 }
 
+// Only the lists are pinned to unfused arithmetic (file header); everything here spells its products and sums as fma.
+template <int MODEL, bool RS>
 __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
                                             f3 scale, float r, float g, float b, float opacity, float extra, float4* rec,
                                             uint4& box) {
     float R[9], inv_norm, qn[4];
     quat_to_rotmat_renorm(qw, qx, qy, qz, R, inv_norm, qn);
     // exponent below which opacity * exp(p) < 1/255 for certain, as float bits in .z
-    const uint32_t thr_bits = __float_as_uint(-logf(fmaxf(255.0f * opacity, 1e-30f)) - 0.02f);
+    const float thr = -logf(fmaxf(255.0f * opacity, 1e-30f)) - 0.02f;
+    const uint32_t thr_bits = __float_as_uint(thr);
     const uint32_t extra_bits = __float_as_uint(extra);  // blended into the last channel of 1- and 4-channel renders
     box = make_uint4(0xFFFF0000u, 0xFFFF0000u, thr_bits, extra_bits);  // (lo | hi << 16) per axis: everything
-    if (cam.model != LFS_EQUIRECTANGULAR && cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {   // one pose for every pixel
-        const float rho2 = 2.0f * (logf(fmaxf(255.0f * opacity, 1.0f)) + 0.03f);
-        // V = R_c R with R_c = Rinv^T ; Sigma_c = rho2 V S^2 V^T ; mu_c = R_c mean + t
-        float V[9];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                V[a * 3 + c] = cam.Rinv[0 * 3 + a] * R[0 * 3 + c] + cam.Rinv[1 * 3 + a] * R[1 * 3 + c] + cam.Rinv[2 * 3 + a] * R[2 * 3 + c];
-        const float s2[3] = {rho2 * scale.x * scale.x, rho2 * scale.y * scale.y, rho2 * scale.z * scale.z};
-        const float mc[3] = {cam.Rinv[0] * mean.x + cam.Rinv[3] * mean.y + cam.Rinv[6] * mean.z + cam.tx,
-                             cam.Rinv[1] * mean.x + cam.Rinv[4] * mean.y + cam.Rinv[7] * mean.z + cam.ty,
-                             cam.Rinv[2] * mean.x + cam.Rinv[5] * mean.y + cam.Rinv[8] * mean.z + cam.tz};
-        auto sig = [&](int a, int c) { return V[a * 3] * s2[0] * V[c * 3] + V[a * 3 + 1] * s2[1] * V[c * 3 + 1] + V[a * 3 + 2] * s2[2] * V[c * 3 + 2]; };
-        float lo[2], hi[2];   // in units of the focal length, before the principal point
-        bool bounded = false;
-        if (cam.model == LFS_FISHEYE) {
-            bounded = fisheye_box(cam, mc, sig(0, 0), sig(0, 1), sig(0, 2), sig(1, 1), sig(1, 2), sig(2, 2), lo, hi);
-        } else {
-            const float B22 = mc[2] * mc[2] - sig(2, 2);
-            if (mc[2] > 0.f && B22 > 0.02f * mc[2] * mc[2]) {
-#pragma unroll
-                for (int ax = 0; ax < 2; ++ax) {
-                    const float Ba2 = mc[ax] * mc[2] - sig(ax, 2);
-                    const float Baa = mc[ax] * mc[ax] - sig(ax, ax);
-                    const float disc = sqrtf(fmaxf(0.f, Ba2 * Ba2 - Baa * B22));
-                    lo[ax] = (Ba2 - disc) / B22; hi[ax] = (Ba2 + disc) / B22;
-                }
-                bounded = cam.model == LFS_PINHOLE || opencv_box(cam, lo, hi);
-            }
-        }
-        if (bounded) {
-            uint32_t packed[2];
-            const float f[2] = {cam.fx, cam.fy}, c0[2] = {cam.cx, cam.cy};
-#pragma unroll
-            for (int ax = 0; ax < 2; ++ax) {
-                const float fl = fabsf(f[ax]);
-                const float lo_px = fminf(f[ax] * lo[ax], f[ax] * hi[ax]) + c0[ax], hi_px = fmaxf(f[ax] * lo[ax], f[ax] * hi[ax]) + c0[ax];
-                const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * fl * (hi[ax] - lo[ax]);
-                // pixel j has its centre at j + 0.5
-                const float lo_j = floorf(lo_px - 0.5f - margin), hi_j = ceilf(hi_px - 0.5f + margin);
-                const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo_j, 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi_j, 0.f), 65535.f);
-                packed[ax] = lo_u | (hi_u << 16);
-            }
-            box = make_uint4(packed[0], packed[1], thr_bits, extra_bits);
-        }
-    }
     const float is[3] = {1.0f / scale.x, 1.0f / scale.y, 1.0f / scale.z};
     const f3 om{cam.ro[0] - mean.x, cam.ro[1] - mean.y, cam.ro[2] - mean.z};
-    if (cam.rs_type == LFS_SHUTTER_GLOBAL && !cam.has_end) {
-        RayFrame f;
-        ray_frame(cam, R, om, scale, is, f);
-        const float m2 = f.m[0] * f.m[0] + f.m[1] * f.m[1] + f.m[2] * f.m[2];
-        const float lambda = m2 > 0.f ? sqrtf(m2) / f.gamma : 1.0f;
-        float p1[3], p3[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            p1[k] = lambda * (f.O[0] * is[0] * f.V[k * 3] + f.O[1] * is[1] * f.V[k * 3 + 1] + f.O[2] * is[2] * f.V[k * 3 + 2]);
-            p3[k] = lambda * (f.O[6] * is[0] * f.V[k * 3] + f.O[7] * is[1] * f.V[k * 3 + 1] + f.O[8] * is[2] * f.V[k * 3 + 2]);
-        }
-        const float n2 = lambda * f.inv_nv;
-        float p2[3] = {f.v[0] * n2, f.v[1] * n2, f.v[2] * n2};
-        // e1 and e2 vanish along the ray through the centre: what rounding left of p . mu_c is taken out of the coefficient that
-        // mu_c weighs most (z for the planar models)
-        const int km = (cam.model == LFS_PINHOLE || cam.model == LFS_PINHOLE_OPENCV) ? 2
-                       : fabsf(f.m[2]) >= fmaxf(fabsf(f.m[0]), fabsf(f.m[1]))       ? 2
-                       : fabsf(f.m[1]) >= fabsf(f.m[0])                             ? 1 : 0;
-        if (m2 > 0.f) {
-            const float im = 1.0f / (km == 2 ? f.m[2] : km == 1 ? f.m[1] : f.m[0]);
-            const float t1 = residual3(p1, f.m) * im, t2 = residual3(p2, f.m) * im;
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if (k == km) { p1[k] -= t1; p2[k] -= t2; }
-        }
-        const float G = f.gamma * f.gamma;
-        rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
-        rec[1] = make_float4(p2[0], p2[1], p2[2], -2.0f * __uint_as_float(thr_bits) / fmaxf(G, 1e-30f));
-        // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
-        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], 0.f) : make_float4(0.6101f, 0.5303f, 0.5887f, 0.f);
-    } else {
+    rec[3] = make_float4(r, g, b, opacity);
+    if (RS) {
         float M[9];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
@@ -509,15 +436,84 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         rec[0] = make_float4(M[0], M[1], M[2], g0);
         rec[1] = make_float4(M[3], M[4], M[5], g1);
         rec[2] = make_float4(M[6], M[7], M[8], g2);
+        return;
     }
-    rec[3] = make_float4(r, g, b, opacity);
+    RayFrame f;
+    ray_frame(cam, R, om, scale, is, f);
+    {
+        const float m2 = fdot3(f.m[0], f.m[0], f.m[1], f.m[1], f.m[2], f.m[2]);
+        const float lambda = m2 > 0.f ? sqrtf(m2) / f.gamma : 1.0f;
+        const float a0 = lambda * is[0], a1 = lambda * is[1], a2 = lambda * is[2];
+        const float n2 = lambda * f.inv_nv;
+        float p1[3], p3[3], p2[3] = {f.v[0] * n2, f.v[1] * n2, f.v[2] * n2};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            p1[k] = fdot3(f.O[0] * a0, f.V[k * 3], f.O[1] * a1, f.V[k * 3 + 1], f.O[2] * a2, f.V[k * 3 + 2]);
+            p3[k] = fdot3(f.O[6] * a0, f.V[k * 3], f.O[7] * a1, f.V[k * 3 + 1], f.O[8] * a2, f.V[k * 3 + 2]);
+        }
+        // e1 and e2 vanish along the ray through the centre: what rounding left of p . mu_c is taken out of the coefficient that
+        // mu_c weighs most (z for the planar models)
+        const int km = (MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV)       ? 2
+                       : fabsf(f.m[2]) >= fmaxf(fabsf(f.m[0]), fabsf(f.m[1]))       ? 2
+                       : fabsf(f.m[1]) >= fabsf(f.m[0])                             ? 1 : 0;
+        if (m2 > 0.f) {
+            const float im = 1.0f / (km == 2 ? f.m[2] : km == 1 ? f.m[1] : f.m[0]);
+            const float t1 = residual3(p1, f.m) * im, t2 = residual3(p2, f.m) * im;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (k == km) { p1[k] -= t1; p2[k] -= t2; }
+        }
+        const float G = f.gamma * f.gamma;
+        rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
+        rec[1] = make_float4(p2[0], p2[1], p2[2], -2.0f * thr / fmaxf(G, 1e-30f));
+        // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
+        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], 0.f) : make_float4(0.6101f, 0.5303f, 0.5887f, 0.f);
+    }
+    if (MODEL == LFS_EQUIRECTANGULAR) return;
+    const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);
+    const float s0 = rho2 * scale.x * scale.x, s1 = rho2 * scale.y * scale.y, s2 = rho2 * scale.z * scale.z;
+    auto sig = [&](int a, int c) { return fdot3(f.V[a * 3] * s0, f.V[c * 3], f.V[a * 3 + 1] * s1, f.V[c * 3 + 1], f.V[a * 3 + 2] * s2, f.V[c * 3 + 2]); };
+    float lo[2], hi[2];   // in units of the focal length, before the principal point
+    bool bounded = false;
+    if (MODEL == LFS_FISHEYE) {
+        bounded = fisheye_box(cam, f.m, sig(0, 0), sig(0, 1), sig(0, 2), sig(1, 1), sig(1, 2), sig(2, 2), lo, hi);
+    } else {
+        const float B22 = fmaf(f.m[2], f.m[2], -sig(2, 2));
+        if (f.m[2] > 0.f && B22 > 0.02f * f.m[2] * f.m[2]) {
+            const float iB = 1.0f / B22;
+#pragma unroll
+            for (int ax = 0; ax < 2; ++ax) {
+                const float Ba2 = fmaf(f.m[ax], f.m[2], -sig(ax, 2));
+                const float Baa = fmaf(f.m[ax], f.m[ax], -sig(ax, ax));
+                const float disc = sqrtf(fmaxf(0.f, fmaf(Ba2, Ba2, -Baa * B22)));
+                lo[ax] = (Ba2 - disc) * iB; hi[ax] = (Ba2 + disc) * iB;
+            }
+            bounded = MODEL == LFS_PINHOLE || opencv_box(cam, lo, hi);
+        }
+    }
+    if (bounded) {
+        uint32_t packed[2];
+        const float fc[2] = {cam.fx, cam.fy}, c0[2] = {cam.cx, cam.cy};
+#pragma unroll
+        for (int ax = 0; ax < 2; ++ax) {
+            const float pa = fmaf(fc[ax], lo[ax], c0[ax]), pb = fmaf(fc[ax], hi[ax], c0[ax]);
+            const float lo_px = fminf(pa, pb), hi_px = fmaxf(pa, pb);
+            const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * (hi_px - lo_px);
+            // pixel j has its centre at j + 0.5
+            const float lo_j = floorf(lo_px - 0.5f - margin), hi_j = ceilf(hi_px - 0.5f + margin);
+            const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo_j, 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi_j, 0.f), 65535.f);
+            packed[ax] = lo_u | (hi_u << 16);
+        }
+        box = make_uint4(packed[0], packed[1], thr_bits, extra_bits);
+    }
 }
 
+template <int MODEL, bool RS>
 __global__ void __launch_bounds__(256) pack_records_kernel(
     int N, const float* __restrict__ means, const float* __restrict__ quats, const float* __restrict__ scales,
     const float* __restrict__ colors, int channels, const float* __restrict__ opacities, const CamDev* __restrict__ cams,
     float4* __restrict__ records, uint4* __restrict__ bounds, float4* __restrict__ accum, float* __restrict__ accum_extra) {
-    const CamDev cam = cams[0];
+    const CamDev& cam = cams[0];
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < N; g += gridDim.x * blockDim.x) {
         const f3 mean{means[g * 3], means[g * 3 + 1], means[g * 3 + 2]};
         const f3 scale{scales[g * 3], scales[g * 3 + 1], scales[g * 3 + 2]};
@@ -527,7 +523,7 @@ __global__ void __launch_bounds__(256) pack_records_kernel(
         // colours [N, channels]: channels 3 = rgb; 4 = rgb + extra; 1 = extra only
         const float* col = colors + (size_t)g * channels;
         const bool has_rgb = channels >= 3;
-        make_record(cam, mean, q.x, q.y, q.z, q.w, scale, has_rgb ? col[0] : 0.f, has_rgb ? col[1] : 0.f, has_rgb ? col[2] : 0.f,
+        make_record<MODEL, RS>(cam, mean, q.x, q.y, q.z, q.w, scale, has_rgb ? col[0] : 0.f, has_rgb ? col[1] : 0.f, has_rgb ? col[2] : 0.f,
                     opacities[g], channels != 3 ? col[channels - 1] : 0.f, rec, box);
 #pragma unroll
         for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
@@ -541,12 +537,22 @@ __global__ void __launch_bounds__(256) pack_records_kernel(
 }
 
 int launch_pack_records(int N, const float* means, const float* quats, const float* scales, const float* colors, int channels,
-                        const float* opacities, const CamDev* cam, float4* records, uint4* bounds, float4* accum,
-                        float* accum_extra, cudaStream_t st) {
+                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, uint4* bounds,
+                        float4* accum, float* accum_extra, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     LFS_TIMED("pack_records", st);
-    pack_records_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, means, quats, scales, colors, channels, opacities, cam, records,
-                                                          bounds, accum, accum_extra);
+#define LFS_PACKREC2(MODEL, RS)                                                                                              \
+    pack_records_kernel<MODEL, RS><<<grid_for(N, 256), 256, 0, st>>>(N, means, quats, scales, colors, channels, opacities, cam, \
+                                                                     records, bounds, accum, accum_extra)
+#define LFS_PACKREC(MODEL) do { if (rolling) LFS_PACKREC2(MODEL, true); else LFS_PACKREC2(MODEL, false); } while (0)
+    switch (model) {
+        case LFS_PINHOLE: LFS_PACKREC(LFS_PINHOLE); break;
+        case LFS_PINHOLE_OPENCV: LFS_PACKREC(LFS_PINHOLE_OPENCV); break;
+        case LFS_EQUIRECTANGULAR: LFS_PACKREC2(LFS_EQUIRECTANGULAR, false); break;
+        default: LFS_PACKREC(LFS_FISHEYE); break;
+    }
+#undef LFS_PACKREC
+#undef LFS_PACKREC2
     return check_launch("pack_records");
 }
 
@@ -555,8 +561,12 @@ int launch_pack_records(int N, const float* means, const float* quats, const flo
 // tile count, depth sort key, SH colour (+0.5, clamped at 0), packed record, zeroed gradient
 // accumulator row. Invisible Gaussians get radii 0, tile count 0 and the sort key 0xFFFFFFFF.
 // ---------------------------------------------------------------------------------------------
+// Bound by instruction issue and the latency of the per-Gaussian chain, not by memory: 64 registers and four CTAs per SM for the
+// models that project in single precision (1 M Gaussians 127 us against 135 with three CTAs, 6 M at 4K 655 against 720); the
+// fisheye evaluates seven double-precision arc tangents per Gaussian and wants its 128 registers instead (6 M: 1120 us against
+// 1176 with three CTAs and 1249 with four).
 template <int MODEL, bool RS>
-__global__ void __launch_bounds__(256, 3) project_pack_kernel(
+__global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pack_kernel(
     int N, int K, int sh_degree, const float* __restrict__ means, const float* __restrict__ sh0,
     const float* __restrict__ shN, const float* __restrict__ scaling_raw, const float* __restrict__ rotation_raw,
     const float* __restrict__ opacity_raw, const CamDev* __restrict__ cams, ProjParams pp, PackOptions opt, float tile_size,
@@ -568,7 +578,7 @@ __global__ void __launch_bounds__(256, 3) project_pack_kernel(
     // each, contiguous in memory) are fetched as one coalesced run into shared memory when any of the 32
     // is visible, and every visible lane then reads its own row from there.
     extern __shared__ __align__(16) float s_rows[];
-    const CamDev cam = cams[0];
+    const CamDev& cam = cams[0];
     const int rest = (K - 1) * 3;
     const int nb = (sh_degree + 1) * (sh_degree + 1);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -641,7 +651,7 @@ __global__ void __launch_bounds__(256, 3) project_pack_kernel(
                 const float* row = my + lane * rest;
                 for (int k = 1; k < nb; ++k) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) rgb[c] += B[k] * row[(k - 1) * 3 + c];
+                    for (int c = 0; c < 3; ++c) rgb[c] = fmaf(B[k], row[(k - 1) * 3 + c], rgb[c]);
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c) rgb[c] = fmaxf(rgb[c] + 0.5f, 0.0f);
@@ -651,7 +661,7 @@ __global__ void __launch_bounds__(256, 3) project_pack_kernel(
 
             float4 rec[4];
             uint4 box;
-            make_record(cam, mean, qw, qx, qy, qz, scale, rgb[0], rgb[1], rgb[2], opacity, o.depth, rec, box);
+            make_record<MODEL, RS>(cam, mean, qw, qx, qy, qz, scale, rgb[0], rgb[1], rgb[2], opacity, o.depth, rec, box);
 #pragma unroll
             for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
             bounds[g] = box;
@@ -707,7 +717,7 @@ __global__ void __launch_bounds__(256) sh_color_kernel(int N, int K, int sh_degr
             const float* row = my + lane * rest;
             for (int k = 1; k < nb; ++k) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) rgb[c] += B[k] * row[(k - 1) * 3 + c];
+                for (int c = 0; c < 3; ++c) rgb[c] = fmaf(B[k], row[(k - 1) * 3 + c], rgb[c]);
             }
             float* out = reinterpret_cast<float*>(records + (size_t)g * 4 + 3);
 #pragma unroll

@@ -29,8 +29,8 @@ int launch_projection_ut(int C, int N, const float* means, const float* quats, c
 // colours [N, channels] with channels 1 (extra only), 3 (rgb) or 4 (rgb + extra); accum / accum_extra (may be null)
 // are zeroed for the backward.
 int launch_pack_records(int N, const float* means, const float* quats, const float* scales, const float* colors, int channels,
-                        const float* opacities, const CamDev* cam, float4* records, uint4* bounds, float4* accum,
-                        float* accum_extra, cudaStream_t st);
+                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, uint4* bounds,
+                        float4* accum, float* accum_extra, cudaStream_t st);
 
 // Per-render switches of the fused path (FusedRasterizationSettings, src/training/rasterization/rasterizer_autograd.hpp).
 struct PackOptions {

@@ -320,15 +320,11 @@ __device__ __forceinline__ float __reduce_add_sync_f32(float x) {
 //   q omega e1, q omega e2 | the same two times phi | q omega^2 e1^2, q omega^2 e1 e2, q omega^2 e2^2 | q phi | rgb | q
 // Rolling shutter: 16 = sum v_u (x) d, sum v_gro, rgb, opacity.
 constexpr int kSums = 12, kSumsRs = 16;
-#ifndef LFS_BWD_PX
-#define LFS_BWD_PX 2
-#endif
-constexpr int kBwdPx = LFS_BWD_PX, kBwdBlock = 256 / kBwdPx;
-template <int BATCH, int NS>
+template <int BATCH, int NS, int PX>
 struct BwdShared {
     Stage<BATCH> stage[3];       // batch b is walked while b+1 and b+2 are in flight
     uint32_t sid[3][BATCH];      // Gaussian index per slot
-    float red[kBwdBlock / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
+    float red[256 / PX / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
 };
 
 // 1 / x for x in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23).
@@ -342,9 +338,9 @@ __device__ __forceinline__ float rcp_newton(float x) {
 // the fused render modes drop it like gsplat/Rasterization.cpp:575-590 does).
 // One thread owns PX horizontally adjacent pixels, a warp a patch of 4 PX x 8: the two pixels' terms are added in registers,
 // so the warp reduction (12 stores, 4 wide loads, the reduction to memory), the record loads and the list walk are paid once
-// for two pixels.
-template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS>
-__global__ void __launch_bounds__(kBwdBlock) raster_bwd_kernel(
+// for two pixels, at the price of more idle lanes in the larger patch. launch_raster_bwd says where which PX runs.
+template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS, int PX>
+__global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds,
     const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
@@ -355,8 +351,7 @@ __global__ void __launch_bounds__(kBwdBlock) raster_bwd_kernel(
     float* __restrict__ accum_extra) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int NS = RS ? kSumsRs : kSums;
-    constexpr int PX = kBwdPx;
-    BwdShared<BATCH, NS>& sm = *reinterpret_cast<BwdShared<BATCH, NS>*>(smem_raw);
+    BwdShared<BATCH, NS, PX>& sm = *reinterpret_cast<BwdShared<BATCH, NS, PX>*>(smem_raw);
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
@@ -419,7 +414,7 @@ __global__ void __launch_bounds__(kBwdBlock) raster_bwd_kernel(
     float* red = sm.red[warp];
 
     // batches run back to front: slot e of batch b holds list position batch_end - e
-    StageIds<BATCH, kBwdBlock> ids;
+    StageIds<BATCH, 256 / PX> ids;
     auto batch_count = [&](int k) { return min(BATCH, range_end - k * BATCH - range_start); };
     auto batch_top = [&](int k) { return range_end - 1 - k * BATCH; };
     if (n_batches > 0) {
@@ -1108,46 +1103,42 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     if (a.channels != 1 && a.channels != 3 && a.channels != 4) { set_error("raster_bwd: channels must be 1, 3 or 4"); return LFS_EINVAL; }
     if (a.normalize && !extra_sum) { set_error("raster_bwd: expected-depth modes need the forward's blended sum"); return LFS_EINVAL; }
     LFS_TIMED("raster_bwd", st);
-#ifndef LFS_BWD_BATCH
-#define LFS_BWD_BATCH 64
-#endif
-    constexpr int kBwdBatch = LFS_BWD_BATCH;
-    constexpr size_t smem = sizeof(BwdShared<kBwdBatch, kSums>), smem_rs = sizeof(BwdShared<kBwdBatch, kSumsRs>);
-    static bool attr_set = false;
-#define LFS_BWD_ATTR(MODEL, EXTRA, XGRAD)                                                                                     \
-    cudaFuncSetAttribute(raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                         (int)smem);                                                                                           \
-    cudaFuncSetAttribute(raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                         (int)smem_rs)
-    if (!attr_set) {
-        LFS_BWD_ATTR(LFS_PINHOLE, false, false); LFS_BWD_ATTR(LFS_PINHOLE, true, false); LFS_BWD_ATTR(LFS_PINHOLE, true, true);
-        LFS_BWD_ATTR(LFS_FISHEYE, false, false); LFS_BWD_ATTR(LFS_FISHEYE, true, false); LFS_BWD_ATTR(LFS_FISHEYE, true, true);
-        LFS_BWD_ATTR(LFS_PINHOLE_OPENCV, false, false); LFS_BWD_ATTR(LFS_PINHOLE_OPENCV, true, false);
-        LFS_BWD_ATTR(LFS_PINHOLE_OPENCV, true, true);
-        LFS_BWD_ATTR(LFS_EQUIRECTANGULAR, false, false); LFS_BWD_ATTR(LFS_EQUIRECTANGULAR, true, false); LFS_BWD_ATTR(LFS_EQUIRECTANGULAR, true, true);
-        attr_set = true;
-    }
-#undef LFS_BWD_ATTR
-#define LFS_BWD4(MODEL, EXTRA, XGRAD, RS)                                                                                     \
-    raster_bwd_kernel<MODEL, kBwdBatch, EXTRA, XGRAD, RS><<<n_tiles, kBwdBlock, RS ? smem_rs : smem, st>>>(                       \
-        a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
-        a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
-        v_alphas, accum, accum_extra)
-#define LFS_BWD(MODEL, EXTRA, XGRAD) do { if (a.rolling) LFS_BWD4(MODEL, EXTRA, XGRAD, true); else LFS_BWD4(MODEL, EXTRA, XGRAD, false); } while (0)
+    // Two pixels per thread where the patches are filled and the CTAs of half the threads still fill the GPU: planar cameras and
+    // at least eight tiles per SM (1 M Gaussians, 1296x840, 4,293 tiles: 889 us against 999 with one; 256 tiles of 256x256:
+    // 127 us against 94). A wide-angle camera shows Gaussians a few pixels across in the middle of its image, where the larger
+    // patch wastes lanes and few tiles carry the work (250 k Gaussians, 1024x1024 fisheye: 478 us against 392).
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
-    if (a.model == LFS_PINHOLE) {
-        if (!extra) LFS_BWD(LFS_PINHOLE, false, false); else if (!xgrad) LFS_BWD(LFS_PINHOLE, true, false); else LFS_BWD(LFS_PINHOLE, true, true);
-    } else if (a.model == LFS_PINHOLE_OPENCV) {
-        if (!extra) LFS_BWD(LFS_PINHOLE_OPENCV, false, false); else if (!xgrad) LFS_BWD(LFS_PINHOLE_OPENCV, true, false);
-        else LFS_BWD(LFS_PINHOLE_OPENCV, true, true);
-    } else if (a.model == LFS_EQUIRECTANGULAR) {
-        if (!extra) LFS_BWD4(LFS_EQUIRECTANGULAR, false, false, false); else if (!xgrad) LFS_BWD4(LFS_EQUIRECTANGULAR, true, false, false);
-        else LFS_BWD4(LFS_EQUIRECTANGULAR, true, true, false);
-    } else {
-        if (!extra) LFS_BWD(LFS_FISHEYE, false, false); else if (!xgrad) LFS_BWD(LFS_FISHEYE, true, false); else LFS_BWD(LFS_FISHEYE, true, true);
-    }
-#undef LFS_BWD4
+    const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
+    const bool wide = planar && !a.rolling && n_tiles >= 8 * num_sms();
+    constexpr int kBatch = 64;
+#define LFS_BWD6(MODEL, EXTRA, XGRAD, RS, PX)                                                                                  \
+    do {                                                                                                                       \
+        constexpr int smem = (int)sizeof(BwdShared<kBatch, RS ? kSumsRs : kSums, PX>);                                         \
+        raster_bwd_kernel<MODEL, kBatch, EXTRA, XGRAD, RS, PX><<<n_tiles, 256 / PX, smem, st>>>(                               \
+            a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
+            a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
+            v_alphas, accum, accum_extra);                                                                                     \
+    } while (0)
+#define LFS_BWD_PLANAR(MODEL, EXTRA, XGRAD)                                                                                    \
+    do {                                                                                                                       \
+        if (a.rolling) LFS_BWD6(MODEL, EXTRA, XGRAD, true, 1);                                                                 \
+        else if (wide) LFS_BWD6(MODEL, EXTRA, XGRAD, false, 2);                                                                \
+        else LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1);                                                                          \
+    } while (0)
+#define LFS_BWD_FISHEYE(MODEL, EXTRA, XGRAD)                                                                                   \
+    do { if (a.rolling) LFS_BWD6(MODEL, EXTRA, XGRAD, true, 1); else LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1); } while (0)
+#define LFS_BWD_EQUIRECT(MODEL, EXTRA, XGRAD) LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1)
+#define LFS_BWD(KIND, MODEL)                                                                                                   \
+    do { if (!extra) KIND(MODEL, false, false); else if (!xgrad) KIND(MODEL, true, false); else KIND(MODEL, true, true); } while (0)
+    if (a.model == LFS_PINHOLE) LFS_BWD(LFS_BWD_PLANAR, LFS_PINHOLE);
+    else if (a.model == LFS_PINHOLE_OPENCV) LFS_BWD(LFS_BWD_PLANAR, LFS_PINHOLE_OPENCV);
+    else if (a.model == LFS_EQUIRECTANGULAR) LFS_BWD(LFS_BWD_EQUIRECT, LFS_EQUIRECTANGULAR);
+    else LFS_BWD(LFS_BWD_FISHEYE, LFS_FISHEYE);
 #undef LFS_BWD
+#undef LFS_BWD_EQUIRECT
+#undef LFS_BWD_FISHEYE
+#undef LFS_BWD_PLANAR
+#undef LFS_BWD6
     return check_launch("raster_bwd");
 }
 
