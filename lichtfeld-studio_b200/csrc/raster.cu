@@ -67,6 +67,12 @@ __device__ __forceinline__ RayForms ray_forms(const float4& r0, const float4& r1
     f.den = f.w * f.w + f.E;
     return f;
 }
+// One special-function instruction (relative error 2^-23); __fdividef spends four more on denominators above 2^126.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ float exp2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                     if (!RS) {
                         const RayForms f = ray_forms<MODEL>(r0, r1, r2, d);
                         if (f.E > r1.w * f.den) continue;
-                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * exp2_approx(r0.w * __fdividef(f.E, f.den)));
+                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * exp2_approx(r0.w * (f.E * rcp_approx(f.den))));
                     } else {
                         const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
                         const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
@@ -329,7 +335,7 @@ struct BwdShared {
 
 // 1 / x for x in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23).
 __device__ __forceinline__ float rcp_newton(float x) {
-    const float y = __fdividef(1.0f, x);
+    const float y = rcp_approx(x);
     return fmaf(y, fmaf(-x, y, 1.0f), y);
 }
 
@@ -495,7 +501,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
                 for (int p = 0; p < PX; ++p) {
                     rden[p] = phi[p] = 0.f;
                     if (!RS) {
-                        rden[p] = __fdividef(1.0f, f[p].den);
+                        rden[p] = rcp_approx(f[p].den);
                         phi[p] = f[p].E * rden[p];
                         vis[p] = exp2_approx(r0.w * phi[p]);
                     } else {
