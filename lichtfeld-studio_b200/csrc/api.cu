@@ -51,8 +51,7 @@ int sorted_sel(int key_bits) { return ((key_bits + 7) / 8) & 1; }
 
 SortScratch carve_scratch(Carver& c) {
     SortScratch s;
-    s.hist = c.take<uint32_t>((size_t)kRadixBlocks * 256);
-    s.block_sums = c.take<uint32_t>(kScanBlocks + 320);  // also holds the 256 digit totals of a radix pass
+    s.block_sums = c.take<uint32_t>(kScanBlocks + 1);
     return s;
 }
 
@@ -60,12 +59,12 @@ SortScratch carve_scratch(Carver& c) {
 struct RenderWs {
     CamDev* cam;
     int32_t* counters;  // [0] overflow, [1] n_isects, [2] n_visible
-    int32_t *radii, *tiles, *offs, *tile_offsets, *last_ids, *tile_order;
+    int32_t *radii, *tiles, *tile_offsets, *last_ids, *tile_order;
     float *means2d, *depths, *accum, *extra_sum;
     float4* records;
     uint4* bounds;
     uint32_t *gkeys[2], *gvals[2], *tkeys[2], *tvals[2];
-    SortScratch scratch;
+    uint32_t* list_state;
     size_t bytes;
 };
 
@@ -82,7 +81,6 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
     w.means2d = c.take<float>(N * 2);
     w.depths = c.take<float>(N);
     w.tiles = c.take<int32_t>(N);
-    w.offs = c.take<int32_t>(N);
     for (int k = 0; k < 2; ++k) { w.gkeys[k] = c.take<uint32_t>(N); w.gvals[k] = c.take<uint32_t>(N); }
     w.records = c.take<float4>(N * 4);
     w.bounds = c.take<uint4>(N);
@@ -92,7 +90,7 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
     w.tile_order = c.take<int32_t>((size_t)tw * th);
     w.last_ids = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
     w.extra_sum = c.take<float>((size_t)cfg.image_width * cfg.image_height);  // blended depth before the division (ED modes)
-    w.scratch = carve_scratch(c);
+    w.list_state = c.take<uint32_t>(tile_list_state_words((int64_t)N, (int64_t)cap, (int)bit_width_u32((uint32_t)tw * th) + 1));
     w.bytes = c.total();
     return w;
 }
@@ -100,12 +98,12 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
 // ---- EWA workspace ----------------------------------------------------------------------------
 struct EwaWs {
     int32_t* counters;  // [0] overflow, [1] n_instances, [2] n_visible
-    int32_t *n_touched, *offs, *tile_offsets, *n_contrib, *tile_order;
+    int32_t *n_touched, *tile_offsets, *n_contrib, *tile_order;
     ushort4* bounds;
     float4* records;
     float* accum;
     uint32_t *gkeys[2], *gvals[2], *tkeys[2], *tvals[2];
-    SortScratch scratch;
+    uint32_t* list_state;
     size_t bytes;
 };
 
@@ -116,7 +114,6 @@ EwaWs carve_ewa(const lfs_ewa_config& cfg, void* base) {
     const int tw = (cfg.image_width + 15) / 16, th = (cfg.image_height + 15) / 16;
     w.counters = c.take<int32_t>(16);
     w.n_touched = c.take<int32_t>(N);
-    w.offs = c.take<int32_t>(N);
     w.bounds = c.take<ushort4>(N);
     w.records = c.take<float4>(N * 3);
     w.accum = c.take<float>(N * 12);
@@ -125,7 +122,7 @@ EwaWs carve_ewa(const lfs_ewa_config& cfg, void* base) {
     w.tile_offsets = c.take<int32_t>((size_t)tw * th + 1);
     w.n_contrib = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
     w.tile_order = c.take<int32_t>((size_t)tw * th);
-    w.scratch = carve_scratch(c);
+    w.list_state = c.take<uint32_t>(tile_list_state_words((int64_t)N, (int64_t)cap, (int)bit_width_u32((uint32_t)tw * th) + 1));
     w.bytes = c.total();
     return w;
 }
@@ -250,23 +247,23 @@ int lfs_intersect_tile_count(int C, int N, const float* means2d, const int32_t* 
     return launch_sum_i32(total, tiles_per_gauss, n_isects_dev, S(stream));
 }
 
-static size_t isect_ws(int C, int N, int64_t n_isects, void* base, uint32_t** gk, uint32_t** gv, int32_t** offs,
-                       int32_t** n_dev, uint32_t** tk, uint32_t** tv, SortScratch* s) {
+// (camera, tile) keys of the operator: the tile grid is not known to the workspace query, so their look-back words are sized
+// for 32-bit keys
+static size_t isect_ws(int C, int N, int64_t n_isects, void* base, uint32_t** gk, uint32_t** gv,
+                       int32_t** n_dev, uint32_t** tk, uint32_t** tv, uint32_t** state) {
     Carver c(base);
     const size_t total = (size_t)C * N, cap = (size_t)(n_isects > 0 ? n_isects : 1);
     for (int k = 0; k < 2; ++k) { gk[k] = c.take<uint32_t>(total); gv[k] = c.take<uint32_t>(total); }
-    *offs = c.take<int32_t>(total);
     *n_dev = c.take<int32_t>(16);
     for (int k = 0; k < 2; ++k) { tk[k] = c.take<uint32_t>(cap); tv[k] = c.take<uint32_t>(cap); }
-    *s = carve_scratch(c);
+    *state = c.take<uint32_t>(tile_list_state_words((int64_t)total, (int64_t)cap, 32));
     return c.total();
 }
 
 size_t lfs_intersect_tile_workspace_bytes(int C, int N, int64_t n_isects) {
-    uint32_t *gk[2], *gv[2], *tk[2], *tv[2];
-    int32_t *offs, *n_dev;
-    SortScratch s;
-    return isect_ws(C, N, n_isects, nullptr, gk, gv, &offs, &n_dev, tk, tv, &s);
+    uint32_t *gk[2], *gv[2], *tk[2], *tv[2], *state;
+    int32_t* n_dev;
+    return isect_ws(C, N, n_isects, nullptr, gk, gv, &n_dev, tk, tv, &state);
 }
 
 int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* radii, const float* depths,
@@ -276,7 +273,7 @@ int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* r
     if (n_isects == 0 || (int64_t)C * N == 0) return LFS_OK;
     LFS_REQUIRE(means2d && radii && depths && tiles_per_gauss && isect_ids && flatten_ids && workspace, "null pointer");
     TileListArgs a{};
-    const size_t need = isect_ws(C, N, n_isects, workspace, a.gkeys, a.gvals, &a.offs, &a.n_isects_dev, a.tkeys, a.tvals, &a.scratch);
+    const size_t need = isect_ws(C, N, n_isects, workspace, a.gkeys, a.gvals, &a.n_isects_dev, a.tkeys, a.tvals, &a.state);
     if (workspace_bytes < need) { set_error("lfs_intersect_tile_emit: workspace too small (%zu < %zu)", workspace_bytes, need); return LFS_ECAPACITY; }
     a.C = C; a.N = N; a.tw = tw; a.th = th; a.tile_size = tile_size; a.sort = sort ? 1 : 0; a.keys_ready = 0;
     a.means2d = means2d; a.radii = radii; a.depths = depths; a.tiles = tiles_per_gauss;
@@ -668,10 +665,10 @@ int lfs_ewa_forward(const lfs_ewa_config* cfg, const lfs_splats* params, const f
     a.C = 1; a.N = cfg->N; a.tw = cam.tw; a.th = cam.th; a.tile_size = 16; a.sort = 1; a.keys_ready = 1;
     a.tiles = w.n_touched;
     for (int k = 0; k < 2; ++k) { a.gkeys[k] = w.gkeys[k]; a.gvals[k] = w.gvals[k]; a.tkeys[k] = w.tkeys[k]; a.tvals[k] = w.tvals[k]; }
-    a.offs = w.offs; a.n_isects_dev = w.counters + 1; a.capacity = cfg->instance_capacity; a.overflow = w.counters + 0;
+    a.n_isects_dev = w.counters + 1; a.capacity = cfg->instance_capacity; a.overflow = w.counters + 0;
     int sel = 0;
     a.sel_out = &sel;
-    a.tile_offsets = w.tile_offsets; a.scratch = w.scratch;
+    a.tile_offsets = w.tile_offsets; a.state = w.list_state;
     a.ewa_bounds = w.bounds; a.ewa_records = w.records;
     rc = build_tile_lists(a, st);
     if (rc != LFS_OK) return rc;
@@ -794,9 +791,9 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
     a.C = 1; a.N = cfg->N; a.tw = tw; a.th = th; a.tile_size = cfg->tile_size; a.sort = 1; a.keys_ready = 1;
     a.means2d = w.means2d; a.radii = w.radii; a.depths = w.depths; a.tiles = w.tiles;
     for (int k = 0; k < 2; ++k) { a.gkeys[k] = w.gkeys[k]; a.gvals[k] = w.gvals[k]; a.tkeys[k] = w.tkeys[k]; a.tvals[k] = w.tvals[k]; }
-    a.offs = w.offs; a.n_isects_dev = w.counters + 1; a.capacity = cfg->isect_capacity; a.overflow = w.counters + 0;
+    a.n_isects_dev = w.counters + 1; a.capacity = cfg->isect_capacity; a.overflow = w.counters + 0;
     a.sel_out = sel_out;
-    a.tile_offsets = w.tile_offsets; a.scratch = w.scratch;
+    a.tile_offsets = w.tile_offsets; a.state = w.list_state;
     rc = build_tile_lists(a, st);
     if (rc != LFS_OK) return rc;
     return launch_tile_order(tw * th, w.tile_offsets, w.tile_order, st);

@@ -100,19 +100,10 @@ int launch_camera_setup(int C, const float* viewmats, const float* viewmats1, in
 
 // ---- sort.cu -------------------------------------------------------------------------------
 struct SortScratch {
-    uint32_t* hist;       // [kRadixBlocks * 256]
     uint32_t* block_sums; // [kScanBlocks + 1]
 };
-// Capacity of the scratch arrays; the launches use min(4 x SM count, capacity) blocks.
-constexpr int kRadixBlocks = 1024;
+// Capacity of the scratch array; the launches use min(4 x SM count, capacity) blocks.
 constexpr int kScanBlocks = 1024;
-size_t sort_scratch_bytes();
-
-// Stable LSD radix sort of (key, value) uint32 pairs over key bits [0, key_bits). n is read from
-// *n_dev when n_dev != nullptr (device-side count, bounded by n_max), else n_max is the count.
-// Returns the index (0 or 1) of the buffer pair holding the result.
-int radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], const int32_t* n_dev, int64_t n_max, int key_bits,
-                     const SortScratch& scratch, cudaStream_t st);
 
 // out[i] = exclusive prefix sum of gather(i) = src[idx ? idx[i] : i]; total written to *total_dev.
 int exclusive_scan_gather(const int32_t* src, const uint32_t* idx, int64_t n, int32_t* out, int32_t* total_dev,

@@ -83,7 +83,6 @@ extern "C" int lfs_mcmc_classify_noalloc(int N, const float* opacity_raw, const 
     int32_t* offs = reinterpret_cast<int32_t*>(base + kOffsOff);
     int32_t* total = reinterpret_cast<int32_t*>(base + kTotalOff);
     SortScratch s;
-    s.hist = nullptr;  // only the prefix scan runs here; it does not touch the radix histogram
     s.block_sums = reinterpret_cast<uint32_t*>(base + kSumsOff);
     // The scratch still holds the previous call's flags, prefix and count. Flags and prefix are rewritten
     // for [0, N) before they are read; the count is the one value a reader could see stale, so clear it.

@@ -16,7 +16,6 @@ struct TileListArgs {
     const int32_t* tiles;  // [C*N] tiles per Gaussian
     uint32_t* gkeys[2];    // [C*N] each
     uint32_t* gvals[2];    // [C*N] each
-    int32_t* offs;         // [C*N] exclusive prefix of tiles in emission order
     int32_t* n_isects_dev; // device int32: total number of instances
     int64_t capacity;      // room in tkeys / tvals
     uint32_t* tkeys[2];
@@ -24,7 +23,7 @@ struct TileListArgs {
     int32_t* overflow;     // device flag set when an instance does not fit (may be null)
     int* sel_out;          // host: which of tkeys/tvals holds the result
     int32_t* tile_offsets; // [C*tw*th + 1] or null
-    SortScratch scratch;
+    uint32_t* state;       // [tile_list_state_words], 16-byte aligned
     // EWA path (C = 1): when set, a Gaussian's instances are the tiles of its bounds rectangle that pass the exact
     // ellipse test (`tiles` holds that count); means2d / radii are unused
     const ushort4* ewa_bounds = nullptr;  // [N] (x_min, x_max, y_min, y_max) in tiles
@@ -32,6 +31,8 @@ struct TileListArgs {
 };
 
 int build_tile_lists(const TileListArgs& a, cudaStream_t st);
+// key_bits: bits of the (camera, tile) key
+size_t tile_list_state_words(int64_t total, int64_t capacity, int key_bits);
 
 // order [n_tiles]: tile indices, longest lists first; offsets [n_tiles + 1]
 int launch_tile_order(int n_tiles, const int32_t* offsets, int32_t* order, cudaStream_t st);
