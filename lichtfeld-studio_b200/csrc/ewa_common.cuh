@@ -24,6 +24,9 @@ constexpr int kEwaRecordVec4 = 3;
 // [min_x, max_x] x [min_y, max_y]? (mx, my) is the 2-D mean shifted by -0.5 so that pixel centres sit on integers.
 // The point of the rectangle with the smallest exponent lies either inside (mean inside) or on the two edges that
 // face the mean; each edge is searched by the closed-form minimiser of the quadratic along it, clamped to the edge.
+// FAST: hardware division (for callers that only cull, with a margin on the threshold; the minimiser along an edge moves the
+// exponent in second order). The lists are pinned to the exact one.
+template <bool FAST = false>
 __device__ __forceinline__ bool ewa_rect_contributes(float mx, float my, float ca, float cb, float cc, float min_x, float max_x,
                                                      float min_y, float max_y, float power_threshold) {
     const float x_min_diff = min_x - mx;
@@ -37,8 +40,10 @@ __device__ __forceinline__ bool ewa_rect_contributes(float mx, float my, float c
     const float corner_y = max_y + y_above * (min_y - max_y);
     const float diff_x = mx - corner_x, diff_y = my - corner_y;
     const float dx = copysignf(max_x - min_x, x_min_diff), dy = copysignf(max_y - min_y, y_min_diff);
-    const float t_x = not_in_y * __saturatef((dx * ca * diff_x + dx * cb * diff_y) / (dx * ca * dx));
-    const float t_y = not_in_x * __saturatef((dy * cb * diff_x + dy * cc * diff_y) / (dy * cc * dy));
+    const float num_x = dx * ca * diff_x + dx * cb * diff_y, den_x = dx * ca * dx;
+    const float num_y = dy * cb * diff_x + dy * cc * diff_y, den_y = dy * cc * dy;
+    const float t_x = not_in_y * __saturatef(FAST ? __fdividef(num_x, den_x) : num_x / den_x);
+    const float t_y = not_in_x * __saturatef(FAST ? __fdividef(num_y, den_y) : num_y / den_y);
     const float px = corner_x + t_x * dx, py = corner_y + t_y * dy;
     const float ex = mx - px, ey = my - py;
     const float power = 0.5f * (ca * ex * ex + cc * ey * ey) + cb * ex * ey;

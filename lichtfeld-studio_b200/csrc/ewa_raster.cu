@@ -14,6 +14,7 @@
 // coalesced reduction of nine words per (warp, Gaussian), so that the per-entry costs are paid once for two pixels.
 #include "ewa.cuh"
 #include "ewa_common.cuh"
+#include "gsmath.cuh"
 
 namespace lfs {
 namespace {
@@ -64,7 +65,7 @@ __device__ __forceinline__ void cull_batch(const float4* rec, int lo, int hi, fl
         if (e >= lo && e < hi) {
             const float4 r0 = rec[e * 3], r1 = rec[e * 3 + 1], r2 = rec[e * 3 + 2];
             // a small margin on the threshold keeps the test conservative under rounding
-            ok = ewa_rect_contributes(r0.x - 0.5f, r0.y - 0.5f, r0.z, r0.w, r1.x, px0, px0 + (PW - 1.0f), py0, py0 + (PH - 1.0f), r2.z + 0.01f);
+            ok = ewa_rect_contributes<true>(r0.x - 0.5f, r0.y - 0.5f, r0.z, r0.w, r1.x, px0, px0 + (PW - 1.0f), py0, py0 + (PH - 1.0f), r2.z + 0.01f);
         }
         live[w] = __ballot_sync(0xffffffffu, ok);
     }
@@ -308,8 +309,10 @@ __global__ void __launch_bounds__(256, 4) ewa_epilogue_kernel(
     const float* __restrict__ accum, float* __restrict__ g_means, float* __restrict__ g_sh0, float* __restrict__ g_shN,
     float* __restrict__ g_scaling, float* __restrict__ g_rotation, float* __restrict__ g_opacity, int accumulate,
     float* __restrict__ densification_info, float* __restrict__ grad_w2c) {
-    extern __shared__ float s_rows[];
+    extern __shared__ __align__(16) float s_rows[];
     __shared__ float s_pose[8][12];
+    const bool rows_aligned = (reinterpret_cast<uintptr_t>(shN) & 15) == 0;
+    const bool out_aligned = (reinterpret_cast<uintptr_t>(g_shN) & 15) == 0;
     if (W2C) {
         if (threadIdx.x < 96) s_pose[threadIdx.x / 12][threadIdx.x % 12] = 0.f;
         __syncthreads();
@@ -347,8 +350,14 @@ __global__ void __launch_bounds__(256, 4) ewa_epilogue_kernel(
             continue;
         }
         if (nb > 1) {
+            // 16-byte asynchronous copies where the tensor allows it (a chunk starts at a multiple of 32 rows): one round trip
+            // for the chunk instead of one per register batch
             const float* src_rows = shN + (size_t)chunk * 32 * rest;
-            for (int k = lane; k < total; k += 32) my[k] = src_rows[k];
+            const int total4 = rows_aligned ? total >> 2 : 0;
+            for (int k = lane; k < total4; k += 32) cp_async16(my + k * 4, src_rows + k * 4);
+            cp_async_commit();
+            for (int k = total4 * 4 + lane; k < total; k += 32) my[k] = src_rows[k];
+            cp_async_wait<0>();
         }
         __syncwarp();
         float* out_rest = my + lane * rest;   // this lane's row: coefficients now, gradients afterwards
@@ -534,10 +543,8 @@ __global__ void __launch_bounds__(256, 4) ewa_epilogue_kernel(
         }
         if (!g_shN) {
             // the caller rebuilds these rows from the sh0 gradient (lfs_ewa_adam_step_rank1_sh)
-        } else if (accumulate) {
-            for (int k = lane; k < total; k += 32) dst_rows[k] += my[k];
         } else {
-            for (int k = lane; k < total; k += 32) dst_rows[k] = my[k];
+            store_rows(dst_rows, my, total, lane, out_aligned, accumulate != 0);
         }
         __syncwarp();
         if (in_range && (visible || !accumulate)) {

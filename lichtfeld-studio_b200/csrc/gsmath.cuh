@@ -476,6 +476,33 @@ __device__ __forceinline__ void ray_frame(const CamDev& cam, const float* R, f3 
     f.O[2] = fmaf(f.O[3], f.O[7], -f.O[4] * f.O[6]);
 }
 
+// A warp writes (or adds) a contiguous run of floats from shared memory, 16 bytes per lane and four of them in flight where the
+// destination is 16-byte aligned (the source is).
+__device__ __forceinline__ void store_rows(float* __restrict__ dst, const float* __restrict__ src, int total, int lane, bool aligned,
+                                           bool add) {
+    const int n4 = aligned ? total >> 2 : 0;
+    float4* d4 = reinterpret_cast<float4*>(dst);
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    if (add) {
+        for (int i0 = lane; i0 < n4; i0 += 128) {
+            float4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + 32 * u < n4) x[u] = d4[i0 + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + 32 * u < n4) {
+                    const float4 y = s4[i0 + 32 * u];
+                    d4[i0 + 32 * u] = make_float4(x[u].x + y.x, x[u].y + y.y, x[u].z + y.z, x[u].w + y.w);
+                }
+        }
+        for (int i = n4 * 4 + lane; i < total; i += 32) dst[i] += src[i];
+    } else {
+        for (int i = lane; i < n4; i += 32) d4[i] = s4[i];
+        for (int i = n4 * 4 + lane; i < total; i += 32) dst[i] = src[i];
+    }
+}
+
 // Tile rectangle covered by a projected Gaussian: [x0,x1) x [y0,y1) in tile units. The float ->
 // unsigned conversion saturates (negative -> 0), which is what clips boxes that start left of /
 // above the image.

@@ -4,8 +4,11 @@
 // Replaces src/training/kernels/ssim.cu:64 (K9) and :284 (K10), the crop / pad / mean glue of
 // include/kernels/fused_ssim.cuh:59-67, :85-96, :117-122, torch::l1_loss of
 // src/training/trainer.cpp:126 and the clamp + permute of src/training/rasterization/rasterizer.cpp:205.
-// Stencil work: each CTA stages the 42x42 halo tile of a 32x32 output tile of one channel in shared memory and runs
-// the 11-tap horizontal and vertical passes from register windows (4 outputs per 14 loaded values).
+// Stencil work, bound by instruction issue and shared-memory accesses: each CTA stages the 42x42 halo tile of a 32x32 output
+// tile of one channel in shared memory and runs the 11-tap horizontal and vertical passes from register windows. The planes
+// that are filtered alike are kept as pairs (x, y), (x^2, y^2) and filtered two at a time with the packed fp32 instructions
+// (one issue slot and one 8-byte shared load for both, each element rounded as by the scalar instruction). 352 threads: the
+// 42 rows x 8 column groups of the horizontal pass and the 32 columns x 11 strips of the vertical pass each fill them once.
 #include "common.cuh"
 #include "loss.cuh"
 
@@ -18,8 +21,10 @@ constexpr int kHalo = 5;
 constexpr int kS = kT + 2 * kHalo;   // 42: halo tile edge
 constexpr int kSX = kS + 1;          // 43: row stride of the staged images (conflict-free for lanes that walk rows)
 constexpr int kSH = kT + 1;          // 33: row stride of the horizontally filtered planes
-constexpr int kThreadsLoss = 256;
+constexpr int kThreadsLoss = 352;
 constexpr int kColGroups = kT / 4;   // a horizontal work item filters 4 adjacent columns of one row
+constexpr int kStrip = 3;            // a vertical work item filters 3 stacked rows of one column
+static_assert(kS * kColGroups <= kThreadsLoss && kThreadsLoss / 32 * kStrip >= kT, "one round per pass");
 
 __constant__ float cTaps[11] = {
     0.001028380123898387f, 0.0075987582094967365f, 0.036000773310661316f, 0.10936068743467331f,
@@ -46,80 +51,128 @@ __device__ __forceinline__ float tap11(const float* v, int ci) {
     return a + v[ci] * cTaps[kHalo];
 }
 
+// Two fp32 values in one register pair.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// tap11 on pairs, the same operations on both elements; taps = the six distinct weights, each in both halves
+__device__ __forceinline__ f32x2 tap11x2(const f32x2* v, int ci, const f32x2* taps) {
+    f32x2 a = mul2(add2(v[ci - 1], v[ci + 1]), taps[kHalo - 1]);
+#pragma unroll
+    for (int d = 2; d <= kHalo; ++d) a = fma2(add2(v[ci - d], v[ci + d]), taps[kHalo - d], a);
+    return fma2(v[ci], taps[kHalo], a);
+}
+
 // One CTA filters a 32x32 output tile of one channel (blockIdx.z). The 42x42 halo tile is staged in shared memory;
-// the horizontal pass gives every thread 4 adjacent outputs of one row from a 14-value register window (7 shared
-// loads per output instead of 44), the vertical pass 4 stacked outputs of one column from 14-value windows of the five
-// filtered planes.
+// the horizontal pass gives every thread 4 adjacent outputs of one row from a 14-value register window, the vertical pass 3
+// stacked outputs of one column from 13-value windows of the filtered planes.
 //
 // Forward. Plain mode writes ssim_map and the three derivative maps. Fused mode writes the derivative maps already
 // multiplied by dL/dmap (map_grad inside the valid crop, 0 outside) and accumulates sum(ssim over the crop) and
 // sum(|img1 - img2|) into sums[0], sums[1].
 template <bool FUSED>
-__global__ void __launch_bounds__(kThreadsLoss) ssim_fwd_kernel(int CH, int H, int W, float C1, float C2,
-                                                               const float* __restrict__ img1, const float* __restrict__ img2,
-                                                               float* __restrict__ ssim_map, float* __restrict__ dm_dmu1,
-                                                               float* __restrict__ dm_dsigma1_sq, float* __restrict__ dm_dsigma12,
-                                                               float map_grad, int crop, double* __restrict__ sums) {
-    __shared__ float sX[kS][kSX], sY[kS][kSX];
-    __shared__ float sH[5][kS][kSH];
+__global__ void __launch_bounds__(kThreadsLoss, 3) ssim_fwd_kernel(int CH, int H, int W, float C1, float C2,
+                                                                  const float* __restrict__ img1, const float* __restrict__ img2,
+                                                                  float* __restrict__ ssim_map, float* __restrict__ dm_dmu1,
+                                                                  float* __restrict__ dm_dsigma1_sq, float* __restrict__ dm_dsigma12,
+                                                                  float map_grad, int crop, double* __restrict__ sums) {
+    __shared__ f32x2 sXY[kS][kSX];            // (img1, img2)
+    __shared__ f32x2 sM[kS][kSH], sQ[kS][kSH];  // filtered (x, y) and (x^2, y^2)
+    __shared__ float sP[kS][kSH];               // filtered x y
     __shared__ float red[2][kThreadsLoss / 32];
     const int tid = threadIdx.x, c = blockIdx.z;
     const int bx0 = blockIdx.x * kT, by0 = blockIdx.y * kT;
+    f32x2 taps[kHalo + 1];
+#pragma unroll
+    for (int d = 0; d <= kHalo; ++d) taps[d] = pack2(cTaps[d], cTaps[d]);
     for (int q = tid; q < kS * kS; q += kThreadsLoss) {
         const int ly = q / kS, lx = q - ly * kS;
-        sX[ly][lx] = load_img1<FUSED>(img1, c, by0 + ly - kHalo, bx0 + lx - kHalo, H, W);
-        sY[ly][lx] = load_chw(img2, c, by0 + ly - kHalo, bx0 + lx - kHalo, H, W);
+        sXY[ly][lx] = pack2(load_img1<FUSED>(img1, c, by0 + ly - kHalo, bx0 + lx - kHalo, H, W),
+                            load_chw(img2, c, by0 + ly - kHalo, bx0 + lx - kHalo, H, W));
     }
     __syncthreads();
-    for (int item = tid; item < kS * kColGroups; item += kThreadsLoss) {
-        const int cg = item / kS, row = item - cg * kS;
-        float xv[14], yv[14], q[14];
+    if (tid < kS * kColGroups) {
+        const int cg = tid / kS, row = tid - cg * kS;
+        f32x2 w[14];
+        float xy[14];
 #pragma unroll
-        for (int j = 0; j < 14; ++j) { xv[j] = sX[row][cg * 4 + j]; yv[j] = sY[row][cg * 4 + j]; }
+        for (int j = 0; j < 14; ++j) {
+            w[j] = sXY[row][cg * 4 + j];
+            const float2 v = unpack2(w[j]);
+            xy[j] = v.x * v.y;
+        }
 #pragma unroll
-        for (int o = 0; o < 4; ++o) sH[0][row][cg * 4 + o] = tap11(xv, o + kHalo);
+        for (int o = 0; o < 4; ++o) sP[row][cg * 4 + o] = tap11(xy, o + kHalo);
 #pragma unroll
-        for (int o = 0; o < 4; ++o) sH[2][row][cg * 4 + o] = tap11(yv, o + kHalo);
+        for (int o = 0; o < 4; ++o) sM[row][cg * 4 + o] = tap11x2(w, o + kHalo, taps);
 #pragma unroll
-        for (int j = 0; j < 14; ++j) q[j] = xv[j] * xv[j];
+        for (int j = 0; j < 14; ++j) w[j] = mul2(w[j], w[j]);
 #pragma unroll
-        for (int o = 0; o < 4; ++o) sH[1][row][cg * 4 + o] = tap11(q, o + kHalo);
-#pragma unroll
-        for (int j = 0; j < 14; ++j) q[j] = yv[j] * yv[j];
-#pragma unroll
-        for (int o = 0; o < 4; ++o) sH[3][row][cg * 4 + o] = tap11(q, o + kHalo);
-#pragma unroll
-        for (int j = 0; j < 14; ++j) q[j] = xv[j] * yv[j];
-#pragma unroll
-        for (int o = 0; o < 4; ++o) sH[4][row][cg * 4 + o] = tap11(q, o + kHalo);
+        for (int o = 0; o < 4; ++o) sQ[row][cg * 4 + o] = tap11x2(w, o + kHalo, taps);
     }
     __syncthreads();
-    const int col = tid & 31, strip = tid >> 5;
-    float out[4][5];
+    const int col = tid & 31, strip = (tid >> 5) * kStrip;
+    float2 mu[kStrip], sq[kStrip];
+    float sxy[kStrip];
+    constexpr int kWin = kStrip + 2 * kHalo;
+    {
+        // windows past the last strip read the last row again; those outputs lie outside the tile
+        f32x2 h[kWin];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        float h[14];
+        for (int j = 0; j < kWin; ++j) h[j] = sM[min(strip + j, kS - 1)][col];
 #pragma unroll
-        for (int j = 0; j < 14; ++j) h[j] = sH[k][strip * 4 + j][col];
+        for (int o = 0; o < kStrip; ++o) mu[o] = unpack2(tap11x2(h, o + kHalo, taps));
 #pragma unroll
-        for (int o = 0; o < 4; ++o) out[o][k] = tap11(h, o + kHalo);
+        for (int j = 0; j < kWin; ++j) h[j] = sQ[min(strip + j, kS - 1)][col];
+#pragma unroll
+        for (int o = 0; o < kStrip; ++o) sq[o] = unpack2(tap11x2(h, o + kHalo, taps));
+        float g[kWin];
+#pragma unroll
+        for (int j = 0; j < kWin; ++j) g[j] = sP[min(strip + j, kS - 1)][col];
+#pragma unroll
+        for (int o = 0; o < kStrip; ++o) sxy[o] = tap11(g, o + kHalo);
     }
     float ssim_acc = 0.f, l1_acc = 0.f;
     const int x = bx0 + col;
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {
-        const int y = by0 + strip * 4 + o;
-        if (x < W && y < H) {
-            const float mu1 = out[o][0], mu2 = out[o][2];
+    for (int o = 0; o < kStrip; ++o) {
+        const int y = by0 + strip + o;
+        if (strip + o < kT && x < W && y < H) {
+            const float mu1 = mu[o].x, mu2 = mu[o].y;
             const float mu1_sq = mu1 * mu1, mu2_sq = mu2 * mu2;
-            const float sigma1_sq = out[o][1] - mu1_sq, sigma2_sq = out[o][3] - mu2_sq, sigma12 = out[o][4] - mu1 * mu2;
+            const float sigma1_sq = sq[o].x - mu1_sq, sigma2_sq = sq[o].y - mu2_sq, sigma12 = sxy[o] - mu1 * mu2;
             const float A = mu1_sq + mu2_sq + C1, B = sigma1_sq + sigma2_sq + C2;
             const float C_ = 2.f * mu1 * mu2 + C1, D_ = 2.f * sigma12 + C2;
-            const float val = (C_ * D_) / (A * B);
-            const float g_mu1 = ((mu2 * 2.f * D_) / (A * B) - (mu2 * 2.f * C_) / (A * B) -
-                                 (mu1 * 2.f * C_ * D_) / (A * A * B) + (mu1 * 2.f * C_ * D_) / (A * B * B));
-            const float g_s1 = (-C_ * D_) / (A * B * B);
-            const float g_s12 = (2.f * C_) / (A * B);
+            // two divisions serve the map and its derivatives
+            const float rA = 1.0f / A, rB = 1.0f / B;
+            const float cA = C_ * rA, dB = D_ * rB;
+            const float val = cA * dB;
+            const float g_mu1 = 2.f * (mu2 * rA * dB - mu2 * rB * cA - mu1 * rA * val + mu1 * rB * val);
+            const float g_s1 = -val * rB;
+            const float g_s12 = 2.f * cA * rB;
             const size_t gi = (size_t)c * H * W + (size_t)y * W + x;
             if (FUSED) {
                 const bool in_crop = !crop || (x >= kHalo && x < W - kHalo && y >= kHalo && y < H - kHalo);
@@ -128,8 +181,8 @@ __global__ void __launch_bounds__(kThreadsLoss) ssim_fwd_kernel(int CH, int H, i
                 dm_dsigma1_sq[gi] = g_s1 * chain;
                 dm_dsigma12[gi] = g_s12 * chain;
                 if (in_crop) ssim_acc += val;
-                const int ly = strip * 4 + o + kHalo, lx = col + kHalo;
-                l1_acc += fabsf(sX[ly][lx] - sY[ly][lx]);
+                const float2 v = unpack2(sXY[strip + o + kHalo][col + kHalo]);
+                l1_acc += fabsf(v.x - v.y);
             } else {
                 ssim_map[gi] = val;
                 if (dm_dmu1) { dm_dmu1[gi] = g_mu1; dm_dsigma1_sq[gi] = g_s1; dm_dsigma12[gi] = g_s12; }
@@ -157,56 +210,68 @@ __global__ void __launch_bounds__(kThreadsLoss) ssim_fwd_kernel(int CH, int H, i
 // are pre-multiplied, the L1 sign term and the clamp mask are applied and the output is the HWC gradient of the
 // unclamped render, scaled by grad_scale.
 template <bool FUSED>
-__global__ void __launch_bounds__(kThreadsLoss) ssim_bwd_kernel(int CH, int H, int W, const float* __restrict__ img1,
-                                                               const float* __restrict__ img2, const float* __restrict__ dL_dmap,
-                                                               const float* __restrict__ dm_dmu1, const float* __restrict__ dm_dsigma1_sq,
-                                                               const float* __restrict__ dm_dsigma12, float* __restrict__ dL_dimg1,
-                                                               float l1_grad, float grad_scale) {
-    __shared__ float sD[3][kS][kSX];
-    __shared__ float sH[3][kS][kSH];
+__global__ void __launch_bounds__(kThreadsLoss, 4) ssim_bwd_kernel(int CH, int H, int W, const float* __restrict__ img1,
+                                                                  const float* __restrict__ img2, const float* __restrict__ dL_dmap,
+                                                                  const float* __restrict__ dm_dmu1, const float* __restrict__ dm_dsigma1_sq,
+                                                                  const float* __restrict__ dm_dsigma12, float* __restrict__ dL_dimg1,
+                                                                  float l1_grad, float grad_scale) {
+    __shared__ f32x2 sD[kS][kSX];    // (d mu1, d sigma1^2)
+    __shared__ float sE[kS][kSX];    // d sigma12
+    __shared__ f32x2 sHD[kS][kSH];
+    __shared__ float sHE[kS][kSH];
     const int tid = threadIdx.x, c = blockIdx.z;
     const int bx0 = blockIdx.x * kT, by0 = blockIdx.y * kT;
+    f32x2 taps[kHalo + 1];
+#pragma unroll
+    for (int d = 0; d <= kHalo; ++d) taps[d] = pack2(cTaps[d], cTaps[d]);
     for (int q = tid; q < kS * kS; q += kThreadsLoss) {
         const int ly = q / kS, lx = q - ly * kS;
         const int gy = by0 + ly - kHalo, gx = bx0 + lx - kHalo;
         const float chain = FUSED ? 1.f : load_chw(dL_dmap, c, gy, gx, H, W);
-        sD[0][ly][lx] = load_chw(dm_dmu1, c, gy, gx, H, W) * chain;
-        sD[1][ly][lx] = load_chw(dm_dsigma1_sq, c, gy, gx, H, W) * chain;
-        sD[2][ly][lx] = load_chw(dm_dsigma12, c, gy, gx, H, W) * chain;
+        sD[ly][lx] = pack2(load_chw(dm_dmu1, c, gy, gx, H, W) * chain, load_chw(dm_dsigma1_sq, c, gy, gx, H, W) * chain);
+        sE[ly][lx] = load_chw(dm_dsigma12, c, gy, gx, H, W) * chain;
     }
     __syncthreads();
-    for (int item = tid; item < kS * kColGroups; item += kThreadsLoss) {
-        const int cg = item / kS, row = item - cg * kS;
+    if (tid < kS * kColGroups) {
+        const int cg = tid / kS, row = tid - cg * kS;
+        f32x2 w[14];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            float v[14];
+        for (int j = 0; j < 14; ++j) w[j] = sD[row][cg * 4 + j];
 #pragma unroll
-            for (int j = 0; j < 14; ++j) v[j] = sD[k][row][cg * 4 + j];
+        for (int o = 0; o < 4; ++o) sHD[row][cg * 4 + o] = tap11x2(w, o + kHalo, taps);
+        float v[14];
 #pragma unroll
-            for (int o = 0; o < 4; ++o) sH[k][row][cg * 4 + o] = tap11(v, o + kHalo);
-        }
+        for (int j = 0; j < 14; ++j) v[j] = sE[row][cg * 4 + j];
+#pragma unroll
+        for (int o = 0; o < 4; ++o) sHE[row][cg * 4 + o] = tap11(v, o + kHalo);
     }
     __syncthreads();
-    const int col = tid & 31, strip = tid >> 5;
-    float s[4][3];
+    const int col = tid & 31, strip = (tid >> 5) * kStrip;
+    constexpr int kWin = kStrip + 2 * kHalo;
+    float2 s01[kStrip];
+    float s2[kStrip];
+    {
+        f32x2 h[kWin];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float h[14];
+        for (int j = 0; j < kWin; ++j) h[j] = sHD[min(strip + j, kS - 1)][col];
 #pragma unroll
-        for (int j = 0; j < 14; ++j) h[j] = sH[k][strip * 4 + j][col];
+        for (int o = 0; o < kStrip; ++o) s01[o] = unpack2(tap11x2(h, o + kHalo, taps));
+        float g[kWin];
 #pragma unroll
-        for (int o = 0; o < 4; ++o) s[o][k] = tap11(h, o + kHalo);
+        for (int j = 0; j < kWin; ++j) g[j] = sHE[min(strip + j, kS - 1)][col];
+#pragma unroll
+        for (int o = 0; o < kStrip; ++o) s2[o] = tap11(g, o + kHalo);
     }
     const int x = bx0 + col;
 #pragma unroll
-    for (int o = 0; o < 4; ++o) {
-        const int y = by0 + strip * 4 + o;
-        if (x < W && y < H) {
+    for (int o = 0; o < kStrip; ++o) {
+        const int y = by0 + strip + o;
+        if (strip + o < kT && x < W && y < H) {
             if (FUSED) {
                 const float raw = img1[((size_t)y * W + x) * 3 + c];
                 const float p1 = fminf(1.f, fmaxf(0.f, raw));
                 const float p2 = img2[(size_t)c * H * W + (size_t)y * W + x];
-                float g = s[o][0] + (2.f * p1) * s[o][1] + (p2)*s[o][2];
+                float g = s01[o].x + (2.f * p1) * s01[o].y + (p2)*s2[o];
                 const float diff = p1 - p2;
                 g += l1_grad * (diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f));
                 if (!(raw >= 0.f && raw <= 1.f)) g = 0.f;
@@ -214,7 +279,7 @@ __global__ void __launch_bounds__(kThreadsLoss) ssim_bwd_kernel(int CH, int H, i
             } else {
                 const size_t gi = (size_t)c * H * W + (size_t)y * W + x;
                 const float p1 = img1[gi], p2 = img2[gi];
-                dL_dimg1[gi] = s[o][0] + (2.f * p1) * s[o][1] + (p2)*s[o][2];
+                dL_dimg1[gi] = s01[o].x + (2.f * p1) * s01[o].y + (p2)*s2[o];
             }
         }
     }

@@ -719,15 +719,17 @@ __device__ __forceinline__ void adam_small_row(const AdamSmall& A, int gi, size_
 // ADAM: the five small groups (means, sh0, scales, rotations, opacities) are not written as gradients but applied at
 // once, in place, with the moments in A (the parameter pointers below alias A.p, hence no __restrict__ on them); the
 // shN gradient leaves as its two rank-1 factors (sh_factors) for adam_sh_rank1_kernel.
-template <bool ADAM>
-__global__ void __launch_bounds__(256, 4) grad_epilogue_fused_kernel(
+// ROWS: the shN gradient leaves as rows; without them the kernel neither holds their staging nor the registers of its stores.
+template <bool ADAM, bool ROWS>
+__global__ void __launch_bounds__(256, ROWS ? 3 : 4) grad_epilogue_fused_kernel(
     int N, int K, int sh_degree, const CamDev* __restrict__ cams, const float* accum /* ADAM: aliased by g_shN */,
     const float4* __restrict__ records, const int32_t* __restrict__ radii,
     const float* means, const float* sh0, const float* scaling_raw, const float* rotation_raw, const float* opacity_raw,
     float* __restrict__ g_means, float* __restrict__ g_sh0, float* g_shN, float* __restrict__ g_scaling,
     float* __restrict__ g_rotation, float* __restrict__ g_opacity, int accumulate, float scaling_modifier, int sh_factors,
     AdamSmall A) {
-    extern __shared__ float s_rows[];
+    extern __shared__ __align__(16) float s_rows[];
+    const bool rows_aligned = (reinterpret_cast<uintptr_t>(g_shN) & 15) == 0;
     const CamDev& cam = cams[0];
     const int rest = (K - 1) * 3;
     const int nb = (sh_degree + 1) * (sh_degree + 1);
@@ -794,7 +796,7 @@ __global__ void __launch_bounds__(256, 4) grad_epilogue_fused_kernel(
 #pragma unroll
             for (int k = 0; k < 3; ++k) g0[k] = B[0] * vc[k];
         }
-        if (g_shN && sh_factors) {
+        if (!ROWS && g_shN && sh_factors) {
             // the two factors of the rank-1 rows instead of the rows: [N,6] = (clamped colour gradient, unit view direction)
             // at the start of the shN gradient tensor, for the data-parallel exchange that sums the outer products
             if (in_range) {
@@ -808,7 +810,7 @@ __global__ void __launch_bounds__(256, 4) grad_epilogue_fused_kernel(
                 float2* f = ADAM ? reinterpret_cast<float2*>(g_shN) + (size_t)g * 8 : reinterpret_cast<float2*>(g_shN) + (size_t)g * 3;
                 f[0] = make_float2(vc[0], vc[1]); f[1] = make_float2(vc[2], dx); f[2] = make_float2(dy, dz);
             }
-        } else if (g_shN) {  // NULL: the caller forms these rows itself from the sh0 gradient (adam_sh_rank1_kernel)
+        } else if (ROWS) {  // otherwise the caller forms these rows itself from the sh0 gradient (adam_sh_rank1_kernel)
             for (int k = 1; k < K; ++k) {
                 const float w = k < nb ? B[k] : 0.f;
 #pragma unroll
@@ -818,12 +820,7 @@ __global__ void __launch_bounds__(256, 4) grad_epilogue_fused_kernel(
             const int n_rows = min(32, N - chunk * 32);
             const int total = n_rows * rest;
             float* dst = g_shN + (size_t)chunk * 32 * rest;
-            if (accumulate) {
-                if (__any_sync(0xffffffffu, visible))
-                    for (int i = lane; i < total; i += 32) dst[i] += my[i];
-            } else {
-                for (int i = lane; i < total; i += 32) dst[i] = my[i];
-            }
+            if (!accumulate || __any_sync(0xffffffffu, visible)) store_rows(dst, my, total, lane, rows_aligned, accumulate != 0);
             __syncwarp();
         }
         if (ADAM) {
@@ -1163,20 +1160,23 @@ int launch_grad_epilogue_fused(int N, int K, int sh_degree, const CamDev* cam, c
                                int accumulate, float scaling_modifier, int sh_factors, cudaStream_t st, const AdamSmall* adam) {
     if (N == 0) return LFS_OK;
     LFS_TIMED(adam ? "grad_epilogue_adam" : "grad_epilogue", st);
-    const size_t smem = (size_t)8 * 32 * (K - 1) * 3 * sizeof(float);
-    if (smem > 200 * 1024) { set_error("grad_epilogue_fused: too many SH coefficients"); return LFS_EINVAL; }
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(grad_epilogue_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(grad_epilogue_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
-    if (adam)
-        grad_epilogue_fused_kernel<true><<<grid_for(N, 256), 256, smem, st>>>(
+    const bool rows = !adam && g.shN && !sh_factors;
+    const size_t row_bytes = (size_t)8 * 32 * (K - 1) * 3 * sizeof(float), smem = rows ? row_bytes : 0;
+    if (row_bytes > 200 * 1024) { set_error("grad_epilogue_fused: too many SH coefficients"); return LFS_EINVAL; }
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(grad_epilogue_fused_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (adam) {
+        grad_epilogue_fused_kernel<true, false><<<grid_for(N, 256), 256, 0, st>>>(
             N, K, sh_degree, cam, accum, records, radii, p.means, p.sh0, p.scaling_raw, p.rotation_raw, p.opacity_raw, nullptr,
             nullptr, const_cast<float*>(accum), nullptr, nullptr, nullptr, 0, scaling_modifier, 1, *adam);
-    else
-        grad_epilogue_fused_kernel<false><<<grid_for(N, 256), 256, smem, st>>>(
-            N, K, sh_degree, cam, accum, records, radii, p.means, p.sh0, p.scaling_raw, p.rotation_raw, p.opacity_raw, g.means,
-            g.sh0, g.shN, g.scaling_raw, g.rotation_raw, g.opacity_raw, accumulate, scaling_modifier, sh_factors, AdamSmall{});
+    } else {
+#define LFS_EPILOGUE(ROWS)                                                                                                          \
+    grad_epilogue_fused_kernel<false, ROWS><<<grid_for(N, 256), 256, smem, st>>>(                                                   \
+        N, K, sh_degree, cam, accum, records, radii, p.means, p.sh0, p.scaling_raw, p.rotation_raw, p.opacity_raw, g.means, g.sh0,  \
+        g.shN, g.scaling_raw, g.rotation_raw, g.opacity_raw, accumulate, scaling_modifier, sh_factors, AdamSmall{})
+        if (rows) LFS_EPILOGUE(true); else LFS_EPILOGUE(false);
+#undef LFS_EPILOGUE
+    }
     return check_launch("grad_epilogue_fused");
 }
 
