@@ -55,7 +55,7 @@ __device__ __forceinline__ void stage_batch(float4* rec, uint32_t* sid, const fl
 }
 
 // one ballot word per 32 staged entries: which of them can reach this warp's patch
-template <int BATCH, int PW, int PH>
+template <int BATCH>
 __device__ __forceinline__ void cull_batch(const float4* rec, int lo, int hi, float px0, float py0, uint32_t* live) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -65,7 +65,7 @@ __device__ __forceinline__ void cull_batch(const float4* rec, int lo, int hi, fl
         if (e >= lo && e < hi) {
             const float4 r0 = rec[e * 3], r1 = rec[e * 3 + 1], r2 = rec[e * 3 + 2];
             // a small margin on the threshold keeps the test conservative under rounding
-            ok = ewa_rect_contributes<true>(r0.x - 0.5f, r0.y - 0.5f, r0.z, r0.w, r1.x, px0, px0 + (PW - 1.0f), py0, py0 + (PH - 1.0f), r2.z + 0.01f);
+            ok = ewa_rect_contributes<true>(r0.x - 0.5f, r0.y - 0.5f, r0.z, r0.w, r1.x, px0, px0 + 7.0f, py0, py0 + 3.0f, r2.z + 0.01f);
         }
         live[w] = __ballot_sync(0xffffffffu, ok);
     }
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kBlock, 5) ewa_blend_fwd_kernel(
         const float4* st = rec[b & 1];
         if (!__all_sync(0xffffffffu, done)) {
             uint32_t live[BATCH / 32];
-            cull_batch<BATCH, 8, 4>(st, 0, batch_size, patch_x, patch_y, live);
+            cull_batch<BATCH>(st, 0, batch_size, patch_x, patch_y, live);
 #pragma unroll
             for (int w = 0; w < BATCH / 32; ++w) {
                 uint32_t bits = live[w];
@@ -187,10 +187,9 @@ __global__ void __launch_bounds__(256 / PX) ewa_blend_bwd_kernel(
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // warps tile the 16x16 block as patches of 4 PX x 8 pixels
-    constexpr int kPatchesX = 16 / (4 * PX);
-    const int patch_j = (tile % tw) * 16 + (warp % kPatchesX) * 4 * PX, patch_i = (tile / tw) * 16 + (warp / kPatchesX) * 8;
-    const int i = patch_i + (lane >> 2), j0 = patch_j + PX * (lane & 3);
+    // warps tile the 16x16 block as patches of 8 x 4 PX pixels: one or two of the forward's 8x4 patches, one above the other
+    const int patch_j = (tile % tw) * 16 + (warp & 1) * 8, patch_i = (tile / tw) * 16 + (warp >> 1) * 4 * PX;
+    const int i = patch_i + (PX == 2 ? lane >> 2 : lane >> 3), j0 = patch_j + (PX == 2 ? 2 * (lane & 3) : lane & 7);
     const float py = (float)i + 0.5f;
     const size_t np = (size_t)W * H;
     const int32_t range_start = tile_offsets[tile];
@@ -242,13 +241,24 @@ __global__ void __launch_bounds__(256 / PX) ewa_blend_bwd_kernel(
         const uint32_t* sid = sid_all[b % 3];
         // slots whose tile-local position is at or beyond this warp's deepest contributor are dropped up front
         const int t_begin = max(0, (batch_top - range_start) - (warp_last - 1));
-        uint32_t live[BATCH / 32];
-        cull_batch<BATCH, 4 * PX, 8>(st, t_begin, batch_size, (float)patch_j, (float)patch_i, live);
+        // The ellipse-versus-rectangle test is not exact for a rectangle that faces the ellipse with a corner, so a pair counts only
+        // if the forward's own 8x4 patch kept it: a pixel that the forward skipped must not enter the transmittance here.
+        uint32_t live[BATCH / 32], lower[BATCH / 32], mine[BATCH / 32];
+        cull_batch<BATCH>(st, t_begin, batch_size, (float)patch_j, (float)patch_i, live);
+        if (PX == 2) {
+            cull_batch<BATCH>(st, t_begin, batch_size, (float)patch_j, (float)(patch_i + 4), lower);
+#pragma unroll
+            for (int w = 0; w < BATCH / 32; ++w) {
+                mine[w] = lane < 16 ? live[w] : lower[w];
+                live[w] |= lower[w];
+            }
+        }
 #pragma unroll
         for (int w = 0; w < BATCH / 32; ++w) {
             uint32_t bits = live[w];
             while (bits) {
                 const int t = w * 32 + __ffs(bits) - 1;
+                const bool kept = PX == 1 || (mine[w] & bits & (0u - bits)) != 0u;
                 bits &= bits - 1;
                 const float4 r0 = st[t * 3], r1 = st[t * 3 + 1];
                 const float dy = r0.y - py;
@@ -259,7 +269,7 @@ __global__ void __launch_bounds__(256 / PX) ewa_blend_bwd_kernel(
                     dx[p] = r0.x - px[p];
                     const float sigma = 0.5f * (r0.z * dx[p] * dx[p] + r1.x * dy * dy) + r0.w * dx[p] * dy;
                     a[p] = fminf(r1.y * __expf(-sigma), kEwaMaxAlpha);
-                    valid[p] = (batch_top - range_start - t) < my_last[p] && !(sigma < 0.0f) && !(a[p] < kEwaMinAlpha);
+                    valid[p] = kept && (batch_top - range_start - t) < my_last[p] && !(sigma < 0.0f) && !(a[p] < kEwaMinAlpha);
                     any_valid = any_valid || valid[p];
                 }
                 if (!__any_sync(0xffffffffu, any_valid)) continue;
@@ -593,8 +603,8 @@ int launch_ewa_blend_bwd(const EwaBlendArgs& a, const float* alpha, const int32_
     ewa_blend_bwd_kernel<PX><<<n_tiles, 256 / PX, 0, st>>>(a.records, a.instance_ids, a.tile_offsets, a.overflow, a.background,      \
                                                            a.tile_order, a.W, a.H, a.tw, alpha, n_contrib, grad_image, grad_alpha,   \
                                                            accum)
-    // two pixels per thread while the CTAs of half the threads still fill the GPU (1 M Gaussians, 1296x840: 573 us against 753
-    // with one and 905 with the sums combined in shared memory first; 60 k, 777x519, 1,617 tiles: 133 against 175 and 201)
+    // two pixels per thread while the CTAs of half the threads still fill the GPU (1 M Gaussians, 1296x840: 617 us against 753
+    // with one and 905 with the sums combined in shared memory first; 60 k, 777x519, 1,617 tiles: 143 against 175 and 201)
     if (n_tiles >= 8 * num_sms()) LFS_EWA_BWD(2); else LFS_EWA_BWD(1);
 #undef LFS_EWA_BWD
     return check_launch("ewa_blend_bwd");
