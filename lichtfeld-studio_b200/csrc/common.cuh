@@ -85,7 +85,7 @@ inline int effective_model(int model, const float* radial, const float* tangenti
 // camera-space direction, (e1, e2, w) = (p1, p2, p3) . d, phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) (RayFrame in gsmath.cuh):
 //   r0 = (p1, c)              c = -|g|^2 log2(e) / 2: the response is exp2(c phi)
 //   r1 = (p2, phi_max)        p2.x = 0 for the planar models (pinhole, OpenCV); alpha < 1/255 for certain when phi > phi_max
-//   r2 = (p3, 0)
+//   r2 = (p3, slope)          slope = sqrt(phi_max / (1 - phi_max)): phi <= phi_max where |(e1, e2)| <= slope |w|
 //   r3 = (red, green, blue, opacity)
 // Rolling shutter, where the ray origin differs from pixel to pixel:
 //   r0 .. r2 = rows of M = diag(1/scale) R^T, each followed by its element of gro = M (start-pose origin - mean); r3 as above

@@ -465,9 +465,12 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         }
         const float G = f.gamma * f.gamma;
         rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
-        rec[1] = make_float4(p2[0], p2[1], p2[2], -2.0f * thr / fmaxf(G, 1e-30f));
+        const float phi_max = -2.0f * thr / fmaxf(G, 1e-30f);
+        // |(e1, e2)| <= slope |w| wherever phi <= phi_max
+        const float slope = phi_max >= 1.0f ? 1e30f : sqrtf(fmaxf(phi_max, 0.f) / (1.0f - phi_max));
+        rec[1] = make_float4(p2[0], p2[1], p2[2], phi_max);
         // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
-        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], 0.f) : make_float4(0.6101f, 0.5303f, 0.5887f, 0.f);
+        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], slope) : make_float4(0.6101f, 0.5303f, 0.5887f, 1e30f);
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);

@@ -9,10 +9,11 @@
 //  * one CTA per 16x16 tile, one thread per pixel, warps cover 8x4 pixel patches;
 //  * the tile's depth-sorted Gaussians are staged in shared memory in batches (192 records forward, 64 backward) of
 //    packed 64-byte records built once per Gaussian, so no per-Gaussian work is repeated per tile or per pixel;
-//  * per warp, a ballot over the batch keeps the records whose screen-space box overlaps the warp's 8x4 patch;
+//  * per warp, a ballot over the batch keeps the records whose screen-space box overlaps the warp's patch and whose forms
+//    reach the cut on it (patch_reached);
 //  * per pair the response is exp(-|g|^2 phi / 2), phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) with three linear forms of the
 //    pixel direction (RayFrame, gsmath.cuh): 10 instructions up to the exp-free rejection test for the planar camera models
-//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840: forward 624 -> 430 us, backward 1441 -> 1065);
+//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840: forward 624 -> 430 us, backward 1441 -> 1065 with nothing else changed);
 //  * backward: every (warp, Gaussian) contribution is 12 numbers that are LINEAR in the per-pixel terms (kSums). They
 //    are summed over the warp by a transpose through padded shared-memory rows (warp_reduce), combined across the 8 warps
 //    by shared-memory atomics, and leave the CTA as 16-byte reductions per (tile, Gaussian). The nonlinear quaternion / scale
@@ -77,6 +78,55 @@ __device__ __forceinline__ float exp2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// The directions of a warp's patch as an axis-aligned box around a centre (camera space; depth 0 for the planar models), over
+// the pixels that take part.
+struct PatchRays { f3 c, h; };
+__device__ __forceinline__ void patch_axis(float lo, float hi, float& c, float& h) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    c = 0.5f * (lo + hi);
+    h = 0.5f * (hi - lo) * 1.00001f;
+}
+template <int MODEL, int PX>
+__device__ __forceinline__ PatchRays patch_rays(const f3* d, const bool* takes_part) {
+    f3 lo{1e30f, 1e30f, 1e30f}, hi{-1e30f, -1e30f, -1e30f};
+#pragma unroll
+    for (int p = 0; p < PX; ++p)
+        if (takes_part[p]) {
+            lo = f3{fminf(lo.x, d[p].x), fminf(lo.y, d[p].y), fminf(lo.z, d[p].z)};
+            hi = f3{fmaxf(hi.x, d[p].x), fmaxf(hi.y, d[p].y), fmaxf(hi.z, d[p].z)};
+        }
+    PatchRays r;
+    patch_axis(lo.x, hi.x, r.c.x, r.h.x);
+    patch_axis(lo.y, hi.y, r.c.y, r.h.y);
+    r.c.z = 1.f;
+    r.h.z = 0.f;
+    if (MODEL != LFS_PINHOLE && MODEL != LFS_PINHOLE_OPENCV) patch_axis(lo.z, hi.z, r.c.z, r.h.z);
+    return r;
+}
+// Can a ray of the patch reach alpha >= 1/255? The forms are linear, so (e1, e2) of the patch lie in a parallelogram around its
+// centre's e_c; along e_c it comes no closer to the origin than |e_c| - ext, and it is out of reach when that exceeds slope times
+// the largest |w|. The axis-aligned screen box has already passed: this takes out its corners (slanted and round footprints).
+// The rounding of the forms is covered by a multiple of their coefficients. Some 35 instructions per (entry, patch), one lane
+// each, against the 40 - 140 of a walked entry: 1 M Gaussians at 1296x840 forward 429 -> 382 us, backward 816 -> 759; 6 M at 4K
+// 1440 -> 1224; 6 M 180 degree fisheye, whose boxes are ring sectors, 1382 -> 1129.
+template <int MODEL>
+__device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, const PatchRays& P) {
+    constexpr bool planar = MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV;
+    const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
+    const RayForms f = ray_forms<MODEL>(r0, r1, r2, P.c);
+    const float inv = rsqrtf(fmaxf(f.E, 1e-37f));
+    const float u1 = f.e1 * inv, u2 = f.e2 * inv;
+    float ext = fabsf(u1 * r0.x + u2 * r1.x) * P.h.x + fabsf(u1 * r0.y + u2 * r1.y) * P.h.y;
+    float w = fabsf(f.w) + fabsf(r2.x) * P.h.x + fabsf(r2.y) * P.h.y;
+    if (!planar) { ext += fabsf(u1 * r0.z + u2 * r1.z) * P.h.z; w += fabsf(r2.z) * P.h.z; }
+    const float slack = 1e-6f * (fabsf(r0.x) + fabsf(r0.y) + fabsf(r0.z) + fabsf(r1.x) + fabsf(r1.y) + fabsf(r1.z));
+    return !(f.E * inv - ext > r2.w * w * 1.001f + slack);   // true for NaN
 }
 
 __device__ __forceinline__ int32_t load_count(const int32_t* n_dev, int64_t n_host) {
@@ -181,6 +231,8 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
     const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
                            : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
     bool done = !inside || !ray_ok;
+    const bool takes_part = !done;
+    const PatchRays rays = RS ? PatchRays{} : patch_rays<MODEL, 1>(&d, &takes_part);
     uint32_t patch_x, patch_y;
     warp_patch(tile, tw, patch_x, patch_y);
 
@@ -222,7 +274,11 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
             for (int w = 0; w < BATCH / 32; ++w) {
                 const int e = w * 32 + (threadIdx.x & 31);
                 bool ov = false;
-                if (e < batch_size) { const uint4 bx = st.box[e]; ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y); }
+                if (e < batch_size) {
+                    const uint4 bx = st.box[e];
+                    ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
+                    if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], rays);
+                }
                 live[w] = __ballot_sync(0xffffffffu, ov);
             }
 #pragma unroll
@@ -376,6 +432,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
     // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
     // (colour . v_colour) alpha T of every entry behind
     float behind[PX];
+    bool takes_part[PX];
     int32_t warp_bin_final = 0;
 #pragma unroll
     for (int p = 0; p < PX; ++p) {
@@ -384,6 +441,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
         const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], oo[p])
                                : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p]);
         const bool active = i < H && j < W && ray_ok;
+        takes_part[p] = active;
         const int pid = min(i * W + j, W * H - 1);
         const float T_final = 1.0f - render_alphas[pid];
         T[p] = T_final;
@@ -412,6 +470,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
         behind[p] = T_final * (v_a - bg_dot);
     }
     warp_bin_final = __reduce_max_sync(0xffffffffu, warp_bin_final);
+    const PatchRays rays = RS ? PatchRays{} : patch_rays<MODEL, PX>(d, takes_part);
 
     const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
     const int32_t range_start = tile_offsets[tile];
@@ -453,7 +512,11 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
         for (int w = 0; w < BATCH / 32; ++w) {
             const int e = w * 32 + lane;
             bool ov = false;
-            if (e >= t_begin && e < batch_size) { const uint4 bx = st.box[e]; ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y); }
+            if (e >= t_begin && e < batch_size) {
+                const uint4 bx = st.box[e];
+                ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
+                if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], rays);
+            }
             live[w] = __ballot_sync(0xffffffffu, ov);
         }
 #pragma unroll
