@@ -45,9 +45,9 @@ METRIC = "train steps/s (fwd+loss+bwd+Adam)"
 # Profiler counters of ONE raster_bwd_kernel launch on train_1m (ncu, --clock-control none): DRAM bytes read + written,
 # share of issue slots used, share of issued warp instructions on the FMA pipe relative to the FP32 peak rate. They are
 # reported next to the event-timed figures because a kernel's traffic and pipe utilisation cannot be read outside a profiler.
-NCU_RASTER_BWD = {"dram_bytes": 180.7e6, "issue_slots_active": 0.82, "fma_pipe_of_fp32_peak": 0.42, "shared_pipe": 0.77,
-                  # 666e6 warp instructions on the FMA pipe x 32 lanes x 2 flop over the 4.25e8 pairs of the captured launch
-                  "executed_flop_per_pair": 100.3}
+NCU_RASTER_BWD = {"dram_bytes": 182.6e6, "issue_slots_active": 0.78, "fma_pipe_of_fp32_peak": 0.42, "shared_pipe": 0.72,
+                  # 371e6 warp instructions on the FMA pipe x 32 lanes x 2 flop over the 4.24e8 pairs of the captured launch
+                  "executed_flop_per_pair": 56.1}
 
 
 def load_peaks():
