@@ -314,7 +314,7 @@ int lfs_render_backward(const lfs_render_config* cfg, const lfs_splats* params, 
  * (gsplat/Ops.h:171-185) — radii [N,2], means2d [N,2], depths [N] (meaningful where radii > 0) — plus
  * tiles_per_gauss [N], tile_offsets [tile_h*tile_w + 1] (last entry = n_isects), flatten_ids
  * [n_isects], last_ids [H,W] and the packed 16-float rasterizer records [N,16] whose floats 12..14
- * are the clamped colours. */
+ * are the clamped colours and float 15 the blended opacity (floats 0..11 are the rasterizer's own). */
 typedef struct lfs_render_view {
     const int32_t* radii;
     const float* means2d;
