@@ -61,7 +61,7 @@ struct RenderWs {
     int32_t* counters;  // [0] overflow, [1] n_isects, [2] n_visible
     int32_t *radii, *tiles, *tile_offsets, *last_ids, *tile_order;
     float *means2d, *depths, *accum, *extra_sum;
-    float4* records;
+    float4 *records, *cuts;
     uint4* bounds;
     uint32_t *gkeys[2], *gvals[2], *tkeys[2], *tvals[2];
     uint32_t* list_state;
@@ -83,6 +83,7 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
     w.tiles = c.take<int32_t>(N);
     for (int k = 0; k < 2; ++k) { w.gkeys[k] = c.take<uint32_t>(N); w.gvals[k] = c.take<uint32_t>(N); }
     w.records = c.take<float4>(N * 4);
+    w.cuts = c.take<float4>(N * 3);
     w.bounds = c.take<uint4>(N);
     w.accum = c.take<float>(N * 16);
     for (int k = 0; k < 2; ++k) { w.tkeys[k] = c.take<uint32_t>(cap); w.tvals[k] = c.take<uint32_t>(cap); }
@@ -297,6 +298,7 @@ size_t lfs_rasterize_workspace_bytes(int N) {
     Carver c(nullptr);
     c.take<CamDev>(1);
     c.take<float4>((size_t)N * 4);
+    c.take<float4>((size_t)N * 3);
     c.take<uint4>((size_t)N);
     c.take<float>((size_t)N * 16);
     c.take<float>((size_t)N);
@@ -331,6 +333,7 @@ int lfs_rasterize_to_pixels_from_world_3dgs_fwd(int N, int64_t n_isects, int cha
     Carver c(workspace);
     CamDev* cam = c.take<CamDev>(1);
     float4* records = c.take<float4>((size_t)N * 4);
+    float4* cuts = c.take<float4>((size_t)N * 3);
     uint4* bounds = c.take<uint4>((size_t)N);
     LFS_REQUIRE(camera_model == LFS_PINHOLE || (!tangential_coeffs && !thin_prism_coeffs),
                 "tangential / thin-prism coefficients belong to the pinhole model");
@@ -342,10 +345,10 @@ int lfs_rasterize_to_pixels_from_world_3dgs_fwd(int N, int64_t n_isects, int cha
     LFS_REQUIRE(camera_model != LFS_EQUIRECTANGULAR || (!rolling && !radial_coeffs),
                 "the equirectangular model has a global shutter and no distortion coefficients");
     if (rc != LFS_OK) return rc;
-    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, bounds, nullptr, nullptr,
+    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, cuts, bounds, nullptr, nullptr,
                              S(stream));
     if (rc != LFS_OK) return rc;
-    RasterArgs a{cam, records, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,
+    RasterArgs a{cam, records, cuts, N, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,
                  nullptr, W, H, (W + 15) / 16, (H + 15) / 16, eff_model, channels, 0, masks, nullptr, rolling};
     return launch_raster_fwd(a, renders, alphas, last_ids, nullptr, S(stream));
 }
@@ -369,6 +372,7 @@ int lfs_rasterize_to_pixels_from_world_3dgs_bwd(int N, int64_t n_isects, int cha
     Carver c(workspace);
     CamDev* cam = c.take<CamDev>(1);
     float4* records = c.take<float4>((size_t)N * 4);
+    float4* cuts = c.take<float4>((size_t)N * 3);
     uint4* bounds = c.take<uint4>((size_t)N);
     float* accum = c.take<float>((size_t)N * 16);
     float* accum_extra = channels != 3 ? c.take<float>((size_t)N) : nullptr;
@@ -382,10 +386,10 @@ int lfs_rasterize_to_pixels_from_world_3dgs_bwd(int N, int64_t n_isects, int cha
     LFS_REQUIRE(camera_model != LFS_EQUIRECTANGULAR || (!rolling && !radial_coeffs),
                 "the equirectangular model has a global shutter and no distortion coefficients");
     if (rc != LFS_OK) return rc;
-    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, bounds,
+    rc = launch_pack_records(N, means, quats, scales, colors, channels, opacities, cam, eff_model, rolling, records, cuts, bounds,
                              reinterpret_cast<float4*>(accum), accum_extra, S(stream));
     if (rc != LFS_OK) return rc;
-    RasterArgs a{cam, records, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,
+    RasterArgs a{cam, records, cuts, N, bounds, reinterpret_cast<const uint32_t*>(flatten_ids), tile_offsets, nullptr, n_isects, backgrounds,
                  nullptr, W, H, (W + 15) / 16, (H + 15) / 16, eff_model, channels, 0, masks, nullptr, rolling};
     rc = launch_raster_bwd(a, render_alphas, last_ids, nullptr, v_render_colors, v_render_alphas, accum, accum_extra, S(stream));
     if (rc != LFS_OK) return rc;
@@ -783,7 +787,7 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
     opt.calc_compensations = cfg->calc_compensations;
     opt.want_rgb = with_colors && mode_channels(cfg->render_mode) != 1;
     rc = launch_project_pack(cfg->N, cfg->sh_coeffs, cfg->sh_degree, *params, w.cam, pp, opt, cfg_model(*cfg), cfg_rolling(*cfg), cfg->tile_size, tw,
-                             th, w.radii, w.means2d, w.depths, w.tiles, w.gkeys[0], w.gvals[0], w.records, w.bounds,
+                             th, w.radii, w.means2d, w.depths, w.tiles, w.gkeys[0], w.gvals[0], w.records, w.cuts, w.bounds,
                              reinterpret_cast<float4*>(w.accum), w.counters + 2, st);
     if (rc != LFS_OK) return rc;
     if (projected && cudaEventRecord(projected, st) != cudaSuccess) { set_error("cudaEventRecord failed"); return LFS_ECUDA; }
@@ -802,7 +806,7 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
 static int render_forward_blend(const lfs_render_config* cfg, const float* background, float* render, float* alpha,
                                 int32_t* status_dev, RenderWs& w, int sel, cudaStream_t st) {
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    RasterArgs ra{w.cam, w.records, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     int rc = launch_raster_fwd(ra, render, alpha, w.last_ids, w.extra_sum, st);
@@ -879,7 +883,7 @@ int lfs_render_backward(const lfs_render_config* cfg, const lfs_splats* params, 
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
     const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
-    RasterArgs ra{w.cam, w.records, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     rc = launch_raster_bwd(ra, alpha, w.last_ids, w.extra_sum, v_render, v_alpha, w.accum, nullptr, st);
@@ -923,7 +927,7 @@ int lfs_render_backward_adam(const lfs_render_config* cfg, const lfs_splats* par
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
     const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
-    RasterArgs ra{w.cam, w.records, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     rc = launch_raster_bwd(ra, alpha, w.last_ids, w.extra_sum, v_render, v_alpha, w.accum, nullptr, st);

@@ -84,9 +84,11 @@ inline int effective_model(int model, const float* radial, const float* tangenti
 // One packed 64-byte record per Gaussian for the rasterizer. Cameras with one ray origin (global shutter), d = the pixel's
 // camera-space direction, (e1, e2, w) = (p1, p2, p3) . d, phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) (RayFrame in gsmath.cuh):
 //   r0 = (p1, c)              c = -|g|^2 log2(e) / 2: the response is exp2(c phi)
-//   r1 = (p2, phi_max)        p2.x = 0 for the planar models (pinhole, OpenCV); alpha < 1/255 for certain when phi > phi_max
-//   r2 = (p3, slope)          slope = sqrt(phi_max / (1 - phi_max)): phi <= phi_max where |(e1, e2)| <= slope |w|
+//   r1 = (p2, phi_cut)        p2.x = 0 for the planar models (pinhole, OpenCV); alpha < 1/255 for certain when phi > phi_cut
+//   r2 = (p3, alpha_cut)      alpha >= 1/255 for certain when it is not below alpha_cut
 //   r3 = (red, green, blue, opacity)
+// Between the two cuts the pair is decided by the product form |u x g|^2 / |u|^2, u = M d, from the cut record
+//   c0 .. c2 = rows of M = diag(1/scale) R^T, each followed by its element of g = M (ray origin - mean)
 // Rolling shutter, where the ray origin differs from pixel to pixel:
 //   r0 .. r2 = rows of M = diag(1/scale) R^T, each followed by its element of gro = M (start-pose origin - mean); r3 as above
 constexpr int kRecordFloats = 16;

@@ -259,11 +259,10 @@ __device__ __forceinline__ bool pixel_world_dir(const CamDev& c, float px, float
 }
 
 // Camera-space direction of a pixel centre, not normalised: (x, y, 1) for the planar models. It is the float32 world-space
-// unit ray, the one on which a pair's alpha falls on either side of its cut, taken back through Rinv in double (once per
+// unit ray wd, the one on which a pair's alpha falls on either side of its cut, taken back through Rinv in double (once per
 // pixel): the ray itself stays the one every other use of the camera sees.
 template <int MODEL>
-__device__ __forceinline__ bool pixel_cam_dir(const CamDev& c, float px, float py, f3& d) {
-    f3 wd;
+__device__ __forceinline__ bool pixel_cam_dir(const CamDev& c, float px, float py, f3& d, f3& wd) {
     const bool valid = pixel_world_dir<MODEL>(c, px, py, wd);
     const double w[3] = {wd.x, wd.y, wd.z};
     double v[3], r[3];

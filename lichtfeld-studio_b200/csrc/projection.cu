@@ -413,36 +413,28 @@ __device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, 
 template <int MODEL, bool RS>
 __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
                                             f3 scale, float r, float g, float b, float opacity, float extra, float4* rec,
-                                            uint4& box) {
+                                            float4* __restrict__ cut, int64_t n, uint4& box) {
     float R[9], inv_norm, qn[4];
     quat_to_rotmat_renorm(qw, qx, qy, qz, R, inv_norm, qn);
-    // exponent below which opacity * exp(p) < 1/255 for certain, as float bits in .z
-    const float thr = -logf(fmaxf(255.0f * opacity, 1e-30f)) - 0.02f;
-    const uint32_t thr_bits = __float_as_uint(thr);
+    // exponent below which opacity * exp(p) < 1/255 for certain
+    const float ln_o = logf(fmaxf(255.0f * opacity, 1e-30f)), thr = -ln_o - 0.02f;
     const uint32_t extra_bits = __float_as_uint(extra);  // blended into the last channel of 1- and 4-channel renders
-    box = make_uint4(0xFFFF0000u, 0xFFFF0000u, thr_bits, extra_bits);  // (lo | hi << 16) per axis: everything
+    box = make_uint4(0xFFFF0000u, 0xFFFF0000u, __float_as_uint(thr), extra_bits);  // (lo | hi << 16) per axis: everything
     const float is[3] = {1.0f / scale.x, 1.0f / scale.y, 1.0f / scale.z};
     const f3 om{cam.ro[0] - mean.x, cam.ro[1] - mean.y, cam.ro[2] - mean.z};
     rec[3] = make_float4(r, g, b, opacity);
-    if (RS) {
-        float M[9];
+    // M = diag(1/scale) R^T and g = M om, unfused: the record of a rolling shutter, the cut record of the others
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) M[a * 3 + c] = is[a] * R[c * 3 + a];
-        const float g0 = M[0] * om.x + M[1] * om.y + M[2] * om.z;
-        const float g1 = M[3] * om.x + M[4] * om.y + M[5] * om.z;
-        const float g2 = M[6] * om.x + M[7] * om.y + M[8] * om.z;
-        rec[0] = make_float4(M[0], M[1], M[2], g0);
-        rec[1] = make_float4(M[3], M[4], M[5], g1);
-        rec[2] = make_float4(M[6], M[7], M[8], g2);
-        return;
+    for (int a = 0; a < 3; ++a) {
+        const float M0 = is[a] * R[a], M1 = is[a] * R[3 + a], M2 = is[a] * R[6 + a];
+        (RS ? rec[a] : cut[a * n]) = make_float4(M0, M1, M2, M0 * om.x + M1 * om.y + M2 * om.z);
     }
+    if (RS) return;
     RayFrame f;
     ray_frame(cam, R, om, scale, is, f);
     {
         const float m2 = fdot3(f.m[0], f.m[0], f.m[1], f.m[1], f.m[2], f.m[2]);
-        const float lambda = m2 > 0.f ? sqrtf(m2) / f.gamma : 1.0f;
+        const float dist = sqrtf(m2), lambda = m2 > 0.f ? dist / f.gamma : 1.0f;
         const float a0 = lambda * is[0], a1 = lambda * is[1], a2 = lambda * is[2];
         const float n2 = lambda * f.inv_nv;
         float p1[3], p3[3], p2[3] = {f.v[0] * n2, f.v[1] * n2, f.v[2] * n2};
@@ -465,12 +457,23 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         }
         const float G = f.gamma * f.gamma;
         rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
-        const float phi_max = -2.0f * thr / fmaxf(G, 1e-30f);
+        // How far the exponents of the forms and of the product form can lie apart where alpha is 1/255. The rounding of M d, of some
+        // 2^-24 max(1/scale) for a unit direction, moves the distance |u x g| / |u| by that times |o - mu|, and its half square by
+        // that times the distance itself, sqrt(2 ln 255 o). Measured on 12 M pairs at the cut (pinhole and fisheye, scales of 1e-4
+        // to 0.2, distances of 0.5 to 20), in units of that product + 1e-6: median 0.2, one in a thousand above 1.7, one in ten
+        // thousand above 2.1, largest 4.0.
+        const float off = 2.5f * 5.9604645e-8f * fmaxf(is[0], fmaxf(is[1], is[2])) * dist;
+        const float two_ln_o = fmaxf(2.0f * ln_o, 0.f);
+        const float band = fmaf(off, fmaf(two_ln_o, rsqrtf(fmaxf(two_ln_o, 1e-30f)), off), 2.5e-6f);
+        const float rG = 2.0f / fmaxf(G, 1e-30f);
+        const float phi_cut = (ln_o + band) * rG, phi_max = (ln_o + fmaxf(band, 0.02f)) * rG;
         // |(e1, e2)| <= slope |w| wherever phi <= phi_max
         const float slope = phi_max >= 1.0f ? 1e30f : sqrtf(fmaxf(phi_max, 0.f) / (1.0f - phi_max));
-        rec[1] = make_float4(p2[0], p2[1], p2[2], phi_max);
+        box.z = __float_as_uint(m2 > 0.f ? slope : 1e30f);
+        rec[1] = make_float4(p2[0], p2[1], p2[2], phi_cut);
+        const float alpha_cut = (1.0f / 255.0f) * __expf(fminf(band, 8.0f));
         // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
-        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], slope) : make_float4(0.6101f, 0.5303f, 0.5887f, 1e30f);
+        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], alpha_cut) : make_float4(0.6101f, 0.5303f, 0.5887f, alpha_cut);
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);
@@ -507,7 +510,8 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
             const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo_j, 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi_j, 0.f), 65535.f);
             packed[ax] = lo_u | (hi_u << 16);
         }
-        box = make_uint4(packed[0], packed[1], thr_bits, extra_bits);
+        box.x = packed[0];
+        box.y = packed[1];
     }
 }
 
@@ -515,7 +519,8 @@ template <int MODEL, bool RS>
 __global__ void __launch_bounds__(256) pack_records_kernel(
     int N, const float* __restrict__ means, const float* __restrict__ quats, const float* __restrict__ scales,
     const float* __restrict__ colors, int channels, const float* __restrict__ opacities, const CamDev* __restrict__ cams,
-    float4* __restrict__ records, uint4* __restrict__ bounds, float4* __restrict__ accum, float* __restrict__ accum_extra) {
+    float4* __restrict__ records, float4* __restrict__ cuts, uint4* __restrict__ bounds, float4* __restrict__ accum,
+    float* __restrict__ accum_extra) {
     const CamDev& cam = cams[0];
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < N; g += gridDim.x * blockDim.x) {
         const f3 mean{means[g * 3], means[g * 3 + 1], means[g * 3 + 2]};
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(256) pack_records_kernel(
         const float* col = colors + (size_t)g * channels;
         const bool has_rgb = channels >= 3;
         make_record<MODEL, RS>(cam, mean, q.x, q.y, q.z, q.w, scale, has_rgb ? col[0] : 0.f, has_rgb ? col[1] : 0.f, has_rgb ? col[2] : 0.f,
-                    opacities[g], channels != 3 ? col[channels - 1] : 0.f, rec, box);
+                    opacities[g], channels != 3 ? col[channels - 1] : 0.f, rec, cuts + g, N, box);
 #pragma unroll
         for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
         bounds[g] = box;
@@ -540,13 +545,13 @@ __global__ void __launch_bounds__(256) pack_records_kernel(
 }
 
 int launch_pack_records(int N, const float* means, const float* quats, const float* scales, const float* colors, int channels,
-                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, uint4* bounds,
-                        float4* accum, float* accum_extra, cudaStream_t st) {
+                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, float4* cuts,
+                        uint4* bounds, float4* accum, float* accum_extra, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     LFS_TIMED("pack_records", st);
 #define LFS_PACKREC2(MODEL, RS)                                                                                              \
     pack_records_kernel<MODEL, RS><<<grid_for(N, 256), 256, 0, st>>>(N, means, quats, scales, colors, channels, opacities, cam, \
-                                                                     records, bounds, accum, accum_extra)
+                                                                     records, cuts, bounds, accum, accum_extra)
 #define LFS_PACKREC(MODEL) do { if (rolling) LFS_PACKREC2(MODEL, true); else LFS_PACKREC2(MODEL, false); } while (0)
     switch (model) {
         case LFS_PINHOLE: LFS_PACKREC(LFS_PINHOLE); break;
@@ -576,7 +581,8 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
     uint32_t tw, uint32_t th,
     int32_t* __restrict__ radii, float* __restrict__ means2d, float* __restrict__ depths,
     int32_t* __restrict__ tiles, uint32_t* __restrict__ sort_keys, uint32_t* __restrict__ sort_vals,
-    float4* __restrict__ records, uint4* __restrict__ bounds, float4* __restrict__ accum, int32_t* __restrict__ n_visible) {
+    float4* __restrict__ records, float4* __restrict__ cuts, uint4* __restrict__ bounds, float4* __restrict__ accum,
+    int32_t* __restrict__ n_visible) {
     // Each warp handles 32 consecutive Gaussians per iteration. Their higher-order SH rows ((K-1)*3 floats
     // each, contiguous in memory) are fetched as one coalesced run into shared memory when any of the 32
     // is visible, and every visible lane then reads its own row from there.
@@ -664,7 +670,8 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
 
             float4 rec[4];
             uint4 box;
-            make_record<MODEL, RS>(cam, mean, qw, qx, qy, qz, scale, rgb[0], rgb[1], rgb[2], opacity, o.depth, rec, box);
+            make_record<MODEL, RS>(cam, mean, qw, qx, qy, qz, scale, rgb[0], rgb[1], rgb[2], opacity, o.depth, rec,
+                                   cuts + g, N, box);
 #pragma unroll
             for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
             bounds[g] = box;
@@ -743,8 +750,8 @@ int launch_sh_color(int N, int K, int sh_degree, const lfs_splats& p, const CamD
 
 int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const ProjParams& pp,
                         const PackOptions& opt, int model, int rolling, int tile_size, int tw, int th, int32_t* radii, float* means2d, float* depths,
-                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, uint4* bounds, float4* accum,
-                        int32_t* n_visible, cudaStream_t st) {
+                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, float4* cuts,
+                        uint4* bounds, float4* accum, int32_t* n_visible, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     const int grid = grid_for(N, 256);
     const size_t smem = (size_t)8 * 32 * (K - 1) * 3 * sizeof(float);
@@ -760,7 +767,7 @@ int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const 
 #define LFS_PACK2(MODEL, RS)                                                                                                       \
     project_pack_kernel<MODEL, RS><<<grid, 256, smem, st>>>(N, K, sh_degree, p.means, p.sh0, p.shN, p.scaling_raw, p.rotation_raw,  \
                                                             p.opacity_raw, cam, pp, opt, (float)tile_size, tw, th, radii, means2d, \
-                                                            depths, tiles, sort_keys, sort_vals, records, bounds, accum, n_visible)
+                                                            depths, tiles, sort_keys, sort_vals, records, cuts, bounds, accum, n_visible)
 #define LFS_PACK(MODEL) do { if (rolling) LFS_PACK2(MODEL, true); else LFS_PACK2(MODEL, false); } while (0)
     switch (model) {
         case LFS_PINHOLE: LFS_PACK(LFS_PINHOLE); break;

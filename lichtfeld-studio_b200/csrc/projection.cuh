@@ -29,8 +29,8 @@ int launch_projection_ut(int C, int N, const float* means, const float* quats, c
 // colours [N, channels] with channels 1 (extra only), 3 (rgb) or 4 (rgb + extra); accum / accum_extra (may be null)
 // are zeroed for the backward.
 int launch_pack_records(int N, const float* means, const float* quats, const float* scales, const float* colors, int channels,
-                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, uint4* bounds,
-                        float4* accum, float* accum_extra, cudaStream_t st);
+                        const float* opacities, const CamDev* cam, int model, int rolling, float4* records, float4* cuts,
+                        uint4* bounds, float4* accum, float* accum_extra, cudaStream_t st);
 
 // Per-render switches of the fused path (FusedRasterizationSettings, src/training/rasterization/rasterizer_autograd.hpp).
 struct PackOptions {
@@ -42,8 +42,8 @@ struct PackOptions {
 // model: the effective (internal) model id, see effective_model(); rolling: the camera has a rolling shutter or an end pose
 int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const ProjParams& pp,
                         const PackOptions& opt, int model, int rolling, int tile_size, int tw, int th, int32_t* radii, float* means2d, float* depths,
-                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, uint4* bounds, float4* accum,
-                        int32_t* n_visible, cudaStream_t st);
+                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, float4* cuts,
+                        uint4* bounds, float4* accum, int32_t* n_visible, cudaStream_t st);
 
 // colours (SH + 0.5, clamped at 0) of the visible Gaussians into records[g*4+3].xyz
 int launch_sh_color(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const int32_t* radii, float4* records,

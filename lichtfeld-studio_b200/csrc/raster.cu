@@ -116,7 +116,7 @@ __device__ __forceinline__ PatchRays patch_rays(const f3* d, const bool* takes_p
 // each, against the 40 - 140 of a walked entry: 1 M Gaussians at 1296x840 forward 429 -> 382 us, backward 816 -> 759; 6 M at 4K
 // 1440 -> 1224; 6 M 180 degree fisheye, whose boxes are ring sectors, 1382 -> 1129.
 template <int MODEL>
-__device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, const PatchRays& P) {
+__device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, float slope, const PatchRays& P) {
     constexpr bool planar = MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV;
     const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
     const RayForms f = ray_forms<MODEL>(r0, r1, r2, P.c);
@@ -126,7 +126,33 @@ __device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, co
     float w = fabsf(f.w) + fabsf(r2.x) * P.h.x + fabsf(r2.y) * P.h.y;
     if (!planar) { ext += fabsf(u1 * r0.z + u2 * r1.z) * P.h.z; w += fabsf(r2.z) * P.h.z; }
     const float slack = 1e-6f * (fabsf(r0.x) + fabsf(r0.y) + fabsf(r0.z) + fabsf(r1.x) + fabsf(r1.y) + fabsf(r1.z));
-    return !(f.E * inv - ext > r2.w * w * 1.001f + slack);   // true for NaN
+    return !(f.E * inv - ext > slope * w * 1.001f + slack);   // true for NaN
+}
+
+// Which side of alpha = 1/255 a pair near it falls on: |u x g|^2 / |u|^2 with u = M d in float32, d the pixel's world-space unit
+// ray, as the kernels with one ray origin per pixel compute it. The three forms round differently (make_record bounds by how
+// much), and a pair that changes side moves a pixel by up to 1/255 of a colour and the gradient of a small Gaussian by percents:
+// the set of blended pairs must not depend on which expression is the faster one.
+// The products and sums are spelled out, so that the set does not depend on a compiler's contraction either.
+// For PX pixels of one thread, as bits. cut: the first row of the Gaussian's cut record, the others n apart; rays: stride apart.
+// A call, since fewer than one walked entry in a hundred comes here and the registers of the callers' loops should not be shaped
+// by it (1 M Gaussians, 1296x840: backward 786 us against 845 inlined; forward 398 either way. Without this test 760 and 382).
+template <int PX>
+__device__ __noinline__ uint32_t kept_at_cut(const float4* cut, int64_t n, const f3* rays, int stride, float opacity) {
+    auto dot = [](float a0, float b0, float a1, float b1, float a2, float b2) { return fmaf(a2, b2, fmaf(a0, b0, __fmul_rn(a1, b1))); };
+    auto det = [](float a, float b, float c, float e) { return fmaf(a, b, -__fmul_rn(c, e)); };
+    const float4 r0 = cut[0], r1 = cut[n], r2 = cut[2 * n];
+    uint32_t kept = 0;
+#pragma unroll
+    for (int p = 0; p < PX; ++p) {
+        const f3 d = rays[p * stride];
+        const float ux = dot(r0.x, d.x, r0.y, d.y, r0.z, d.z), uy = dot(r1.x, d.x, r1.y, d.y, r1.z, d.z), uz = dot(r2.x, d.x, r2.y, d.y, r2.z, d.z);
+        const float cx = det(uy, r2.w, r1.w, uz), cy = det(uz, r0.w, r2.w, ux), cz = det(ux, r1.w, r0.w, uy);
+        const float cc = dot(cx, cx, cy, cy, cz, cz), uu = dot(ux, ux, uy, uy, uz, uz);
+        const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
+        if (!(fminf(0.999f, opacity * __expf(power)) < kAlphaMin)) kept |= 1u << p;
+    }
+    return kept;
 }
 
 __device__ __forceinline__ int32_t load_count(const int32_t* n_dev, int64_t n_host) {
@@ -140,7 +166,7 @@ __device__ __forceinline__ int32_t load_count(const int32_t* n_dev, int64_t n_ho
 template <int BATCH>
 struct Stage {
     float4 rec[BATCH * 4];  // packed records
-    uint4 box[BATCH];       // (x box, y box, rejection exponent as float bits, unused)
+    uint4 box[BATCH];       // rows of RasterArgs::bounds
 };
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
@@ -200,14 +226,15 @@ __device__ __forceinline__ void issue_stage(Stage<BATCH>& st, uint32_t* sid, con
 // (30 KB for the two staging buffers), six CTAs per SM; the other instantiations keep their 48 - 64 registers.
 template <int MODEL, bool EXTRA, bool RS>
 __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA) ? 6 : 4) raster_fwd_kernel(
-    const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds,
-    const uint32_t* __restrict__ flatten_ids,
+    const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
+    const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
     const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
     float* __restrict__ render, float* __restrict__ alphas, int32_t* __restrict__ last_ids, float* __restrict__ extra_sum) {
     constexpr int BATCH = 192;
     __shared__ Stage<BATCH> stage[2];
+    __shared__ f3 ray[RS ? 1 : kBlock];   // world-space unit rays, for kept_at_cut
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
@@ -227,9 +254,10 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
         return;
     }
     const CamDev& cam = cams[0];
-    f3 d, oo{0.f, 0.f, 0.f};
+    f3 d, wd, oo{0.f, 0.f, 0.f};
     const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
-                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d);
+                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, wd);
+    if (!RS) ray[threadIdx.x] = wd;
     bool done = !inside || !ray_ok;
     const bool takes_part = !done;
     const PatchRays rays = RS ? PatchRays{} : patch_rays<MODEL, 1>(&d, &takes_part);
@@ -268,22 +296,21 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
         if (__syncthreads_count(done) >= kBlock) break;
         const Stage<BATCH>& st = stage[b & 1];
         if (!__all_sync(0xffffffffu, done)) {
-            // entries of this batch whose box overlaps this warp's 8x4 patch: one ballot word per 32 entries
-            uint32_t live[BATCH / 32];
-#pragma unroll
-            for (int w = 0; w < BATCH / 32; ++w) {
+            // entries of this batch whose box overlaps this warp's 8x4 patch: one ballot word per 32 entries, formed when its
+            // turn comes (six words kept at once are five registers more, at 40 in all: 413 us against 398)
+            auto reach = [&](int w) {
                 const int e = w * 32 + (threadIdx.x & 31);
                 bool ov = false;
                 if (e < batch_size) {
                     const uint4 bx = st.box[e];
                     ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
-                    if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], rays);
+                    if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], __uint_as_float(bx.z), rays);
                 }
-                live[w] = __ballot_sync(0xffffffffu, ov);
-            }
+                return __ballot_sync(0xffffffffu, ov);
+            };
 #pragma unroll
             for (int w = 0; w < BATCH / 32; ++w) {
-                uint32_t bits = live[w];
+                uint32_t bits = reach(w);
                 while (bits && !done) {
                     const int t = w * 32 + __ffs(bits) - 1;
                     bits &= bits - 1;
@@ -292,7 +319,12 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                     if (!RS) {
                         const RayForms f = ray_forms<MODEL>(r0, r1, r2, d);
                         if (f.E > r1.w * f.den) continue;
-                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * exp2_approx(r0.w * (f.E * rcp_approx(f.den))));
+                        const float o = st.rec[t * 4 + 3].w;
+                        alpha = fminf(0.999f, o * exp2_approx(r0.w * (f.E * rcp_approx(f.den))));
+                        if (__builtin_expect(alpha < r2.w, 0)) {
+                            const uint32_t g = flatten_ids[batch_start + t];
+                            if (!kept_at_cut<1>(cuts + g, n_cuts, ray + threadIdx.x, 0, o)) continue;
+                        }
                     } else {
                         const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
                         const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
@@ -309,9 +341,9 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                         if (cc > -2.0f * __uint_as_float(st.box[t].z) * uu) continue;
                         const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
                         alpha = fminf(0.999f, st.rec[t * 4 + 3].w * __expf(power));
+                        if (alpha < kAlphaMin) continue;
                     }
                     const float4 r3 = st.rec[t * 4 + 3];
-                    if (alpha < kAlphaMin) continue;
                     const float next_T = T * (1.0f - alpha);
                     if (next_T <= 1e-4f) { done = true; break; }
                     const float vis = alpha * T;
@@ -382,11 +414,12 @@ __device__ __forceinline__ float __reduce_add_sync_f32(float x) {
 //   q omega e1, q omega e2 | the same two times phi | q omega^2 e1^2, q omega^2 e1 e2, q omega^2 e2^2 | q phi | rgb | q
 // Rolling shutter: 16 = sum v_u (x) d, sum v_gro, rgb, opacity.
 constexpr int kSums = 12, kSumsRs = 16;
-template <int BATCH, int NS, int PX>
+template <int BATCH, int NS, int PX, bool RAYS>
 struct BwdShared {
     Stage<BATCH> stage[3];       // batch b is walked while b+1 and b+2 are in flight
     uint32_t sid[3][BATCH];      // Gaussian index per slot
     float red[256 / PX / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
+    f3 ray[RAYS ? PX : 1][RAYS ? 256 / PX : 1];  // world-space unit rays, for kept_at_cut
 };
 
 // 1 / x for x in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23).
@@ -402,9 +435,10 @@ __device__ __forceinline__ float rcp_newton(float x) {
 // so the warp reduction (12 stores, 4 wide loads, the reduction to memory), the record loads and the list walk are paid once
 // for two pixels, at the price of more idle lanes in the larger patch. launch_raster_bwd says where which PX runs.
 template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS, int PX>
-__global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
-    const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds,
-    const uint32_t* __restrict__ flatten_ids,
+__global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd_kernel(
+
+    const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
+    const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
     const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
@@ -413,7 +447,8 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
     float* __restrict__ accum_extra) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int NS = RS ? kSumsRs : kSums;
-    BwdShared<BATCH, NS, PX>& sm = *reinterpret_cast<BwdShared<BATCH, NS, PX>*>(smem_raw);
+    using Shared = BwdShared<BATCH, NS, PX, !RS>;
+    Shared& sm = *reinterpret_cast<Shared*>(smem_raw);
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
@@ -438,8 +473,10 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
     for (int p = 0; p < PX; ++p) {
         const int j = j0 + p;
         oo[p] = f3{0.f, 0.f, 0.f};
+        f3 wd;
         const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], oo[p])
-                               : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p]);
+                               : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], wd);
+        if (!RS) sm.ray[p][threadIdx.x] = wd;
         const bool active = i < H && j < W && ray_ok;
         takes_part[p] = active;
         const int pid = min(i * W + j, W * H - 1);
@@ -515,7 +552,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
             if (e >= t_begin && e < batch_size) {
                 const uint4 bx = st.box[e];
                 ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
-                if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], rays);
+                if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], __uint_as_float(bx.z), rays);
             }
             live[w] = __ballot_sync(0xffffffffu, ov);
         }
@@ -559,6 +596,7 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
                 if (!__any_sync(0xffffffffu, any_valid)) continue;
                 const float4 r3 = st.rec[t * 4 + 3];
                 float rden[PX], phi[PX], alpha[PX];
+                bool near_cut = false;
                 any_valid = false;
 #pragma unroll
                 for (int p = 0; p < PX; ++p) {
@@ -571,8 +609,18 @@ __global__ void __launch_bounds__(256 / PX) raster_bwd_kernel(
                         vis[p] = __expf(vis[p]);
                     }
                     alpha[p] = fminf(0.999f, r3.w * vis[p]);
-                    valid[p] = valid[p] && !(alpha[p] < kAlphaMin);
+                    if (RS) valid[p] = valid[p] && !(alpha[p] < kAlphaMin);
+                    else near_cut = near_cut || (valid[p] && alpha[p] < r2.w);
                     any_valid = any_valid || valid[p];
+                }
+                if (!RS && __any_sync(0xffffffffu, near_cut)) {
+                    any_valid = false;
+                    const uint32_t kept = kept_at_cut<PX>(cuts + sid[t], n_cuts, sm.ray[0] + threadIdx.x, 256 / PX, r3.w);
+#pragma unroll
+                    for (int p = 0; p < PX; ++p) {
+                        valid[p] = valid[p] && ((kept >> p & 1u) || !(alpha[p] < r2.w));
+                        any_valid = any_valid || valid[p];
+                    }
                 }
                 if (!__any_sync(0xffffffffu, any_valid)) continue;
                 float v[NS];
@@ -1147,7 +1195,7 @@ int launch_raster_fwd(const RasterArgs& a, float* render, float* alphas, int32_t
     if (a.channels != 1 && a.channels != 3 && a.channels != 4) { set_error("raster_fwd: channels must be 1, 3 or 4"); return LFS_EINVAL; }
     LFS_TIMED("raster_fwd", st);
 #define LFS_FWD3(MODEL, EXTRA, RS)                                                                                         \
-    raster_fwd_kernel<MODEL, EXTRA, RS><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets,   \
+    raster_fwd_kernel<MODEL, EXTRA, RS><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets,   \
                                                                     a.n_isects_dev, a.n_isects_host, a.overflow, a.background,  \
                                                                     a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H,   \
                                                                     a.tw, n_tiles, render, alphas, last_ids, extra_sum)
@@ -1179,9 +1227,10 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     constexpr int kBatch = 64;
 #define LFS_BWD6(MODEL, EXTRA, XGRAD, RS, PX)                                                                                  \
     do {                                                                                                                       \
-        constexpr int smem = (int)sizeof(BwdShared<kBatch, RS ? kSumsRs : kSums, PX>);                                         \
+        constexpr int smem = (int)sizeof(BwdShared<kBatch, RS ? kSumsRs : kSums, PX, !RS>);                                \
         raster_bwd_kernel<MODEL, kBatch, EXTRA, XGRAD, RS, PX><<<n_tiles, 256 / PX, smem, st>>>(                               \
-            a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
+            a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow,    \
+            a.background,                                                                                                      \
             a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
             v_alphas, accum, accum_extra);                                                                                     \
     } while (0)

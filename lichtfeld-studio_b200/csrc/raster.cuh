@@ -8,9 +8,12 @@ namespace lfs {
 struct RasterArgs {
     const CamDev* cam;            // one camera
     const float4* records;        // [N] packed 64-byte records
-    const uint4* bounds;          // [N] (x box, y box, rejection exponent, extra): inclusive pixel box (lo | hi << 16)
-                                  //     outside of which alpha < 1/255, -ln(255 opacity) - margin as float bits, and the
-                                  //     value blended into the last channel when channels is 1 or 4 (the depth)
+    const float4* cuts;           // [3][N] rows of the cut records (not for a rolling shutter)
+    int64_t n_cuts;               // N
+    const uint4* bounds;          // [N] (x box, y box, limit, extra): inclusive pixel box (lo | hi << 16) outside of which
+                                  //     alpha < 1/255; as float bits sqrt(phi_max / (1 - phi_max)) with phi_max somewhat above
+                                  //     the record's phi_cut (rolling shutter: -ln(255 opacity) - margin); the value blended
+                                  //     into the last channel when channels is 1 or 4 (the depth)
     const uint32_t* flatten_ids;  // depth-sorted Gaussian index per instance
     const int32_t* tile_offsets;  // [tw*th] first instance of each tile
     const int32_t* n_isects_dev;  // device-side instance count, or null to use n_isects_host
