@@ -376,21 +376,33 @@ __device__ __forceinline__ bool opencv_box(const CamDev& cam, float* lo, float* 
 // Fisheye: the rays lie in the cone of half angle beta around the centre, tan beta = the largest tangent-plane extent of the
 // dual quadric over all directions; the image of the cone lies in the ring sector theta0 +- beta, psi0 +- asin(sin beta /
 // sin theta0). The radius is monotone in theta up to max_angle, which bounds every valid ray (known for k4 = 0 only).
-__device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, float s00, float s01, float s02, float s11,
-                                            float s12, float s22, float* lo, float* hi) {
-    const float m2 = mc[0] * mc[0] + mc[1] * mc[1] + mc[2] * mc[2];
+// V: camera-space axes of the Gaussian (columns), s[i]: their half lengths squared. The extents across the centre direction e are
+// summed over the axes in a basis (a, b) across e: a needle that points at the camera is up to a thousand times longer than wide,
+// and what is left of its squares after subtracting the part along e would be rounding.
+__device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, const float* V, const float* s, float* lo, float* hi) {
+    const float m2 = fdot3(mc[0], mc[0], mc[1], mc[1], mc[2], mc[2]);
     if (cam.k[3] != 0.f || !(m2 > 0.f)) return false;
     const float im = 1.0f / sqrtf(m2);
-    const float e0 = mc[0] * im, e1 = mc[1] * im, e2 = mc[2] * im;
-    const float t0 = s00 * e0 + s01 * e1 + s02 * e2, t1 = s01 * e0 + s11 * e1 + s12 * e2, t2 = s02 * e0 + s12 * e1 + s22 * e2;
-    const float along = t0 * e0 + t1 * e1 + t2 * e2, tt = t0 * t0 + t1 * t1 + t2 * t2;
-    const float B22 = m2 - along;
+    const float e[3] = {mc[0] * im, mc[1] * im, mc[2] * im};
+    // a = e x (the x or the y axis, whichever is farther from e)
+    const bool use_x = fabsf(e[0]) < 0.7f;
+    const float an = rsqrtf(use_x ? fmaf(e[1], e[1], e[2] * e[2]) : fmaf(e[0], e[0], e[2] * e[2]));
+    const float a[3] = {use_x ? 0.f : -e[2] * an, use_x ? e[2] * an : 0.f, use_x ? -e[1] * an : e[0] * an};
+    const float b[3] = {fmaf(e[1], a[2], -e[2] * a[1]), fmaf(e[2], a[0], -e[0] * a[2]), fmaf(e[0], a[1], -e[1] * a[0])};
+    float saa = 0.f, sbb = 0.f, sab = 0.f, sea = 0.f, seb = 0.f, see = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float ai = fdot3(a[0], V[i], a[1], V[3 + i], a[2], V[6 + i]), bi = fdot3(b[0], V[i], b[1], V[3 + i], b[2], V[6 + i]);
+        const float ei = fdot3(e[0], V[i], e[1], V[3 + i], e[2], V[6 + i]);
+        const float sa = s[i] * ai, sb = s[i] * bi;
+        saa = fmaf(sa, ai, saa); sbb = fmaf(sb, bi, sbb); sab = fmaf(sa, bi, sab);
+        sea = fmaf(sa, ei, sea); seb = fmaf(sb, ei, seb); see = fmaf(s[i] * ei, ei, see);
+    }
+    const float B22 = m2 - see;
     if (!(B22 > 0.02f * m2)) return false;
-    const float cross2 = fmaxf(0.f, tt - along * along);             // |part of Sigma e across e|^2
-    const float tr = s00 + s11 + s22 - along;                        // trace and squared norm of Sigma across e
-    const float fro = s00 * s00 + s11 * s11 + s22 * s22 + 2.f * (s01 * s01 + s02 * s02 + s12 * s12) - 2.f * tt + along * along;
-    const float lmax = 0.5f * (tr + sqrtf(fmaxf(0.f, 2.f * fro - tr * tr))) * 1.001f;
-    const float ext = (sqrtf(cross2) + sqrtf(cross2 + lmax * B22)) / B22;
+    const float lmax = 0.5f * (saa + sbb + sqrtf(fmaf(saa - sbb, saa - sbb, 4.f * sab * sab))) * 1.001f;
+    const float cross2 = fmaf(sea, sea, seb * seb);
+    const float ext = (sqrtf(cross2) + sqrtf(fmaf(lmax, B22, cross2))) / B22;
     const float beta = atanf(ext) * 1.001f;
     const float n = sqrtf(mc[0] * mc[0] + mc[1] * mc[1]), theta0 = atan2f(n, mc[2]);
     const float th_lo = fmaxf(theta0 - beta, 0.f) * 0.9999f, th_hi = fminf(theta0 + beta, cam.max_angle) * 1.0001f;
@@ -482,7 +494,8 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
     float lo[2], hi[2];   // in units of the focal length, before the principal point
     bool bounded = false;
     if (MODEL == LFS_FISHEYE) {
-        bounded = fisheye_box(cam, f.m, sig(0, 0), sig(0, 1), sig(0, 2), sig(1, 1), sig(1, 2), sig(2, 2), lo, hi);
+        const float s[3] = {s0, s1, s2};
+        bounded = fisheye_box(cam, f.m, f.V, s, lo, hi);
     } else {
         const float B22 = fmaf(f.m[2], f.m[2], -sig(2, 2));
         if (f.m[2] > 0.f && B22 > 0.02f * f.m[2] * f.m[2]) {

@@ -84,3 +84,90 @@ def test_pairs_at_the_cut_are_those_of_the_product_form(pkg, f, seed, decided):
                                                             v_render_colors=torch.ones_like(image), v_render_alphas=torch.zeros_like(alphas))
     v_colors = grads[3][0, :, 0].cpu().numpy()
     assert np.abs(v_colors - got.astype(np.float64).sum(1)).max() < 1e-3
+
+
+# ---- boxes and patches: one Gaussian per tile list, every pair against float64 -----------------------------------------
+def _quat(R):
+    """float32 quaternions (w, x, y, z) of rotation matrices [n, 3, 3]"""
+    q = np.sqrt(np.maximum(0, 1 + np.stack([R[:, 0, 0] + R[:, 1, 1] + R[:, 2, 2], R[:, 0, 0] - R[:, 1, 1] - R[:, 2, 2],
+                                            R[:, 1, 1] - R[:, 0, 0] - R[:, 2, 2], R[:, 2, 2] - R[:, 0, 0] - R[:, 1, 1]], -1))) / 2
+    q[:, 1] = np.copysign(q[:, 1], R[:, 2, 1] - R[:, 1, 2])
+    q[:, 2] = np.copysign(q[:, 2], R[:, 0, 2] - R[:, 2, 0])
+    q[:, 3] = np.copysign(q[:, 3], R[:, 1, 0] - R[:, 0, 1])
+    return q.astype(np.float32)
+
+
+def _rotmat(q):
+    w, x, y, z = (q / np.linalg.norm(q, axis=1, keepdims=True)).T
+    return np.array([[1 - 2 * (y * y + z * z), 2 * (x * y - w * z), 2 * (x * z + w * y)],
+                     [2 * (x * y + w * z), 1 - 2 * (x * x + z * z), 2 * (y * z - w * x)],
+                     [2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)]]).transpose(2, 0, 1)
+
+
+def _alpha64(means, quats, scales, opac, owner, d):
+    """[H, W] alpha of each pixel's own Gaussian (owner, -1 = none) along the line of its ray d [H, W, 3]"""
+    M = _rotmat(quats.astype(np.float64)).transpose(0, 2, 1) / scales.astype(np.float64)[:, :, None]
+    g = (M @ -means.astype(np.float64)[:, :, None])[:, :, 0]
+    at = np.maximum(owner, 0)
+    u = np.einsum("hwij,hwj->hwi", M[at], d)
+    c = np.cross(u, g[at])
+    return np.where(owner >= 0, opac[at] * np.exp(-0.5 * (c * c).sum(-1) / (u * u).sum(-1)), 0.0)
+
+
+def _check_single_lists(pkg, means, quats, scales, opac, tile_owner, W, H, f):
+    """Equidistant fisheye at the origin. Every pair with alpha clearly above 1/255 is blended, none clearly below, and the backward
+    walks the same pairs."""
+    n, th, tw = len(means), H // 16, W // 16
+    j, i = np.meshgrid(np.arange(W) + 0.5, np.arange(H) + 0.5)
+    ux, uy = (j - W / 2) / f, (i - H / 2) / f
+    theta = np.hypot(ux, uy)
+    d = np.stack([np.sin(theta) / theta * ux, np.sin(theta) / theta * uy, np.cos(theta)], -1)
+    owner = np.repeat(np.repeat(tile_owner, 16, 0), 16, 1)
+    alpha = _alpha64(means, quats, scales, opac, owner, d)
+    valid = theta < np.hypot(W / 2, H / 2) / f * (1 - 1e-6)
+    K = np.array([[[f, 0, W / 2], [0, f, H / 2], [0, 0, 1]]], np.float32)
+    front = (T(means), T(quats), T(scales), torch.ones((1, n, 3), device=DEV), T(opac[None]), None, None, W, H, 16,
+             T(np.eye(4, dtype=np.float32)[None]), None, T(K), pkg._capi.FISHEYE)
+    has = tile_owner.reshape(-1) >= 0
+    lists = dict(tile_offsets=T((np.cumsum(has) - has).astype(np.int32).reshape(1, th, tw)),
+                 flatten_ids=T(tile_owner.reshape(-1)[has].astype(np.int32)))
+    radial = torch.zeros((1, 4), device=DEV)
+    image, alphas, last_ids = pkg.ops.rasterize_to_pixels_from_world_3dgs_fwd(*front, radial_coeffs=radial, **lists)
+    got = alphas[0, ..., 0].cpu().numpy().astype(np.float64)
+    # the kernels' float32 response errs by a few 2^-24 (distance / smallest scale): 2 % where that ratio is 1e4 or less
+    assert (1 / scales.min(1) * np.linalg.norm(means, axis=1)).max() < 1e4
+    lost, extra = valid & (alpha > 1.02 / 255) & (got == 0), (alpha < 0.98 / 255) & (got > 0)
+    assert lost.sum() == 0 and extra.sum() == 0, (lost.sum(), alpha[lost].max() if lost.any() else 0, extra.sum())
+    grads = pkg.ops.rasterize_to_pixels_from_world_3dgs_bwd(*front, radial_coeffs=radial, **lists, render_alphas=alphas, last_ids=last_ids,
+                                                            v_render_colors=torch.ones_like(image), v_render_alphas=torch.zeros_like(alphas))
+    # one entry per pixel: the colour's gradient is the sum of the blended alphas. A pair more or less moves it by 3.9e-3 and more, the
+    # float32 sum of up to 3e4 alphas by their rounding
+    total = np.array([got[owner == g].sum() for g in range(n)])
+    assert np.abs(grads[3][0, :, 0].cpu().numpy() - total).max() < 2e-3 + 2e-6 * total.max()
+
+
+# needles that point at the camera and reach close to it: sixty to a thousand times longer than wide, twice to ten times wider than thick
+@pytest.mark.parametrize("seed", range(4))
+def test_fisheye_keeps_the_pairs_of_needles_along_the_ray(pkg, seed):
+    rng = np.random.default_rng(seed)
+    W = H = 2048
+    block = 8                                   # tiles of a needle's own square
+    by, bx = np.divmod(np.arange(256), 16)
+    f = 1400.0                                  # 84 degrees across the image
+    px = np.stack([bx * 128 + 64 + rng.uniform(-8, 8, 256), by * 128 + 64 + rng.uniform(-8, 8, 256)], -1)
+    u = (px - 1024) / f
+    theta = np.linalg.norm(u, axis=1)
+    e = np.stack([np.sin(theta) / theta * u[:, 0], np.sin(theta) / theta * u[:, 1], np.cos(theta)], -1)
+    n = len(e)
+    dist = np.exp(rng.uniform(-1, 1, n))
+    opac = rng.uniform(0.3, 0.95, n).astype(np.float32)
+    length = dist * rng.uniform(0.5, 0.98, n) / np.sqrt(2 * np.log(255 * opac))
+    width = length / 10 ** rng.uniform(1.8, 2.3, n)
+    scales = np.stack([length, width, np.maximum(width * rng.uniform(0.1, 0.5, n), dist / 9000)], -1).astype(np.float32)
+    a = e + 10 ** rng.uniform(-6, -4, (n, 1)) * rng.normal(size=(n, 3))
+    a /= np.linalg.norm(a, axis=1, keepdims=True)
+    b = np.cross(a, rng.normal(size=(n, 3)))
+    b /= np.linalg.norm(b, axis=1, keepdims=True)
+    quats = _quat(np.stack([a, b, np.cross(a, b)], -1))
+    owner = np.arange(256).reshape(16, 16).repeat(block, 0).repeat(block, 1)
+    _check_single_lists(pkg, (e * dist[:, None]).astype(np.float32), quats, scales, opac, owner, W, H, f)
