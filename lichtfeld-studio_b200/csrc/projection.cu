@@ -329,7 +329,8 @@ int launch_projection_ut(int C, int N, const float* means, const float* quats, c
 // B = mu_c mu_c^T - Sigma_c: x_n = (B02 -+ sqrt(B02^2 - B00 B22)) / B22 (same with index 1 for y). A distorted pinhole maps
 // that rectangle by interval arithmetic (opencv_box); a fisheye takes the cone around the ellipsoid to a ring sector
 // (fisheye_box). A margin keeps the box conservative under rounding; when the ellipsoid reaches the camera plane (B22 <= 0,
-// for a fisheye: the origin) or the camera is none of the three the box is the whole image. The rasterizer uses it only to
+// for a fisheye: the plane across its direction), when a fisheye sees it from behind as well, or when the camera is none of the
+// three, the box is the whole image. The rasterizer uses it only to
 // skip (warp patch, Gaussian) pairs that cannot contribute.
 // a . b for nearly orthogonal vectors, as if summed in twice the precision (products split by fma, sums by two-sum;
 // Ogita, Rump and Oishi's Dot2)
@@ -376,12 +377,45 @@ __device__ __forceinline__ bool opencv_box(const CamDev& cam, float* lo, float* 
 // Fisheye: the rays lie in the cone of half angle beta around the centre, tan beta = the largest tangent-plane extent of the
 // dual quadric over all directions; the image of the cone lies in the ring sector theta0 +- beta, psi0 +- asin(sin beta /
 // sin theta0). The radius is monotone in theta up to max_angle, which bounds every valid ray (known for k4 = 0 only).
+// The response does not know the sign of a ray: one that leaves the Gaussian behind it, in the cone around -mu, is answered too. A
+// lens that sees past the plane of the camera may show both cones. One box does not hold both, so where the second one can meet the
+// tiles that list the Gaussian (`tiles`, in pixels: x0, y0, and past the end x1, y1) there is none.
 // V: camera-space axes of the Gaussian (columns), s[i]: their half lengths squared. The extents across the centre direction e are
 // summed over the axes in a basis (a, b) across e: a needle that points at the camera is up to a thousand times longer than wide,
 // and what is left of its squares after subtracting the part along e would be rounding.
-__device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, const float* V, const float* s, float* lo, float* hi) {
+struct Box { float lo[2], hi[2]; };   // in units of the focal length, from the principal point
+__device__ __forceinline__ void box_pixels(const CamDev& cam, const Box& box, float* lo_j, float* hi_j) {
+    const float fc[2] = {cam.fx, cam.fy}, c0[2] = {cam.cx, cam.cy};
+#pragma unroll
+    for (int ax = 0; ax < 2; ++ax) {
+        const float pa = fmaf(fc[ax], box.lo[ax], c0[ax]), pb = fmaf(fc[ax], box.hi[ax], c0[ax]);
+        const float lo_px = fminf(pa, pb), hi_px = fmaxf(pa, pb);
+        const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * (hi_px - lo_px);
+        // pixel j has its centre at j + 0.5
+        lo_j[ax] = floorf(lo_px - 0.5f - margin); hi_j[ax] = ceilf(hi_px - 0.5f + margin);
+    }
+}
+// Image of the cone of half angle beta (sine sb) around the direction (theta0, psi0), of which st = sin theta0, cp = cos psi0, sp =
+// sin psi0; false when no ray of the lens lies in it.
+__device__ __forceinline__ bool fisheye_sector(const CamDev& cam, float theta0, float st, float cp, float sp, float beta, float sb, Box& box) {
+    const float th_lo = fmaxf(theta0 - beta, 0.f) * 0.9999f, th_hi = fminf(theta0 + beta, cam.max_angle) * 1.0001f;
+    if (!(th_hi >= th_lo)) return false;
+    const float r_lo = fisheye_poly_odd(cam.k, th_lo), r_hi = fmaxf(r_lo, fisheye_poly_odd(cam.k, th_hi));
+    float cmin = -1.f, cmax = 1.f, smin = -1.f, smax = 1.f;          // ranges of cos psi and sin psi
+    if (beta < 1.5f && sb < st) {
+        const float sd = sb / st, cd = sqrtf(fmaxf(0.f, 1.f - sd * sd));
+        const float ca = cp * cd - sp * sd, cb = cp * cd + sp * sd, sa = sp * cd + cp * sd, sc = sp * cd - cp * sd;
+        cmax = cp >= cd ? 1.f : fmaxf(ca, cb); cmin = -cp >= cd ? -1.f : fminf(ca, cb);
+        smax = sp >= cd ? 1.f : fmaxf(sa, sc); smin = -sp >= cd ? -1.f : fminf(sa, sc);
+    }
+    box.lo[0] = fminf(cmin * r_lo, cmin * r_hi); box.hi[0] = fmaxf(cmax * r_lo, cmax * r_hi);
+    box.lo[1] = fminf(smin * r_lo, smin * r_hi); box.hi[1] = fmaxf(smax * r_lo, smax * r_hi);
+    return true;
+}
+__device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, const float* V, const float* s, const float4& tiles, Box& box) {
     const float m2 = fdot3(mc[0], mc[0], mc[1], mc[1], mc[2], mc[2]);
-    if (cam.k[3] != 0.f || !(m2 > 0.f)) return false;
+    // rays past 180 degrees from the axis repeat the directions of others
+    if (cam.k[3] != 0.f || !(m2 > 0.f) || cam.max_angle > 3.1415f) return false;
     const float im = 1.0f / sqrtf(m2);
     const float e[3] = {mc[0] * im, mc[1] * im, mc[2] * im};
     // a = e x (the x or the y axis, whichever is farther from e)
@@ -405,27 +439,21 @@ __device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, 
     const float ext = (sqrtf(cross2) + sqrtf(fmaf(lmax, B22, cross2))) / B22;
     const float beta = atanf(ext) * 1.001f;
     const float n = sqrtf(mc[0] * mc[0] + mc[1] * mc[1]), theta0 = atan2f(n, mc[2]);
-    const float th_lo = fmaxf(theta0 - beta, 0.f) * 0.9999f, th_hi = fminf(theta0 + beta, cam.max_angle) * 1.0001f;
-    if (!(th_hi >= th_lo)) return false;
-    const float r_lo = fisheye_poly_odd(cam.k, th_lo), r_hi = fmaxf(r_lo, fisheye_poly_odd(cam.k, th_hi));
-    const float sb = sinf(beta) * 1.001f, st = n * im;
-    float cmin = -1.f, cmax = 1.f, smin = -1.f, smax = 1.f;          // ranges of cos psi and sin psi
-    if (beta < 1.5f && sb < st) {
-        const float cp = mc[0] / n, sp = mc[1] / n, sd = sb / st, cd = sqrtf(fmaxf(0.f, 1.f - sd * sd));
-        const float ca = cp * cd - sp * sd, cb = cp * cd + sp * sd, sa = sp * cd + cp * sd, sc = sp * cd - cp * sd;
-        cmax = cp >= cd ? 1.f : fmaxf(ca, cb); cmin = -cp >= cd ? -1.f : fminf(ca, cb);
-        smax = sp >= cd ? 1.f : fmaxf(sa, sc); smin = -sp >= cd ? -1.f : fminf(sa, sc);
+    const float sb = sinf(beta) * 1.001f, st = n * im, in = 1.0f / fmaxf(n, 1e-30f), cp = mc[0] * in, sp = mc[1] * in;
+    const float behind = 3.14159265f - theta0;
+    if ((behind - beta) * 0.9999f <= cam.max_angle && fisheye_sector(cam, behind, st, -cp, -sp, beta, sb, box)) {
+        float lo[2], hi[2];
+        box_pixels(cam, box, lo, hi);
+        if (lo[0] < tiles.z && hi[0] >= tiles.x && lo[1] < tiles.w && hi[1] >= tiles.y) return false;
     }
-    lo[0] = fminf(cmin * r_lo, cmin * r_hi); hi[0] = fmaxf(cmax * r_lo, cmax * r_hi);
-    lo[1] = fminf(smin * r_lo, smin * r_hi); hi[1] = fmaxf(smax * r_lo, smax * r_hi);
-    return true;
+    return fisheye_sector(cam, theta0, st, cp, sp, beta, sb, box);
 }
 
 // Only the lists are pinned to unfused arithmetic (file header); everything here spells its products and sums as fma.
 template <int MODEL, bool RS>
 __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
                                             f3 scale, float r, float g, float b, float opacity, float extra, float4* rec,
-                                            float4* __restrict__ cut, int64_t n, uint4& box) {
+                                            float4* __restrict__ cut, int64_t n, const float4& tiles, uint4& box) {
     float R[9], inv_norm, qn[4];
     quat_to_rotmat_renorm(qw, qx, qy, qz, R, inv_norm, qn);
     // exponent below which opacity * exp(p) < 1/255 for certain
@@ -491,11 +519,11 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);
     const float s0 = rho2 * scale.x * scale.x, s1 = rho2 * scale.y * scale.y, s2 = rho2 * scale.z * scale.z;
     auto sig = [&](int a, int c) { return fdot3(f.V[a * 3] * s0, f.V[c * 3], f.V[a * 3 + 1] * s1, f.V[c * 3 + 1], f.V[a * 3 + 2] * s2, f.V[c * 3 + 2]); };
-    float lo[2], hi[2];   // in units of the focal length, before the principal point
+    Box image;
     bool bounded = false;
     if (MODEL == LFS_FISHEYE) {
         const float s[3] = {s0, s1, s2};
-        bounded = fisheye_box(cam, f.m, f.V, s, lo, hi);
+        bounded = fisheye_box(cam, f.m, f.V, s, tiles, image);
     } else {
         const float B22 = fmaf(f.m[2], f.m[2], -sig(2, 2));
         if (f.m[2] > 0.f && B22 > 0.02f * f.m[2] * f.m[2]) {
@@ -505,22 +533,18 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
                 const float Ba2 = fmaf(f.m[ax], f.m[2], -sig(ax, 2));
                 const float Baa = fmaf(f.m[ax], f.m[ax], -sig(ax, ax));
                 const float disc = sqrtf(fmaxf(0.f, fmaf(Ba2, Ba2, -Baa * B22)));
-                lo[ax] = (Ba2 - disc) * iB; hi[ax] = (Ba2 + disc) * iB;
+                image.lo[ax] = (Ba2 - disc) * iB; image.hi[ax] = (Ba2 + disc) * iB;
             }
-            bounded = MODEL == LFS_PINHOLE || opencv_box(cam, lo, hi);
+            bounded = MODEL == LFS_PINHOLE || opencv_box(cam, image.lo, image.hi);
         }
     }
     if (bounded) {
+        float lo[2], hi[2];
         uint32_t packed[2];
-        const float fc[2] = {cam.fx, cam.fy}, c0[2] = {cam.cx, cam.cy};
+        box_pixels(cam, image, lo, hi);
 #pragma unroll
         for (int ax = 0; ax < 2; ++ax) {
-            const float pa = fmaf(fc[ax], lo[ax], c0[ax]), pb = fmaf(fc[ax], hi[ax], c0[ax]);
-            const float lo_px = fminf(pa, pb), hi_px = fmaxf(pa, pb);
-            const float margin = 0.75f + 2e-4f * (fabsf(lo_px) + fabsf(hi_px)) + 1e-3f * (hi_px - lo_px);
-            // pixel j has its centre at j + 0.5
-            const float lo_j = floorf(lo_px - 0.5f - margin), hi_j = ceilf(hi_px - 0.5f + margin);
-            const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo_j, 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi_j, 0.f), 65535.f);
+            const uint32_t lo_u = (uint32_t)fminf(fmaxf(lo[ax], 0.f), 65535.f), hi_u = (uint32_t)fminf(fmaxf(hi[ax], 0.f), 65535.f);
             packed[ax] = lo_u | (hi_u << 16);
         }
         box.x = packed[0];
@@ -545,7 +569,8 @@ __global__ void __launch_bounds__(256) pack_records_kernel(
         const float* col = colors + (size_t)g * channels;
         const bool has_rgb = channels >= 3;
         make_record<MODEL, RS>(cam, mean, q.x, q.y, q.z, q.w, scale, has_rgb ? col[0] : 0.f, has_rgb ? col[1] : 0.f, has_rgb ? col[2] : 0.f,
-                    opacities[g], channels != 3 ? col[channels - 1] : 0.f, rec, cuts + g, N, box);
+                    opacities[g], channels != 3 ? col[channels - 1] : 0.f, rec, cuts + g, N,
+                    make_float4(0.f, 0.f, 65536.f, 65536.f), box);   // whatever lists the caller has
 #pragma unroll
         for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
         bounds[g] = box;
@@ -684,7 +709,7 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
             float4 rec[4];
             uint4 box;
             make_record<MODEL, RS>(cam, mean, qw, qx, qy, qz, scale, rgb[0], rgb[1], rgb[2], opacity, o.depth, rec,
-                                   cuts + g, N, box);
+                                   cuts + g, N, make_float4(x0 * tile_size, y0 * tile_size, x1 * tile_size, y1 * tile_size), box);
 #pragma unroll
             for (int k = 0; k < 4; ++k) records[(size_t)g * 4 + k] = rec[k];
             bounds[g] = box;
