@@ -193,13 +193,15 @@ def test_fisheye_keeps_the_pairs_behind_the_ray(pkg, fov):
         _check_single_lists(pkg, means[one], quats[one], scales[one], opac[one], np.zeros((H // 16, W // 16), int), W, H, f)
 
 
-@pytest.mark.parametrize("fov,grow", [(180, 1.2), (200, 1.0), (220, 1.0)])
-def test_fisheye_inside_a_scene(pkg, orc, synth, fov, grow):
+@pytest.mark.parametrize("n,fov,grow,fade", [(20000, 180, 1.2, 0.0), (20000, 200, 1.0, 0.0), (1000, 220, 2.2, 2.0)])
+def test_fisheye_inside_a_scene(pkg, orc, synth, n, fov, grow, fade):
     tr, capi = pkg.trainer, pkg._capi
-    n, W, H, deg = 3000, 208, 176, 1
+    W = H = 256
+    deg = 1
     P = synth.make_gaussians(n, 5, "cube", deg)
     P["scaling_raw"] = (P["scaling_raw"] + np.float32(grow)).astype(np.float32)
-    vm = synth.look_at_origin([0.25, -0.3, 0.2])
+    P["opacity_raw"] = (P["opacity_raw"] - np.float32(fade)).astype(np.float32)
+    vm = synth.look_at_origin([0.1, -0.2, 0.1])
     f = min(W, H) / np.radians(fov)
     K = synth.intrinsics(f, f, W / 2.0, H / 2.0)
     radial = np.zeros(4, np.float32)
@@ -211,7 +213,7 @@ def test_fisheye_inside_a_scene(pkg, orc, synth, fov, grow):
     out = rast.forward(tr.Camera(T(vm), T(K), W, H, capi.FISHEYE, radial=T(radial)), None)
     diff = np.abs(out.image.cpu().numpy() - fwd["render"]).max(-1)
     # The oracle rounds the product form without fused operations: a pair within that of the cut falls on either side, 4e-3 of a colour
-    # of up to 1.5. A lost pair of alpha 0.02 in an unsaturated pixel shows as 1e-2 and more
+    # of up to 1.5 in a pixel here and there. Lost cones show as larger differences or in many pixels
     assert diff.max() < 8e-3 and (diff > 1e-4).sum() <= 20, (diff.max(), (diff > 1e-4).sum())
     rng = np.random.default_rng(1)
     v_r, v_a = (rng.normal(size=(H, W, k)).astype(np.float32) * 1e-3 for k in (3, 1))
