@@ -674,19 +674,24 @@ size_t emit_state_words(int64_t total) { return ((size_t)((total + kThreads - 1)
 // kernels; 250 k 51 against 68; 1 M 79 against 94); on long lists its waves of tiles queue behind one another's words and the
 // three-kernel pass with one chunk per CTA is the faster one (6 M keys: 217 us against 279; 7 M instances, two passes: 291
 // against 360). A device-side count is bounded by the list's capacity, which users leave a few times larger than the list.
-bool sort_by_lookback(const int32_t* n_dev, int64_t n_max) { return n_max <= (n_dev ? (int64_t)6 << 20 : (int64_t)2 << 20); }
+int64_t lookback_limit(bool count_on_device) { return count_on_device ? (int64_t)6 << 20 : (int64_t)2 << 20; }
 constexpr int64_t kMaxChunks = 1024;   // the size query must not depend on a device
 int chunk_blocks(int64_t n_max) { return (int)min((n_max + kTile - 1) / kTile, min((int64_t)4 * num_sms(), kMaxChunks)); }
-size_t sort_state_words(bool lookback, int64_t n, int passes) {
-    return lookback ? (size_t)((n + kTile - 1) / kTile) * 256 * passes : (size_t)256 * (min((n + kTile - 1) / kTile, kMaxChunks) + 1);
+// Never less for a longer list, although a chunked sort needs less than the longest look-back: a workspace made for a capacity
+// serves every list up to it.
+size_t sort_state_words(bool count_on_device, int64_t n, int passes) {
+    const int64_t limit = lookback_limit(count_on_device);
+    const size_t lookback = (size_t)((min(n, limit) + kTile - 1) / kTile) * 256 * passes;
+    const size_t chunked = n > limit ? (size_t)256 * (min((n + kTile - 1) / kTile, kMaxChunks) + 1) : 0;
+    return lookback > chunked ? lookback : chunked;
 }
 int tile_sort_passes(int key_bits) { return (key_bits + 7) / 8; }
 }  // namespace
 
 size_t tile_list_state_words(int64_t total, int64_t capacity, int key_bits) {
-    const int32_t on_device = 0;   // the instance count is read on the device, the number of Gaussians is not
-    const size_t depth = sort_state_words(sort_by_lookback(nullptr, total), total, 4);
-    const size_t tile = sort_state_words(sort_by_lookback(&on_device, capacity), capacity, tile_sort_passes(key_bits));
+    // the instance count is read on the device, the number of Gaussians is not
+    const size_t depth = sort_state_words(false, total, 4);
+    const size_t tile = sort_state_words(true, capacity, tile_sort_passes(key_bits));
     return kTicketWords + kHistWords + emit_state_words(total) + (depth > tile ? depth : tile);
 }
 
@@ -701,7 +706,7 @@ static int radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], const int32_t*
     const uint32_t mask = (1u << bits) - 1u;
     int cur = 0;
     LFS_TIMED(n_dev ? "radix_sort_tile" : "radix_sort_depth", st);
-    if (sort_by_lookback(n_dev, n_max)) {
+    if (n_max <= lookback_limit(n_dev != nullptr)) {
         const int64_t max_tiles = (n_max + kTile - 1) / kTile;
         // six CTAs per SM (27 KB of shared memory each) keep enough keys in flight; more only queue for tickets
         const int nb = (int)min(max_tiles, (int64_t)6 * num_sms());

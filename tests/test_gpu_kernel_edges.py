@@ -131,3 +131,25 @@ def test_ssim_tile_edges(pkg, orc, H, W):
     dl = rng.normal(size=(1, 3, H, W)).astype(np.float32)
     g = pkg.ops.fusedssim_backward(0.01 ** 2, 0.03 ** 2, T(a), T(b), T(dl), *out[1:])
     assert rel_l2(g.cpu().numpy(), orc.fusedssim_backward(a[0], b[0], dl[0], *ref[1:])) < 1e-4
+
+
+# A model with room for 2,100,000 Gaussians that holds 2,090,000: the workspace is made for the former, whose depth sort is of the
+# other kind than the latter's
+@pytest.mark.parametrize("ewa", [False, True])
+def test_fewer_gaussians_than_the_workspace_was_made_for(pkg, synth, ewa):
+    tr = pkg.trainer
+    W, H, n, capacity = 96, 64, 2_090_000, 2_100_000
+    _, P, vm, K = make_scene(synth, 1000, W, H, 0)
+    model = tr.SplatData(n, 1, DEV, capacity=capacity)
+    for name in NAMES:
+        t = model.tensor(name)
+        if t.numel():
+            t.copy_(T(P[name]).repeat(n // 1000, *[1] * (t.dim() - 1)).view(t.shape))
+    cam, bg = tr.Camera(T(vm), T(K), W, H), torch.zeros(3, device=DEV)
+    make = (lambda m: tr.FastRasterizer(m, W, H, 0, instance_capacity=1 << 25)) if ewa else (lambda m: tr.Rasterizer(m, W, H, 0, isect_capacity=1 << 25))
+    image = make(model).forward(cam, bg).image.clone()
+    exact = tr.SplatData(n, 1, DEV)
+    for name in NAMES:
+        exact.tensor(name).copy_(model.tensor(name))
+    assert torch.isfinite(image).all() and image.abs().max() > 0.1
+    assert torch.equal(image, make(exact).forward(cam, bg).image)
