@@ -479,6 +479,9 @@ __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd
         if (!RS) sm.ray[p][threadIdx.x] = wd;
         const bool active = i < H && j < W && ray_ok;
         takes_part[p] = active;
+        // What a lens leaves for a pixel without a ray may be anything, NaN too. Such a pixel's terms are multiplied by zero below,
+        // which takes finite ones.
+        if (!active) { d[p] = f3{0.f, 0.f, 1.f}; oo[p] = f3{0.f, 0.f, 0.f}; }
         const int pid = min(i * W + j, W * H - 1);
         const float T_final = 1.0f - render_alphas[pid];
         T[p] = T_final;

@@ -221,3 +221,27 @@ def test_fisheye_inside_a_scene(pkg, orc, synth, n, fov, grow, fade):
     rast.backward(T(v_r), grads, None, T(v_a))
     for name in ("means", "sh0", "shN", "scaling_raw", "rotation_raw", "opacity_raw"):
         assert rel_l2(grads.tensor(name).cpu().numpy(), bwd[name]) < 2e-3, name   # as at the backward's other parity tests
+
+
+# Lenses whose inversion runs away to infinity in pixels that share a warp's patch with valid ones (some two dozen of them each)
+@pytest.mark.parametrize("rolling", [False, True])
+@pytest.mark.parametrize("k,f", [((-0.0813082829, -0.525065839, 0.20530051), 111.764832), ((-0.119644128, -0.4756459, 0.237992167), 85.6079636),
+                                 ((-0.101954706, -0.259541839, 0.101956189), 70.9386826)])
+def test_pixels_without_a_ray_leave_the_gradients_finite(pkg, synth, k, f, rolling):
+    tr, capi = pkg.trainer, pkg._capi
+    n, W, H, deg = 3000, 208, 144, 1
+    P = synth.make_gaussians(n, 7, "cube", deg)
+    vm = synth.look_at_origin([0.3, -2.0, 0.4])
+    K = synth.intrinsics(f, f, W / 2.0, H / 2.0)
+    radial = np.zeros(6, np.float32)
+    radial[:3] = k
+    model = tr.SplatData(n, (deg + 1) ** 2, DEV).load(P)
+    grads = model.like()
+    rast = tr.Rasterizer(model, W, H, deg)
+    end = dict(viewmat_end=T(synth.look_at_origin([0.31, -2.0, 0.4])), shutter=1) if rolling else {}
+    out = rast.forward(tr.Camera(T(vm), T(K), W, H, radial=T(radial), **end), None)
+    assert torch.isfinite(out.image).all()
+    rast.backward(torch.full((H, W, 3), 1e-3, device=DEV), grads, None)
+    for name in ("means", "sh0", "shN", "scaling_raw", "rotation_raw", "opacity_raw"):
+        g = grads.tensor(name)
+        assert torch.isfinite(g).all() and g.abs().max() > 0, name
