@@ -496,6 +496,8 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
                 if (k == km) { p1[k] -= t1; p2[k] -= t2; }
         }
         const float G = f.gamma * f.gamma;
+        // camera on the centre: P = 0 along every ray (G = 0) whatever the forms; these have no common zero
+        if (!(m2 > 0.f)) { p1[0] = 1.f; p1[1] = p1[2] = 0.f; p2[1] = 1.f; p2[0] = p2[2] = 0.f; p3[0] = p3[1] = 0.f; p3[2] = 1.f; }
         rec[0] = make_float4(p1[0], p1[1], p1[2], -0.72134752044448f * G);
         // How far the exponents of the forms and of the product form can lie apart where alpha is 1/255. The rounding of M d, of some
         // 2^-24 max(1/scale) for a unit direction, moves the distance |u x g| / |u| by that times |o - mu|, and its half square by
@@ -509,11 +511,9 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         const float phi_cut = (ln_o + band) * rG, phi_max = (ln_o + fmaxf(band, 0.02f)) * rG;
         // |(e1, e2)| <= slope |w| wherever phi <= phi_max
         const float slope = phi_max >= 1.0f ? 1e30f : sqrtf(fmaxf(phi_max, 0.f) / (1.0f - phi_max));
-        box.z = __float_as_uint(m2 > 0.f ? slope : 1e30f);
+        box.z = __float_as_uint(m2 > 0.f ? slope : INFINITY);
         rec[1] = make_float4(p2[0], p2[1], p2[2], phi_cut);
-        const float alpha_cut = (1.0f / 255.0f) * __expf(fminf(band, 8.0f));
-        // camera on the centre: e1 = e2 = 0, and a form of w that no pixel ray makes zero
-        rec[2] = m2 > 0.f ? make_float4(p3[0], p3[1], p3[2], alpha_cut) : make_float4(0.6101f, 0.5303f, 0.5887f, alpha_cut);
+        rec[2] = make_float4(p3[0], p3[1], p3[2], (1.0f / 255.0f) * __expf(fminf(band, 8.0f)));
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);

@@ -245,3 +245,28 @@ def test_pixels_without_a_ray_leave_the_gradients_finite(pkg, synth, k, f, rolli
     for name in ("means", "sh0", "shN", "scaling_raw", "rotation_raw", "opacity_raw"):
         g = grads.tensor(name)
         assert torch.isfinite(g).all() and g.abs().max() > 0, name
+
+
+# A Gaussian centred on the camera answers every ray with its opacity, in front of the camera or behind it
+@pytest.mark.parametrize("fisheye", [False, True])
+def test_camera_on_the_centre(pkg, fisheye):
+    W = H = 512
+    tiles = (W // 16) * (H // 16)
+    one = lambda *v: torch.tensor([v], dtype=torch.float32, device=DEV)
+    eye = torch.eye(4, device=DEV)[None]
+    lists = dict(tile_offsets=torch.arange(tiles, dtype=torch.int32, device=DEV).view(1, H // 16, W // 16),
+                 flatten_ids=torch.zeros(tiles, dtype=torch.int32, device=DEV))
+    if fisheye:
+        lists["radial_coeffs"] = torch.zeros((1, 4), device=DEV)
+    for shift in range(2):
+        f = W / 3.5 if fisheye else W / 3.0
+        K = torch.tensor([[[f, 0, W / 2 + 0.37 * shift], [0, f, H / 2 - 0.21 * shift], [0, 0, 1]]], device=DEV)
+        front = (one(0, 0, 0), one(0.8, 0.2, -0.4, 0.4), one(0.3, 0.2, 0.1), torch.ones((1, 1, 3), device=DEV), one(0.5), None, None, W, H, 16,
+                 eye, None, K, pkg._capi.FISHEYE if fisheye else pkg._capi.PINHOLE)
+        image, alphas, last_ids = pkg.ops.rasterize_to_pixels_from_world_3dgs_fwd(*front, **lists)
+        inside = alphas > 0 if fisheye else torch.ones_like(alphas, dtype=torch.bool)   # a fisheye's corners have no ray
+        assert inside.float().mean() > 0.7 and (alphas[inside] == 0.5).all()
+        grads = pkg.ops.rasterize_to_pixels_from_world_3dgs_bwd(*front, **lists, render_alphas=alphas, last_ids=last_ids,
+                                                                v_render_colors=torch.ones_like(image), v_render_alphas=torch.zeros_like(alphas))
+        assert all(torch.isfinite(g).all() for g in grads)
+        assert (grads[0] == 0).all() and (grads[2] == 0).all()
