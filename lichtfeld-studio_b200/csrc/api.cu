@@ -283,7 +283,7 @@ int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* r
     a.sel_out = &sel;
     int rc = build_tile_lists(a, S(stream));
     if (rc != LFS_OK) return rc;
-    return launch_compose_isect_ids(n_isects, a.tkeys[sel], a.tvals[sel], depths, isect_ids, flatten_ids, S(stream));
+    return launch_compose_isect_ids(n_isects, a.tkeys[sel], a.tvals[sel], depths, a.state, isect_ids, flatten_ids, S(stream));
 }
 
 int lfs_intersect_offset(int64_t n_isects, const int64_t* isect_ids, int C, int tw, int th, int32_t* offsets, void* stream) {

@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int32_t* __r
 // One word per list tile (and digit): 0 = nothing yet, top bit clear = the tile's own count + 1, top bit set = the count of this
 // and all earlier tiles. Value and flag share the word, so relaxed accesses are enough. Tiles are numbered by a ticket, so every
 // predecessor of a tile belongs to a CTA that is already running and publishes its own count without waiting for anybody:
-// each wait ends. The poll limit only bounds the damage of a defect: it raises the overflow flag, and every store below
-// checks its position.
+// each wait ends. The poll limit only bounds the damage of a defect: it raises a flag, after which nobody reads the list, and every
+// store below checks its position.
 constexpr uint32_t kInclusive = 0x80000000u;
 constexpr int kPollLimit = 1 << 21;
 
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreads) radix_scatter_chunk_kernel(
 __global__ void __launch_bounds__(kThreads) radix_scatter_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, const int32_t* n_dev, int64_t n_max, int shift, uint32_t mask,
-    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* state, int32_t* overflow) {
+    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* state, int32_t* gave_up) {
     __shared__ uint32_t cnt[kWarps][256];   // per-warp digit counts, then per-warp start inside the tile
     __shared__ uint32_t gbase[256];         // where the items of digit d of this tile go
     __shared__ uint32_t tstart[256];        // start of digit d inside the reordered tile
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) radix_scatter_kernel(
                     --left;
                 }
                 if (++polls > kPollLimit) {
-                    if (overflow) atomicExch(overflow, 1);
+                    atomicExch(gave_up, 1);
                     break;
                 }
             }
@@ -431,8 +431,8 @@ __global__ void __launch_bounds__(kThreads) emit_instances_kernel(
     int64_t total, int N, const uint32_t* __restrict__ order, const int32_t* __restrict__ tiles,
     const float* __restrict__ means2d, const int32_t* __restrict__ radii, const ushort4* __restrict__ ewa_bounds,
     const float4* __restrict__ rec, float tile_size, uint32_t tw, uint32_t th, uint32_t tile_n_bits, int64_t capacity,
-    uint32_t* __restrict__ tkeys, uint32_t* __restrict__ tvals, int32_t* overflow, int32_t* __restrict__ n_out, uint32_t* ticket,
-    uint32_t* state) {
+    uint32_t* __restrict__ tkeys, uint32_t* __restrict__ tvals, int32_t* overflow, int32_t* gave_up, int32_t* __restrict__ n_out,
+    uint32_t* ticket, uint32_t* state) {
     constexpr int kList = kThreads * ITEMS;
     __shared__ int sm[33];
     __shared__ uint32_t s_tile, s_prefix;
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kThreads) emit_instances_kernel(
                 const int last = incl ? __ffs(incl) - 1 : 31;   // nearest predecessor whose total covers everything before it
                 if (empty & (last == 31 ? 0xffffffffu : (2u << last) - 1u)) {
                     if (++polls > kPollLimit) {
-                        if (lane == 0 && overflow) atomicExch(overflow, 1);
+                        if (lane == 0) atomicExch(gave_up, 1);
                         break;
                     }
                     continue;
@@ -588,15 +588,18 @@ __global__ void __launch_bounds__(kThreads) tile_offsets_kernel(const uint32_t* 
     }
 }
 
-// Operator-level output: 64-bit keys (camera | tile | depth bits) and int32 flattened ids.
+// Operator-level output: 64-bit keys (camera | tile | depth bits) and int32 flattened ids. A list that was given up (some of its
+// slots were never written) comes out as the largest key and id 0 throughout, beyond every tile.
 __global__ void __launch_bounds__(kThreads) compose_isect_ids_kernel(int64_t n, const uint32_t* __restrict__ tkeys,
                                                                      const uint32_t* __restrict__ tvals,
                                                                      const float* __restrict__ depths,
+                                                                     const int32_t* __restrict__ gave_up,
                                                                      int64_t* __restrict__ isect_ids,
                                                                      int32_t* __restrict__ flatten_ids) {
+    const bool failed = *gave_up != 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = tvals[i];
-        isect_ids[i] = ((int64_t)tkeys[i] << 32) | (int64_t)__float_as_uint(depths[v]);
+        const uint32_t v = failed ? 0u : tvals[i];
+        isect_ids[i] = failed ? INT64_MAX : ((int64_t)tkeys[i] << 32) | (int64_t)__float_as_uint(depths[v]);
         flatten_ids[i] = (int32_t)v;
     }
 }
@@ -668,7 +671,8 @@ int exclusive_scan_gather(const int32_t* src, const uint32_t* idx, int64_t n, in
 // Words of the list state: tickets [64] | digit counts [2 sorts][4 passes][256] | emission look-back | sort look-back. The first three
 // are zeroed by one memset per list build, the last by the histogram kernel of each sort, which knows the count.
 namespace {
-constexpr size_t kTicketWords = 64, kHistWords = 2 * 4 * 256;
+constexpr size_t kTicketWords = 64, kHistWords = 2 * 4 * 256;   // tickets: nine, and at 32 the word of list_gave_up
+int32_t* list_gave_up(uint32_t* state) { return reinterpret_cast<int32_t*>(state) + 32; }
 size_t emit_state_words(int64_t total) { return ((size_t)((total + kThreads - 1) / kThreads) + 63) / 64 * 64; }
 // Look-back serves short lists, where a sort is mostly launches (16 k keys, four passes: 42 us against 66 with separate counting
 // kernels; 250 k 51 against 68; 1 M 79 against 94); on long lists its waves of tiles queue behind one another's words and the
@@ -699,7 +703,7 @@ size_t tile_list_state_words(int64_t total, int64_t capacity, int key_bits) {
 // (device-side count, bounded by n_max), else n_max is the count. Returns the index (0 or 1) of the pair holding the result.
 // tickets [4], hist [4 * 256]: zero on entry. state: sort_state_words.
 static int radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], const int32_t* n_dev, int64_t n_max, int key_bits,
-                            uint32_t* tickets, uint32_t* hist, uint32_t* state, int32_t* overflow, cudaStream_t st) {
+                            uint32_t* tickets, uint32_t* hist, uint32_t* state, int32_t* gave_up, cudaStream_t st) {
     if (n_max <= 0 || key_bits <= 0) return 0;
     const int passes = tile_sort_passes(key_bits);
     const int bits = (key_bits + passes - 1) / passes;
@@ -715,7 +719,7 @@ static int radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], const int32_t*
         for (int p = 0; p < passes; ++p) {
             radix_scatter_kernel<<<nb, kThreads, 0, st>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n_dev, n_max,
                                                                  p * bits, mask, hist + p * 256, tickets + p,
-                                                                 state + (size_t)p * max_tiles * 256, overflow);
+                                                                 state + (size_t)p * max_tiles * 256, gave_up);
             cur ^= 1;
         }
     } else {
@@ -751,6 +755,9 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
     const int key_bits = (int)(tile_n_bits + cam_n_bits);
     uint32_t *tickets = a.state, *hist = tickets + kTicketWords, *emit_state = hist + kHistWords;
     uint32_t* sort_state = emit_state + emit_state_words(total);
+    // raised by a look-back that ran out of polls; without an overflow flag of the caller's a word behind the tickets, read by
+    // compose_isect_ids_kernel
+    int32_t* gave_up = a.overflow ? a.overflow : list_gave_up(a.state);
     cudaMemsetAsync(a.state, 0, (kTicketWords + kHistWords + emit_state_words(total)) * sizeof(uint32_t), st);
     const uint32_t* order = nullptr;
     if (a.sort) {
@@ -759,7 +766,7 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
         }
         uint32_t* k[2] = {a.gkeys[0], a.gkeys[1]};
         uint32_t* v[2] = {a.gvals[0], a.gvals[1]};
-        const int sel = radix_sort_pairs(k, v, nullptr, total, 32, tickets, hist, sort_state, a.overflow, st);
+        const int sel = radix_sort_pairs(k, v, nullptr, total, 32, tickets, hist, sort_state, gave_up, st);
         if (sel < 0) return LFS_ECUDA;
         order = v[sel];
     }
@@ -774,7 +781,7 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
 #define LFS_EMIT(EWA, ITEMS)                                                                                                                 \
     emit_instances_kernel<EWA, ITEMS><<<nb, kThreads, 0, st>>>(total, a.N, order, a.tiles, a.means2d, a.radii, a.ewa_bounds, a.ewa_records,    \
                                                         (float)a.tile_size, (uint32_t)a.tw, (uint32_t)a.th, tile_n_bits, a.capacity,   \
-                                                        a.tkeys[0], a.tvals[0], a.overflow, a.n_isects_dev, tickets + 8, emit_state)
+                                                        a.tkeys[0], a.tvals[0], a.overflow, gave_up, a.n_isects_dev, tickets + 8, emit_state)
         if (a.ewa_bounds) { if (four) LFS_EMIT(true, kEmitItems); else LFS_EMIT(true, 1); }
         else { if (four) LFS_EMIT(false, kEmitItems); else LFS_EMIT(false, 1); }
 #undef LFS_EMIT
@@ -785,7 +792,7 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
     if (a.sort && a.capacity > 0) {
         uint32_t* k[2] = {a.tkeys[0], a.tkeys[1]};
         uint32_t* v[2] = {a.tvals[0], a.tvals[1]};
-        sel = radix_sort_pairs(k, v, a.n_isects_dev, a.capacity, key_bits, tickets + 4, hist + 4 * 256, sort_state, a.overflow, st);
+        sel = radix_sort_pairs(k, v, a.n_isects_dev, a.capacity, key_bits, tickets + 4, hist + 4 * 256, sort_state, gave_up, st);
         if (sel < 0) return LFS_ECUDA;
     }
     if (a.sel_out) *a.sel_out = sel;
@@ -833,10 +840,11 @@ int launch_tile_order(int n_tiles, const int32_t* offsets, int32_t* order, cudaS
     return check_launch("tile_order");
 }
 
-int launch_compose_isect_ids(int64_t n, const uint32_t* tkeys, const uint32_t* tvals, const float* depths,
+int launch_compose_isect_ids(int64_t n, const uint32_t* tkeys, const uint32_t* tvals, const float* depths, const uint32_t* list_state,
                              int64_t* isect_ids, int32_t* flatten_ids, cudaStream_t st) {
     if (n <= 0) return LFS_OK;
-    compose_isect_ids_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, tkeys, tvals, depths, isect_ids, flatten_ids);
+    compose_isect_ids_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, tkeys, tvals, depths, list_gave_up(const_cast<uint32_t*>(list_state)), isect_ids,
+                                                                flatten_ids);
     return check_launch("compose_isect_ids");
 }
 

@@ -36,10 +36,9 @@ size_t tile_list_state_words(int64_t total, int64_t capacity, int key_bits);
 
 // order [n_tiles]: tile indices, longest lists first; offsets [n_tiles + 1]
 int launch_tile_order(int n_tiles, const int32_t* offsets, int32_t* order, cudaStream_t st);
-int launch_compose_isect_ids(int64_t n, const uint32_t* tkeys, const uint32_t* tvals, const float* depths,
+int launch_compose_isect_ids(int64_t n, const uint32_t* tkeys, const uint32_t* tvals, const float* depths, const uint32_t* list_state,
                              int64_t* isect_ids, int32_t* flatten_ids, cudaStream_t st);
 int launch_isect_offset(int64_t n, const int64_t* isect_ids, int C, int tw, int th, int32_t* offsets, cudaStream_t st);
-int launch_total_to_i64(const int32_t* total, int64_t* out, cudaStream_t st);
 int launch_sum_i32(int64_t n, const int32_t* src, int64_t* out_dev, cudaStream_t st);
 
 }  // namespace lfs

@@ -153,3 +153,10 @@ def test_fewer_gaussians_than_the_workspace_was_made_for(pkg, synth, ewa):
         exact.tensor(name).copy_(model.tensor(name))
     assert torch.isfinite(image).all() and image.abs().max() > 0.1
     assert torch.equal(image, make(exact).forward(cam, bg).image)
+
+
+# What the list build leaves when it gives up: the largest key throughout. Its offsets are empty lists for every tile.
+@pytest.mark.parametrize("n,C,tw,th", [(1, 1, 3, 2), (5000, 1, 81, 53), (300, 3, 7, 5)])
+def test_offsets_of_a_list_that_was_given_up(pkg, n, C, tw, th):
+    ids = torch.full((n,), torch.iinfo(torch.int64).max, dtype=torch.int64, device=DEV)
+    assert (pkg.ops.intersect_offset(ids, C, tw, th) == 0).all()
