@@ -107,9 +107,8 @@ struct SortScratch {
 // Capacity of the scratch array; the launches use min(4 x SM count, capacity) blocks.
 constexpr int kScanBlocks = 1024;
 
-// out[i] = exclusive prefix sum of gather(i) = src[idx ? idx[i] : i]; total written to *total_dev.
-int exclusive_scan_gather(const int32_t* src, const uint32_t* idx, int64_t n, int32_t* out, int32_t* total_dev,
-                          const SortScratch& scratch, cudaStream_t st);
+// out[i] = exclusive prefix sum of src; total written to *total_dev.
+int exclusive_scan(const int32_t* src, int64_t n, int32_t* out, int32_t* total_dev, const SortScratch& scratch, cudaStream_t st);
 
 // One 16-byte store to an NVSwitch multicast address: the switch writes it into the same offset of every GPU bound to the
 // multicast object (this GPU included), so a broadcast leaves this GPU's NVLink ports once instead of once per peer.

@@ -575,7 +575,7 @@ int launch_mcmc_classify(int N, const float* opacity_raw, const float* rotation_
                          int32_t* total_dev, const SortScratch& s, cudaStream_t st) {
     if (N == 0) { cudaMemsetAsync(counts_dev, 0, 2 * sizeof(int32_t), st); return LFS_OK; }
     mcmc_flags_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, opacity_raw, rotation_raw, min_opacity, flags);
-    const int rc = exclusive_scan_gather(flags, nullptr, N, offs, total_dev, s, st);
+    const int rc = exclusive_scan(flags, N, offs, total_dev, s, st);
     if (rc != LFS_OK) return rc;
     mcmc_compact_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, flags, offs, total_dev, opacity_raw, dead_indices, alive_indices,
                                                           alive_opacities, counts_dev);

@@ -62,12 +62,11 @@ __device__ __forceinline__ int64_t device_count(const int32_t* n_dev, int64_t n_
 }
 
 // ---- prefix sum -----------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) scan_reduce_kernel(const int32_t* __restrict__ src, const uint32_t* __restrict__ idx,
-                                                               int64_t n, int64_t chunk, uint32_t* __restrict__ block_sums) {
+__global__ void __launch_bounds__(kThreads) scan_reduce_kernel(const int32_t* __restrict__ src, int64_t n, int64_t chunk, uint32_t* __restrict__ block_sums) {
     __shared__ int sm[33];
     const int64_t lo = (int64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
     int s = 0;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) s += idx ? src[idx[i]] : src[i];
+    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) s += src[i];
     int total;
     block_excl_scan(s, total, sm);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = (uint32_t)total;
@@ -91,15 +90,14 @@ __global__ void __launch_bounds__(1024) scan_block_sums_kernel(uint32_t* __restr
     if (threadIdx.x == 0 && total_dev) *total_dev = carry;
 }
 
-__global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int32_t* __restrict__ src, const uint32_t* __restrict__ idx,
-                                                              int64_t n, int64_t chunk, const uint32_t* __restrict__ block_sums,
+__global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int32_t* __restrict__ src, int64_t n, int64_t chunk, const uint32_t* __restrict__ block_sums,
                                                               int32_t* __restrict__ out) {
     __shared__ int sm[33];
     const int64_t lo = (int64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
     int carry = (int)block_sums[blockIdx.x];
     for (int64_t base = lo; base < hi; base += kThreads) {
         const int64_t i = base + threadIdx.x;
-        const int v = i < hi ? (idx ? src[idx[i]] : src[i]) : 0;
+        const int v = i < hi ? src[i] : 0;
         int total;
         const int ex = block_excl_scan(v, total, sm);
         if (i < hi) out[i] = carry + ex;
@@ -640,8 +638,6 @@ __global__ void depth_keys_kernel(int64_t total, const float* __restrict__ depth
     }
 }
 
-__global__ void total_to_i64_kernel(const int32_t* total, int64_t* out) { *out = (int64_t)*total; }
-
 __global__ void __launch_bounds__(kThreads) sum_i32_kernel(int64_t n, const int32_t* __restrict__ src, unsigned long long* out) {
     long long s = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) s += src[i];
@@ -652,8 +648,7 @@ __global__ void __launch_bounds__(kThreads) sum_i32_kernel(int64_t n, const int3
 
 }  // namespace
 
-int exclusive_scan_gather(const int32_t* src, const uint32_t* idx, int64_t n, int32_t* out, int32_t* total_dev,
-                          const SortScratch& s, cudaStream_t st) {
+int exclusive_scan(const int32_t* src, int64_t n, int32_t* out, int32_t* total_dev, const SortScratch& s, cudaStream_t st) {
     if (n <= 0) {
         if (total_dev) cudaMemsetAsync(total_dev, 0, sizeof(int32_t), st);
         return LFS_OK;
@@ -662,9 +657,9 @@ int exclusive_scan_gather(const int32_t* src, const uint32_t* idx, int64_t n, in
     nb = min(nb, min(4 * num_sms(), kScanBlocks));
     const int64_t chunk = (n + nb - 1) / nb;
     LFS_TIMED("exclusive_scan", st);
-    scan_reduce_kernel<<<nb, kThreads, 0, st>>>(src, idx, n, chunk, s.block_sums);
+    scan_reduce_kernel<<<nb, kThreads, 0, st>>>(src, n, chunk, s.block_sums);
     scan_block_sums_kernel<<<1, 1024, 0, st>>>(s.block_sums, nb, total_dev);
-    scan_apply_kernel<<<nb, kThreads, 0, st>>>(src, idx, n, chunk, s.block_sums, out);
+    scan_apply_kernel<<<nb, kThreads, 0, st>>>(src, n, chunk, s.block_sums, out);
     return check_launch("exclusive_scan");
 }
 
@@ -860,11 +855,6 @@ int launch_sum_i32(int64_t n, const int32_t* src, int64_t* out_dev, cudaStream_t
     cudaMemsetAsync(out_dev, 0, sizeof(int64_t), st);
     if (n > 0) sum_i32_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, src, reinterpret_cast<unsigned long long*>(out_dev));
     return check_launch("sum_i32");
-}
-
-int launch_total_to_i64(const int32_t* total, int64_t* out, cudaStream_t st) {
-    total_to_i64_kernel<<<1, 1, 0, st>>>(total, out);
-    return check_launch("total_to_i64");
 }
 
 }  // namespace lfs
