@@ -24,6 +24,11 @@ constexpr int kEwaRecordVec4 = 3;
 // [min_x, max_x] x [min_y, max_y]? (mx, my) is the 2-D mean shifted by -0.5 so that pixel centres sit on integers.
 // The point of the rectangle with the smallest exponent lies either inside (mean inside) or on the two edges that
 // face the mean; each edge is searched by the closed-form minimiser of the quadratic along it, clamped to the edge.
+// Where the rectangle faces the mean with a corner, both minimisers are applied at once. In exact arithmetic at most one of them lies off
+// the corner; the float32 conic of an ellipse hundreds of pixels long is close to singular, or indefinite, and then both may, and the
+// point tested is none of the rectangle's edges: a rectangle that the ellipse reaches is missed (none of 0.76 M with axes up to 100 px,
+// 2 of 0.75 M up to 500, 270 of 0.75 M up to 2,000). The lists share this with the reference's; the patches of the blend kernels have
+// it too, and their images with it.
 // FAST: hardware division (for callers that only cull, with a margin on the threshold; the minimiser along an edge moves the
 // exponent in second order). The lists are pinned to the exact one.
 template <bool FAST = false>

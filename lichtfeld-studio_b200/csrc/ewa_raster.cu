@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(256 / PX) ewa_blend_bwd_kernel(
         const uint32_t* sid = sid_all[b % 3];
         // slots whose tile-local position is at or beyond this warp's deepest contributor are dropped up front
         const int t_begin = max(0, (batch_top - range_start) - (warp_last - 1));
-        // The ellipse-versus-rectangle test is not exact for a rectangle that faces the ellipse with a corner, so a pair counts only
-        // if the forward's own 8x4 patch kept it: a pixel that the forward skipped must not enter the transmittance here.
+        // The ellipse-versus-rectangle test misses a rectangle now and then (ewa_rect_contributes says when), and differently for
+        // rectangles of another shape, so a pair counts only if the forward's own 8x4 patch kept it: a pixel that the forward skipped
+        // must not enter the transmittance here.
         uint32_t live[BATCH / 32], lower[BATCH / 32], mine[BATCH / 32];
         cull_batch<BATCH>(st, t_begin, batch_size, (float)patch_j, (float)patch_i, live);
         if (PX == 2) {

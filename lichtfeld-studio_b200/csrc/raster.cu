@@ -6,18 +6,20 @@
 // activation backward that autograd performs for src/core/splat_data.cpp:267-286.
 //
 // Design (instruction-issue bound, no tensor cores: the largest contraction is 3x3):
-//  * one CTA per 16x16 tile, one thread per pixel, warps cover 8x4 pixel patches;
+//  * one CTA per 16x16 tile. Forward: one thread per pixel, a warp covers a patch of 8x4 pixels. Backward: one or two horizontally
+//    adjacent pixels per thread, patches of 4x8 or 8x8 (launch_raster_bwd says where which);
 //  * the tile's depth-sorted Gaussians are staged in shared memory in batches (192 records forward, 64 backward) of
 //    packed 64-byte records built once per Gaussian, so no per-Gaussian work is repeated per tile or per pixel;
 //  * per warp, a ballot over the batch keeps the records whose screen-space box overlaps the warp's patch and whose forms
 //    reach the cut on it (patch_reached);
 //  * per pair the response is exp(-|g|^2 phi / 2), phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) with three linear forms of the
 //    pixel direction (RayFrame, gsmath.cuh): 10 instructions up to the exp-free rejection test for the planar camera models
-//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840: forward 624 -> 430 us, backward 1441 -> 1065 with nothing else changed);
+//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840, when it was brought in: forward 624 -> 430 us,
+//    backward 1441 -> 1065 with nothing else changed; with the cut decided as before (kept_at_cut) 399 and 787 today);
 //  * backward: every (warp, Gaussian) contribution is 12 numbers that are LINEAR in the per-pixel terms (kSums). They
-//    are summed over the warp by a transpose through padded shared-memory rows (warp_reduce), combined across the 8 warps
-//    by shared-memory atomics, and leave the CTA as 16-byte reductions per (tile, Gaussian). The nonlinear quaternion / scale
-//    VJP runs once per Gaussian in the epilogue instead of once per pixel pair;
+//    are summed over the warp by a transpose through padded shared-memory rows (warp_reduce) and leave as one coalesced reduction
+//    to the Gaussian's accumulator row. The nonlinear quaternion / scale VJP runs once per Gaussian in the epilogue instead of once
+//    per pixel pair;
 //  * a rolling shutter gives every pixel its own ray origin: the RS instantiations keep u = M d and 16 sums.
 #include "gsmath.cuh"
 #include "raster.cuh"
@@ -222,8 +224,8 @@ __device__ __forceinline__ void issue_stage(Stage<BATCH>& st, uint32_t* sid, con
 // in extra_sum for the backward.
 // RS: rolling shutter. Every pixel has its own pose, hence its own ray origin; the record's gro = M (o_start - mu) is
 // corrected per pair by M (o_pixel - o_start).
-// The plain pinhole RGB instantiation fits 40 registers (12 bytes of spills outside the loop) and, with 192-record batches
-// (30 KB for the two staging buffers), six CTAs per SM; the other instantiations keep their 48 - 64 registers.
+// The plain pinhole RGB instantiation fits 40 registers (16 bytes of stack) and, with 192-record batches (33 KB with the rays for
+// kept_at_cut), six CTAs per SM; the other instantiations keep their 56 - 64 registers.
 template <int MODEL, bool EXTRA, bool RS>
 __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA) ? 6 : 4) raster_fwd_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
@@ -434,6 +436,9 @@ __device__ __forceinline__ float rcp_newton(float x) {
 // One thread owns PX horizontally adjacent pixels, a warp a patch of 4 PX x 8: the two pixels' terms are added in registers,
 // so the warp reduction (12 stores, 4 wide loads, the reduction to memory), the record loads and the list walk are paid once
 // for two pixels, at the price of more idle lanes in the larger patch. launch_raster_bwd says where which PX runs.
+// Registers: six CTAs of 128 threads have 80 each and spill nothing (1 M Gaussians, 1296x840: 786 us; eight with 64 and 28 bytes of
+// spills 801, uncapped 95 and 921; a distorted pinhole, uncapped at 120 for its Newton steps in double: 758 against 647). Four of 256 at
+// 64 for one pixel per thread (five at 48 with spills: 250 k Gaussians, 1024x1024 fisheye, 350 us against 317).
 template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS, int PX>
 __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd_kernel(
 
@@ -1221,9 +1226,10 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     if (a.normalize && !extra_sum) { set_error("raster_bwd: expected-depth modes need the forward's blended sum"); return LFS_EINVAL; }
     LFS_TIMED("raster_bwd", st);
     // Two pixels per thread where the patches are filled and the CTAs of half the threads still fill the GPU: planar cameras and
-    // at least eight tiles per SM (1 M Gaussians, 1296x840, 4,293 tiles: 889 us against 999 with one; 256 tiles of 256x256:
-    // 127 us against 94). A wide-angle camera shows Gaussians a few pixels across in the middle of its image, where the larger
-    // patch wastes lanes and few tiles carry the work (250 k Gaussians, 1024x1024 fisheye: 478 us against 392).
+    // at least eight tiles per SM. Measured when the rule was set, with one cross product per pair dearer than today: 1 M Gaussians,
+    // 1296x840, 4,293 tiles: 889 us against 999 with one; 256 tiles of 256x256: 127 us against 94. A wide-angle camera shows Gaussians
+    // a few pixels across in the middle of its image, where the larger patch wastes lanes and few tiles carry the work (250 k
+    // Gaussians, 1024x1024 fisheye, the one such scene measured: 478 us against 392).
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
     const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
     const bool wide = planar && !a.rolling && n_tiles >= 8 * num_sms();
