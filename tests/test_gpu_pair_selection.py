@@ -270,3 +270,30 @@ def test_camera_on_the_centre(pkg, fisheye):
                                                                 v_render_colors=torch.ones_like(image), v_render_alphas=torch.zeros_like(alphas))
         assert all(torch.isfinite(g).all() for g in grads)
         assert (grads[0] == 0).all() and (grads[2] == 0).all()
+
+
+# Large Gaussians close to a strongly distorted pinhole, image and gradients: the backward's patches have another shape than the forward's
+@pytest.mark.parametrize("k,f,dist,grow", [([-0.3, 0.12, -0.02, 0.01, 0.0, 0.0], 90.0, 1.5, 0.8), ([0.25, 0.05, 0.0, 0.0, 0.02, 0.0], 120.0, 2.2, 0.3),
+                                           ([-0.2, 0.05, 0.0, 0.0, 0.0, 0.0], 300.0, 1.2, 1.0)])
+def test_distorted_pinhole_close_to_a_scene(pkg, orc, synth, k, f, dist, grow):
+    tr = pkg.trainer
+    n, W, H, deg = 6000, 308, 236, 1
+    P = synth.make_gaussians(n, 3, "cube", deg)
+    P["scaling_raw"] = (P["scaling_raw"] + np.float32(grow)).astype(np.float32)
+    vm = synth.look_at_origin([0.3, -dist, 0.4])
+    K = synth.intrinsics(f, f * 0.97, W / 2 + 5.0, H / 2 - 3.0)
+    radial, tangential = np.array(k, np.float32), np.array([1e-3, -5e-4], np.float32)
+    packed = orc.pack_distortion(radial=radial, tangential=tangential)
+    fwd = orc.render_fwd(P, vm, K, W, H, deg, radial=packed)
+    model = tr.SplatData(n, (deg + 1) ** 2, DEV).load(P)
+    grads = model.like()
+    rast = tr.Rasterizer(model, W, H, deg)
+    out = rast.forward(tr.Camera(T(vm), T(K), W, H, radial=T(radial), tangential=T(tangential)), None)
+    diff = np.abs(out.image.cpu().numpy() - fwd["render"]).max(-1)
+    assert diff.max() < 8e-3 and (diff > 1e-4).sum() <= 20, (diff.max(), (diff > 1e-4).sum())   # pairs at the cut, as above
+    rng = np.random.default_rng(1)
+    v_r, v_a = (rng.normal(size=(H, W, c)).astype(np.float32) * 1e-3 for c in (3, 1))
+    bwd = orc.render_bwd(P, fwd, vm, K, W, H, deg, v_r, v_a, radial=packed)
+    rast.backward(T(v_r), grads, None, T(v_a))
+    for name in ("means", "sh0", "shN", "scaling_raw", "rotation_raw", "opacity_raw"):
+        assert rel_l2(grads.tensor(name).cpu().numpy(), bwd[name]) < 2e-3, name
