@@ -610,7 +610,8 @@ int launch_pack_records(int N, const float* means, const float* quats, const flo
 // Bound by instruction issue and the latency of the per-Gaussian chain, not by memory: 64 registers and four CTAs per SM for the
 // models that project in single precision (1 M Gaussians 127 us against 135 with three CTAs, 6 M at 4K 655 against 720); the
 // fisheye evaluates seven double-precision arc tangents per Gaussian and wants its 128 registers instead (6 M: 1120 us against
-// 1176 with three CTAs and 1249 with four).
+// 1176 with three CTAs and 1249 with four). Since the cut record (48 bytes and some 30 instructions per visible Gaussian) 136 and
+// 697 us; the fisheye, with its box for either side of the camera too, 1329.
 template <int MODEL, bool RS>
 __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pack_kernel(
     int N, int K, int sh_degree, const float* __restrict__ means, const float* __restrict__ sh0,
