@@ -1226,10 +1226,11 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     if (a.normalize && !extra_sum) { set_error("raster_bwd: expected-depth modes need the forward's blended sum"); return LFS_EINVAL; }
     LFS_TIMED("raster_bwd", st);
     // Two pixels per thread where the patches are filled and the CTAs of half the threads still fill the GPU: planar cameras and
-    // at least eight tiles per SM. Measured when the rule was set, with one cross product per pair dearer than today: 1 M Gaussians,
-    // 1296x840, 4,293 tiles: 889 us against 999 with one; 256 tiles of 256x256: 127 us against 94. A wide-angle camera shows Gaussians
-    // a few pixels across in the middle of its image, where the larger patch wastes lanes and few tiles carry the work (250 k
-    // Gaussians, 1024x1024 fisheye, the one such scene measured: 478 us against 392).
+    // at least eight tiles per SM. 4,293 tiles (1 M Gaussians, 1296x840) 787 us against 992 with one pixel; 2,170 (120 k, 979x547) 241
+    // against 306; 1,080 (250 k, 640x427, the other side of the line, which could lie lower) 302 against 335; 256 (16 k, 256x256) 111
+    // against 88. A wide-angle camera shows Gaussians a few pixels across in the middle of its image, where the larger patch wastes lanes
+    // and few tiles carry the work (250 k Gaussians, 1024x1024 fisheye, the one such scene measured, with earlier kernels: 478 us against
+    // 392).
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
     const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
     const bool wide = planar && !a.rolling && n_tiles >= 8 * num_sms();

@@ -272,8 +272,9 @@ def test_camera_on_the_centre(pkg, fisheye):
         assert (grads[0] == 0).all() and (grads[2] == 0).all()
 
 
-# Large Gaussians close to a strongly distorted pinhole, image and gradients: the backward's patches have another shape than the forward's
-@pytest.mark.parametrize("k,f,dist,grow", [([-0.3, 0.12, -0.02, 0.01, 0.0, 0.0], 90.0, 1.5, 0.8), ([0.25, 0.05, 0.0, 0.0, 0.02, 0.0], 120.0, 2.2, 0.3),
+# Large Gaussians close to a strongly distorted pinhole, image and gradients: the backward's patches have another shape than the forward's.
+# Every pixel's ray converges: where the inversion hardly does, fused operations decide whether a pixel has one.
+@pytest.mark.parametrize("k,f,dist,grow", [([-0.3, 0.12, -0.02, 0.01, 0.0, 0.0], 200.0, 1.5, 0.8), ([0.25, 0.05, 0.0, 0.0, 0.02, 0.0], 120.0, 2.2, 0.3),
                                            ([-0.2, 0.05, 0.0, 0.0, 0.0, 0.0], 300.0, 1.2, 1.0)])
 def test_distorted_pinhole_close_to_a_scene(pkg, orc, synth, k, f, dist, grow):
     tr = pkg.trainer
