@@ -767,10 +767,10 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
     }
     if (total > 0) {
         LFS_TIMED("emit_instances", st);
-        // Four Gaussians per thread make fewer tickets and a shorter look-back, one makes more CTAs in flight. Measured: 400 k 30 us
-        // with one against 60 with four, 1 M 50 against 63, 3 M 149 against 125, 6 M (all visible) 265 against 203; EWA, whose
-        // rectangle walk is longer than the scan: 60 k 31 against 80, 1 M 118 against 103.
-        const bool four = total > (a.ewa_bounds ? (int64_t)300000 : (int64_t)2 << 20);
+        // Four Gaussians per thread make fewer tickets and a shorter look-back, one makes more CTAs in flight. us with one and with four,
+        // 1296x840 (in thousands of Gaussians): 450: 33 / 57, 1000: 54 / 71, 1500: 69 / 66, 2000: 93 / 76, 3000: 137 / 118. EWA, whose
+        // rectangle walk is longer than the scan: 300: 58 / 133, 450: 67 / 111, 700: 99 / 124, 1000: 123 / 107, 2000: 259 / 185.
+        const bool four = total > (a.ewa_bounds ? (int64_t)850000 : (int64_t)2 << 20);
         const int64_t list = four ? kThreads * kEmitItems : kThreads;
         const int nb = (int)min((total + list - 1) / list, (int64_t)8 * num_sms());
 #define LFS_EMIT(EWA, ITEMS)                                                                                                                 \
