@@ -613,10 +613,8 @@ def run_ours(args):
         small = dp_self_check(pkg, dev, rank, world, args.dp_mode, dp_split, dp_rank1, args.dp_ordering, args.dp_multicast, args.dp_color_after_projection)
         dp_check = {"ok": bool(same_params and small["ok"]), "bench_parameters_identical_on_all_ranks": bool(same_params), **small}
     if rank == 0:
-        # launches inside one call that are not individually bracketed: a short list is sorted by a histogram kernel and one kernel per
-        # pass, a long one by three per pass (four passes over the depths, two over the tiles)
-        per_step_kernels = {"radix_sort_depth": 5 if n <= 2 << 20 else 12, "radix_sort_tile": 3 if rast.cfg.isect_capacity <= 6 << 20 else 6}
-        gpu_launches_step = sum(per_step_kernels.get(k, 1) * len(vs) / n_prof for k, vs in kernels.items()) + 4
+        # every bracket holds one launch; camera set-up and the loss' last kernel have none
+        gpu_launches_step = sum(len(vs) / n_prof for vs in kernels.values()) + 2
         st = rast.state()
         last, offs = st["last_ids"].long(), st["tile_offsets"].long()
         tw = (W + 15) // 16
@@ -660,7 +658,7 @@ def run_ours(args):
             adam_kernel = "adam_sh_rank1_kernel"
             adam_note = f"(24 B x {rest} shN floats + 24 B) x {n} Gaussians"
         adam_gbs = adam_bytes / (t_adam * 1e-3) / 1e9 if np.isfinite(t_adam) else None   # N > 1: Adam runs inside the exchange
-        list_keys = ("radix_sort_depth", "exclusive_scan", "emit_instances", "radix_sort_tile", "tile_offsets", "tile_order")
+        list_keys = ("tile_scan", "tile_scatter", "tile_sort")
         t_lists = sum(float(np.sum(kernels[k])) / calls for k in list_keys if k in kernels)
         V, I = float(status[2]), float(status[1])
         tiles = ((W + 15) // 16) * ((H + 15) // 16)
@@ -675,7 +673,7 @@ def run_ours(args):
                                          "frac": ach_fwd / fp32_peak if ncu else None,
                                          "reference_arithmetic": 70.0 * q_list / (t_fwd * 1e-3) / 1e12,
                                          "note": f"executed flops from the profiler capture; reference_arithmetic: 70 flop x {q_list} list entries x pixels (upper bound of pairs visited), may exceed the peak"},
-                 "roofline_tile_lists": {"kernel": "depth sort + scan + emit + tile sort + offsets + order", "bound": "hbm",
+                 "roofline_tile_lists": {"kernel": "tile_scan + tile_scatter + tile_sort", "bound": "hbm",
                                          "achieved": list_bytes / (t_lists * 1e-3) / 1e9 if t_lists else None, "peak": hbm_peak, "unit": "GB/s",
                                          "frac": list_bytes / (t_lists * 1e-3) / 1e9 / hbm_peak if t_lists else None, "ms": t_lists,
                                          "note": f"20 V + 36 I + 4 tiles bytes, of {peak_kind}"},
@@ -840,7 +838,7 @@ def run_forward_only(args):
     torch.cuda.synchronize()
     km = {k: float(np.mean(v)) for k, v in _kernel_means(capi.profile_collect()).items()}
     capi.profile_enable(False)
-    sort_ms = sum(km.get(k, 0.0) for k in ("radix_sort_depth", "exclusive_scan", "emit_instances", "radix_sort_tile", "tile_offsets"))
+    sort_ms = sum(km.get(k, 0.0) for k in ("tile_scan", "tile_scatter", "tile_sort"))
     hbm_peak, kind = load_peaks()
     V, I = float(np.mean(n_vis)), float(np.mean(n_isects))
     tiles = ((W + 15) // 16) * ((H + 15) // 16)
@@ -850,11 +848,11 @@ def run_forward_only(args):
            "data": "synthetic", "config": {"workload": args.workload, "gaussians": n, "image": [W, H], "poses": len(cams),
                                            "camera": "fisheye" if cfg["model"] == 2 else "pinhole"},
            "clocks": clocks, "n_isects_mean": I, "n_isects_max": int(np.max(n_isects)), "n_visible_mean": V, "tile_list_ms": sort_ms,
-           "kernel_ms": km, "gpu_launches": int(reps * len(cams) * 30),
-           "roofline": {"kernel": "tile-list stage (radix_* + scan_* + emit + offsets)", "bound": "hbm",
+           "kernel_ms": km, "gpu_launches": int(reps * len(cams) * 6),
+           "roofline": {"kernel": "tile-list stage (scan + scatter + sort)", "bound": "hbm",
                         "achieved": sort_bytes / (sort_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                         "frac": sort_bytes / (sort_ms * 1e-3) / 1e9 / hbm_peak, "traffic": None,
-                        "note": f"20 V + 36 I + 4 tiles bytes, of {kind}; 21 launches, launch-latency bound at this size"}}
+                        "note": f"20 V + 36 I + 4 tiles bytes, of {kind}; three launches"}}
     print(json.dumps(_finite(out)), flush=True)
 
 
@@ -923,7 +921,7 @@ def run_ewa(args):
            "dtype": "f32", "data": "synthetic",
            "config": {"workload": "ewa_1m", "gaussians": n, "image": [W, H], "sh_degree": deg, "path": "default (non --gut) EWA rasterizer",
                       "l2": "inputs larger than L2 (parameters, moments and gradients streamed per step)"},
-           "clocks": clocks, "n_instances": int(st[1]), "n_visible": int(st[2]), "kernel_ms": km, "gpu_launches": int(args.steps * 36),
+           "clocks": clocks, "n_instances": int(st[1]), "n_visible": int(st[2]), "kernel_ms": km, "gpu_launches": int(args.steps * 12),
            "roofline": {"kernel": "adam_groups_kernel", "bound": "hbm", "achieved": adam_bytes / (t_adam * 1e-3) / 1e9, "peak": hbm_peak,
                         "unit": "GB/s", "frac": adam_bytes / (t_adam * 1e-3) / 1e9 / hbm_peak, "traffic": None,
                         "note": f"the blend kernels are instruction-issue bound; the streaming kernel shown is Adam, of {kind}"}}

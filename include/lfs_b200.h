@@ -103,8 +103,7 @@ size_t lfs_intersect_tile_workspace_bytes(int C, int N, int64_t n_isects);
 /* gsplat/Ops.h:28-38 intersect_tile, second pass + sort (gsplat/Intersect.cpp:79-121,
  * gsplat/IntersectTile.cu:290-328). isect_ids [n_isects] int64 and flatten_ids [n_isects] int32 come
  * out in the order a stable ascending radix sort of the (camera | tile | depth-bits) key gives.
- * With sort == 0 they are written in emission order. Every isect_id INT64_MAX and every flatten_id 0: the list could not be
- * built (a wait inside the sort ran out, which a sound device does not let happen). */
+ * With sort == 0 they are written in emission order. */
 int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* radii, const float* depths,
                             const int32_t* tiles_per_gauss, int tile_size, int tile_width, int tile_height,
                             int sort, int64_t n_isects, int64_t* isect_ids, int32_t* flatten_ids,

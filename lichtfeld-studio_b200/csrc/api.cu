@@ -40,15 +40,6 @@ struct Carver {
     size_t total() const { return (off + 255) & ~(size_t)255; }
 };
 
-uint32_t bit_width_u32(uint32_t v) {
-    uint32_t b = 0;
-    while (v) { ++b; v >>= 1; }
-    return b;
-}
-
-// which buffer of a ping-pong pair holds the result after sorting key_bits bits
-int sorted_sel(int key_bits) { return ((key_bits + 7) / 8) & 1; }
-
 SortScratch carve_scratch(Carver& c) {
     SortScratch s;
     s.block_sums = c.take<uint32_t>(kScanBlocks + 1);
@@ -59,12 +50,13 @@ SortScratch carve_scratch(Carver& c) {
 struct RenderWs {
     CamDev* cam;
     int32_t* counters;  // [0] overflow, [1] n_isects, [2] n_visible
-    int32_t *radii, *tiles, *tile_offsets, *last_ids, *tile_order;
+    int32_t *radii, *tiles, *tile_offsets, *last_ids, *flatten_ids;
     float *means2d, *depths, *accum, *extra_sum;
     float4 *records, *cuts;
     uint4* bounds;
-    uint32_t *gkeys[2], *gvals[2], *tkeys[2], *tvals[2];
-    uint32_t* list_state;
+    uint64_t* entries;
+    int32_t* list_state;
+    const int32_t* tile_order;
     size_t bytes;
 };
 
@@ -81,17 +73,17 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
     w.means2d = c.take<float>(N * 2);
     w.depths = c.take<float>(N);
     w.tiles = c.take<int32_t>(N);
-    for (int k = 0; k < 2; ++k) { w.gkeys[k] = c.take<uint32_t>(N); w.gvals[k] = c.take<uint32_t>(N); }
     w.records = c.take<float4>(N * 4);
     w.cuts = c.take<float4>(N * 3);
     w.bounds = c.take<uint4>(N);
     w.accum = c.take<float>(N * 16);
-    for (int k = 0; k < 2; ++k) { w.tkeys[k] = c.take<uint32_t>(cap); w.tvals[k] = c.take<uint32_t>(cap); }
+    w.entries = c.take<uint64_t>(cap);
+    w.flatten_ids = c.take<int32_t>(cap);
     w.tile_offsets = c.take<int32_t>((size_t)tw * th + 1);
-    w.tile_order = c.take<int32_t>((size_t)tw * th);
     w.last_ids = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
     w.extra_sum = c.take<float>((size_t)cfg.image_width * cfg.image_height);  // blended depth before the division (ED modes)
-    w.list_state = c.take<uint32_t>(tile_list_state_words((int64_t)N, (int64_t)cap, (int)bit_width_u32((uint32_t)tw * th) + 1));
+    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th));
+    w.tile_order = tile_list_order(w.list_state, (int64_t)tw * th);
     w.bytes = c.total();
     return w;
 }
@@ -99,12 +91,14 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
 // ---- EWA workspace ----------------------------------------------------------------------------
 struct EwaWs {
     int32_t* counters;  // [0] overflow, [1] n_instances, [2] n_visible
-    int32_t *n_touched, *tile_offsets, *n_contrib, *tile_order;
+    int32_t *n_touched, *tile_offsets, *n_contrib, *flatten_ids;
     ushort4* bounds;
     float4* records;
     float* accum;
-    uint32_t *gkeys[2], *gvals[2], *tkeys[2], *tvals[2];
-    uint32_t* list_state;
+    uint32_t* depth_bits;
+    uint64_t *masks, *entries;
+    int32_t* list_state;
+    const int32_t* tile_order;
     size_t bytes;
 };
 
@@ -118,12 +112,14 @@ EwaWs carve_ewa(const lfs_ewa_config& cfg, void* base) {
     w.bounds = c.take<ushort4>(N);
     w.records = c.take<float4>(N * 3);
     w.accum = c.take<float>(N * 12);
-    for (int k = 0; k < 2; ++k) { w.gkeys[k] = c.take<uint32_t>(N); w.gvals[k] = c.take<uint32_t>(N); }
-    for (int k = 0; k < 2; ++k) { w.tkeys[k] = c.take<uint32_t>(cap); w.tvals[k] = c.take<uint32_t>(cap); }
+    w.depth_bits = c.take<uint32_t>(N);
+    w.masks = c.take<uint64_t>(N);
+    w.entries = c.take<uint64_t>(cap);
+    w.flatten_ids = c.take<int32_t>(cap);
     w.tile_offsets = c.take<int32_t>((size_t)tw * th + 1);
     w.n_contrib = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
-    w.tile_order = c.take<int32_t>((size_t)tw * th);
-    w.list_state = c.take<uint32_t>(tile_list_state_words((int64_t)N, (int64_t)cap, (int)bit_width_u32((uint32_t)tw * th) + 1));
+    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th));
+    w.tile_order = tile_list_order(w.list_state, (int64_t)tw * th);
     w.bytes = c.total();
     return w;
 }
@@ -248,23 +244,8 @@ int lfs_intersect_tile_count(int C, int N, const float* means2d, const int32_t* 
     return launch_sum_i32(total, tiles_per_gauss, n_isects_dev, S(stream));
 }
 
-// (camera, tile) keys of the operator: the tile grid is not known to the workspace query, so their look-back words are sized
-// for 32-bit keys
-static size_t isect_ws(int C, int N, int64_t n_isects, void* base, uint32_t** gk, uint32_t** gv,
-                       int32_t** n_dev, uint32_t** tk, uint32_t** tv, uint32_t** state) {
-    Carver c(base);
-    const size_t total = (size_t)C * N, cap = (size_t)(n_isects > 0 ? n_isects : 1);
-    for (int k = 0; k < 2; ++k) { gk[k] = c.take<uint32_t>(total); gv[k] = c.take<uint32_t>(total); }
-    *n_dev = c.take<int32_t>(16);
-    for (int k = 0; k < 2; ++k) { tk[k] = c.take<uint32_t>(cap); tv[k] = c.take<uint32_t>(cap); }
-    *state = c.take<uint32_t>(tile_list_state_words((int64_t)total, (int64_t)cap, 32));
-    return c.total();
-}
-
 size_t lfs_intersect_tile_workspace_bytes(int C, int N, int64_t n_isects) {
-    uint32_t *gk[2], *gv[2], *tk[2], *tv[2], *state;
-    int32_t* n_dev;
-    return isect_ws(C, N, n_isects, nullptr, gk, gv, &n_dev, tk, tv, &state);
+    return isect_lists_bytes((int64_t)C * N, n_isects > 0 ? n_isects : 1, nullptr, nullptr);
 }
 
 int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* radii, const float* depths,
@@ -273,17 +254,10 @@ int lfs_intersect_tile_emit(int C, int N, const float* means2d, const int32_t* r
     LFS_REQUIRE(C >= 0 && N >= 0 && tile_size > 0 && n_isects >= 0 && n_isects < ((int64_t)1 << 31), "bad sizes");
     if (n_isects == 0 || (int64_t)C * N == 0) return LFS_OK;
     LFS_REQUIRE(means2d && radii && depths && tiles_per_gauss && isect_ids && flatten_ids && workspace, "null pointer");
-    TileListArgs a{};
-    const size_t need = isect_ws(C, N, n_isects, workspace, a.gkeys, a.gvals, &a.n_isects_dev, a.tkeys, a.tvals, &a.state);
+    IsectBuffers b;
+    const size_t need = isect_lists_bytes((int64_t)C * N, n_isects, &b, workspace);
     if (workspace_bytes < need) { set_error("lfs_intersect_tile_emit: workspace too small (%zu < %zu)", workspace_bytes, need); return LFS_ECAPACITY; }
-    a.C = C; a.N = N; a.tw = tw; a.th = th; a.tile_size = tile_size; a.sort = sort ? 1 : 0; a.keys_ready = 0;
-    a.means2d = means2d; a.radii = radii; a.depths = depths; a.tiles = tiles_per_gauss;
-    a.capacity = n_isects; a.overflow = nullptr; a.tile_offsets = nullptr;
-    int sel = 0;
-    a.sel_out = &sel;
-    int rc = build_tile_lists(a, S(stream));
-    if (rc != LFS_OK) return rc;
-    return launch_compose_isect_ids(n_isects, a.tkeys[sel], a.tvals[sel], depths, a.state, isect_ids, flatten_ids, S(stream));
+    return build_isect_lists(C, N, tw, th, tile_size, sort, means2d, radii, depths, tiles_per_gauss, n_isects, b, isect_ids, flatten_ids, S(stream));
 }
 
 int lfs_intersect_offset(int64_t n_isects, const int64_t* isect_ids, int C, int tw, int th, int32_t* offsets, void* stream) {
@@ -661,24 +635,22 @@ int lfs_ewa_forward(const lfs_ewa_config* cfg, const lfs_splats* params, const f
     if (workspace_bytes < w.bytes) { set_error("lfs_ewa_forward: workspace too small (%zu < %zu)", workspace_bytes, w.bytes); return LFS_ECAPACITY; }
     cudaStream_t st = S(stream);
     const EwaCamera cam = ewa_camera(*cfg, w2c, cam_position);
+    const size_t bins = (size_t)cam.tw * cam.th;
+    const TileCounters counters = tile_list_counters(w.list_state, (int64_t)bins);
     cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st);
-    rc = launch_ewa_preprocess(cfg->N, *params, cam, w.n_touched, w.bounds, w.records, w.gkeys[0], w.gvals[0],
+    clear_tile_counters(counters, st);
+    rc = launch_ewa_preprocess(cfg->N, *params, cam, w.n_touched, w.bounds, w.records, w.depth_bits, w.masks, counters,
                                reinterpret_cast<float4*>(w.accum), w.counters + 2, st);
     if (rc != LFS_OK) return rc;
     TileListArgs a{};
-    a.C = 1; a.N = cfg->N; a.tw = cam.tw; a.th = cam.th; a.tile_size = 16; a.sort = 1; a.keys_ready = 1;
-    a.tiles = w.n_touched;
-    for (int k = 0; k < 2; ++k) { a.gkeys[k] = w.gkeys[k]; a.gvals[k] = w.gvals[k]; a.tkeys[k] = w.tkeys[k]; a.tvals[k] = w.tvals[k]; }
+    a.N = cfg->N; a.tw = cam.tw; a.th = cam.th; a.tile_size = 16;
+    a.tiles = w.n_touched; a.entries = w.entries; a.flatten_ids = w.flatten_ids;
     a.n_isects_dev = w.counters + 1; a.capacity = cfg->instance_capacity; a.overflow = w.counters + 0;
-    int sel = 0;
-    a.sel_out = &sel;
     a.tile_offsets = w.tile_offsets; a.state = w.list_state;
-    a.ewa_bounds = w.bounds; a.ewa_records = w.records;
+    a.ewa_bounds = w.bounds; a.ewa_records = w.records; a.ewa_masks = w.masks; a.ewa_depth_bits = w.depth_bits;
     rc = build_tile_lists(a, st);
     if (rc != LFS_OK) return rc;
-    rc = launch_tile_order(cam.tw * cam.th, w.tile_offsets, w.tile_order, st);
-    if (rc != LFS_OK) return rc;
-    EwaBlendArgs b{w.records, w.tvals[sel], w.tile_offsets, w.counters + 0, background, cfg->image_width, cfg->image_height, cam.tw, cam.th,
+    EwaBlendArgs b{w.records, reinterpret_cast<const uint32_t*>(w.flatten_ids), w.tile_offsets, w.counters + 0, background, cfg->image_width, cfg->image_height, cam.tw, cam.th,
                    w.tile_order};
     rc = launch_ewa_blend_fwd(b, image, alpha, w.n_contrib, st);
     if (rc != LFS_OK) return rc;
@@ -698,8 +670,7 @@ int lfs_ewa_backward(const lfs_ewa_config* cfg, const lfs_splats* params, const 
     if (workspace_bytes < w.bytes) { set_error("lfs_ewa_backward: workspace too small"); return LFS_ECAPACITY; }
     cudaStream_t st = S(stream);
     const EwaCamera cam = ewa_camera(*cfg, w2c, cam_position);
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)cam.tw * cam.th) + 1));  // tile bits + one camera bit
-    EwaBlendArgs b{w.records, w.tvals[sel], w.tile_offsets, w.counters + 0, background, cfg->image_width, cfg->image_height, cam.tw, cam.th,
+    EwaBlendArgs b{w.records, reinterpret_cast<const uint32_t*>(w.flatten_ids), w.tile_offsets, w.counters + 0, background, cfg->image_width, cfg->image_height, cam.tw, cam.th,
                    w.tile_order};
     rc = launch_ewa_blend_bwd(b, alpha, w.n_contrib, grad_image, grad_alpha, w.accum, st);
     if (rc != LFS_OK) return rc;
@@ -738,11 +709,10 @@ int lfs_ewa_workspace_view(const lfs_ewa_config* cfg, void* workspace, size_t wo
     EwaWs w = carve_ewa(*cfg, workspace);
     if (workspace_bytes < w.bytes) { set_error("lfs_ewa_workspace_view: workspace too small"); return LFS_ECAPACITY; }
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
     out->n_touched = w.n_touched;
     out->bounds = reinterpret_cast<const uint16_t*>(w.bounds);
     out->records = reinterpret_cast<const float*>(w.records);
-    out->instance_ids = w.tvals[sel];
+    out->instance_ids = reinterpret_cast<const uint32_t*>(w.flatten_ids);
     out->tile_offsets = w.tile_offsets;
     out->n_contrib = w.n_contrib;
     return LFS_OK;
@@ -775,38 +745,37 @@ size_t lfs_render_workspace_bytes(const lfs_render_config* cfg) {
 
 // Shared body of the forward: per-Gaussian stage + tile lists (stage 1), shading + blending (stage 2).
 static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* params, const float* viewmat, const float* K,
-                                int with_colors, RenderWs& w, int* sel_out, cudaStream_t st, cudaEvent_t projected = nullptr) {
+                                int with_colors, RenderWs& w, cudaStream_t st, cudaEvent_t projected = nullptr) {
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
     int rc = launch_camera_setup(1, viewmat, cfg->viewmat_end, cfg_rs_type(*cfg), K, cfg->radial_coeffs, cfg->tangential_coeffs,
                                  cfg->thin_prism_coeffs, cfg->image_width, cfg->image_height, cfg->camera_model, w.cam, st);
     if (rc != LFS_OK) return rc;
     cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st);
+    const TileCounters counters = tile_list_counters(w.list_state, (int64_t)tw * th);
+    clear_tile_counters(counters, st);
     const ProjParams pp = make_proj_params(cfg->eps2d, cfg->near_plane, cfg->far_plane, cfg->radius_clip, cfg->ut);
     PackOptions opt;
     opt.scaling_modifier = cfg_modifier(*cfg);
     opt.calc_compensations = cfg->calc_compensations;
     opt.want_rgb = with_colors && mode_channels(cfg->render_mode) != 1;
     rc = launch_project_pack(cfg->N, cfg->sh_coeffs, cfg->sh_degree, *params, w.cam, pp, opt, cfg_model(*cfg), cfg_rolling(*cfg), cfg->tile_size, tw,
-                             th, w.radii, w.means2d, w.depths, w.tiles, w.gkeys[0], w.gvals[0], w.records, w.cuts, w.bounds,
+                             th, w.radii, w.means2d, w.depths, w.tiles, counters, w.records, w.cuts, w.bounds,
                              reinterpret_cast<float4*>(w.accum), w.counters + 2, st);
     if (rc != LFS_OK) return rc;
     if (projected && cudaEventRecord(projected, st) != cudaSuccess) { set_error("cudaEventRecord failed"); return LFS_ECUDA; }
     TileListArgs a{};
-    a.C = 1; a.N = cfg->N; a.tw = tw; a.th = th; a.tile_size = cfg->tile_size; a.sort = 1; a.keys_ready = 1;
+    a.N = cfg->N; a.tw = tw; a.th = th; a.tile_size = cfg->tile_size;
     a.means2d = w.means2d; a.radii = w.radii; a.depths = w.depths; a.tiles = w.tiles;
-    for (int k = 0; k < 2; ++k) { a.gkeys[k] = w.gkeys[k]; a.gvals[k] = w.gvals[k]; a.tkeys[k] = w.tkeys[k]; a.tvals[k] = w.tvals[k]; }
     a.n_isects_dev = w.counters + 1; a.capacity = cfg->isect_capacity; a.overflow = w.counters + 0;
-    a.sel_out = sel_out;
+    a.entries = w.entries; a.flatten_ids = w.flatten_ids;
     a.tile_offsets = w.tile_offsets; a.state = w.list_state;
-    rc = build_tile_lists(a, st);
-    if (rc != LFS_OK) return rc;
-    return launch_tile_order(tw * th, w.tile_offsets, w.tile_order, st);
+    return build_tile_lists(a, st);
 }
 
 static int render_forward_blend(const lfs_render_config* cfg, const float* background, float* render, float* alpha,
-                                int32_t* status_dev, RenderWs& w, int sel, cudaStream_t st) {
+                                int32_t* status_dev, RenderWs& w, cudaStream_t st) {
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, reinterpret_cast<const uint32_t*>(w.flatten_ids), w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     int rc = launch_raster_fwd(ra, render, alpha, w.last_ids, w.extra_sum, st);
@@ -825,10 +794,9 @@ int lfs_render_forward(const lfs_render_config* cfg, const lfs_splats* params, c
     RenderWs w = carve_render(*cfg, workspace);
     if (workspace_bytes < w.bytes) { set_error("lfs_render_forward: workspace too small (%zu < %zu)", workspace_bytes, w.bytes); return LFS_ECAPACITY; }
     cudaStream_t st = S(stream);
-    int sel = 0;
-    rc = render_forward_lists(cfg, params, viewmat, K, 1, w, &sel, st);
+    rc = render_forward_lists(cfg, params, viewmat, K, 1, w, st);
     if (rc != LFS_OK) return rc;
-    rc = render_forward_blend(cfg, background, render, alpha, status_dev, w, sel, st);
+    rc = render_forward_blend(cfg, background, render, alpha, status_dev, w, st);
     if (rc != LFS_OK) return rc;
     return check_launch("lfs_render_forward");
 }
@@ -841,8 +809,7 @@ int lfs_render_forward_lists_event(const lfs_render_config* cfg, const lfs_splat
     LFS_REQUIRE(aligned16(params->rotation_raw), "rotation_raw must be 16-byte aligned");
     RenderWs w = carve_render(*cfg, workspace);
     if (workspace_bytes < w.bytes) { set_error("lfs_render_forward_lists: workspace too small"); return LFS_ECAPACITY; }
-    int sel = 0;
-    rc = render_forward_lists(cfg, params, viewmat, K, 0, w, &sel, S(stream), reinterpret_cast<cudaEvent_t>(projected_event));
+    rc = render_forward_lists(cfg, params, viewmat, K, 0, w, S(stream), reinterpret_cast<cudaEvent_t>(projected_event));
     if (rc != LFS_OK) return rc;
     return check_launch("lfs_render_forward_lists");
 }
@@ -861,12 +828,11 @@ int lfs_render_forward_shade(const lfs_render_config* cfg, const lfs_splats* par
     if (workspace_bytes < w.bytes) { set_error("lfs_render_forward_shade: workspace too small"); return LFS_ECAPACITY; }
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
     if (mode_channels(cfg->render_mode) != 1) {
         rc = launch_sh_color(cfg->N, cfg->sh_coeffs, cfg->sh_degree, *params, w.cam, w.radii, w.records, st);
         if (rc != LFS_OK) return rc;
     }
-    rc = render_forward_blend(cfg, background, render, alpha, status_dev, w, sel, st);
+    rc = render_forward_blend(cfg, background, render, alpha, status_dev, w, st);
     if (rc != LFS_OK) return rc;
     return check_launch("lfs_render_forward_shade");
 }
@@ -882,8 +848,7 @@ int lfs_render_backward(const lfs_render_config* cfg, const lfs_splats* params, 
     if (workspace_bytes < w.bytes) { set_error("lfs_render_backward: workspace too small"); return LFS_ECAPACITY; }
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
-    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, reinterpret_cast<const uint32_t*>(w.flatten_ids), w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     rc = launch_raster_bwd(ra, alpha, w.last_ids, w.extra_sum, v_render, v_alpha, w.accum, nullptr, st);
@@ -926,8 +891,7 @@ int lfs_render_backward_adam(const lfs_render_config* cfg, const lfs_splats* par
     if (with_shN) LFS_REQUIRE(params->shN && exp_avg->shN && exp_avg_sq->shN, "null tensor in a parameter group");
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
-    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, w.tvals[sel], w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
+    RasterArgs ra{w.cam, w.records, w.cuts, cfg->N, w.bounds, reinterpret_cast<const uint32_t*>(w.flatten_ids), w.tile_offsets, w.counters + 1, 0, background, w.counters + 0,
                   cfg->image_width, cfg->image_height, tw, th, cfg_model(*cfg), mode_channels(cfg->render_mode),
                   mode_normalize(cfg->render_mode), cfg->tile_masks, w.tile_order, cfg_rolling(*cfg)};
     rc = launch_raster_bwd(ra, alpha, w.last_ids, w.extra_sum, v_render, v_alpha, w.accum, nullptr, st);
@@ -974,9 +938,8 @@ int lfs_render_workspace_view(const lfs_render_config* cfg, void* workspace, siz
     RenderWs w = carve_render(*cfg, workspace);
     if (workspace_bytes < w.bytes) { set_error("lfs_render_workspace_view: workspace too small"); return LFS_ECAPACITY; }
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
-    const int sel = sorted_sel((int)(bit_width_u32((uint32_t)tw * th) + 1));
     view->radii = w.radii; view->means2d = w.means2d; view->depths = w.depths; view->tiles_per_gauss = w.tiles;
-    view->tile_offsets = w.tile_offsets; view->flatten_ids = reinterpret_cast<const int32_t*>(w.tvals[sel]);
+    view->tile_offsets = w.tile_offsets; view->flatten_ids = w.flatten_ids;
     view->last_ids = w.last_ids; view->records = reinterpret_cast<const float*>(w.records);
     return LFS_OK;
 }

@@ -100,6 +100,14 @@ int launch_camera_setup(int C, const float* viewmats, const float* viewmats1, in
                         const float* tangential, const float* thin_prism, int W, int H, int model, CamDev* cams,
                         cudaStream_t st);
 
+// Instances per tile, and where the next one goes. The counters exist `replicas` times (a power of two), `stride` apart; the Gaussians
+// g .. g + 31, g a multiple of 32, use the same ones when they are counted and when they are written.
+struct TileCounters {
+    int32_t *counts, *cursors;
+    int32_t replicas, stride;
+    __device__ __forceinline__ size_t replica(int64_t g) const { return (size_t)((g >> 5) & (replicas - 1)) * stride; }
+};
+
 // ---- sort.cu -------------------------------------------------------------------------------
 struct SortScratch {
     uint32_t* block_sums; // [kScanBlocks + 1]

@@ -5,6 +5,7 @@
 // double and are rounded once (the reference calls expf / logf) so that a host evaluation gives the same floats.
 #include "ewa.cuh"
 #include "ewa_common.cuh"
+#include "gsmath.cuh"
 
 namespace lfs {
 namespace {
@@ -32,19 +33,21 @@ __global__ void __launch_bounds__(256, 4) ewa_preprocess_kernel(
     int N, const float* __restrict__ means, const float* __restrict__ sh0, const float* __restrict__ shN,
     const float* __restrict__ scaling_raw, const float* __restrict__ rotation_raw, const float* __restrict__ opacity_raw,
     EwaCamera cam, int32_t* __restrict__ n_touched, ushort4* __restrict__ bounds, float4* __restrict__ records,
-    uint32_t* __restrict__ sort_keys, uint32_t* __restrict__ sort_vals, float4* __restrict__ accum, int32_t* __restrict__ n_visible) {
+    uint32_t* __restrict__ depth_bits, uint64_t* __restrict__ masks, TileCounters tile_counters, float4* __restrict__ accum,
+    int32_t* __restrict__ n_visible) {
     int local_visible = 0;
     float r1[4], r2[4], r3[4], campos[3];
 #pragma unroll
     for (int k = 0; k < 4; ++k) { r1[k] = cam.w2c[k]; r2[k] = cam.w2c[4 + k]; r3[k] = cam.w2c[8 + k]; }
 #pragma unroll
     for (int k = 0; k < 3; ++k) campos[k] = cam.campos[k];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        sort_vals[i] = (uint32_t)i;
-        int count = 0;
-        const float m0 = means[i * 3], m1 = means[i * 3 + 1], m2 = means[i * 3 + 2];
+    const int lane = threadIdx.x & 31;
+    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < N; base += gridDim.x * blockDim.x) {
+        const int i = base + lane;
+        const bool in_range = i < N;
+        const float m0 = in_range ? means[i * 3] : 0.f, m1 = in_range ? means[i * 3 + 1] : 0.f, m2 = in_range ? means[i * 3 + 2] : 0.f;
         const float depth = r3[0] * m0 + r3[1] * m1 + r3[2] * m2 + r3[3];
-        bool active = !(depth < cam.near_plane || depth > cam.far_plane);
+        bool active = in_range && !(depth < cam.near_plane || depth > cam.far_plane);
         float opacity = 0.f, ca = 0.f, cb = 0.f, cc = 0.f, mx = 0.f, my = 0.f, thr = 0.f;
         uint32_t x0 = 0, x1 = 0, y0 = 0, y1 = 0;
         if (active) {
@@ -101,19 +104,37 @@ __global__ void __launch_bounds__(256, 4) ewa_preprocess_kernel(
                 x1 = min((uint32_t)cam.tw, (uint32_t)max(0, __float2int_ru((mx + ex) / 16.0f)));
                 y0 = min((uint32_t)cam.th, (uint32_t)max(0, __float2int_rd((my - ey) / 16.0f)));
                 y1 = min((uint32_t)cam.th, (uint32_t)max(0, __float2int_ru((my + ey) / 16.0f)));
-                // exact number of tiles the ellipse reaches
-                for (uint32_t tyi = y0; tyi < y1; ++tyi)
-                    for (uint32_t txi = x0; txi < x1; ++txi)
-                        count += ewa_tile_contributes(mx - 0.5f, my - 0.5f, ca, cb, cc, txi, tyi, thr) ? 1 : 0;
             }
         }
+        // Which tiles of the rectangle the ellipse reaches. The 32 rectangles of a warp are tested 32 tiles at a time, and the ballot gives
+        // every lane its own answers.
+        int count = 0;
+        uint64_t reached = 0;
+        const int width = (int)(x1 - x0), area = active && x1 > x0 && y1 > y0 ? width * (int)(y1 - y0) : 0;
+        const int start = warp_incl_scan(area) - area;
+        int round = 0;
+        int32_t* counts = tile_counters.counts + tile_counters.replica(base);
+        for_each_tile(area, x0, y0, width, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
+            const bool hit = ewa_tile_contributes(__shfl_sync(0xffffffffu, mx, owner) - 0.5f, __shfl_sync(0xffffffffu, my, owner) - 0.5f,
+                                                  __shfl_sync(0xffffffffu, ca, owner), __shfl_sync(0xffffffffu, cb, owner),
+                                                  __shfl_sync(0xffffffffu, cc, owner), tx, ty, __shfl_sync(0xffffffffu, thr, owner)) && on;
+            if (hit) atomicAdd(counts + (size_t)ty * cam.tw + tx, 1);
+            const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+            // this lane's tiles among the 32 of this round: [from, to)
+            const int from = max(start - round, 0), to = min(start + area - round, 32);
+            if (from < to) {
+                const uint32_t mine = (hits >> from) & (to - from == 32 ? 0xffffffffu : (1u << (to - from)) - 1u);
+                count += __popc(mine);
+                if (area <= 64) reached |= (uint64_t)mine << (round + from - start);
+            }
+            round += 32;
+        });
+        if (!in_range) continue;
         n_touched[i] = count;
-        if (count == 0) {
-            sort_keys[i] = 0xFFFFFFFFu;
-            continue;
-        }
+        if (count == 0) continue;
         ++local_visible;
-        sort_keys[i] = __float_as_uint(depth);
+        depth_bits[i] = __float_as_uint(depth);
+        masks[i] = reached;
         bounds[i] = make_ushort4((unsigned short)x0, (unsigned short)x1, (unsigned short)y0, (unsigned short)y1);
         // colour
         float rgb[3];
@@ -145,12 +166,12 @@ __global__ void __launch_bounds__(256, 4) ewa_preprocess_kernel(
 }  // namespace
 
 int launch_ewa_preprocess(int N, const lfs_splats& p, const EwaCamera& cam, int32_t* n_touched,
-                          ushort4* bounds, float4* records, uint32_t* sort_keys, uint32_t* sort_vals, float4* accum,
+                          ushort4* bounds, float4* records, uint32_t* depth_bits, uint64_t* masks, const TileCounters& tile_counters, float4* accum,
                           int32_t* n_visible, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     LFS_TIMED("ewa_preprocess", st);
     ewa_preprocess_kernel<<<grid_for(N, 256), 256, 0, st>>>(N, p.means, p.sh0, p.shN, p.scaling_raw, p.rotation_raw, p.opacity_raw,
-                                                            cam, n_touched, bounds, records, sort_keys, sort_vals, accum, n_visible);
+                                                            cam, n_touched, bounds, records, depth_bits, masks, tile_counters, accum, n_visible);
     return check_launch("ewa_preprocess");
 }
 

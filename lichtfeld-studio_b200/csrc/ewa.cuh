@@ -14,11 +14,11 @@ struct EwaCamera {       // passed by value to the kernels
     int active_sh_bases, total_rest;  // SH bases in use (1, 4, 9, 16), rows stored per Gaussian in shN
 };
 
-// preprocess_cu: activations, 3-D and 2-D covariance, exact tile count, SH colour; packed record, depth sort key
-// (0xFFFFFFFF when culled), zeroed gradient accumulators, visible count.
+// preprocess_cu: activations, 3-D and 2-D covariance, exact tile count, SH colour; packed record, depth bits, which tiles of
+// the bounds rectangle are reached (rectangles of up to 64), instances per tile, zeroed gradient accumulators, visible count.
 int launch_ewa_preprocess(int N, const lfs_splats& p, const EwaCamera& cam,
-                          int32_t* n_touched, ushort4* bounds, float4* records, uint32_t* sort_keys, uint32_t* sort_vals,
-                          float4* accum, int32_t* n_visible, cudaStream_t st);
+                          int32_t* n_touched, ushort4* bounds, float4* records, uint32_t* depth_bits, uint64_t* masks,
+                          const TileCounters& tile_counters, float4* accum, int32_t* n_visible, cudaStream_t st);
 
 struct EwaBlendArgs {
     const float4* records;        // [N*3]

@@ -502,6 +502,46 @@ __device__ __forceinline__ void store_rows(float* __restrict__ dst, const float*
     }
 }
 
+__device__ __forceinline__ int warp_incl_scan(int v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) >= o) v += t;
+    }
+    return v;
+}
+
+// The tiles of the 32 rectangles that the lanes of a warp hold (count tiles each, in row-major order from (x0, y0), `width` wide), 32 at a time:
+// every lane gets one tile and the lane that owns it, so that a rectangle of many tiles does not hold up 31 lanes. All lanes call;
+// f(on, owner, tile x, tile y, index in the rectangle) is called with on = false past the last tile. With U > 1 the results of U calls
+// are collected before then(owner, result) takes them, so that U requests to memory are in flight.
+template <int U, class F, class Then>
+__device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y0, uint32_t width, F f, Then then) {
+    const int incl = warp_incl_scan(count), total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int base = 0; base < total; base += 32 * U) {
+        int owners[U], got[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = base + 32 * u + (threadIdx.x & 31);
+            int owner = 0;   // lanes whose last tile comes before k
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, owner + step - 1) <= k) owner += step;
+            const uint32_t local = (uint32_t)(k - __shfl_sync(0xffffffffu, incl - count, owner));
+            const uint32_t w = max(__shfl_sync(0xffffffffu, width, owner), 1u), y = local / w;
+            owners[u] = owner;
+            got[u] = f(k < total, owner, __shfl_sync(0xffffffffu, x0, owner) + (local - y * w), __shfl_sync(0xffffffffu, y0, owner) + y, local);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) then(owners[u], got[u]);
+    }
+}
+template <class F>
+__device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y0, uint32_t width, F f) {
+    for_each_tile<1>(count, x0, y0, width, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) { f(on, owner, tx, ty, local); return 0; },
+                     [](int, int) {});
+}
+
 // Tile rectangle covered by a projected Gaussian: [x0,x1) x [y0,y1) in tile units. The float ->
 // unsigned conversion saturates (negative -> 0), which is what clips boxes that start left of /
 // above the image.

@@ -604,8 +604,8 @@ int launch_pack_records(int N, const float* means, const float* quats, const flo
 
 // ---------------------------------------------------------------------------------------------
 // Fused per-Gaussian forward stage of the training path (one camera): activations, projection,
-// tile count, depth sort key, SH colour (+0.5, clamped at 0), packed record, zeroed gradient
-// accumulator row. Invisible Gaussians get radii 0, tile count 0 and the sort key 0xFFFFFFFF.
+// tile count, instances per tile, SH colour (+0.5, clamped at 0), packed record, zeroed gradient
+// accumulator row. Invisible Gaussians get radii 0 and tile count 0.
 // ---------------------------------------------------------------------------------------------
 // Bound by instruction issue and the latency of the per-Gaussian chain, not by memory: 64 registers and four CTAs per SM for the
 // models that project in single precision (1 M Gaussians 127 us against 135 with three CTAs, 6 M at 4K 655 against 720); the
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
     const float* __restrict__ opacity_raw, const CamDev* __restrict__ cams, ProjParams pp, PackOptions opt, float tile_size,
     uint32_t tw, uint32_t th,
     int32_t* __restrict__ radii, float* __restrict__ means2d, float* __restrict__ depths,
-    int32_t* __restrict__ tiles, uint32_t* __restrict__ sort_keys, uint32_t* __restrict__ sort_vals,
+    int32_t* __restrict__ tiles, TileCounters tile_counters,
     float4* __restrict__ records, float4* __restrict__ cuts, uint4* __restrict__ bounds, float4* __restrict__ accum,
     int32_t* __restrict__ n_visible) {
     // Each warp handles 32 consecutive Gaussians per iteration. Their higher-order SH rows ((K-1)*3 floats
@@ -654,11 +654,9 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
             const float nrm = fmaxf(sqrtf(n2), 1e-12f);
             qw = qr.x / nrm; qx = qr.y / nrm; qy = qr.z / nrm; qz = qr.w / nrm;
             vis = project_gaussian<MODEL, RS>(cam, pp, mean, qw, qx, qy, qz, scale, true, opacity, o);
-            sort_vals[g] = (uint32_t)g;
             if (!vis) {
                 radii[g * 2] = 0; radii[g * 2 + 1] = 0;
                 tiles[g] = 0;
-                sort_keys[g] = 0xFFFFFFFFu;
             }
         }
         const bool any_vis = __any_sync(0xffffffffu, vis);
@@ -675,19 +673,27 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pac
             }
             asm volatile("cp.async.commit_group;\n" ::);
             for (int i = total16 * 4 + lane; i < total; i += 32) my[i] = src[i];
-            asm volatile("cp.async.wait_group 0;\n" ::);
         }
-        __syncwarp();
+        uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0;
+        int nt = 0;
         if (vis) {
             radii[g * 2] = o.rx; radii[g * 2 + 1] = o.ry;
             means2d[g * 2] = o.mx; means2d[g * 2 + 1] = o.my;
             depths[g] = o.depth;
-            uint32_t x0, y0, x1, y1;
             tile_rect(o.mx, o.my, o.rx, o.ry, tile_size, tw, th, x0, y0, x1, y1);
-            const int nt = (int)((y1 - y0) * (x1 - x0));
+            nt = (int)((y1 - y0) * (x1 - x0));
             tiles[g] = nt;
-            sort_keys[g] = nt > 0 ? __float_as_uint(o.depth) : 0xFFFFFFFFu;
             ++local_visible;
+        }
+        // the lists' lengths, in the shadow of the SH rows
+        int32_t* counts = tile_counters.counts + tile_counters.replica((int64_t)chunk * 32);
+        if (any_vis)
+            for_each_tile(nt, x0, y0, x1 - x0, [&](bool on, int, uint32_t tx, uint32_t ty, uint32_t) {
+                if (on && tx < tw && ty < th) atomicAdd(counts + (size_t)ty * tw + tx, 1);
+            });
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncwarp();
+        if (vis) {
 
             // colour from SH along (mean - camera position)
             float rgb[3] = {0.f, 0.f, 0.f};
@@ -789,7 +795,7 @@ int launch_sh_color(int N, int K, int sh_degree, const lfs_splats& p, const CamD
 
 int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const ProjParams& pp,
                         const PackOptions& opt, int model, int rolling, int tile_size, int tw, int th, int32_t* radii, float* means2d, float* depths,
-                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, float4* cuts,
+                        int32_t* tiles, const TileCounters& tile_counters, float4* records, float4* cuts,
                         uint4* bounds, float4* accum, int32_t* n_visible, cudaStream_t st) {
     if (N == 0) return LFS_OK;
     const int grid = grid_for(N, 256);
@@ -806,7 +812,7 @@ int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const 
 #define LFS_PACK2(MODEL, RS)                                                                                                       \
     project_pack_kernel<MODEL, RS><<<grid, 256, smem, st>>>(N, K, sh_degree, p.means, p.sh0, p.shN, p.scaling_raw, p.rotation_raw,  \
                                                             p.opacity_raw, cam, pp, opt, (float)tile_size, tw, th, radii, means2d, \
-                                                            depths, tiles, sort_keys, sort_vals, records, cuts, bounds, accum, n_visible)
+                                                            depths, tiles, tile_counters, records, cuts, bounds, accum, n_visible)
 #define LFS_PACK(MODEL) do { if (rolling) LFS_PACK2(MODEL, true); else LFS_PACK2(MODEL, false); } while (0)
     switch (model) {
         case LFS_PINHOLE: LFS_PACK(LFS_PINHOLE); break;

@@ -42,7 +42,7 @@ struct PackOptions {
 // model: the effective (internal) model id, see effective_model(); rolling: the camera has a rolling shutter or an end pose
 int launch_project_pack(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const ProjParams& pp,
                         const PackOptions& opt, int model, int rolling, int tile_size, int tw, int th, int32_t* radii, float* means2d, float* depths,
-                        int32_t* tiles, uint32_t* sort_keys, uint32_t* sort_vals, float4* records, float4* cuts,
+                        int32_t* tiles, const TileCounters& tile_counters, float4* records, float4* cuts,
                         uint4* bounds, float4* accum, int32_t* n_visible, cudaStream_t st);
 
 // colours (SH + 0.5, clamped at 0) of the visible Gaussians into records[g*4+3].xyz

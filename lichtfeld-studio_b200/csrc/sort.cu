@@ -1,38 +1,28 @@
-// Tile-list construction: prefix sums, a stable LSD radix sort on (uint32 key, uint32 value) pairs,
-// instance emission and per-tile offsets.
+// Tile-list construction: the depth-sorted list of Gaussians of every tile, and prefix sums.
 //
 // Replaces gsplat/IntersectTile.cu:24 (second pass), the at::cumsum + CUB DeviceRadixSort::SortPairs
 // call of gsplat/Intersect.cpp:75 / gsplat/IntersectTile.cu:290-328, and gsplat/IntersectTile.cu:206.
 //
-// The reference sorts n_isects 12-byte (int64 key, int32 value) pairs over 32 + tile_bits + cam_bits
-// bits. The same order (camera, tile, depth bits, ties by ascending flattened Gaussian index) is
-// produced here with far less traffic: the Gaussians are sorted once by their 32 depth bits, the
-// instances are emitted in that order, and a stable sort on the (camera, tile) key alone finishes.
-// All passes are HBM-bound integer work; nothing here is shaped for tensor cores. Prefixes over the tiles of a list travel by
-// decoupled look-back (Merrill and Garland) inside the kernel that uses them, so a short sort is one histogram kernel and one
-// kernel per digit, and the prefix over the Gaussians' tile counts and the emission of their instances are one kernel: 9 launches
-// where separate histogram, scan and scatter kernels took 22.
+// The reference sorts n_isects 12-byte (int64 key, int32 value) pairs over 32 + tile_bits + cam_bits bits. The order that comes out
+// (camera, tile, depth bits, ties by ascending flattened Gaussian index) is a total one inside each tile, so nothing has to be stable:
+// the per-Gaussian stage counts the instances of every tile (one reduction to memory per instance), one CTA turns the counts into
+// offsets, the instances drop into their tile's range in any order (8 bytes each, one returning atomic), and every range is sorted by
+// (depth bits, index) where it fits into shared memory. Against two global radix sorts (depth of N, then tile of the instances) the
+// instances are written twice instead of six times and there are three launches instead of eleven. All of the list build, projection's
+// extra counting included, in us, before and now: 16 k Gaussians at 256x256 90 and 36, 150 k at 640x360 126 and 53, 1 M at 1296x840
+// 253 and 131, 3 M at 1600x1064 632 and 420, 6 M at 3840x2160 743 and 320.
 #include "gsmath.cuh"
 #include "sort.cuh"
 #include "ewa_common.cuh"
+
+#include <cooperative_groups.h>
 
 namespace lfs {
 
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
-constexpr int kItems = 8;
-constexpr int kTile = kThreads * kItems;
-
-__device__ __forceinline__ int warp_incl_scan(int v) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) >= o) v += t;
-    }
-    return v;
-}
+constexpr int kTile = 2048;
 
 // Exclusive scan over the block (any multiple of 32 threads up to 1024); returns the block total.
 __device__ __forceinline__ int block_excl_scan(int v, int& total, int* smem /*[33]*/) {
@@ -51,14 +41,6 @@ __device__ __forceinline__ int block_excl_scan(int v, int& total, int* smem /*[3
     total = smem[32];
     __syncthreads();
     return base + incl - v;
-}
-
-__device__ __forceinline__ int64_t device_count(const int32_t* n_dev, int64_t n_max) {
-    if (n_dev == nullptr) return n_max;
-    int64_t n = *n_dev;
-    if (n > n_max) n = n_max;
-    if (n < 0) n = 0;
-    return n;
 }
 
 // ---- prefix sum -----------------------------------------------------------------------------
@@ -105,500 +87,563 @@ __global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int32_t* __r
     }
 }
 
-// ---- decoupled look-back ------------------------------------------------------------------------
-// One word per list tile (and digit): 0 = nothing yet, top bit clear = the tile's own count + 1, top bit set = the count of this
-// and all earlier tiles. Value and flag share the word, so relaxed accesses are enough. Tiles are numbered by a ticket, so every
-// predecessor of a tile belongs to a CTA that is already running and publishes its own count without waiting for anybody:
-// each wait ends. The poll limit only bounds the damage of a defect: it raises a flag, after which nobody reads the list, and every
-// store below checks its position.
-constexpr uint32_t kInclusive = 0x80000000u;
-constexpr int kPollLimit = 1 << 21;
-
-__device__ __forceinline__ uint32_t ld_state(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_state(uint32_t* p, uint32_t v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// ---- radix sort -------------------------------------------------------------------------------
-// Digit counts of all passes in one read of the keys; zeroes the look-back words of the passes that follow.
-__global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint32_t* __restrict__ keys, const int32_t* n_dev,
-                                                              int64_t n_max, int bits, int passes,
-                                                              uint32_t* __restrict__ hist, uint4* __restrict__ state,
-                                                              int64_t pass_stride4) {
-    __shared__ uint32_t h[4][256];
-    const int64_t n = device_count(n_dev, n_max);
-    const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x, stride = (int64_t)gridDim.x * kThreads;
-    const int64_t n_words4 = (n + kTile - 1) / kTile * 64;
-    for (int p = 0; p < passes; ++p)
-        for (int64_t i = tid; i < n_words4; i += stride) state[p * pass_stride4 + i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int p = 0; p < 4; ++p) h[p][threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t mask = (1u << bits) - 1u;
-    for (int64_t i = tid; i < n; i += stride) {
-        const uint32_t k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&h[p][(k >> (p * bits)) & mask], 1u);
-    }
-    __syncthreads();
-    for (int p = 0; p < passes; ++p)
-        if (h[p][threadIdx.x]) atomicAdd(&hist[p * 256 + threadIdx.x], h[p][threadIdx.x]);
-}
-
-// Long lists: one digit count per CTA and pass over its chunk of the list (row d of a digit-major table), ...
-__global__ void __launch_bounds__(kThreads) radix_count_kernel(const uint32_t* __restrict__ keys, const int32_t* n_dev,
-                                                               int64_t n_max, int shift, uint32_t mask, int nb,
-                                                               uint32_t* __restrict__ table) {
-    __shared__ uint32_t h[256];
-    const int64_t n = device_count(n_dev, n_max);
-    const int64_t chunk = (n + nb - 1) / nb;
-    const int64_t lo = (int64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    for (int64_t i = lo + threadIdx.x; i < hi; i += kThreads) atomicAdd(&h[(keys[i] >> shift) & mask], 1u);
-    __syncthreads();
-    table[(size_t)threadIdx.x * nb + blockIdx.x] = h[threadIdx.x];
-}
-
-// ... and one CTA per digit: exclusive scan of that digit's counts and the digit total.
-__global__ void __launch_bounds__(kThreads) radix_scan_kernel(uint32_t* __restrict__ table, int nb, uint32_t* __restrict__ digit_totals) {
-    __shared__ int sm[33];
-    uint32_t* row = table + (size_t)blockIdx.x * nb;
-    int carry = 0;
-    for (int base = 0; base < nb; base += kThreads) {
-        const int i = base + threadIdx.x;
-        const int v = i < nb ? (int)row[i] : 0;
-        int total;
-        const int ex = block_excl_scan(v, total, sm);
-        if (i < nb) row[i] = (uint32_t)(carry + ex);
-        carry += total;
-    }
-    if (threadIdx.x == 0) digit_totals[blockIdx.x] = (uint32_t)carry;
-}
-
-// Scatter of the chunked pass: the CTA walks its chunk in tiles of 2048 pairs. Every item gets its rank among the equal digits
-// of the tile (warp match + per-warp counters), the tile is reordered by digit in shared memory, and consecutive threads write
-// consecutive addresses of each digit's output run, so the global stores are contiguous runs instead of 4-byte scatters.
-__global__ void __launch_bounds__(kThreads) radix_scatter_chunk_kernel(
-    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
-    uint32_t* __restrict__ vals_out, const int32_t* n_dev, int64_t n_max, int shift, uint32_t mask, int nb,
-    const uint32_t* __restrict__ table, const uint32_t* __restrict__ digit_totals) {
-    __shared__ uint32_t cnt[kWarps][256];   // per-warp digit counts, then per-warp start inside the tile
-    __shared__ uint32_t gbase[256];         // where the next item of digit d from this CTA goes
-    __shared__ uint32_t tstart[256];        // start of digit d inside the reordered tile
-    __shared__ uint32_t skeys[kTile], svals[kTile];
-    __shared__ int sm[33];
-    const int64_t n = device_count(n_dev, n_max);
-    const int64_t chunk = (n + nb - 1) / nb;
-    const int64_t lo = (int64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    {
-        // start of digit d = totals of the smaller digits + this digit's counts in the earlier blocks
-        int total;
-        const int digit_base = block_excl_scan((int)digit_totals[threadIdx.x], total, sm);
-        gbase[threadIdx.x] = (uint32_t)digit_base + table[(size_t)threadIdx.x * nb + blockIdx.x];
-    }
-    for (int64_t tile_lo = lo; tile_lo < hi; tile_lo += kTile) {
-        const int tile_n = (int)min((int64_t)kTile, hi - tile_lo);
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        uint32_t key[kItems], val[kItems], rank[kItems];
-        const int64_t wbase = tile_lo + (int64_t)warp * (32 * kItems);
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int64_t i = wbase + r * 32 + lane;
-            const bool ok = i < hi;
-            key[r] = ok ? keys_in[i] : 0u;
-            val[r] = ok ? vals_in[i] : 0u;
-        }
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int64_t i = wbase + r * 32 + lane;
-            const bool ok = i < hi;
-            const uint32_t d = ok ? ((key[r] >> shift) & mask) : 0xFFFFFFFFu;
-            const uint32_t peers = __match_any_sync(0xffffffffu, d);
-            uint32_t prev = 0;
-            if (ok) prev = cnt[warp][d];
-            __syncwarp();
-            if (ok && (peers & lt_mask) == 0) cnt[warp][d] = prev + __popc(peers);
-            __syncwarp();
-            rank[r] = prev + __popc(peers & lt_mask);
-        }
-        __syncthreads();
-        {
-            // digit threadIdx.x: exclusive prefix over the warps and the digit's total in this tile
-            uint32_t run = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = cnt[w][threadIdx.x];
-                cnt[w][threadIdx.x] = run;
-                run += c;
-            }
-            int total;
-            const int start = block_excl_scan((int)run, total, sm);  // start of this digit inside the tile
-            tstart[threadIdx.x] = (uint32_t)start;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] += (uint32_t)start;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int64_t i = wbase + r * 32 + lane;
-            if (i < hi) {
-                const uint32_t d = (key[r] >> shift) & mask;
-                const uint32_t pos = cnt[warp][d] + rank[r];
-                skeys[pos] = key[r];
-                svals[pos] = val[r];
-            }
-        }
-        __syncthreads();
-        // write out: item j of the reordered tile belongs to digit d = digit(skeys[j]) and goes to
-        // gbase[d] + (j - tstart[d]); neighbouring j of one digit are neighbouring addresses
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int j = r * kThreads + threadIdx.x;
-            if (j < tile_n) {
-                const uint32_t k = skeys[j];
-                const uint32_t d = (k >> shift) & mask;
-                const uint32_t pos = gbase[d] + ((uint32_t)j - tstart[d]);
-                keys_out[pos] = k;
-                vals_out[pos] = svals[j];
-            }
-        }
-        __syncthreads();
-        {
-            // advance the global bases by this tile's digit totals
-            const uint32_t next = threadIdx.x + 1 < 256 ? tstart[threadIdx.x + 1] : (uint32_t)tile_n;
-            gbase[threadIdx.x] += next - tstart[threadIdx.x];
-        }
-        __syncthreads();
-    }
-}
-
-// Stable scatter of one radix pass. A CTA takes tiles of 2048 pairs by ticket: every item gets its rank among the equal
-// digits of the tile (warp match + per-warp counters), the tile's digit counts are published, the tile is reordered by
-// digit in shared memory, the counts of the earlier tiles are looked up (one thread per digit, four tiles at a time), and then
-// consecutive threads write consecutive addresses of each digit's output run.
-__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(
-    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
-    uint32_t* __restrict__ vals_out, const int32_t* n_dev, int64_t n_max, int shift, uint32_t mask,
-    const uint32_t* __restrict__ hist, uint32_t* ticket, uint32_t* state, int32_t* gave_up) {
-    __shared__ uint32_t cnt[kWarps][256];   // per-warp digit counts, then per-warp start inside the tile
-    __shared__ uint32_t gbase[256];         // where the items of digit d of this tile go
-    __shared__ uint32_t tstart[256];        // start of digit d inside the reordered tile
-    __shared__ uint32_t skeys[kTile], svals[kTile];
-    __shared__ int sm[33];
-    __shared__ uint32_t s_tile;
-    const int64_t n = device_count(n_dev, n_max);
-    const uint32_t n_list_tiles = (uint32_t)((n + kTile - 1) / kTile);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    uint32_t digit_base;   // start of digit threadIdx.x in the output: totals of the smaller digits
-    {
-        int total;
-        digit_base = (uint32_t)block_excl_scan((int)hist[threadIdx.x], total, sm);
-    }
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= n_list_tiles) break;
-        const int64_t tile_lo = (int64_t)tile * kTile;
-        const int tile_n = (int)min((int64_t)kTile, n - tile_lo);
-        uint32_t key[kItems], val[kItems], rank[kItems];
-        const int wbase = warp * (32 * kItems);
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int i = wbase + r * 32 + lane;
-            const bool ok = i < tile_n;
-            key[r] = ok ? keys_in[tile_lo + i] : 0u;
-            val[r] = ok ? vals_in[tile_lo + i] : 0u;
-        }
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const bool ok = wbase + r * 32 + lane < tile_n;
-            const uint32_t d = (key[r] >> shift) & mask;
-            // lanes with the same digit: one ballot per digit bit. The warp's match instruction works through the distinct values
-            // one by one, which a tile that its successors wait for feels (60 k keys 48 us with it, 42 with ballots).
-            uint32_t peers = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-            for (int bit = 0; bit < 8; ++bit) {
-                if (mask >> bit) {
-                    const bool one = (d >> bit) & 1u;
-                    const uint32_t b = __ballot_sync(0xffffffffu, one);
-                    peers &= one ? b : ~b;
-                }
-            }
-            uint32_t prev = 0;
-            if (ok) prev = cnt[warp][d];
-            __syncwarp();
-            if (ok && (peers & lt_mask) == 0) cnt[warp][d] = prev + __popc(peers);
-            __syncwarp();
-            rank[r] = prev + __popc(peers & lt_mask);
-        }
-        __syncthreads();
-        uint32_t* my_state = state + (size_t)tile * 256 + threadIdx.x;
-        uint32_t run = 0;   // items of digit threadIdx.x in this tile
-        {
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = cnt[w][threadIdx.x];
-                cnt[w][threadIdx.x] = run;
-                run += c;
-            }
-            st_state(my_state, tile == 0 ? (kInclusive | run) : run + 1u);
-            int total;
-            const int start = block_excl_scan((int)run, total, sm);  // start of this digit inside the tile
-            tstart[threadIdx.x] = (uint32_t)start;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] += (uint32_t)start;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            if (wbase + r * 32 + lane < tile_n) {
-                const uint32_t d = (key[r] >> shift) & mask;
-                const uint32_t pos = cnt[warp][d] + rank[r];
-                skeys[pos] = key[r];
-                svals[pos] = val[r];
-            }
-        }
-        uint32_t prefix = 0;
-        if (tile > 0) {
-            int polls = 0;
-            const uint32_t* p = my_state - 256;
-            int64_t left = tile;   // predecessors not yet counted
-            bool found = false;
-            while (!found && left > 0) {
-                uint32_t v[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) v[q] = q < left ? ld_state(p - q * 256) : 0u;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (found || v[q] == 0u) break;
-                    prefix += (v[q] & kInclusive) ? (v[q] & ~kInclusive) : v[q] - 1u;
-                    found = (v[q] & kInclusive) != 0u;
-                    p -= 256;
-                    --left;
-                }
-                if (++polls > kPollLimit) {
-                    atomicExch(gave_up, 1);
-                    break;
-                }
-            }
-            st_state(my_state, kInclusive | (prefix + run));
-        }
-        gbase[threadIdx.x] = digit_base + prefix;
-        __syncthreads();
-        // write out: item j of the reordered tile belongs to digit d = digit(skeys[j]) and goes to
-        // gbase[d] + (j - tstart[d]); neighbouring j of one digit are neighbouring addresses
-#pragma unroll
-        for (int r = 0; r < kItems; ++r) {
-            const int j = r * kThreads + threadIdx.x;
-            if (j < tile_n) {
-                const uint32_t k = skeys[j];
-                const uint32_t d = (k >> shift) & mask;
-                const uint32_t pos = gbase[d] + ((uint32_t)j - tstart[d]);
-                if (pos < (uint32_t)n) {
-                    keys_out[pos] = k;
-                    vals_out[pos] = svals[j];
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// ---- instance emission ----------------------------------------------------------------------
-// Prefix over the Gaussians' tile counts (in emission order) and their instances, in one kernel. A CTA takes 256 or
-// 1024 Gaussians by ticket, scans their counts, finds the instances of the earlier tiles by look-back (one warp, 32 tiles at a time)
-// and writes its instances as one contiguous run: thread k of a round finds the owner of instance k by bisection, so the stores
-// are coalesced and a Gaussian that covers the whole image does not hold up one thread.
-// EWA: a Gaussian's instances are the tiles of the bounds rectangle that the ellipse reaches (create_instances_cu,
-// src/training/fastgs/rasterization/include/kernels_forward.cuh:205-309), in row-major tile order: no closed form for the k-th,
-// so eight lanes walk a rectangle together.
-constexpr int kEmitItems = 4;
-template <bool EWA, int ITEMS>
-__global__ void __launch_bounds__(kThreads) emit_instances_kernel(
-    int64_t total, int N, const uint32_t* __restrict__ order, const int32_t* __restrict__ tiles,
-    const float* __restrict__ means2d, const int32_t* __restrict__ radii, const ushort4* __restrict__ ewa_bounds,
-    const float4* __restrict__ rec, float tile_size, uint32_t tw, uint32_t th, uint32_t tile_n_bits, int64_t capacity,
-    uint32_t* __restrict__ tkeys, uint32_t* __restrict__ tvals, int32_t* overflow, int32_t* gave_up, int32_t* __restrict__ n_out,
-    uint32_t* ticket, uint32_t* state) {
-    constexpr int kList = kThreads * ITEMS;
-    __shared__ int sm[33];
-    __shared__ uint32_t s_tile, s_prefix;
-    __shared__ int s_off[kList + 1];
-    __shared__ uint32_t s_idx[kList], s_w[EWA ? 1 : kList];
-    __shared__ uint2 s_xy[EWA ? 1 : kList];
-    const uint32_t n_list_tiles = (uint32_t)((total + kList - 1) / kList);
+// ---- scatter ------------------------------------------------------------------------------------
+// One entry per instance, (depth bits, flattened Gaussian index), to the next free place of its tile's range. Bound by the latency of the
+// returning atomics, so a lane has kInFlight of them under way (8.3 M instances of 6 M Gaussians at 3840x2160: 195 us with one, 171 with two, 152
+// with four, 269 with eight; 1 M at 1296x840 no difference).
+constexpr int kInFlight = 4;
+__global__ void __launch_bounds__(kThreads) tile_scatter_kernel(int64_t total, int N, int tw, int th, float tile_size, const int32_t* __restrict__ tiles,
+                                                                const float* __restrict__ means2d, const int32_t* __restrict__ radii,
+                                                                const float* __restrict__ depths, int64_t first_bin, int64_t n_bins, int64_t capacity,
+                                                                const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries) {
+    if (overflow && *overflow) return;
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= n_list_tiles) break;
-        const int64_t r0 = (int64_t)tile * kList + threadIdx.x * ITEMS;
-        uint32_t idx[ITEMS];
-        int nt[ITEMS], sum = 0;
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            const int64_t r = r0 + k;
-            idx[k] = r < total ? (order ? order[r] : (uint32_t)r) : 0u;
-            nt[k] = r < total && idx[k] < (uint64_t)total ? max(tiles[idx[k]], 0) : 0;
-        }
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) sum += nt[k];
-        int block_total;
-        int off = block_excl_scan(sum, block_total, sm);
-        if (threadIdx.x == 0) st_state(state + tile, tile == 0 ? (kInclusive | (uint32_t)block_total) : (uint32_t)block_total + 1u);
-        if (threadIdx.x == 0) s_off[kList] = block_total;
-        {
-            int o = off;
-#pragma unroll
-            for (int k = 0; k < ITEMS; ++k) {
-                const int e = threadIdx.x * ITEMS + k;
-                s_off[e] = o;
-                s_idx[e] = idx[k];
-                if (!EWA && nt[k] > 0) {
-                    const size_t g = (size_t)idx[k] * 2;
-                    uint32_t x0, y0, x1, y1;
-                    tile_rect(means2d[g], means2d[g + 1], radii[g], radii[g + 1], tile_size, tw, th, x0, y0, x1, y1);
-                    s_xy[e] = make_uint2(x0, y0);
-                    s_w[e] = max(x1 - x0, 1u);
-                }
-                o += nt[k];
-            }
-        }
-        if (threadIdx.x < 32) {
-            uint32_t prefix = 0;
-            int64_t j = (int64_t)tile - 1;
-            int polls = 0;
-            while (j >= 0) {
-                const uint32_t v = j - lane >= 0 ? ld_state(state + (j - lane)) : kInclusive;
-                const uint32_t incl = __ballot_sync(0xffffffffu, (v & kInclusive) != 0u), empty = __ballot_sync(0xffffffffu, v == 0u);
-                const int last = incl ? __ffs(incl) - 1 : 31;   // nearest predecessor whose total covers everything before it
-                if (empty & (last == 31 ? 0xffffffffu : (2u << last) - 1u)) {
-                    if (++polls > kPollLimit) {
-                        if (lane == 0) atomicExch(gave_up, 1);
-                        break;
-                    }
-                    continue;
-                }
-                const uint32_t c = lane > last ? 0u : (v & kInclusive) ? (v & ~kInclusive) : v - 1u;
-                prefix = min(prefix + __reduce_add_sync(0xffffffffu, c), 0x7fffffffu);
-                if (incl) break;
-                j -= 32;
-            }
-            if (lane == 0) {
-                const uint32_t upto = min(prefix + (uint32_t)block_total, 0x7fffffffu);
-                if (tile > 0) st_state(state + tile, kInclusive | upto);
-                s_prefix = prefix;
-                if (tile == n_list_tiles - 1) *n_out = (int32_t)upto;
-                if ((int64_t)prefix + block_total > capacity && overflow) atomicExch(overflow, 1);
-            }
-        }
-        __syncthreads();
-        const int64_t base = s_prefix;
-        if (!EWA) {
-            for (int k = threadIdx.x; k < block_total; k += kThreads) {
-                int lo = 0;   // last entry whose first instance is at or before k
-#pragma unroll
-                for (int step = kList / 2; step > 0; step >>= 1)
-                    if (s_off[lo + step] <= k) lo += step;
-                const uint32_t local = (uint32_t)(k - s_off[lo]), w = s_w[lo], g = s_idx[lo];
-                const uint32_t y = local / w, x = local - y * w;
-                const uint2 xy = s_xy[lo];
-                if (base + k < capacity) {
-                    tkeys[base + k] = ((g / (uint32_t)N) << tile_n_bits) | ((xy.y + y) * tw + xy.x + x);
-                    tvals[base + k] = g;
-                }
-            }
-        } else {
-            // eight lanes test eight tiles of one rectangle at a time; the ballot gives each reached tile its place
-            const int sub = lane & 7, group = lane >> 3;
-            for (int q0 = (threadIdx.x >> 5) * 4; q0 < kList; q0 += kWarps * 4) {
-                const int q = q0 + group;
-                int64_t at = base + s_off[q];
-                const int64_t end = base + s_off[q + 1];
-                const uint32_t g = s_idx[q];
-                ushort4 b = make_ushort4(0, 0, 0, 0);
-                float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0, c2 = c0;
-                if (at < end && end <= capacity) {
-                    b = ewa_bounds[g];
-                    c0 = rec[(size_t)g * 3]; c1 = rec[(size_t)g * 3 + 1]; c2 = rec[(size_t)g * 3 + 2];
-                }
-                const uint32_t width = b.y - b.x, area = width * (b.w - b.z);
-                for (uint32_t k = sub; __any_sync(0xffffffffu, k - sub < area); k += 8) {
-                    const uint32_t row = k < area ? k / width : 0u, ty = b.z + row, tx = b.x + (k - row * width);
-                    const bool hit = k < area && ewa_tile_contributes(c0.x - 0.5f, c0.y - 0.5f, c0.z, c0.w, c1.x, tx, ty, c2.z);
-                    const uint32_t hits = (__ballot_sync(0xffffffffu, hit) >> (8 * group)) & 0xffu;
-                    const int64_t pos = at + __popc(hits & ((1u << sub) - 1u));
-                    if (hit && pos < end) {
-                        tkeys[pos] = ty * tw + tx;
-                        tvals[pos] = g;
-                    }
-                    at += __popc(hits);
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// offsets[t] = first sorted instance whose (camera, tile) id >= t, for t in [0, n_ids]; entry n_ids
-// (one past the last tile) holds the instance count. Keys hold (cid << tile_n_bits) | tile.
-// When the overflow flag is set the instance list is incomplete (some slots were never written), so
-// the keys cannot be trusted: all offsets are zeroed and the rasterizer draws nothing. Ids are clamped to
-// n_ids in any case so that no key value can direct a store outside the offsets array.
-__global__ void __launch_bounds__(kThreads) tile_offsets_kernel(const uint32_t* __restrict__ tkeys, const int32_t* n_dev,
-                                                                int64_t n_max, uint32_t n_tiles, uint32_t tile_n_bits,
-                                                                int64_t n_ids, const int32_t* __restrict__ overflow,
-                                                                int32_t* __restrict__ offsets) {
-    const int64_t n = (overflow && *overflow) ? 0 : device_count(n_dev, n_max);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n == 0) {
-        for (int64_t i = tid; i <= n_ids; i += stride) offsets[i] = 0;
-        return;
-    }
-    const uint32_t tmask = (1u << tile_n_bits) - 1u;
-    for (int64_t i = tid; i < n; i += stride) {
-        const uint32_t k = tkeys[i];
-        const int64_t id_curr = min((int64_t)(k >> tile_n_bits) * n_tiles + (k & tmask), n_ids - 1);
-        if (i == 0)
-            for (int64_t t = 0; t <= id_curr; ++t) offsets[t] = 0;
-        if (i == n - 1)
-            for (int64_t t = id_curr + 1; t <= n_ids; ++t) offsets[t] = (int32_t)n;
-        if (i > 0) {
-            const uint32_t kp = tkeys[i - 1];
-            if (kp != k) {
-                const int64_t id_prev = min((int64_t)(kp >> tile_n_bits) * n_tiles + (kp & tmask), n_ids - 1);
-                for (int64_t t = id_prev + 1; t <= id_curr; ++t) offsets[t] = (int32_t)i;
-            }
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total; base += stride) {
+        const int64_t i = base + lane;
+        int32_t* cursors = t.cursors + t.replica(base);
+        const int nt = i < total ? max(tiles[i], 0) : 0;
+        uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0, key = 0;
+        if (nt > 0) {
+            tile_rect(means2d[i * 2], means2d[i * 2 + 1], radii[i * 2], radii[i * 2 + 1], tile_size, tw, th, x0, y0, x1, y1);
+            key = __float_as_uint(depths[i]);
         }
+        for_each_tile<kInFlight>(nt, x0, y0, x1 - x0, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
+            const int64_t bin = (N == total ? 0 : (base + owner) / N * ((int64_t)tw * th)) + (int64_t)ty * tw + tx - first_bin;
+            return on && bin >= 0 && bin < n_bins ? atomicAdd(cursors + bin, 1) : -1;
+        }, [&](int owner, int pos) {
+            const uint32_t d = __shfl_sync(0xffffffffu, key, owner);
+            if ((uint32_t)pos < (uint32_t)capacity) entries[pos] = ((uint64_t)d << 32) | (uint64_t)(base + owner);
+        });
     }
 }
 
-// Operator-level output: 64-bit keys (camera | tile | depth bits) and int32 flattened ids. A list that was given up (some of its
-// slots were never written) comes out as the largest key and id 0 throughout, beyond every tile.
-__global__ void __launch_bounds__(kThreads) compose_isect_ids_kernel(int64_t n, const uint32_t* __restrict__ tkeys,
-                                                                     const uint32_t* __restrict__ tvals,
-                                                                     const float* __restrict__ depths,
-                                                                     const int32_t* __restrict__ gave_up,
-                                                                     int64_t* __restrict__ isect_ids,
-                                                                     int32_t* __restrict__ flatten_ids) {
-    const bool failed = *gave_up != 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = failed ? 0u : tvals[i];
-        isect_ids[i] = failed ? INT64_MAX : ((int64_t)tkeys[i] << 32) | (int64_t)__float_as_uint(depths[v]);
-        flatten_ids[i] = (int32_t)v;
+// EWA: the tiles of the bounds rectangle that the ellipse reaches (create_instances_cu,
+// src/training/fastgs/rasterization/include/kernels_forward.cuh:205-309). Rectangles of up to 64 tiles carry the answers of the
+// per-Gaussian stage as a mask, larger ones are tested again.
+__global__ void __launch_bounds__(kThreads) ewa_scatter_kernel(int N, int tw, const int32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds,
+                                                               const uint64_t* __restrict__ masks, const float4* __restrict__ records,
+                                                               const uint32_t* __restrict__ depth_bits, int64_t n_bins, int64_t capacity,
+                                                               const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries) {
+    if (*overflow) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < N; base += stride) {
+        const int64_t i = base + lane;
+        int32_t* cursors = t.cursors + t.replica(base);
+        const bool on_screen = i < N && n_touched[i] > 0;
+        ushort4 b = make_ushort4(0, 0, 0, 0);
+        uint64_t mask = 0;
+        uint32_t key = 0;
+        if (on_screen) { b = bounds[i]; mask = masks[i]; key = depth_bits[i]; }
+        const int width = b.y - b.x, area = width * (b.w - b.z);
+        for_each_tile<kInFlight>(area, b.x, b.z, width, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) {
+            const uint64_t m = __shfl_sync(0xffffffffu, mask, owner);
+            const int owner_area = __shfl_sync(0xffffffffu, area, owner);
+            const int64_t g = base + owner, bin = (int64_t)ty * tw + tx;
+            bool hit = on && bin < n_bins;
+            if (owner_area <= 64) {
+                hit = hit && ((m >> local) & 1u);
+            } else if (hit) {
+                const float4 c0 = records[g * 3], c1 = records[g * 3 + 1], c2 = records[g * 3 + 2];
+                hit = ewa_tile_contributes(c0.x - 0.5f, c0.y - 0.5f, c0.z, c0.w, c1.x, tx, ty, c2.z);
+            }
+            return hit ? atomicAdd(cursors + bin, 1) : -1;
+        }, [&](int owner, int pos) {
+            const uint32_t d = __shfl_sync(0xffffffffu, key, owner);
+            if ((uint32_t)pos < (uint32_t)capacity) entries[pos] = ((uint64_t)d << 32) | (uint64_t)(base + owner);
+        });
+    }
+}
+
+// Operator level: instances per tile.
+__global__ void __launch_bounds__(kThreads) tile_histogram_kernel(int64_t total, int N, int tw, int th, float tile_size, const int32_t* __restrict__ tiles,
+                                                                  const float* __restrict__ means2d, const int32_t* __restrict__ radii, int64_t first_bin,
+                                                                  int64_t n_bins, TileCounters t) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total; base += stride) {
+        const int64_t i = base + lane;
+        int32_t* counts = t.counts + t.replica(base);
+        const int nt = i < total ? max(tiles[i], 0) : 0;
+        uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0;
+        if (nt > 0) tile_rect(means2d[i * 2], means2d[i * 2 + 1], radii[i * 2], radii[i * 2 + 1], tile_size, tw, th, x0, y0, x1, y1);
+        for_each_tile(nt, x0, y0, x1 - x0, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
+            const int64_t bin = (N == total ? 0 : (base + owner) / N * ((int64_t)tw * th)) + (int64_t)ty * tw + tx - first_bin;
+            if (on && bin >= 0 && bin < n_bins) atomicAdd(counts + bin, 1);
+        });
+    }
+}
+
+// Operator level, unsorted: instances in the order of the Gaussians, each Gaussian's tiles in row-major order. offs: exclusive prefix
+// of `tiles`.
+__global__ void __launch_bounds__(kThreads) emit_unsorted_kernel(int64_t total, int N, int tw, int th, float tile_size, uint32_t tile_n_bits,
+                                                                 const int32_t* __restrict__ tiles, const int32_t* __restrict__ offs,
+                                                                 const float* __restrict__ means2d, const int32_t* __restrict__ radii,
+                                                                 const float* __restrict__ depths, int64_t capacity, int64_t* __restrict__ isect_ids,
+                                                                 int32_t* __restrict__ flatten_ids) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total; base += stride) {
+        const int64_t i = base + lane;
+        const int nt = i < total ? max(tiles[i], 0) : 0;
+        uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0, key = 0;
+        int off = 0;
+        if (nt > 0) {
+            tile_rect(means2d[i * 2], means2d[i * 2 + 1], radii[i * 2], radii[i * 2 + 1], tile_size, tw, th, x0, y0, x1, y1);
+            key = __float_as_uint(depths[i]);
+            off = offs[i];
+        }
+        for_each_tile(nt, x0, y0, x1 - x0, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) {
+            const uint32_t d = __shfl_sync(0xffffffffu, key, owner);
+            const int64_t pos = (int64_t)__shfl_sync(0xffffffffu, off, owner) + local, g = base + owner;
+            if (on && pos < capacity) {
+                isect_ids[pos] = (((g / N) << tile_n_bits | ((int64_t)ty * tw + tx)) << 32) | d;
+                flatten_ids[pos] = (int32_t)g;
+            }
+        });
+    }
+}
+
+// ---- offsets, overflow, launch order ---------------------------------------------------------------
+// Launch order of the tile CTAs: tiles with the longest lists first, so that the last wave of a rasterizer launch is made of short tiles.
+// 132 buckets by the leading one and the next two bits of the list length (a floating-point-like key with a 2-bit mantissa); the order
+// inside a bucket is arbitrary.
+__device__ __forceinline__ int tile_order_bucket(int c) {
+    if (c <= 0) return 131;
+    const int lz = __clz(c);                              // 0 .. 31, small = long list
+    const int shift = max(0, 29 - lz);                    // bring the two bits below the leading one down
+    const int mant = (c >> shift) & 3;
+    return lz * 4 + (3 - mant);
+}
+// first bucket of the lists shorter than 2^K
+template <int K>
+constexpr int kBucketBelow = (32 - K) * 4;
+static_assert(kBucketBelow<8> == kBucketBelow<10> + 8, "");
+
+// Words of the list state in front of the per-bin arrays.
+// lists of at least 2^10 and 2^8 entries, and of any
+constexpr int kMetaLists = 0, kMetaWords = 16, kKinds = 3;
+
+// One cluster: counts -> offsets [n_bins + 1] and cursors, the total and the overflow flag (with it all offsets are 0: the list is not
+// built), the launch order, and how many lists each kind of sorting group has. Every CTA takes a run of bins, 1024 at a time; the CTAs
+// exchange their totals and their bucket counts through each other's shared memory. carry: instances of earlier bins (operator
+// level with more bins than the arrays hold), updated.
+// One CTA alone took 52 us for the 32,400 bins of a 4K image.
+constexpr int kScanCluster = 8;
+__global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) tile_scan_kernel(
+    int n_bins, TileCounters t, int64_t capacity, int64_t* carry, int32_t* __restrict__ n_out, int32_t* overflow, int32_t* __restrict__ offsets,
+    int32_t* __restrict__ order, int2* __restrict__ ranges, int32_t* __restrict__ meta) {
+    __shared__ int64_t warp_sums[32], block_sum;
+    __shared__ int hist[132], cursor[132], sm[33];
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = blockIdx.x;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    if (threadIdx.x < 132) hist[threadIdx.x] = 0;
+    __syncthreads();
+    const int run = (n_bins + kScanCluster - 1) / kScanCluster;
+    const int first = min(rank * run, n_bins), last = min(first + run, n_bins);
+    // the replicas of a bin, eight loads in flight
+    auto count = [&](int i) {
+        int c = 0;
+        for (int r0 = 0; r0 < t.replicas; r0 += 8) {
+            int v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = r0 + k < t.replicas ? t.counts[(size_t)(r0 + k) * t.stride + i] : 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c += v[k];
+        }
+        return c;
+    };
+    int64_t sum = 0;
+    int kept = 0;   // the count of the first round
+    for (int base = first; base < last; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int c = i < last ? count(i) : 0;
+        if (base == first) kept = c;
+        sum += c;
+        const int bucket = i < last ? tile_order_bucket(c) : -1;
+        const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
+        if (bucket >= 0 && (peers & lt_mask) == 0) atomicAdd(&hist[bucket], __popc(peers));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) warp_sums[warp] = sum;
+    __syncthreads();
+    if (warp == 0) {
+        int64_t v = warp_sums[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) block_sum = v;
+    }
+    cluster.sync();
+    int64_t at = carry ? *carry : 0, total = at;
+    {
+        // everybody's totals; one thread per bucket: its count in all CTAs and in the earlier ones
+        int64_t v[kScanCluster];
+        int h[kScanCluster], all = 0, earlier = 0;
+#pragma unroll
+        for (int r = 0; r < kScanCluster; ++r) {
+            v[r] = *cluster.map_shared_rank(&block_sum, r);
+            h[r] = threadIdx.x < 132 ? cluster.map_shared_rank(hist, r)[threadIdx.x] : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < kScanCluster; ++r) {
+            total += v[r];
+            all += h[r];
+            if (r < rank) { at += v[r]; earlier += h[r]; }
+        }
+        int sum_all;
+        const int before = block_excl_scan(all, sum_all, sm);
+        if (threadIdx.x < 132) cursor[threadIdx.x] = before + earlier;
+    }
+    cluster.sync();   // nobody reads another CTA's memory, or the carry, from here on
+    const bool dropped = overflow && total > capacity;
+    const int32_t total32 = (int32_t)min(total, (int64_t)0x7fffffff);
+    if (rank == 0) {
+        // the first CTA's share starts where the bucket does
+        if (threadIdx.x < kMetaWords) {
+            const int k = threadIdx.x;
+            meta[k] = k == kKinds - 1 ? cursor[131] : k < kKinds - 1 ? cursor[kBucketBelow<10> + 8 * k] : 0;
+        }
+        if (threadIdx.x == 0) {
+            if (n_out) *n_out = total32;
+            if (dropped) *overflow = 1;
+            if (carry) *carry = total;
+            offsets[n_bins] = dropped ? 0 : total32;
+        }
+    }
+    __syncthreads();
+    for (int base = first; base < last; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int c = base == first ? kept : i < last ? count(i) : 0;
+        int round;
+        const int ex = block_excl_scan(c, round, sm);
+        const int bucket = i < last ? tile_order_bucket(c) : -1;
+        const uint32_t peers = __match_any_sync(0xffffffffu, bucket);
+        int slot = 0;
+        if (bucket >= 0 && (peers & lt_mask) == 0) slot = atomicAdd(&cursor[bucket], __popc(peers));
+        slot = __shfl_sync(0xffffffffu, slot, __ffs(peers) - 1) + __popc(peers & lt_mask);
+        if (i < last) {
+            order[slot] = i;
+            int64_t pos = at + ex;
+            ranges[slot] = make_int2((int)min(pos, capacity), (int)min(pos + c, capacity) - (int)min(pos, capacity));
+            offsets[i] = dropped ? 0 : (int32_t)min(pos, (int64_t)0x7fffffff);
+            for (int r0 = 0; r0 < t.replicas; r0 += 8) {
+                int v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = r0 + k < t.replicas ? t.counts[(size_t)(r0 + k) * t.stride + i] : 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (r0 + k < t.replicas) {
+                        t.cursors[(size_t)(r0 + k) * t.stride + i] = (int32_t)min(pos, (int64_t)0x7fffffff);
+                        pos += v[k];
+                    }
+            }
+        }
+        at += round;
+    }
+}
+
+// ---- sorting a tile's range --------------------------------------------------------------------------
+// A group of G threads sorts n <= K G entries: the range between the smallest and the largest depth is cut into about n buckets of equal
+// width in the bits of the depth, the entries are counted into them (the count's return value is an entry's place inside its bucket),
+// a prefix over the buckets places them bucket by bucket in shared memory, and an entry's final place is the start of its bucket plus the
+// number of smaller entries in it: a handful of compares where depths are spread, which they are except in constructed scenes. Where some
+// bucket holds more than kHeavy entries, a bitonic network sorts the list instead. Issue slots (27 M warp instructions for 4.1 M entries, 59 %) and the
+// barriers between the passes bound it: 45 us for 1 M Gaussians at 1296x840 (lists of 967), 157 for 3 M at 1600x1064 (lists of 2,136).
+// Up to eight entries per thread stay in registers between the passes; with sixteen (RELOAD) they are read again.
+constexpr int kSortThreads = 512, kHeavy = 96, kLongLog = 11;
+constexpr int kRoomCta = 16 * kSortThreads, kRoomGroup = 1024, kRoomWarp = 256;
+struct SortShared {
+    uint64_t entry[kRoomCta];
+    uint32_t start[kRoomCta / 32 * 33 + 64];      // every group has its own run and four more words (bucket_slot)
+    uint32_t cum[(1 << kLongLog) + 1];            // long lists: prefix over the bins
+    uint32_t red[2][kSortThreads / 32][2];
+    uint64_t red64[2][kSortThreads / 32];
+    uint32_t cursor;
+};
+
+template <int G>
+__device__ __forceinline__ void group_sync(int group) {
+    if (G == 32) __syncwarp();
+    else if (G == kSortThreads) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(G) : "memory");
+}
+
+// Where a bucket's word lies: one word is left out after every 32, so that threads that own runs of 2 to 16 buckets read different banks.
+__device__ __forceinline__ uint32_t bucket_slot(uint32_t b) { return b + (b >> 5); }
+
+template <int G, int K, bool RELOAD, class Load, class Out>
+__device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t* __restrict__ entry, uint32_t* __restrict__ start,
+                                             uint32_t (*red)[kSortThreads / 32][2], Load load, Out out) {
+    constexpr int kWarps = G / 32;
+    const int lane = tid & 31, warp = tid >> 5;
+    uint64_t key[RELOAD ? 1 : K];
+    uint32_t rank[K];
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = tid + k * G;
+        if (!RELOAD) key[k] = 0;
+        if (i < n) {
+            const uint64_t x = load(i);
+            if (!RELOAD) key[k] = x;
+            const uint32_t d = (uint32_t)(x >> 32);
+            lo = min(lo, d); hi = max(hi, d);
+        }
+    }
+    // as many buckets as entries, a power of two, at least one per thread
+    const int log_b = max(32 - __clz(n - 1), 31 - __clz(G)), buckets = 1 << log_b, per = buckets / G;
+    for (int i = tid; i < buckets + buckets / 32; i += G) start[i] = 0;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (kWarps > 1) {
+        if (lane == 0) { red[0][warp][0] = lo; red[0][warp][1] = hi; }
+        group_sync<G>(group);
+        lo = __reduce_min_sync(0xffffffffu, red[0][lane & (kWarps - 1)][0]);
+        hi = __reduce_max_sync(0xffffffffu, red[0][lane & (kWarps - 1)][1]);
+    } else {
+        __syncwarp();
+    }
+    const int shift = max(0, 32 - __clz(hi - lo) - log_b);
+    auto bucket = [&](uint64_t k) { return ((uint32_t)(k >> 32) - lo) >> shift; };
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = tid + k * G;
+        rank[k] = 0;
+        if (i < n) rank[k] = atomicAdd(&start[bucket_slot(bucket(RELOAD ? load(i) : key[RELOAD ? 0 : k]))], 1u);
+    }
+    group_sync<G>(group);
+    uint32_t sum = 0, most = 0;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+        if (j < per) {
+            const uint32_t c = start[bucket_slot(tid * per + j)];
+            sum += c;
+            most = max(most, c);
+        }
+    uint32_t at = (uint32_t)warp_incl_scan((int)sum);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (kWarps > 1) {
+        if (lane == 31) { red[1][warp][0] = at; red[1][warp][1] = most; }
+        group_sync<G>(group);
+        const uint32_t v = red[1][lane & (kWarps - 1)][0];
+        most = __reduce_max_sync(0xffffffffu, red[1][lane & (kWarps - 1)][1]);
+        at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u);   // warp < kWarps <= 16 lanes
+    }
+    at -= sum;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+        if (j < per) {
+            const uint32_t c = start[bucket_slot(tid * per + j)];
+            start[bucket_slot(tid * per + j)] = at;
+            at += c;
+        }
+    if (tid == G - 1) start[bucket_slot(buckets)] = (uint32_t)n;
+    group_sync<G>(group);
+    if (most > (uint32_t)kHeavy) {
+        const int width = 1 << (32 - __clz(n - 1));   // n > kHeavy > 1
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int i = tid + k * G;
+            if (i < width) entry[i] = i < n ? (RELOAD ? load(i) : key[RELOAD ? 0 : k]) : ~0ull;
+        }
+        for (int size = 2; size <= width; size <<= 1)
+            for (int step = size >> 1; step > 0; step >>= 1) {
+                group_sync<G>(group);
+                for (int q = tid; q < width / 2; q += G) {
+                    const int i = 2 * q - (q & (step - 1)), j = i + step;   // q with a zero bit inserted at `step`
+                    const uint64_t a = entry[i], b = entry[j];
+                    if ((a > b) == ((i & size) == 0)) { entry[i] = b; entry[j] = a; }
+                }
+            }
+        group_sync<G>(group);
+        for (int i = tid; i < n; i += G) out(i, entry[i]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int i = tid + k * G;
+            if (i < n) {
+                const uint64_t x = RELOAD ? load(i) : key[RELOAD ? 0 : k];
+                entry[start[bucket_slot(bucket(x))] + rank[k]] = x;
+            }
+        }
+        group_sync<G>(group);
+        for (int i = tid; i < n; i += G) {
+            const uint64_t mine = entry[i];
+            const uint32_t b = bucket(mine), from = start[bucket_slot(b)], to = start[bucket_slot(b + 1)];
+            uint32_t pos = from;
+            if (to - from > 1)
+                for (uint32_t j = from; j < to; ++j) pos += entry[j] < mine ? 1u : 0u;
+            out((int)pos, mine);
+        }
+    }
+    group_sync<G>(group);
+}
+// n <= 8 G, or 16 G where the entries can be read again
+template <int G, bool LONG, class Load, class Out>
+__device__ __forceinline__ void sort_group(int tid, int group, int n, uint64_t* __restrict__ entry, uint32_t* __restrict__ start,
+                                           uint32_t (*red)[kSortThreads / 32][2], Load load, Out out) {
+    if (n <= 4 * G) sort_group_k<G, 4, false>(tid, group, n, entry, start, red, load, out);
+    else if (!LONG || n <= 8 * G) sort_group_k<G, 8, false>(tid, group, n, entry, start, red, load, out);
+    else sort_group_k<G, 16, true>(tid, group, n, entry, start, red, load, out);
+}
+
+// A list of any length, by the whole CTA: a histogram over 2048 bins of the keys from `next` on (64 bits, which are all different), then
+// runs of bins that hold up to 4096 entries are gathered into shared memory and sorted. A bin that holds more by itself is cut into
+// 2048 again.
+template <class Out>
+__device__ void sort_long(int n, const uint64_t* __restrict__ list, SortShared& sm, Out out) {
+    constexpr int kBins = 1 << kLongLog, kRoom = 8 * kSortThreads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint64_t lo = ~0ull, hi = 0;
+    for (int i = tid; i < n; i += kSortThreads) {
+        const uint64_t k = list[i];
+        lo = min(lo, k); hi = max(hi, k);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) { sm.red64[0][warp] = lo; sm.red64[1][warp] = hi; }
+    __syncthreads();
+    for (int w = 0; w < kSortThreads / 32; ++w) { lo = min(lo, sm.red64[0][w]); hi = max(hi, sm.red64[1][w]); }
+    uint64_t next = lo;   // every smaller key is out
+    int done = 0;
+    while (done < n) {
+        uint64_t top = hi;
+        int shift;
+        for (;;) {
+            shift = max(0, 64 - __clzll((long long)(top - next)) - kLongLog);
+            __syncthreads();
+            for (int i = tid; i < kBins; i += kSortThreads) sm.cum[i] = 0;
+            __syncthreads();
+            for (int i = tid; i < n; i += kSortThreads) {
+                const uint64_t k = list[i];
+                if (k >= next && k <= top) atomicAdd(&sm.cum[(k - next) >> shift], 1u);
+            }
+            __syncthreads();
+            uint32_t c[kBins / kSortThreads], sum = 0;
+#pragma unroll
+            for (int j = 0; j < kBins / kSortThreads; ++j) { c[j] = sm.cum[tid * (kBins / kSortThreads) + j]; sum += c[j]; }
+            uint32_t at = (uint32_t)warp_incl_scan((int)sum);
+            if (lane == 31) sm.red[1][warp][0] = at;
+            __syncthreads();
+            {
+                const uint32_t v = sm.red[1][lane & (kSortThreads / 32 - 1)][0];
+                at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u) - sum;
+            }
+#pragma unroll
+            for (int j = 0; j < kBins / kSortThreads; ++j) { sm.cum[tid * (kBins / kSortThreads) + j] = at; at += c[j]; }
+            if (tid == kSortThreads - 1) sm.cum[kBins] = at;
+            __syncthreads();
+            // the first bin that holds anything: the last one that starts at 0
+            int b = 0;
+            for (int step = kBins / 2; step > 0; step >>= 1)
+                if (sm.cum[b + step] == 0) b += step;
+            if (shift == 0 || sm.cum[b + 1] <= (uint32_t)kRoom) break;
+            next += (uint64_t)b << shift;
+            top = min(top, next + (((uint64_t)1 << shift) - 1));
+        }
+        int s = 0;
+        while (s < kBins && done < n) {
+            const uint32_t have = sm.cum[s];
+            int e = s;   // the last bin boundary within reach
+            for (int step = kBins; step > 0; step >>= 1)
+                if (e + step <= kBins && sm.cum[e + step] - have <= (uint32_t)kRoom) e += step;
+            if (e == s) {
+                if (shift > 0) break;
+                // more than 4096 equal keys: not from this file's callers, but the loop has to end
+                const int m = (int)(sm.cum[s + 1] - have);
+                for (int i = tid; i < m; i += kSortThreads) out(done + i, next + (uint64_t)s);
+                done += m;
+                ++s;
+                continue;
+            }
+            const int m = (int)(sm.cum[e] - have);
+            if (m > 0) {
+                if (tid == 0) sm.cursor = 0;
+                __syncthreads();
+                for (int i = tid; i < n; i += kSortThreads) {
+                    const uint64_t k = list[i];
+                    if (k >= next && k <= top) {
+                        const int b = (int)((k - next) >> shift);
+                        if (b >= s && b < e) sm.entry[min(atomicAdd(&sm.cursor, 1u), (uint32_t)kRoom - 1u)] = k;
+                    }
+                }
+                __syncthreads();
+                sort_group<kSortThreads, false>(tid, 0, m, sm.entry, sm.start, sm.red, [&](int i) { return sm.entry[i]; },
+                                         [&](int i, uint64_t k) { out(done + i, k); });
+                done += m;
+            }
+            s = e;
+        }
+        if (s == kBins || (uint64_t)s > ((top - next) >> shift)) next = top + 1;   // top == hi: done == n
+        else next += (uint64_t)s << shift;
+    }
+    __syncthreads();
+}
+
+// Groups of G threads share lists first .. last - 1 of the launch order: a round gives one list to every group, the longest to the first group of every
+// CTA, then to the second ones, and every other round runs backwards. (By ticket, thousands of groups queue for one counter: 30 us instead of 15 on
+// the smallest scenes.) The range of the next list is on its way while one is sorted.
+template <int G, class Body>
+__device__ __forceinline__ void share_lists(int tid, int group, int first, int last, const int2* __restrict__ ranges, Body body) {
+    const int groups = (int)gridDim.x * (kSortThreads / G), mine = group * (int)gridDim.x + (int)blockIdx.x;
+    auto list = [&](int round) { return first + round * groups + (round & 1 ? groups - 1 - mine : mine); };
+    int2 r = make_int2(0, 0);
+    if (list(0) < last) r = ranges[list(0)];
+    for (int round = 0; first + round * groups < last; ++round) {
+        const int idx = list(round), after = list(round + 1);
+        const int2 now = r;
+        if (after < last) r = ranges[after];
+        if (idx < last && now.y > 0) body(idx, now.x, now.y);
+    }
+}
+
+// OP: operator level, with the 64-bit keys.
+template <bool OP>
+__global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_t* __restrict__ order, const int2* __restrict__ ranges, const int32_t* __restrict__ meta,
+                                                                    const uint64_t* __restrict__ entries, const int32_t* __restrict__ overflow,
+                                                                    int64_t first_bin, uint32_t n_tiles, uint32_t tile_n_bits,
+                                                                    int32_t* __restrict__ flatten_ids, int64_t* __restrict__ isect_ids) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SortShared& sm = *reinterpret_cast<SortShared*>(smem_raw);
+    if (overflow && *overflow) return;
+    const int tid = threadIdx.x;
+    auto writer = [&](int idx, int from) {
+        const int64_t id = OP ? first_bin + order[idx] : 0;
+        const int64_t tile_key = OP ? (id / n_tiles << tile_n_bits | id % n_tiles) << 32 : 0;
+        return [=](int i, uint64_t k) {
+            flatten_ids[from + i] = (int32_t)(uint32_t)k;
+            if (OP) isect_ids[from + i] = tile_key | (int64_t)(k >> 32);
+        };
+    };
+    const int n_cta = meta[kMetaLists], n_group = meta[kMetaLists + 1], n_warp = meta[kMetaLists + 2];
+    share_lists<kSortThreads>(tid, 0, 0, n_cta, ranges, [&](int idx, int from, int n) {
+        if (n <= kRoomCta)
+            sort_group<kSortThreads, true>(tid, 0, n, sm.entry, sm.start, sm.red, [&](int i) { return entries[from + i]; }, writer(idx, from));
+        else
+            sort_long(n, entries + from, sm, writer(idx, from));
+    });
+    __syncthreads();
+    {
+        const int group = tid / 128, t = tid % 128;
+        uint32_t (*red)[kSortThreads / 32][2] = reinterpret_cast<uint32_t (*)[kSortThreads / 32][2]>(&sm.red[0][group * 4][0]);
+        share_lists<128>(t, group, n_cta, n_group, ranges, [&](int idx, int from, int n) {
+            sort_group<128, false>(t, group, n, sm.entry + group * kRoomGroup, sm.start + group * (kRoomGroup / 32 * 33 + 4), red,
+                                   [&](int i) { return entries[from + i]; }, writer(idx, from));
+        });
+    }
+    __syncthreads();
+    {
+        const int group = tid / 32, t = tid % 32;
+        share_lists<32>(t, group, n_group, n_warp, ranges, [&](int idx, int from, int n) {
+            sort_group<32, false>(t, group, n, sm.entry + group * kRoomWarp, sm.start + group * (kRoomWarp / 32 * 33 + 4), sm.red,
+                                  [&](int i) { return entries[from + i]; }, writer(idx, from));
+        });
     }
 }
 
@@ -630,14 +675,6 @@ __global__ void __launch_bounds__(kThreads) isect_offset_kernel(int64_t n, const
     }
 }
 
-__global__ void depth_keys_kernel(int64_t total, const float* __restrict__ depths, const int32_t* __restrict__ tiles,
-                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        keys[i] = tiles[i] > 0 ? __float_as_uint(depths[i]) : 0xFFFFFFFFu;
-        vals[i] = (uint32_t)i;
-    }
-}
-
 __global__ void __launch_bounds__(kThreads) sum_i32_kernel(int64_t n, const int32_t* __restrict__ src, unsigned long long* out) {
     long long s = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) s += src[i];
@@ -663,184 +700,152 @@ int exclusive_scan(const int32_t* src, int64_t n, int32_t* out, int32_t* total_d
     return check_launch("exclusive_scan");
 }
 
-// Words of the list state: tickets [64] | digit counts [2 sorts][4 passes][256] | emission look-back | sort look-back. The first three
-// are zeroed by one memset per list build, the last by the histogram kernel of each sort, which knows the count.
-namespace {
-constexpr size_t kTicketWords = 64, kHistWords = 2 * 4 * 256;   // tickets: nine, and at 32 the word of list_gave_up
-int32_t* list_gave_up(uint32_t* state) { return reinterpret_cast<int32_t*>(state) + 32; }
-size_t emit_state_words(int64_t total) { return ((size_t)((total + kThreads - 1) / kThreads) + 63) / 64 * 64; }
-// Look-back serves short lists, where a sort is mostly launches (16 k keys, four passes: 42 us against 66 with separate counting
-// kernels; 250 k 51 against 68; 1 M 79 against 94); on long lists its waves of tiles queue behind one another's words and the
-// three-kernel pass with one chunk per CTA is the faster one (6 M keys: 217 us against 279; 7 M instances, two passes: 291
-// against 360). A device-side count is bounded by the list's capacity, which users leave a few times larger than the list.
-int64_t lookback_limit(bool count_on_device) { return count_on_device ? (int64_t)6 << 20 : (int64_t)2 << 20; }
-constexpr int64_t kMaxChunks = 1024;   // the size query must not depend on a device
-int chunk_blocks(int64_t n_max) { return (int)min((n_max + kTile - 1) / kTile, min((int64_t)4 * num_sms(), kMaxChunks)); }
-// Never less for a longer list, although a chunked sort needs less than the longest look-back: a workspace made for a capacity
-// serves every list up to it.
-size_t sort_state_words(bool count_on_device, int64_t n, int passes) {
-    const int64_t limit = lookback_limit(count_on_device);
-    const size_t lookback = (size_t)((min(n, limit) + kTile - 1) / kTile) * 256 * passes;
-    const size_t chunked = n > limit ? (size_t)256 * (min((n + kTile - 1) / kTile, kMaxChunks) + 1) : 0;
-    return lookback > chunked ? lookback : chunked;
-}
-int tile_sort_passes(int key_bits) { return (key_bits + 7) / 8; }
-}  // namespace
-
-size_t tile_list_state_words(int64_t total, int64_t capacity, int key_bits) {
-    // the instance count is read on the device, the number of Gaussians is not
-    const size_t depth = sort_state_words(false, total, 4);
-    const size_t tile = sort_state_words(true, capacity, tile_sort_passes(key_bits));
-    return kTicketWords + kHistWords + emit_state_words(total) + (depth > tile ? depth : tile);
-}
-
-// Stable LSD radix sort of (key, value) uint32 pairs over key bits [0, key_bits). n is read from *n_dev when n_dev != nullptr
-// (device-side count, bounded by n_max), else n_max is the count. Returns the index (0 or 1) of the pair holding the result.
-// tickets [4], hist [4 * 256]: zero on entry. state: sort_state_words.
-static int radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], const int32_t* n_dev, int64_t n_max, int key_bits,
-                            uint32_t* tickets, uint32_t* hist, uint32_t* state, int32_t* gave_up, cudaStream_t st) {
-    if (n_max <= 0 || key_bits <= 0) return 0;
-    const int passes = tile_sort_passes(key_bits);
-    const int bits = (key_bits + passes - 1) / passes;
-    const uint32_t mask = (1u << bits) - 1u;
-    int cur = 0;
-    LFS_TIMED(n_dev ? "radix_sort_tile" : "radix_sort_depth", st);
-    if (n_max <= lookback_limit(n_dev != nullptr)) {
-        const int64_t max_tiles = (n_max + kTile - 1) / kTile;
-        // six CTAs per SM (27 KB of shared memory each) keep enough keys in flight; more only queue for tickets
-        const int nb = (int)min(max_tiles, (int64_t)6 * num_sms());
-        radix_hist_kernel<<<(int)min(max_tiles, (int64_t)4 * num_sms()), kThreads, 0, st>>>(
-            keys[0], n_dev, n_max, bits, passes, hist, reinterpret_cast<uint4*>(state), max_tiles * 64);
-        for (int p = 0; p < passes; ++p) {
-            radix_scatter_kernel<<<nb, kThreads, 0, st>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n_dev, n_max,
-                                                                 p * bits, mask, hist + p * 256, tickets + p,
-                                                                 state + (size_t)p * max_tiles * 256, gave_up);
-            cur ^= 1;
-        }
-    } else {
-        const int nb = chunk_blocks(n_max);
-        uint32_t *table = state, *totals = state + (size_t)256 * nb;
-        for (int p = 0; p < passes; ++p) {
-            radix_count_kernel<<<nb, kThreads, 0, st>>>(keys[cur], n_dev, n_max, p * bits, mask, nb, table);
-            radix_scan_kernel<<<256, kThreads, 0, st>>>(table, nb, totals);
-            radix_scatter_chunk_kernel<<<nb, kThreads, 0, st>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], n_dev, n_max, p * bits,
-                                                                mask, nb, table, totals);
-            cur ^= 1;
-        }
-    }
-    if (check_launch("radix_sort") != LFS_OK) return -1;
-    return cur;
-}
-
 static uint32_t bit_width_u32(uint32_t v) {
     uint32_t b = 0;
     while (v) { ++b; v >>= 1; }
     return b;
 }
 
+// ---- list state: kMetaWords | carry (int64) | counts [replicas][stride] | cursors [replicas][stride] | order [bins] | ranges [bins] | offsets [bins + 1] --------
+namespace {
+int64_t pad8(int64_t n) { return (n + 7) / 8 * 8; }
+// Counters of neighbouring tiles share a 32-byte sector, and the memory system applies one request to a sector at a time: some 12 cycles each.
+// On small images, where a tile has thousands of instances, that is a queue, so the counters exist several times and Gaussians take them
+// in turn, 32 at a time; up to 16 sets and 65,536 counters (more cost the scan what they save, and tear a tile's entries apart). Scatter in us with one set of counters and now: 150 k Gaussians at
+// 640x360 47 and 15, 1 M at 1296x840 116 and 58, 6 M 180 degree fisheye at 1920x1920 322 and 174; counting them inside the projection 33 and 3, 20 and 15.
+int list_replicas(int64_t bins) {
+    int r = 1;
+    while (r < 16 && bins * r * 2 <= 65536) r *= 2;
+    return r;
+}
+struct ListState {
+    int32_t *meta, *order, *offsets;
+    int64_t* carry;
+    int2* ranges;
+    TileCounters t;
+};
+ListState list_state(int32_t* base, int64_t bins) {
+    ListState s;
+    s.meta = base;
+    s.carry = reinterpret_cast<int64_t*>(base + kMetaWords);
+    s.t.replicas = list_replicas(bins);
+    s.t.stride = (int32_t)pad8(bins);
+    s.t.counts = base + kMetaWords + 16;
+    s.t.cursors = s.t.counts + (size_t)s.t.replicas * s.t.stride;
+    s.order = s.t.cursors + (size_t)s.t.replicas * s.t.stride;
+    s.ranges = reinterpret_cast<int2*>(s.order + pad8(bins));
+    s.offsets = s.order + 3 * pad8(bins);
+    return s;
+}
+size_t list_words(int64_t bins, int64_t counters) { return (size_t)(kMetaWords + 16 + 2 * counters + 3 * pad8(bins) + pad8(bins + 1)); }
+}  // namespace
+
+size_t tile_list_state_words(int64_t bins) { return list_words(bins, list_replicas(bins) * pad8(bins)); }
+TileCounters tile_list_counters(int32_t* state, int64_t bins) { return list_state(state, bins).t; }
+const int32_t* tile_list_order(const int32_t* state, int64_t bins) { return list_state(const_cast<int32_t*>(state), bins).order; }
+int clear_tile_counters(const TileCounters& t, cudaStream_t st) {
+    return cudaMemsetAsync(t.counts, 0, (size_t)t.replicas * t.stride * sizeof(int32_t), st) == cudaSuccess ? LFS_OK : LFS_ECUDA;
+}
+
+static int launch_tile_scan(int bins, const ListState& s, int64_t capacity, int64_t* carry, int32_t* n_out, int32_t* overflow, int32_t* offsets, cudaStream_t st) {
+    LFS_TIMED("tile_scan", st);
+    tile_scan_kernel<<<kScanCluster, 1024, 0, st>>>(bins, s.t, capacity, carry, n_out, overflow, offsets, s.order, s.ranges, s.meta);
+    return check_launch("tile_scan");
+}
+
+template <bool OP>
+static int launch_tile_sort(int bins, const ListState& s, const uint64_t* entries, const int32_t* overflow, int64_t first_bin, uint32_t n_tiles,
+                            uint32_t tile_n_bits, int32_t* flatten_ids, int64_t* isect_ids, cudaStream_t st) {
+    LFS_TIMED("tile_sort", st);
+    cudaFuncSetAttribute(tile_sort_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortShared));
+    tile_sort_kernel<OP><<<min(bins, 2 * num_sms()), kSortThreads, sizeof(SortShared), st>>>(s.order, s.ranges, s.meta, entries, overflow, first_bin, n_tiles,
+                                                                                             tile_n_bits, flatten_ids, isect_ids);
+    return check_launch("tile_sort");
+}
+
 int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
-    const int64_t total = (int64_t)a.C * a.N;
-    const uint32_t n_tiles = (uint32_t)a.tw * a.th;
-    const uint32_t tile_n_bits = bit_width_u32(n_tiles);
-    const uint32_t cam_n_bits = bit_width_u32((uint32_t)a.C);
-    if (tile_n_bits + cam_n_bits > 32) {
-        set_error("build_tile_lists: tile and camera ids need more than 32 bits");
-        return LFS_EINVAL;
-    }
-    const int key_bits = (int)(tile_n_bits + cam_n_bits);
-    uint32_t *tickets = a.state, *hist = tickets + kTicketWords, *emit_state = hist + kHistWords;
-    uint32_t* sort_state = emit_state + emit_state_words(total);
-    // raised by a look-back that ran out of polls; without an overflow flag of the caller's a word behind the tickets, read by
-    // compose_isect_ids_kernel
-    int32_t* gave_up = a.overflow ? a.overflow : list_gave_up(a.state);
-    cudaMemsetAsync(a.state, 0, (kTicketWords + kHistWords + emit_state_words(total)) * sizeof(uint32_t), st);
-    const uint32_t* order = nullptr;
-    if (a.sort) {
-        if (!a.keys_ready) {
-            depth_keys_kernel<<<grid_for(total, 256), 256, 0, st>>>(total, a.depths, a.tiles, a.gkeys[0], a.gvals[0]);
+    const int bins = a.tw * a.th;
+    const ListState s = list_state(a.state, bins);
+    int rc = launch_tile_scan(bins, s, a.capacity, nullptr, a.n_isects_dev, a.overflow, a.tile_offsets, st);
+    if (rc != LFS_OK) return rc;
+    if (a.N > 0 && a.capacity > 0 && bins > 0) {
+        {
+            LFS_TIMED("tile_scatter", st);
+            if (a.ewa_bounds)
+                ewa_scatter_kernel<<<grid_for(a.N, kThreads), kThreads, 0, st>>>(a.N, a.tw, a.tiles, a.ewa_bounds, a.ewa_masks, a.ewa_records, a.ewa_depth_bits,
+                                                                                 bins, a.capacity, a.overflow, s.t, a.entries);
+            else
+                tile_scatter_kernel<<<grid_for(a.N, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d, a.radii,
+                                                                                  a.depths, 0, bins, a.capacity, a.overflow, s.t, a.entries);
         }
-        uint32_t* k[2] = {a.gkeys[0], a.gkeys[1]};
-        uint32_t* v[2] = {a.gvals[0], a.gvals[1]};
-        const int sel = radix_sort_pairs(k, v, nullptr, total, 32, tickets, hist, sort_state, gave_up, st);
-        if (sel < 0) return LFS_ECUDA;
-        order = v[sel];
-    }
-    if (total > 0) {
-        LFS_TIMED("emit_instances", st);
-        // Four Gaussians per thread make fewer tickets and a shorter look-back, one makes more CTAs in flight. us with one and with four,
-        // 1296x840 (in thousands of Gaussians): 450: 33 / 57, 1000: 54 / 71, 1500: 69 / 66, 2000: 93 / 76, 3000: 137 / 118. EWA, whose
-        // rectangle walk is longer than the scan: 300: 58 / 133, 450: 67 / 111, 700: 99 / 124, 1000: 123 / 107, 2000: 259 / 185.
-        const bool four = total > (a.ewa_bounds ? (int64_t)850000 : (int64_t)2 << 20);
-        const int64_t list = four ? kThreads * kEmitItems : kThreads;
-        const int nb = (int)min((total + list - 1) / list, (int64_t)8 * num_sms());
-#define LFS_EMIT(EWA, ITEMS)                                                                                                                 \
-    emit_instances_kernel<EWA, ITEMS><<<nb, kThreads, 0, st>>>(total, a.N, order, a.tiles, a.means2d, a.radii, a.ewa_bounds, a.ewa_records,    \
-                                                        (float)a.tile_size, (uint32_t)a.tw, (uint32_t)a.th, tile_n_bits, a.capacity,   \
-                                                        a.tkeys[0], a.tvals[0], a.overflow, gave_up, a.n_isects_dev, tickets + 8, emit_state)
-        if (a.ewa_bounds) { if (four) LFS_EMIT(true, kEmitItems); else LFS_EMIT(true, 1); }
-        else { if (four) LFS_EMIT(false, kEmitItems); else LFS_EMIT(false, 1); }
-#undef LFS_EMIT
-    } else {
-        cudaMemsetAsync(a.n_isects_dev, 0, sizeof(int32_t), st);
-    }
-    int sel = 0;
-    if (a.sort && a.capacity > 0) {
-        uint32_t* k[2] = {a.tkeys[0], a.tkeys[1]};
-        uint32_t* v[2] = {a.tvals[0], a.tvals[1]};
-        sel = radix_sort_pairs(k, v, a.n_isects_dev, a.capacity, key_bits, tickets + 4, hist + 4 * 256, sort_state, gave_up, st);
-        if (sel < 0) return LFS_ECUDA;
-    }
-    if (a.sel_out) *a.sel_out = sel;
-    if (a.tile_offsets) {
-        const int64_t n_ids = (int64_t)a.C * n_tiles;
-        LFS_TIMED("tile_offsets", st);
-        tile_offsets_kernel<<<grid_for(a.capacity > 0 ? a.capacity : 1, 256), 256, 0, st>>>(
-            a.tkeys[sel], a.n_isects_dev, a.capacity, n_tiles, tile_n_bits, n_ids, a.overflow, a.tile_offsets);
+        rc = launch_tile_sort<false>(bins, s, a.entries, a.overflow, 0, 1, 0, a.flatten_ids, nullptr, st);
+        if (rc != LFS_OK) return rc;
     }
     return check_launch("build_tile_lists");
 }
 
-// Launch order of the tile CTAs: tiles with the longest lists first, so that the last wave of a rasterizer launch
-// is made of short tiles. 132 buckets by the leading one and the next two bits of the list length (a
-// floating-point-like key with a 2-bit mantissa); the order inside a bucket is arbitrary. offsets has n_tiles + 1
-// entries.
-__device__ __forceinline__ int tile_order_bucket(int c) {
-    if (c <= 0) return 131;
-    const int lz = __clz(c);                              // 0 .. 31, small = long list
-    const int shift = max(0, 29 - lz);                    // bring the two bits below the leading one down
-    const int mant = (c >> shift) & 3;
-    return lz * 4 + (3 - mant);
+// Operator level. The grid is not known to the workspace query, so the per-bin arrays hold kOperatorBins bins and larger grids take
+// several rounds.
+constexpr int64_t kOperatorBins = 1 << 17;
+
+size_t isect_lists_bytes(int64_t total, int64_t n_isects, IsectBuffers* b, void* base) {
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        off = (off + 255) & ~(size_t)255;
+        void* p = base ? reinterpret_cast<char*>(base) + off : nullptr;
+        off += bytes;
+        return p;
+    };
+    IsectBuffers x;
+    // any number of bins up to kOperatorBins, each with its replicas: 65,536 counters and the padding of 16 sets, or one set
+    x.state = (int32_t*)take(list_words(kOperatorBins, kOperatorBins + 8 * 16) * sizeof(int32_t));
+    x.scratch.block_sums = (uint32_t*)take((kScanBlocks + 1) * sizeof(uint32_t));
+    // sorted: the entries; unsorted: the prefix over the Gaussians
+    const size_t entries = (size_t)n_isects * sizeof(uint64_t), prefix = (size_t)total * sizeof(int32_t);
+    void* p = take(entries > prefix ? entries : prefix);
+    x.entries = (uint64_t*)p;
+    x.prefix = (int32_t*)p;
+    if (b) *b = x;
+    return (off + 255) & ~(size_t)255;
 }
 
-__global__ void __launch_bounds__(1024) tile_order_kernel(int n_tiles, const int32_t* __restrict__ offsets,
-                                                          int32_t* __restrict__ order) {
-    __shared__ int hist[132], cursor[132];
-    if (threadIdx.x < 132) hist[threadIdx.x] = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < n_tiles; t += blockDim.x) atomicAdd(&hist[tile_order_bucket(offsets[t + 1] - offsets[t])], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int b = 0; b < 132; ++b) { cursor[b] = run; run += hist[b]; }
+int build_isect_lists(int C, int N, int tw, int th, int tile_size, int sort, const float* means2d, const int32_t* radii, const float* depths,
+                      const int32_t* tiles, int64_t n_isects, const IsectBuffers& b, int64_t* isect_ids, int32_t* flatten_ids, cudaStream_t st) {
+    const int64_t total = (int64_t)C * N, n_ids = (int64_t)C * tw * th;
+    const uint32_t n_tiles = (uint32_t)tw * th, tile_n_bits = bit_width_u32(n_tiles);
+    if (tile_n_bits + bit_width_u32((uint32_t)C) > 32) {
+        set_error("build_isect_lists: tile and camera ids need more than 32 bits");
+        return LFS_EINVAL;
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < n_tiles; t += blockDim.x)
-        order[atomicAdd(&cursor[tile_order_bucket(offsets[t + 1] - offsets[t])], 1)] = t;
-}
-
-int launch_tile_order(int n_tiles, const int32_t* offsets, int32_t* order, cudaStream_t st) {
-    if (n_tiles <= 0) return LFS_OK;
-    LFS_TIMED("tile_order", st);
-    tile_order_kernel<<<1, 1024, 0, st>>>(n_tiles, offsets, order);
-    return check_launch("tile_order");
-}
-
-int launch_compose_isect_ids(int64_t n, const uint32_t* tkeys, const uint32_t* tvals, const float* depths, const uint32_t* list_state,
-                             int64_t* isect_ids, int32_t* flatten_ids, cudaStream_t st) {
-    if (n <= 0) return LFS_OK;
-    compose_isect_ids_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, tkeys, tvals, depths, list_gave_up(const_cast<uint32_t*>(list_state)), isect_ids,
-                                                                flatten_ids);
-    return check_launch("compose_isect_ids");
+    const int grid = grid_for(total, kThreads);
+    if (!sort) {
+        const int rc = exclusive_scan(tiles, total, b.prefix, nullptr, b.scratch, st);
+        if (rc != LFS_OK) return rc;
+        LFS_TIMED("emit_unsorted", st);
+        emit_unsorted_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tile_n_bits, tiles, b.prefix, means2d, radii, depths, n_isects,
+                                                        isect_ids, flatten_ids);
+        return check_launch("emit_unsorted");
+    }
+    cudaMemsetAsync(list_state(b.state, 1).carry, 0, sizeof(int64_t), st);
+    for (int64_t first = 0; first < n_ids; first += kOperatorBins) {
+        const int bins = (int)min(kOperatorBins, n_ids - first);
+        const ListState s = list_state(b.state, bins);
+        if (clear_tile_counters(s.t, st) != LFS_OK) { set_error("build_isect_lists: memset failed"); return LFS_ECUDA; }
+        {
+            LFS_TIMED("tile_histogram", st);
+            tile_histogram_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, first, bins, s.t);
+        }
+        int rc = launch_tile_scan(bins, s, n_isects, s.carry, nullptr, nullptr, s.offsets, st);
+        if (rc != LFS_OK) return rc;
+        {
+            LFS_TIMED("tile_scatter", st);
+            tile_scatter_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, depths, first, bins, n_isects, nullptr,
+                                                           s.t, b.entries);
+        }
+        rc = launch_tile_sort<true>(bins, s, b.entries, nullptr, first, n_tiles, tile_n_bits, flatten_ids, isect_ids, st);
+        if (rc != LFS_OK) return rc;
+    }
+    return check_launch("build_isect_lists");
 }
 
 int launch_isect_offset(int64_t n, const int64_t* isect_ids, int C, int tw, int th, int32_t* offsets, cudaStream_t st) {

@@ -1,0 +1,66 @@
+"""Tile lists against a stable host sort of the same instances: lists on both sides of every size at which the sorting groups change, depths that
+defeat the buckets (equal, few, one far away, negative), rectangles larger than a warp, several cameras, more tiles than one round holds."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+F = np.float32
+
+
+def _instances(m, r, d, ts, tw, th):
+    """(64-bit key, flattened index) of every instance in emission order."""
+    keys, ids = [], []
+    C, N = d.shape
+    for c in range(C):
+        lo = [np.minimum(np.maximum(np.floor(m[c, :, a] / F(ts) - r[c, :, a].astype(F) / F(ts)), 0), n).astype(np.int64) for a, n in ((0, tw), (1, th))]
+        hi = [np.minimum(np.maximum(np.ceil(m[c, :, a] / F(ts) + r[c, :, a].astype(F) / F(ts)), 0), n).astype(np.int64) for a, n in ((0, tw), (1, th))]
+        w = hi[0] - lo[0]
+        n = np.where((r[c] > 0).all(-1), w * (hi[1] - lo[1]), 0)
+        g = np.repeat(np.arange(N), n)
+        local = np.arange(n.sum()) - (np.cumsum(n) - n)[g]
+        tile = (lo[1][g] + local // np.maximum(w[g], 1)) * tw + lo[0][g] + local % np.maximum(w[g], 1)
+        depth = d[c].view(np.uint32).astype(np.int64)[g]
+        keys.append((((c << int(tw * th).bit_length()) | tile) << 32) | depth)
+        ids.append(g + c * N)
+    return np.concatenate(keys), np.concatenate(ids)
+
+
+def _check(pkg, m, r, d, tw, th, ts=16):
+    m, r, d = m.astype(F), r.astype(np.int32), d.astype(F)
+    keys, ids = _instances(m, r, d, ts, tw, th)
+    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (m, r, d)]
+    for sort in (True, False):
+        _, k, i = pkg.ops.intersect_tile(*t, None, None, d.shape[0], ts, tw, th, sort)
+        o = np.argsort(keys, kind="stable") if sort else slice(None)
+        assert np.array_equal(k.cpu().numpy(), keys[o]) and np.array_equal(i.cpu().numpy(), ids[o])
+
+
+DEPTHS = {
+    "spread": lambda rng, n: rng.random(n) * 5 + 0.5,
+    "equal": lambda rng, n: np.full(n, 3.25),
+    "few": lambda rng, n: rng.integers(1, 5, n).astype(float),
+    "far": lambda rng, n: np.concatenate([[9000.0], rng.random(n - 1) * 1e-3 + 2]),
+    "negative": lambda rng, n: rng.standard_normal(n),
+}
+
+
+@pytest.mark.parametrize("depths", DEPTHS)
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 128, 129, 255, 256, 512, 513, 1023, 1024, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 9000, 70_001])
+def test_one_list(pkg, n, depths):
+    d = DEPTHS[depths](np.random.default_rng(n), n)
+    _check(pkg, np.full((1, n, 2), 8.0), np.ones((1, n, 2)), d[None], 1, 1)
+
+
+@pytest.mark.parametrize("C,N,tw,th,ts,radius", [
+    (1, 20_000, 40, 27, 16, 30),      # lists of all the sizes
+    (2, 5000, 13, 9, 16, 60),
+    (5, 2000, 1, 1, 16, 4),
+    (1, 30, 700, 600, 16, 6000),      # rectangles of thousands of tiles; 420,000 tiles: four rounds
+    (3, 300, 500, 400, 4, 300),       # rounds that end inside a camera
+    (1, 100_000, 3, 2, 16, 12),
+])
+def test_many_lists(pkg, C, N, tw, th, ts, radius):
+    rng = np.random.default_rng(N)
+    m = rng.random((C, N, 2)) * [tw * ts, th * ts]
+    _check(pkg, m, rng.integers(0, radius, (C, N, 2)), np.exp(rng.standard_normal((C, N))), tw, th, ts)
