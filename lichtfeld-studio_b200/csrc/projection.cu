@@ -180,7 +180,9 @@ __device__ __forceinline__ bool project_gaussian(const CamDev& cam, const ProjPa
     float ipx[7], ipy[7];
     float m2x = 0.f, m2y = 0.f;
     bool valid = pp.require_all;
-#pragma unroll
+    AxisAngle first{0.0, 0.0, 0.0};
+    // the fisheye's seven arc tangents would not leave the instruction cache room for the rest of the kernel
+#pragma unroll (MODEL == LFS_FISHEYE && !RS ? 1 : 7)
     for (int i = 0; i < 7; ++i) {
         f3 p = mean;
         if (i > 0) {
@@ -190,7 +192,7 @@ __device__ __forceinline__ bool project_gaussian(const CamDev& cam, const ProjPa
             p = (i <= 3) ? (mean + delta) : (mean - delta);
         }
         float px, py;
-        const bool pv = world_point_to_image<MODEL, RS>(cam, p, pp.margin, px, py);
+        const bool pv = world_point_to_image<MODEL, RS>(cam, p, pp.margin, px, py, &first);
         if (pp.require_all) {
             valid &= pv;
             if (!pv) return false;
@@ -607,13 +609,13 @@ int launch_pack_records(int N, const float* means, const float* quats, const flo
 // tile count, instances per tile, SH colour (+0.5, clamped at 0), packed record, zeroed gradient
 // accumulator row. Invisible Gaussians get radii 0 and tile count 0.
 // ---------------------------------------------------------------------------------------------
-// Bound by instruction issue and the latency of the per-Gaussian chain, not by memory: 64 registers and four CTAs per SM for the
-// models that project in single precision (1 M Gaussians 127 us against 135 with three CTAs, 6 M at 4K 655 against 720); the
-// fisheye evaluates seven double-precision arc tangents per Gaussian and wants its 128 registers instead (6 M: 1120 us against
-// 1176 with three CTAs and 1249 with four). Since the cut record (48 bytes and some 30 instructions per visible Gaussian) 136 and
-// 697 us; the fisheye, with its box for either side of the camera too, 1329.
+// Bound by instruction issue (some 2,900 warp instructions per 32 Gaussians, 60 % of the slots), the latency of the per-Gaussian chain and
+// instruction fetch: four CTAs of 64 registers per SM (1 M Gaussians 152 us, with three 151, with five and 190 bytes of spills 183; 6 M at 4K 762,
+// 799 and 932). Of the 152 us the record takes 39, the colour 37, clearing the gradient rows 10, counting the instances 11, activations in double 9.
+// The fisheye (6 M at 1920x1920) took 1363 us with seven double-precision arc tangents unrolled, 128 registers and two CTAs; 1309 with the arc
+// tangents of angle_near, 1262 with the loop over the points rolled up and four CTAs (1260 with three, 1396 with two).
 template <int MODEL, bool RS>
-__global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE ? 2 : 4) project_pack_kernel(
+__global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE && RS ? 2 : 4) project_pack_kernel(
     int N, int K, int sh_degree, const float* __restrict__ means, const float* __restrict__ sh0,
     const float* __restrict__ shN, const float* __restrict__ scaling_raw, const float* __restrict__ rotation_raw,
     const float* __restrict__ opacity_raw, const CamDev* __restrict__ cams, ProjParams pp, PackOptions opt, float tile_size,
