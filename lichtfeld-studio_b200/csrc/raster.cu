@@ -5,24 +5,28 @@
 // (K8) with the VJPs of gsplat/Utils.cuh:104-194, gsplat/SphericalHarmonicsCUDA.cu:445 (K3) and the
 // activation backward that autograd performs for src/core/splat_data.cpp:267-286.
 //
-// Design (instruction-issue bound, no tensor cores: the largest contraction is 3x3):
-//  * one CTA per 16x16 tile. Forward: one thread per pixel, a warp covers a patch of 8x4 pixels. Backward: one or two horizontally
-//    adjacent pixels per thread, patches of 4x8 or 8x8 (launch_raster_bwd says where which);
-//  * the tile's depth-sorted Gaussians are staged in shared memory in batches (192 records forward, 64 backward) of
-//    packed 64-byte records built once per Gaussian, so no per-Gaussian work is repeated per tile or per pixel;
-//  * per warp, a ballot over the batch keeps the records whose screen-space box overlaps the warp's patch and whose forms
-//    reach the cut on it (patch_reached);
+// Design (bound by instruction issue and the shared-memory pipe; no tensor cores: the largest contraction is 3x3):
+//  * a warp owns a patch of pixels and walks its tile's depth-sorted list by itself, 32 entries at a time: no barrier. (With the four or eight warps of a
+//    tile on one staged batch, a seventh to a fifth of the warps' time was waiting for one another: 1 M Gaussians, 1296x840, backward 760 -> 721 us,
+//    3 M at 1600x1064 2415 -> 1983, where warps also start at their own last contributor);
+//  * the packed 64-byte records are built once per Gaussian, so no per-Gaussian work is repeated per tile or per pixel. A warp looks at the boxes of
+//    32 entries and fetches the records of those that overlap its patch (EntryFeed); a ballot keeps the ones whose forms reach the cut on it
+//    (patch_reached);
 //  * per pair the response is exp(-|g|^2 phi / 2), phi = (e1^2 + e2^2) / (e1^2 + e2^2 + w^2) with three linear forms of the
 //    pixel direction (RayFrame, gsmath.cuh): 10 instructions up to the exp-free rejection test for the planar camera models
-//    against 23 for u = M d, u x g and the two norms (1 M Gaussians, 1296x840, when it was brought in: forward 624 -> 430 us,
-//    backward 1441 -> 1065 with nothing else changed; with the cut decided as before (kept_at_cut) 399 and 787 today);
+//    against 23 for u = M d, u x g and the two norms;
+//  * a thread owns one pixel or two horizontally adjacent ones, held in the halves of 64-bit registers and evaluated by the packed fp32 instructions
+//    (launch_raster_fwd says where which). 1 M Gaussians, 1296x840: backward 719 us against 755 with two scalar evaluations, 579 M warp instructions
+//    against 694; forward 352 against 388;
 //  * backward: every (warp, Gaussian) contribution is 12 numbers that are LINEAR in the per-pixel terms (kSums). They
-//    are summed over the warp by a transpose through padded shared-memory rows (warp_reduce) and leave as one coalesced reduction
-//    to the Gaussian's accumulator row. The nonlinear quaternion / scale VJP runs once per Gaussian in the epilogue instead of once
+//    are summed over the warp by a transpose through padded shared-memory rows, in the shadow of the next entry's evaluation, and leave as one coalesced
+//    reduction to the Gaussian's accumulator row. The nonlinear quaternion / scale VJP runs once per Gaussian in the epilogue instead of once
 //    per pixel pair;
-//  * a rolling shutter gives every pixel its own ray origin: the RS instantiations keep u = M d and 16 sums.
+//  * a rolling shutter gives every pixel its own ray origin: its kernels (_rs) keep u = M d and 16 sums, one pixel per thread and the tile's list staged for
+//    all warps.
 #include "gsmath.cuh"
 #include "raster.cuh"
+#include <math_constants.h>
 
 namespace lfs {
 
@@ -118,9 +122,8 @@ __device__ __forceinline__ PatchRays patch_rays(const f3* d, const bool* takes_p
 // each, against the 40 - 140 of a walked entry: 1 M Gaussians at 1296x840 forward 429 -> 382 us, backward 816 -> 759; 6 M at 4K
 // 1440 -> 1224; 6 M 180 degree fisheye, whose boxes are ring sectors, 1382 -> 1129.
 template <int MODEL>
-__device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, float slope, const PatchRays& P) {
+__device__ __forceinline__ bool patch_reached(const float4& r0, const float4& r1, const float4& r2, float slope, const PatchRays& P) {
     constexpr bool planar = MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV;
-    const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2];
     const RayForms f = ray_forms<MODEL>(r0, r1, r2, P.c);
     const float inv = rsqrtf(fmaxf(f.E, 1e-37f));
     const float u1 = f.e1 * inv, u2 = f.e2 * inv;
@@ -138,7 +141,7 @@ __device__ __forceinline__ bool patch_reached(const float4* __restrict__ rec, fl
 // The products and sums are spelled out, so that the set does not depend on a compiler's contraction either.
 // For PX pixels of one thread, as bits. cut: the first row of the Gaussian's cut record, the others n apart; rays: stride apart.
 // A call, since fewer than one walked entry in a hundred comes here and the registers of the callers' loops should not be shaped
-// by it (1 M Gaussians, 1296x840: backward 786 us against 845 inlined; forward 398 either way. Without this test 760 and 382).
+// by it (1 M Gaussians, 1296x840, with the kernels of the time: backward 786 us against 845 inlined; forward 398 either way).
 template <int PX>
 __device__ __noinline__ uint32_t kept_at_cut(const float4* cut, int64_t n, const f3* rays, int stride, float opacity) {
     auto dot = [](float a0, float b0, float a1, float b1, float a2, float b2) { return fmaf(a2, b2, fmaf(a0, b0, __fmul_rn(a1, b1))); };
@@ -217,26 +220,323 @@ __device__ __forceinline__ void issue_stage(Stage<BATCH>& st, uint32_t* sid, con
 }
 
 // ---------------------------------------------------------------------------------------------
-// EXTRA = false: three colour channels (render mode RGB). EXTRA = true: `channels` is 1 or 4 and the last
+// Two pixels of one thread as one operand of the packed fp32 instructions (one issue slot for both, each half rounded like the
+// scalar instruction). A factor that both pixels share costs nothing to replicate: in a loop of nothing else, four packed fmas with
+// replicated factors take 5.9 issue slots and 0.62 of the time of the eight scalar fmas (10.5).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 both2(float a) { return pair2(a, a); }
+__device__ __forceinline__ float2 halves2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// The same names for one pixel, so that the kernels are written once. Pixels<PX>: what PX pixels of a thread are held in.
+__device__ __forceinline__ float add2(float a, float b) { return a + b; }
+__device__ __forceinline__ float mul2(float a, float b) { return a * b; }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return fmaf(a, b, c); }
+template <int PX>
+struct Pixels {
+    using V = f32x2;
+    static __device__ __forceinline__ V make(const float* a) { return pair2(a[0], a[1]); }
+    static __device__ __forceinline__ V all(float a) { return both2(a); }
+    static __device__ __forceinline__ void get(V v, float* a) { const float2 h = halves2(v); a[0] = h.x; a[1] = h.y; }
+    static __device__ __forceinline__ float sum(V v) { const float2 h = halves2(v); return h.x + h.y; }
+};
+template <>
+struct Pixels<1> {
+    using V = float;
+    static __device__ __forceinline__ V make(const float* a) { return a[0]; }
+    static __device__ __forceinline__ V all(float a) { return a; }
+    static __device__ __forceinline__ void get(V v, float* a) { a[0] = v; }
+    static __device__ __forceinline__ float sum(V v) { return v; }
+};
+template <int PX>
+struct PixelForms { typename Pixels<PX>::V e1, e2, w, E, den; };
+template <int MODEL, int PX>
+__device__ __forceinline__ PixelForms<PX> pixel_forms(const float4& r0, const float4& r1, const float4& r2, typename Pixels<PX>::V dx,
+                                                      typename Pixels<PX>::V dy, typename Pixels<PX>::V dz) {
+    using P = Pixels<PX>;
+    PixelForms<PX> f;
+    if (MODEL == LFS_PINHOLE || MODEL == LFS_PINHOLE_OPENCV) {
+        f.e1 = fma2(P::all(r0.x), dx, fma2(P::all(r0.y), dy, P::all(r0.z)));
+        f.e2 = fma2(P::all(r1.y), dy, P::all(r1.z));
+        f.w = fma2(P::all(r2.x), dx, fma2(P::all(r2.y), dy, P::all(r2.z)));
+    } else {
+        f.e1 = fma2(P::all(r0.x), dx, fma2(P::all(r0.y), dy, mul2(P::all(r0.z), dz)));
+        f.e2 = fma2(P::all(r1.x), dx, fma2(P::all(r1.y), dy, mul2(P::all(r1.z), dz)));
+        f.w = fma2(P::all(r2.x), dx, fma2(P::all(r2.y), dy, mul2(P::all(r2.z), dz)));
+    }
+    f.E = fma2(f.e1, f.e1, mul2(f.e2, f.e2));
+    f.den = fma2(f.w, f.w, f.E);
+    return f;
+}
+
+// A warp's own staging of 32 entries, part by part: lanes that read the same part of 32 entries (the culling) touch consecutive 16-byte
+// words. With the four parts of an entry side by side those loads were 64 bytes apart and took four times as many passes.
+struct WarpStage {
+    float4 rec[4][32];
+    float2 zw[32];       // slope and extra value of the entry's row of RasterArgs::bounds
+    uint32_t sid[32];    // Gaussian
+};
+// Entries of a list for one warp, 32 at a time in three stages: the index of batch b + 3 and the box of b + 2 are on their way to registers and the records of
+// b + 1 to shared memory while b is walked. Only entries whose box overlaps the patch are fetched.
+struct EntryFeed {
+    uint32_t id_box, id_ahead;   // of the batch whose boxes are on their way, and of the one after it
+    uint4 box;
+    uint32_t mask;               // entries of the batch staged last
+    __device__ __forceinline__ void start(uint32_t id0, uint32_t id1, const uint4* __restrict__ bounds) {
+        id_box = id0;
+        id_ahead = id1;
+        box = bounds[id0];
+    }
+    // stages the batch whose boxes have come (n entries), starts on the boxes of the next one; id: of the batch after that
+    __device__ __forceinline__ void stage(WarpStage& st, int n, uint32_t patch_x, uint32_t patch_y, const float4* __restrict__ records,
+                                          const uint4* __restrict__ bounds, uint32_t id, int lane) {
+        const bool ov = lane < n && box_overlaps(make_uint2(box.x, box.y), patch_x, patch_y);
+        mask = __ballot_sync(0xffffffffu, ov);
+        if (ov) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cp_async16(&st.rec[k][lane], records + (size_t)id_box * 4 + k);
+            st.zw[lane] = make_float2(__uint_as_float(box.z), __uint_as_float(box.w));
+            st.sid[lane] = id_box;
+        }
+        cp_async_commit();
+        id_box = id_ahead;
+        id_ahead = id;
+        box = bounds[id_box];
+    }
+};
+
+template <int PX>
+struct FwdPatchWarp {
+    WarpStage stage[2];   // one is walked while the other is filled
+    f3 ray[PX][32];       // world-space unit rays, for kept_at_cut
+};
+
+// Forward for cameras with one ray origin. A warp owns a patch of 8 x 4 PX pixels and stages its own entries: no barrier, and a warp whose pixels are finished
+// stops by itself. EXTRA = false: three colour channels (render mode RGB). EXTRA = true: `channels` is 1 or 4 and the last
 // channel blends the per-Gaussian value kept in bounds.w (the depth in the render modes D / ED / RGB_D /
 // RGB_ED of gsplat/Rasterization.cpp:373-393); `normalize` divides it by max(alpha, 1e-10) on output (the
 // expected-depth modes of src/training/rasterization/rasterizer.cpp:186-198) and keeps the undivided value
 // in extra_sum for the backward.
-// RS: rolling shutter. Every pixel has its own pose, hence its own ray origin; the record's gro = M (o_start - mu) is
-// corrected per pair by M (o_pixel - o_start).
-// The plain pinhole RGB instantiation fits 40 registers (16 bytes of stack) and, with 192-record batches (33 KB with the rays for
-// kept_at_cut), six CTAs per SM; the other instantiations keep their 56 - 64 registers.
-template <int MODEL, bool EXTRA, bool RS>
-__global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA) ? 6 : 4) raster_fwd_kernel(
+// Pixels whose pair is rejected go on with alpha = 0. A wide-angle camera's warps have many entries that reach no pixel, where leaving early pays
+// (6 M fisheye 1300 -> 1164 us); a planar camera's have few (1 M, 1296x840: 352 us against 361 with the vote).
+// Eight CTAs of 64 registers per SM; seven 378 us, nine the same.
+template <int MODEL, bool EXTRA, int PX>
+__global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
     const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
     const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
     float* __restrict__ render, float* __restrict__ alphas, int32_t* __restrict__ last_ids, float* __restrict__ extra_sum) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using P = Pixels<PX>;
+    using V = typename P::V;
+    constexpr bool kVote = MODEL != LFS_PINHOLE && MODEL != LFS_PINHOLE_OPENCV;
+    FwdPatchWarp<PX>& sm = reinterpret_cast<FwdPatchWarp<PX>*>(smem_raw)[threadIdx.x >> 5];
+
+    if (overflow && *overflow) return;
+    const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
+    const int tile = tile_order ? tile_order[slot] : slot;
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
+    // warps tile the 16x16 block as patches of 8 x 4 PX pixels
+    const int patch_x0 = (tile % tw) * 16 + (warp & 1) * 8, patch_y0 = (tile / tw) * 16 + (warp >> 1) * 4 * PX;
+    const uint32_t patch_x = patch_x0 | ((patch_x0 + 7) << 16), patch_y = patch_y0 | ((patch_y0 + 4 * PX - 1) << 16);
+    const int i = patch_y0 + (PX == 2 ? lane >> 2 : lane >> 3), j0 = patch_x0 + (PX == 2 ? 2 * (lane & 3) : lane & 7);
+    if (masks && !masks[tile]) {
+        // a tile labelled false shows the background (gsplat/RasterizeToPixelsFromWorld3DGSFwd.cu:147-155)
+#pragma unroll
+        for (int q = 0; q < PX; ++q)
+            if (i < H && j0 + q < W) {
+                const int pid = i * W + j0 + q;
+                const int ch = EXTRA ? channels : 3;
+                for (int k = 0; k < ch; ++k) render[pid * ch + k] = background ? background[k] : 0.f;
+                alphas[pid] = 0.f;
+                last_ids[pid] = 0;
+                if (EXTRA && extra_sum) extra_sum[pid] = background ? background[ch - 1] : 0.f;
+            }
+        return;
+    }
+    const CamDev& cam = cams[0];
+    f3 d[PX];
+    bool takes_part[PX];
+    float dc[3][PX];
+    uint32_t cur_idx[PX];
+#pragma unroll
+    for (int q = 0; q < PX; ++q) {
+        f3 wd;
+        takes_part[q] = pixel_cam_dir<MODEL>(cam, (float)(j0 + q) + 0.5f, (float)i + 0.5f, d[q], wd) && i < H && j0 + q < W;
+        sm.ray[q][lane] = wd;
+        dc[1][q] = d[q].y; dc[2][q] = d[q].z;
+        // a pixel that takes no part, or no longer, has no direction: every comparison with its distance is false
+        dc[0][q] = takes_part[q] ? d[q].x : CUDART_NAN_F;
+        cur_idx[q] = 0;
+    }
+    const PatchRays rays = patch_rays<MODEL, PX>(d, takes_part);
+    V dx = P::make(dc[0]);
+    const V dy = P::make(dc[1]), dz = P::make(dc[2]), minus_one = P::all(-1.0f);
+    V T = P::all(1.0f), pr = P::all(0.f), pg = P::all(0.f), pb = P::all(0.f), px = P::all(0.f);
+
+    const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
+    const int32_t range_start = tile_offsets[tile];
+    const int32_t range_end = (tile == n_tiles - 1) ? n_isects : tile_offsets[tile + 1];
+    const int total = range_end - range_start, n_batches = (total + 31) / 32;
+    auto batch_ids = [&](int b) { return lane < total - 32 * b ? flatten_ids[range_start + 32 * b + lane] : 0u; };
+    EntryFeed feed;
+    if (n_batches > 0) {
+        feed.start(batch_ids(0), batch_ids(1), bounds);
+        feed.stage(sm.stage[0], total, patch_x, patch_y, records, bounds, batch_ids(2), lane);
+    }
+    for (int b = 0; b < n_batches; ++b) {
+        const int32_t batch_start = range_start + 32 * b;
+        float left[PX];
+        P::get(dx, left);
+        bool any_left = false;
+#pragma unroll
+        for (int q = 0; q < PX; ++q) any_left = any_left || left[q] == left[q];
+        // also: everybody has finished walking batch b - 1, whose buffer is filled next
+        if (!__any_sync(0xffffffffu, any_left)) break;
+        const uint32_t staged = feed.mask;
+        if (b + 1 < n_batches) {
+            feed.stage(sm.stage[(b + 1) & 1], total - 32 * (b + 1), patch_x, patch_y, records, bounds, batch_ids(b + 3), lane);
+            if (!staged) continue;
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncwarp();
+        const WarpStage& st = sm.stage[b & 1];
+        // entries whose forms miss this warp's patch are dropped up front
+        bool reached = staged >> lane & 1u;
+        if (reached) reached = patch_reached<MODEL>(st.rec[0][lane], st.rec[1][lane], st.rec[2][lane], st.zw[lane].x, rays);
+        uint32_t bits = __ballot_sync(0xffffffffu, reached);
+        while (bits) {
+            const int t = __ffs(bits) - 1;
+            bits &= bits - 1;
+            const float4 r0 = st.rec[0][t], r1 = st.rec[1][t], r2 = st.rec[2][t], r3 = st.rec[3][t];
+            const PixelForms<PX> f = pixel_forms<MODEL, PX>(r0, r1, r2, dx, dy, dz);
+            float E[PX], limit[PX], den[PX], ex[PX], vis[PX], alpha[PX];
+            P::get(f.E, E);
+            P::get(mul2(P::all(r1.w), f.den), limit);
+            P::get(f.den, den);
+            bool valid[PX], any_valid = false;
+#pragma unroll
+            for (int q = 0; q < PX; ++q) {
+                valid[q] = E[q] <= limit[q];
+                any_valid = any_valid || valid[q];
+            }
+            if (kVote && !__any_sync(0xffffffffu, any_valid)) continue;
+#pragma unroll
+            for (int q = 0; q < PX; ++q) den[q] = rcp_approx(den[q]);
+            P::get(mul2(P::all(r0.w), mul2(f.E, P::make(den))), ex);
+#pragma unroll
+            for (int q = 0; q < PX; ++q) vis[q] = exp2_approx(ex[q]);
+            P::get(mul2(P::all(r3.w), P::make(vis)), alpha);
+            bool near_cut = false;
+#pragma unroll
+            for (int q = 0; q < PX; ++q) {
+                alpha[q] = fminf(0.999f, alpha[q]);
+                near_cut = near_cut || (valid[q] && alpha[q] < r2.w);
+            }
+            if (near_cut) {
+                const uint32_t kept = kept_at_cut<PX>(cuts + st.sid[t], n_cuts, &sm.ray[0][lane], 32, r3.w);
+#pragma unroll
+                for (int q = 0; q < PX; ++q) valid[q] = valid[q] && ((kept >> q & 1u) || !(alpha[q] < r2.w));
+            }
+#pragma unroll
+            for (int q = 0; q < PX; ++q)
+                if (!valid[q]) alpha[q] = 0.f;
+            V al = P::make(alpha);
+            V next_T = mul2(T, mul2(add2(al, minus_one), minus_one));
+            float nt[PX];
+            P::get(next_T, nt);
+            bool stops = false;
+#pragma unroll
+            for (int q = 0; q < PX; ++q) stops = stops || nt[q] <= 1e-4f;   // no pixel without alpha comes here: its T is above
+            if (stops) {
+                float x[PX], t0[PX];
+                P::get(dx, x);
+                P::get(T, t0);
+#pragma unroll
+                for (int q = 0; q < PX; ++q)
+                    if (nt[q] <= 1e-4f) { valid[q] = false; alpha[q] = 0.f; nt[q] = t0[q]; x[q] = CUDART_NAN_F; }
+                dx = P::make(x);
+                al = P::make(alpha);
+                next_T = P::make(nt);
+            }
+            const V w = mul2(al, T);
+            pr = fma2(P::all(r3.x), w, pr); pg = fma2(P::all(r3.y), w, pg); pb = fma2(P::all(r3.z), w, pb);
+            if (EXTRA) px = fma2(P::all(st.zw[t].y), w, px);
+#pragma unroll
+            for (int q = 0; q < PX; ++q) cur_idx[q] = valid[q] ? (uint32_t)(batch_start + t) : cur_idx[q];
+            T = next_T;
+        }
+    }
+    cp_async_wait<0>();
+    float Tq[PX], rq[PX], gq[PX], bq[PX], xq[PX];
+    P::get(T, Tq); P::get(pr, rq); P::get(pg, gq); P::get(pb, bq); P::get(px, xq);
+#pragma unroll
+    for (int q = 0; q < PX; ++q) {
+        if (!(i < H && j0 + q < W)) continue;
+        const int pid = i * W + j0 + q;
+        alphas[pid] = 1.0f - Tq[q];
+        if (background && (!EXTRA || channels == 4)) { rq[q] += Tq[q] * background[0]; gq[q] += Tq[q] * background[1]; bq[q] += Tq[q] * background[2]; }
+        if (!EXTRA) {
+            render[pid * 3 + 0] = rq[q];
+            render[pid * 3 + 1] = gq[q];
+            render[pid * 3 + 2] = bq[q];
+        } else {
+            if (channels == 4) {
+                render[pid * 4 + 0] = rq[q];
+                render[pid * 4 + 1] = gq[q];
+                render[pid * 4 + 2] = bq[q];
+            }
+            if (background) xq[q] += Tq[q] * background[channels - 1];
+            if (extra_sum) extra_sum[pid] = xq[q];
+            render[pid * channels + channels - 1] = normalize ? xq[q] / fmaxf(1.0f - Tq[q], 1e-10f) : xq[q];
+        }
+        last_ids[pid] = (int32_t)cur_idx[q];
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// EXTRA = false: three colour channels (render mode RGB). EXTRA = true: `channels` is 1 or 4 and the last
+// channel blends the per-Gaussian value kept in bounds.w (the depth in the render modes D / ED / RGB_D /
+// RGB_ED of gsplat/Rasterization.cpp:373-393); `normalize` divides it by max(alpha, 1e-10) on output (the
+// expected-depth modes of src/training/rasterization/rasterizer.cpp:186-198) and keeps the undivided value
+// in extra_sum for the backward.
+// A rolling shutter: every pixel has its own pose, hence its own ray origin; the record's gro = M (o_start - mu) is
+// corrected per pair by M (o_pixel - o_start).
+template <int MODEL, bool EXTRA>
+__global__ void __launch_bounds__(kBlock, 4) raster_fwd_rs_kernel(
+    const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
+    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
+    const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
+    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
+    float* __restrict__ render, float* __restrict__ alphas, int32_t* __restrict__ last_ids, float* __restrict__ extra_sum) {
     constexpr int BATCH = 192;
     __shared__ Stage<BATCH> stage[2];
-    __shared__ f3 ray[RS ? 1 : kBlock];   // world-space unit rays, for kept_at_cut
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
@@ -256,13 +556,9 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
         return;
     }
     const CamDev& cam = cams[0];
-    f3 d, wd, oo{0.f, 0.f, 0.f};
-    const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo)
-                           : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, wd);
-    if (!RS) ray[threadIdx.x] = wd;
+    f3 d, oo{0.f, 0.f, 0.f};
+    const bool ray_ok = pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo);
     bool done = !inside || !ray_ok;
-    const bool takes_part = !done;
-    const PatchRays rays = RS ? PatchRays{} : patch_rays<MODEL, 1>(&d, &takes_part);
     uint32_t patch_x, patch_y;
     warp_patch(tile, tw, patch_x, patch_y);
 
@@ -306,7 +602,6 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                 if (e < batch_size) {
                     const uint4 bx = st.box[e];
                     ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
-                    if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], __uint_as_float(bx.z), rays);
                 }
                 return __ballot_sync(0xffffffffu, ov);
             };
@@ -317,34 +612,22 @@ __global__ void __launch_bounds__(kBlock, (MODEL == LFS_PINHOLE && !RS && !EXTRA
                     const int t = w * 32 + __ffs(bits) - 1;
                     bits &= bits - 1;
                     const float4 r0 = st.rec[t * 4 + 0], r1 = st.rec[t * 4 + 1], r2 = st.rec[t * 4 + 2];
-                    float alpha;
-                    if (!RS) {
-                        const RayForms f = ray_forms<MODEL>(r0, r1, r2, d);
-                        if (f.E > r1.w * f.den) continue;
-                        const float o = st.rec[t * 4 + 3].w;
-                        alpha = fminf(0.999f, o * exp2_approx(r0.w * (f.E * rcp_approx(f.den))));
-                        if (__builtin_expect(alpha < r2.w, 0)) {
-                            const uint32_t g = flatten_ids[batch_start + t];
-                            if (!kept_at_cut<1>(cuts + g, n_cuts, ray + threadIdx.x, 0, o)) continue;
-                        }
-                    } else {
-                        const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
-                        const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
-                        const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
-                        const float gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
-                        const float gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
-                        const float gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
-                        const float cx = uy * gz - gy * uz;
-                        const float cy = uz * gx - gz * ux;
-                        const float cz = ux * gy - gx * uy;
-                        const float cc = cx * cx + cy * cy + cz * cz;
-                        const float uu = ux * ux + uy * uy + uz * uz;
-                        // power = -0.5 cc / uu ; reject when power < thr  <=>  cc > -2 thr uu
-                        if (cc > -2.0f * __uint_as_float(st.box[t].z) * uu) continue;
-                        const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
-                        alpha = fminf(0.999f, st.rec[t * 4 + 3].w * __expf(power));
-                        if (alpha < kAlphaMin) continue;
-                    }
+                    const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
+                    const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
+                    const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
+                    const float gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
+                    const float gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
+                    const float gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
+                    const float cx = uy * gz - gy * uz;
+                    const float cy = uz * gx - gz * ux;
+                    const float cz = ux * gy - gx * uy;
+                    const float cc = cx * cx + cy * cy + cz * cz;
+                    const float uu = ux * ux + uy * uy + uz * uz;
+                    // power = -0.5 cc / uu ; reject when power < thr  <=>  cc > -2 thr uu
+                    if (cc > -2.0f * __uint_as_float(st.box[t].z) * uu) continue;
+                    const float power = -0.5f * __fdividef(cc, fmaxf(uu, 1e-37f));
+                    const float alpha = fminf(0.999f, st.rec[t * 4 + 3].w * __expf(power));
+                    if (alpha < kAlphaMin) continue;
                     const float4 r3 = st.rec[t * 4 + 3];
                     const float next_T = T * (1.0f - alpha);
                     if (next_T <= 1e-4f) { done = true; break; }
@@ -416,12 +699,11 @@ __device__ __forceinline__ float __reduce_add_sync_f32(float x) {
 //   q omega e1, q omega e2 | the same two times phi | q omega^2 e1^2, q omega^2 e1 e2, q omega^2 e2^2 | q phi | rgb | q
 // Rolling shutter: 16 = sum v_u (x) d, sum v_gro, rgb, opacity.
 constexpr int kSums = 12, kSumsRs = 16;
-template <int BATCH, int NS, int PX, bool RAYS>
+template <int BATCH>
 struct BwdShared {
     Stage<BATCH> stage[3];       // batch b is walked while b+1 and b+2 are in flight
     uint32_t sid[3][BATCH];      // Gaussian index per slot
-    float red[256 / PX / 32][NS * kRedStride];  // per-warp transpose rows of warp_reduce
-    f3 ray[RAYS ? PX : 1][RAYS ? 256 / PX : 1];  // world-space unit rays, for kept_at_cut
+    float red[kBlock / 32][kSumsRs * kRedStride];  // per-warp transpose rows of warp_reduce
 };
 
 // 1 / x for x in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23).
@@ -430,20 +712,12 @@ __device__ __forceinline__ float rcp_newton(float x) {
     return fmaf(y, fmaf(-x, y, 1.0f), y);
 }
 
-// EXTRA: the output has 1 or 4 channels and its last one blends bounds.w (see the forward). XGRAD: also return
+// Backward under a rolling shutter. EXTRA: the output has 1 or 4 channels and its last one blends bounds.w (see the forward). XGRAD: also return
 // the gradient of that per-Gaussian value in accum_extra [N] (operator-level colours with 1 or 4 channels;
 // the fused render modes drop it like gsplat/Rasterization.cpp:575-590 does).
-// One thread owns PX horizontally adjacent pixels, a warp a patch of 4 PX x 8: the two pixels' terms are added in registers,
-// so the warp reduction (12 stores, 4 wide loads, the reduction to memory), the record loads and the list walk are paid once
-// for two pixels, at the price of more idle lanes in the larger patch. launch_raster_bwd says where which PX runs.
-// Registers: six CTAs of 128 threads have 80 each and spill nothing (1 M Gaussians, 1296x840: 786 us; eight with 64 and 28 bytes of
-// spills 801, uncapped 95 and 921; a distorted pinhole, uncapped at 120 for its Newton steps in double: 758 against 647). Four of 256 at
-// 64 for one pixel per thread (five at 48 with spills: 250 k Gaussians, 1024x1024 fisheye, 350 us against 317).
-template <int MODEL, int BATCH, bool EXTRA, bool XGRAD, bool RS, int PX>
-__global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd_kernel(
-
-    const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
-    const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
+template <int MODEL, int BATCH, bool EXTRA, bool XGRAD>
+__global__ void __launch_bounds__(kBlock) raster_bwd_rs_kernel(
+    const CamDev* __restrict__ cams, const float4* __restrict__ records, const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
     const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
@@ -451,71 +725,51 @@ __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd
     const float* __restrict__ v_render, const float* __restrict__ v_alphas, float* __restrict__ accum,
     float* __restrict__ accum_extra) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NS = RS ? kSumsRs : kSums;
-    using Shared = BwdShared<BATCH, NS, PX, !RS>;
+    using Shared = BwdShared<BATCH>;
     Shared& sm = *reinterpret_cast<Shared*>(smem_raw);
 
     if (overflow && *overflow) return;
     const int tile = tile_order ? tile_order[blockIdx.x] : blockIdx.x;
     if (masks && !masks[tile]) return;  // gsplat/RasterizeToPixelsFromWorld3DGSBwd.cu:84
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // warps tile the 16x16 block as patches of 4 PX x 8 pixels
-    constexpr int kPatchesX = 16 / (4 * PX);
-    const int patch_x0 = (tile % tw) * 16 + (warp % kPatchesX) * 4 * PX, patch_y0 = (tile / tw) * 16 + (warp / kPatchesX) * 8;
-    const uint32_t patch_x = patch_x0 | ((patch_x0 + 4 * PX - 1) << 16), patch_y = patch_y0 | ((patch_y0 + 7) << 16);
-    const int i = patch_y0 + (lane >> 2), j0 = patch_x0 + PX * (lane & 3);
+    // warps tile the 16x16 block as patches of 4 x 8 pixels
+    const int patch_x0 = (tile % tw) * 16 + (warp & 3) * 4, patch_y0 = (tile / tw) * 16 + (warp >> 2) * 8;
+    const uint32_t patch_x = patch_x0 | ((patch_x0 + 3) << 16), patch_y = patch_y0 | ((patch_y0 + 7) << 16);
+    const int i = patch_y0 + (lane >> 2), j = patch_x0 + (lane & 3);
     const CamDev& cam = cams[0];
 
-    f3 d[PX], oo[PX];
-    int32_t bin_final[PX];   // last list position that reached the pixel; below every position for pixels that take no part
-    float T[PX], vcr[PX], vcg[PX], vcb[PX], vcx[PX];
+    f3 d, oo;
+    const bool ray_ok = pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d, oo);
+    const bool active = i < H && j < W && ray_ok;
+    // What a lens leaves for a pixel without a ray may be anything, NaN too. Such a pixel's terms are multiplied by zero below,
+    // which takes finite ones.
+    if (!active) { d = f3{0.f, 0.f, 1.f}; oo = f3{0.f, 0.f, 0.f}; }
+    const int pid = min(i * W + j, W * H - 1);
+    const float T_final = 1.0f - render_alphas[pid];
+    float T = T_final, vcr = 0.f, vcg = 0.f, vcb = 0.f, vcx = 0.f;
+    const int32_t bin_final = active ? last_ids[pid] : -1;   // last list position that reached the pixel; below every position for pixels that take no part
+    float v_a = v_alphas ? v_alphas[pid] : 0.f;
+    if (!EXTRA) {
+        vcr = v_render[pid * 3 + 0]; vcg = v_render[pid * 3 + 1]; vcb = v_render[pid * 3 + 2];
+    } else {
+        if (channels == 4) { vcr = v_render[pid * 4 + 0]; vcg = v_render[pid * 4 + 1]; vcb = v_render[pid * 4 + 2]; }
+        vcx = v_render[pid * channels + channels - 1];
+        if (normalize) {
+            // output = sum / max(alpha, 1e-10): chain rule of the division and of clamp_min
+            const float a = 1.0f - T_final, ac = fmaxf(a, 1e-10f);
+            if (a > 1e-10f) v_a -= extra_sum[pid] / (ac * ac) * vcx;
+            vcx = vcx / ac;
+        }
+    }
+    float bg_dot = 0.f;
+    if (background) {
+        if (!EXTRA || channels == 4) bg_dot = background[0] * vcr + background[1] * vcg + background[2] * vcb;
+        if (EXTRA) bg_dot += background[channels - 1] * vcx;
+    }
     // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
     // (colour . v_colour) alpha T of every entry behind
-    float behind[PX];
-    bool takes_part[PX];
-    int32_t warp_bin_final = 0;
-#pragma unroll
-    for (int p = 0; p < PX; ++p) {
-        const int j = j0 + p;
-        oo[p] = f3{0.f, 0.f, 0.f};
-        f3 wd;
-        const bool ray_ok = RS ? pixel_world_ray_rs<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], oo[p])
-                               : pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[p], wd);
-        if (!RS) sm.ray[p][threadIdx.x] = wd;
-        const bool active = i < H && j < W && ray_ok;
-        takes_part[p] = active;
-        // What a lens leaves for a pixel without a ray may be anything, NaN too. Such a pixel's terms are multiplied by zero below,
-        // which takes finite ones.
-        if (!active) { d[p] = f3{0.f, 0.f, 1.f}; oo[p] = f3{0.f, 0.f, 0.f}; }
-        const int pid = min(i * W + j, W * H - 1);
-        const float T_final = 1.0f - render_alphas[pid];
-        T[p] = T_final;
-        bin_final[p] = active ? last_ids[pid] : -1;
-        warp_bin_final = max(warp_bin_final, bin_final[p]);
-        float v_a = v_alphas ? v_alphas[pid] : 0.f;
-        vcx[p] = 0.f;
-        if (!EXTRA) {
-            vcr[p] = v_render[pid * 3 + 0]; vcg[p] = v_render[pid * 3 + 1]; vcb[p] = v_render[pid * 3 + 2];
-        } else {
-            vcr[p] = vcg[p] = vcb[p] = 0.f;
-            if (channels == 4) { vcr[p] = v_render[pid * 4 + 0]; vcg[p] = v_render[pid * 4 + 1]; vcb[p] = v_render[pid * 4 + 2]; }
-            vcx[p] = v_render[pid * channels + channels - 1];
-            if (normalize) {
-                // output = sum / max(alpha, 1e-10): chain rule of the division and of clamp_min
-                const float a = 1.0f - T_final, ac = fmaxf(a, 1e-10f);
-                if (a > 1e-10f) v_a -= extra_sum[pid] / (ac * ac) * vcx[p];
-                vcx[p] = vcx[p] / ac;
-            }
-        }
-        float bg_dot = 0.f;
-        if (background) {
-            if (!EXTRA || channels == 4) bg_dot = background[0] * vcr[p] + background[1] * vcg[p] + background[2] * vcb[p];
-            if (EXTRA) bg_dot += background[channels - 1] * vcx[p];
-        }
-        behind[p] = T_final * (v_a - bg_dot);
-    }
-    warp_bin_final = __reduce_max_sync(0xffffffffu, warp_bin_final);
-    const PatchRays rays = RS ? PatchRays{} : patch_rays<MODEL, PX>(d, takes_part);
+    float behind = T_final * (v_a - bg_dot);
+    const int32_t warp_bin_final = __reduce_max_sync(0xffffffffu, max(bin_final, 0));
 
     const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
     const int32_t range_start = tile_offsets[tile];
@@ -524,7 +778,7 @@ __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd
     float* red = sm.red[warp];
 
     // batches run back to front: slot e of batch b holds list position batch_end - e
-    StageIds<BATCH, 256 / PX> ids;
+    StageIds<BATCH, kBlock> ids;
     auto batch_count = [&](int k) { return min(BATCH, range_end - k * BATCH - range_start); };
     auto batch_top = [&](int k) { return range_end - 1 - k * BATCH; };
     if (n_batches > 0) {
@@ -560,7 +814,6 @@ __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd
             if (e >= t_begin && e < batch_size) {
                 const uint4 bx = st.box[e];
                 ov = box_overlaps(make_uint2(bx.x, bx.y), patch_x, patch_y);
-                if (!RS && ov) ov = patch_reached<MODEL>(&st.rec[e * 4], __uint_as_float(bx.z), rays);
             }
             live[w] = __ballot_sync(0xffffffffu, ov);
         }
@@ -574,127 +827,282 @@ __global__ void __launch_bounds__(256 / PX, RS ? 0 : PX == 1 ? 4 : 6) raster_bwd
                 // the image, beyond their last contributor or below the alpha threshold continue with alpha = vis = 0,
                 // which makes every term they add exactly zero, so no per-lane branching is needed below.
                 const float4 r0 = st.rec[t * 4 + 0], r1 = st.rec[t * 4 + 1], r2 = st.rec[t * 4 + 2];
-                bool valid[PX], any_valid = false;
-                float vis[PX];
-                RayForms f[PX];
-                float ux[PX], uy[PX], uz[PX], gx[PX], gy[PX], gz[PX], inv[PX];
-#pragma unroll
-                for (int p = 0; p < PX; ++p) {
-                    if (!RS) {
-                        f[p] = ray_forms<MODEL>(r0, r1, r2, d[p]);
-                        valid[p] = (batch_end - t <= bin_final[p]) && !(f[p].E > r1.w * f[p].den);
-                    } else {
-                        ux[p] = r0.x * d[p].x + r0.y * d[p].y + r0.z * d[p].z;
-                        uy[p] = r1.x * d[p].x + r1.y * d[p].y + r1.z * d[p].z;
-                        uz[p] = r2.x * d[p].x + r2.y * d[p].y + r2.z * d[p].z;
-                        gx[p] = r0.w + (r0.x * oo[p].x + r0.y * oo[p].y + r0.z * oo[p].z);
-                        gy[p] = r1.w + (r1.x * oo[p].x + r1.y * oo[p].y + r1.z * oo[p].z);
-                        gz[p] = r2.w + (r2.x * oo[p].x + r2.y * oo[p].y + r2.z * oo[p].z);
-                        const float cx = uy[p] * gz[p] - gy[p] * uz[p];
-                        const float cy = uz[p] * gx[p] - gz[p] * ux[p];
-                        const float cz = ux[p] * gy[p] - gx[p] * uy[p];
-                        const float cc = cx * cx + cy * cy + cz * cz;
-                        const float uu = ux[p] * ux[p] + uy[p] * uy[p] + uz[p] * uz[p];
-                        valid[p] = (batch_end - t <= bin_final[p]) && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
-                        inv[p] = rsqrtf(fmaxf(uu, 1e-37f));
-                        vis[p] = -0.5f * (cc * (inv[p] * inv[p]));
-                    }
-                    any_valid = any_valid || valid[p];
-                }
-                if (!__any_sync(0xffffffffu, any_valid)) continue;
+                const float ux = r0.x * d.x + r0.y * d.y + r0.z * d.z;
+                const float uy = r1.x * d.x + r1.y * d.y + r1.z * d.z;
+                const float uz = r2.x * d.x + r2.y * d.y + r2.z * d.z;
+                const float gx = r0.w + (r0.x * oo.x + r0.y * oo.y + r0.z * oo.z);
+                const float gy = r1.w + (r1.x * oo.x + r1.y * oo.y + r1.z * oo.z);
+                const float gz = r2.w + (r2.x * oo.x + r2.y * oo.y + r2.z * oo.z);
+                const float cx = uy * gz - gy * uz;
+                const float cy = uz * gx - gz * ux;
+                const float cz = ux * gy - gx * uy;
+                const float cc = cx * cx + cy * cy + cz * cz;
+                const float uu = ux * ux + uy * uy + uz * uz;
+                bool valid = (batch_end - t <= bin_final) && !(cc > -2.0f * __uint_as_float(st.box[t].z) * uu);
+                if (!__any_sync(0xffffffffu, valid)) continue;
+                const float inv = rsqrtf(fmaxf(uu, 1e-37f));
                 const float4 r3 = st.rec[t * 4 + 3];
-                float rden[PX], phi[PX], alpha[PX];
-                bool near_cut = false;
-                any_valid = false;
+                float vis = __expf(-0.5f * (cc * (inv * inv)));
+                float alpha = fminf(0.999f, r3.w * vis);
+                valid = valid && !(alpha < kAlphaMin);
+                if (!__any_sync(0xffffffffu, valid)) continue;
+                if (!valid) { vis = 0.f; alpha = 0.f; }
+                const float ra = rcp_newton(1.0f - alpha);
+                T *= ra;
+                const float fac = alpha * T;
+                // colour . v_colour of this entry: the colours only ever meet the output gradient in this product
+                float cv = r3.x * vcr + r3.y * vcg + r3.z * vcb;
+                if (EXTRA) cv += __uint_as_float(st.box[t].w) * vcx;
+                const float v_alpha = cv * T + ra * behind;
+                behind -= cv * fac;
+                // geometry and opacity only while alpha is not clamped at 0.999
+                const float gate = (r3.w * vis <= 0.999f) ? vis : 0.f;
+                const float q = gate * v_alpha;
+                const float s = -(r3.w * q);  // v_c = s * c with c = n x g
+                // with n = u / |u|, gn = g . n and w = gn n - g (minus the part of g orthogonal to n):
+                //   v_g = v_c x n = -s w,   v_u = (v_n - (v_n . n) n) / |u| = (s gn / |u|) w
+                const float nx = ux * inv, ny = uy * inv, nz = uz * inv;
+                const float gn = gx * nx + gy * ny + gz * nz;
+                const float wx = gn * nx - gx, wy = gn * ny - gy, wz = gn * nz - gz;
+                const float ku = s * gn * inv;
+                const float vu[3] = {ku * wx, ku * wy, ku * wz}, vg[3] = {-s * wx, -s * wy, -s * wz};
+                const float dd[3] = {d.x, d.y, d.z}, od[3] = {oo.x, oo.y, oo.z};
+                float v[kSumsRs];
+                // g = M (o_start - mu) + M (o_pixel - o_start): the second term adds v_g (x) (o_pixel - o_start) to v_M
 #pragma unroll
-                for (int p = 0; p < PX; ++p) {
-                    rden[p] = phi[p] = 0.f;
-                    if (!RS) {
-                        rden[p] = rcp_approx(f[p].den);
-                        phi[p] = f[p].E * rden[p];
-                        vis[p] = exp2_approx(r0.w * phi[p]);
-                    } else {
-                        vis[p] = __expf(vis[p]);
-                    }
-                    alpha[p] = fminf(0.999f, r3.w * vis[p]);
-                    if (RS) valid[p] = valid[p] && !(alpha[p] < kAlphaMin);
-                    else near_cut = near_cut || (valid[p] && alpha[p] < r2.w);
-                    any_valid = any_valid || valid[p];
+                for (int r = 0; r < 3; ++r) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) v[r * 3 + c] = vu[r] * dd[c] + vg[r] * od[c];
+                    v[9 + r] = vg[r];
                 }
-                if (!RS && __any_sync(0xffffffffu, near_cut)) {
-                    any_valid = false;
-                    const uint32_t kept = kept_at_cut<PX>(cuts + sid[t], n_cuts, sm.ray[0] + threadIdx.x, 256 / PX, r3.w);
-#pragma unroll
-                    for (int p = 0; p < PX; ++p) {
-                        valid[p] = valid[p] && ((kept >> p & 1u) || !(alpha[p] < r2.w));
-                        any_valid = any_valid || valid[p];
-                    }
-                }
-                if (!__any_sync(0xffffffffu, any_valid)) continue;
-                float v[NS];
-                float xs = 0.f;
-#pragma unroll
-                for (int p = 0; p < PX; ++p) {
-                    if (!valid[p]) { vis[p] = 0.f; alpha[p] = 0.f; }
-                    const float ra = rcp_newton(1.0f - alpha[p]);
-                    T[p] *= ra;
-                    const float fac = alpha[p] * T[p];
-                    // colour . v_colour of this entry: the colours only ever meet the output gradient in this product
-                    float cv = r3.x * vcr[p] + r3.y * vcg[p] + r3.z * vcb[p];
-                    if (EXTRA) cv += __uint_as_float(st.box[t].w) * vcx[p];
-                    const float v_alpha = cv * T[p] + ra * behind[p];
-                    behind[p] -= cv * fac;
-                    // geometry and opacity only while alpha is not clamped at 0.999
-                    const float gate = (r3.w * vis[p] <= 0.999f) ? vis[p] : 0.f;
-                    const float q = gate * v_alpha;
-                    auto add = [&](int k, float a, float c) { v[k] = p == 0 ? a * c : fmaf(a, c, v[k]); };
-                    if (!RS) {
-                        const float omega = f[p].w * rden[p], qo = q * omega;
-                        const float th1 = qo * f[p].e1, th2 = qo * f[p].e2;
-                        const float t1 = th1 * omega, t2 = th2 * omega;
-                        if (p == 0) { v[0] = th1; v[1] = th2; v[11] = q; } else { v[0] += th1; v[1] += th2; v[11] += q; }
-                        add(2, th1, phi[p]); add(3, th2, phi[p]);
-                        add(4, t1, f[p].e1); add(5, t1, f[p].e2); add(6, t2, f[p].e2);
-                        add(7, q, phi[p]);
-                        add(8, fac, vcr[p]); add(9, fac, vcg[p]); add(10, fac, vcb[p]);
-                    } else {
-                        const float s = -(r3.w * q);  // v_c = s * c with c = n x g
-                        // with n = u / |u|, gn = g . n and w = gn n - g (minus the part of g orthogonal to n):
-                        //   v_g = v_c x n = -s w,   v_u = (v_n - (v_n . n) n) / |u| = (s gn / |u|) w
-                        const float nx = ux[p] * inv[p], ny = uy[p] * inv[p], nz = uz[p] * inv[p];
-                        const float gn = gx[p] * nx + gy[p] * ny + gz[p] * nz;
-                        const float wx = gn * nx - gx[p], wy = gn * ny - gy[p], wz = gn * nz - gz[p];
-                        const float ku = s * gn * inv[p];
-                        const float vu[3] = {ku * wx, ku * wy, ku * wz}, vg[3] = {-s * wx, -s * wy, -s * wz};
-                        const float dd[3] = {d[p].x, d[p].y, d[p].z}, od[3] = {oo[p].x, oo[p].y, oo[p].z};
-                        // g = M (o_start - mu) + M (o_pixel - o_start): the second term adds v_g (x) (o_pixel - o_start) to v_M
-                        const float rgbq[4] = {fac * vcr[p], fac * vcg[p], fac * vcb[p], q};
-#pragma unroll
-                        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) {
-                                const float x = vu[r] * dd[c] + vg[r] * od[c];
-                                if (p == 0) v[r * 3 + c] = x; else v[r * 3 + c] += x;
-                            }
-                            if (p == 0) v[9 + r] = vg[r]; else v[9 + r] += vg[r];
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (p == 0) v[NS - 4 + k] = rgbq[k]; else v[NS - 4 + k] += rgbq[k];
-                    }
-                    if (XGRAD) xs += fac * vcx[p];
-                }
+                v[12] = fac * vcr; v[13] = fac * vcg; v[14] = fac * vcb; v[15] = q;
                 const uint32_t g = sid[t];
                 if (XGRAD) {
-                    xs = __reduce_add_sync_f32(xs);
+                    const float xs = __reduce_add_sync_f32(fac * vcx);
                     if (lane == 0) atomicAdd(accum_extra + g, xs);
                 }
-                const float total = warp_reduce<NS>(v, red, lane);
-                if ((lane & 1) == 0 && lane < 2 * NS) atomicAdd(accum + (size_t)g * 16 + (lane >> 1), total);
+                const float total = warp_reduce<kSumsRs>(v, red, lane);
+                if ((lane & 1) == 0) atomicAdd(accum + (size_t)g * 16 + (lane >> 1), total);
             }
         }
     }
     cp_async_wait<0>();
+}
+
+template <int PX>
+struct BwdPatchWarp {
+    WarpStage stage[2];                      // one is walked while the other is filled
+    float red[kSums * kRedStride];           // transpose rows
+    f3 ray[PX][32];                            // world-space unit rays, for kept_at_cut
+};
+
+// Backward for cameras with one ray origin. A warp owns a patch of 4 PX x 8 pixels. Each warp stages its own entries, from its own last contributor on: no
+// barrier, the warps of a tile run apart. EXTRA, XGRAD: as below (raster_bwd_rs_kernel).
+// Five CTAs of 96 registers per SM (PX = 2: 1 M Gaussians 719 us, six of 80 737, four 751).
+// Predicating the eight idle lanes off the loads of `flush` saves a tenth of the shared-memory passes and loses more to the order it imposes (741).
+template <int MODEL, bool EXTRA, bool XGRAD, int PX>
+__global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
+    const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
+    const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
+    const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
+    const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
+    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
+    const float* __restrict__ render_alphas, const int32_t* __restrict__ last_ids, const float* __restrict__ extra_sum,
+    const float* __restrict__ v_render, const float* __restrict__ v_alphas, float* __restrict__ accum,
+    float* __restrict__ accum_extra) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using P = Pixels<PX>;
+    using V = typename P::V;
+    BwdPatchWarp<PX>& sm = reinterpret_cast<BwdPatchWarp<PX>*>(smem_raw)[threadIdx.x >> 5];
+
+    if (overflow && *overflow) return;
+    const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
+    const int tile = tile_order ? tile_order[slot] : slot;
+    if (masks && !masks[tile]) return;  // gsplat/RasterizeToPixelsFromWorld3DGSBwd.cu:84
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
+    const CamDev& cam = cams[0];
+
+    // warps tile the 16x16 block as patches of 4 PX x 8 pixels
+    constexpr int kPatchesX = 4 / PX;
+    const int patch_x0 = (tile % tw) * 16 + (warp % kPatchesX) * 4 * PX, patch_y0 = (tile / tw) * 16 + (warp / kPatchesX) * 8;
+    const uint32_t patch_x = patch_x0 | ((patch_x0 + 4 * PX - 1) << 16), patch_y = patch_y0 | ((patch_y0 + 7) << 16);
+    const int i = patch_y0 + (lane >> 2), j0 = patch_x0 + PX * (lane & 3);
+    f3 d[PX];
+    bool takes_part[PX];
+    float Tf[PX], vr[PX], vg[PX], vb[PX], vx[PX], bh[PX], dc[3][PX];
+    int32_t bin_final[PX];   // last list position that reached the pixel; below every position for pixels that take no part
+    int32_t warp_bin_final = -1;
+#pragma unroll
+    for (int q = 0; q < PX; ++q) {
+        const int j = j0 + q;
+        f3 wd;
+        const bool active = pixel_cam_dir<MODEL>(cam, (float)j + 0.5f, (float)i + 0.5f, d[q], wd) && i < H && j < W;
+        sm.ray[q][lane] = wd;
+        takes_part[q] = active;
+        // What a lens leaves for a pixel without a ray may be anything, NaN too. Such a pixel's terms are multiplied by zero below,
+        // which takes finite ones.
+        if (!active) d[q] = f3{0.f, 0.f, 1.f};
+        const int pid = min(i * W + j, W * H - 1);
+        Tf[q] = 1.0f - render_alphas[pid];
+        bin_final[q] = active ? last_ids[pid] : -1;
+        warp_bin_final = max(warp_bin_final, bin_final[q]);
+        float v_a = v_alphas ? v_alphas[pid] : 0.f;
+        vx[q] = 0.f;
+        if (!EXTRA) {
+            vr[q] = v_render[pid * 3 + 0]; vg[q] = v_render[pid * 3 + 1]; vb[q] = v_render[pid * 3 + 2];
+        } else {
+            vr[q] = vg[q] = vb[q] = 0.f;
+            if (channels == 4) { vr[q] = v_render[pid * 4 + 0]; vg[q] = v_render[pid * 4 + 1]; vb[q] = v_render[pid * 4 + 2]; }
+            vx[q] = v_render[pid * channels + channels - 1];
+            if (normalize) {
+                // output = sum / max(alpha, 1e-10): chain rule of the division and of clamp_min
+                const float a = 1.0f - Tf[q], ac = fmaxf(a, 1e-10f);
+                if (a > 1e-10f) v_a -= extra_sum[pid] / (ac * ac) * vx[q];
+                vx[q] = vx[q] / ac;
+            }
+        }
+        float bg_dot = 0.f;
+        if (background) {
+            if (!EXTRA || channels == 4) bg_dot = background[0] * vr[q] + background[1] * vg[q] + background[2] * vb[q];
+            if (EXTRA) bg_dot += background[channels - 1] * vx[q];
+        }
+        bh[q] = Tf[q] * (v_a - bg_dot);
+        dc[0][q] = d[q].x; dc[1][q] = d[q].y; dc[2][q] = d[q].z;
+        vr[q] = -vr[q]; vg[q] = -vg[q]; vb[q] = -vb[q]; vx[q] = -vx[q];
+    }
+    const V dx = P::make(dc[0]), dy = P::make(dc[1]), dz = P::make(dc[2]);
+    const V vcr = P::make(vr), vcg = P::make(vg), vcb = P::make(vb), vcx = P::make(vx);   // with the sign turned
+    V T = P::make(Tf);
+    // what lies behind the entry being walked, as seen by the output gradient: T_final (v_a - background . v_colour), minus
+    // (colour . v_colour) alpha T of every entry behind
+    V behind = P::make(bh);
+    warp_bin_final = __reduce_max_sync(0xffffffffu, warp_bin_final);
+    const PatchRays rays = patch_rays<MODEL, PX>(d, takes_part);
+
+    const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
+    const int32_t range_start = tile_offsets[tile];
+    const int32_t range_end = (tile == n_tiles - 1) ? n_isects : tile_offsets[tile + 1];
+    // back to front from the patch's last contributor: slot e of batch b holds list position top - 32 b - e
+    const int32_t top = min(range_end - 1, warp_bin_final);
+    const int total = top - range_start + 1, n_batches = (total + 31) / 32;
+    if (total <= 0) return;
+    auto batch_ids = [&](int b) { return lane < total - 32 * b ? flatten_ids[top - 32 * b - lane] : 0u; };
+
+    const V one = P::all(1.0f), minus_one = P::all(-1.0f);
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    uint32_t pending = kNone;   // Gaussian whose sums lie in `red`
+    const ulonglong2* red_half = reinterpret_cast<const ulonglong2*>(sm.red + min(lane >> 1, kSums - 1) * kRedStride + 16 * (lane & 1));
+    const bool red_lane = (lane & 1) == 0 && lane < 2 * kSums;
+    auto flush = [&](uint32_t g) {
+        const ulonglong2 x0 = red_half[0], x1 = red_half[1], x2 = red_half[2], x3 = red_half[3];
+        const float2 h = halves2(add2(add2(add2(x0.x, x0.y), add2(x1.x, x1.y)), add2(add2(x2.x, x2.y), add2(x3.x, x3.y))));
+        float sum = h.x + h.y;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if (red_lane && g != kNone) atomicAdd(accum + (size_t)g * 16 + (lane >> 1), sum);
+    };
+
+    EntryFeed feed;
+    feed.start(batch_ids(0), batch_ids(1), bounds);
+    feed.stage(sm.stage[0], total, patch_x, patch_y, records, bounds, batch_ids(2), lane);
+    for (int b = 0; b < n_batches; ++b) {
+        const int32_t batch_end = top - 32 * b;
+        const uint32_t staged = feed.mask;
+        if (b + 1 < n_batches) {
+            // (b + 1)'s buffer was last read before the walk of b - 1 ended
+            __syncwarp();
+            feed.stage(sm.stage[(b + 1) & 1], total - 32 * (b + 1), patch_x, patch_y, records, bounds, batch_ids(b + 3), lane);
+            if (!staged) continue;
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        __syncwarp();
+        const WarpStage& st = sm.stage[b & 1];
+        // entries whose forms miss this warp's patch are dropped up front
+        bool reached = staged >> lane & 1u;
+        if (reached) reached = patch_reached<MODEL>(st.rec[0][lane], st.rec[1][lane], st.rec[2][lane], st.zw[lane].x, rays);
+        uint32_t bits = __ballot_sync(0xffffffffu, reached);
+        while (bits) {
+            const int t = __ffs(bits) - 1;
+            bits &= bits - 1;
+            // Every lane evaluates the pair (the record reads are warp-wide broadcasts); pixels that are outside
+            // the image, beyond their last contributor or below the alpha threshold continue with alpha = vis = 0,
+            // which makes every term they add exactly zero, so no per-lane branching is needed below.
+            const float4 r0 = st.rec[0][t], r1 = st.rec[1][t], r2 = st.rec[2][t], r3 = st.rec[3][t];
+            flush(pending);   // in the shadow of this entry's evaluation
+            pending = kNone;
+            const PixelForms<PX> f = pixel_forms<MODEL, PX>(r0, r1, r2, dx, dy, dz);
+            float E[PX], limit[PX], den[PX], ex[PX], vis[PX], ov[PX], alpha[PX];
+            P::get(f.E, E);
+            P::get(mul2(P::all(r1.w), f.den), limit);
+            P::get(f.den, den);
+            bool valid[PX], any_valid = false, near_cut = false;
+#pragma unroll
+            for (int q = 0; q < PX; ++q) {
+                valid[q] = batch_end - t <= bin_final[q] && !(E[q] > limit[q]);
+                any_valid = any_valid || valid[q];
+                den[q] = rcp_approx(den[q]);
+            }
+            const V rden = P::make(den), phi = mul2(f.E, rden);
+            P::get(mul2(P::all(r0.w), phi), ex);
+#pragma unroll
+            for (int q = 0; q < PX; ++q) vis[q] = exp2_approx(ex[q]);
+            P::get(mul2(P::all(r3.w), P::make(vis)), ov);
+#pragma unroll
+            for (int q = 0; q < PX; ++q) {
+                alpha[q] = fminf(0.999f, ov[q]);
+                near_cut = near_cut || (valid[q] && alpha[q] < r2.w);
+            }
+            const uint32_t some = __ballot_sync(0xffffffffu, any_valid), ask = __ballot_sync(0xffffffffu, near_cut);
+            if (!some) continue;
+            if (ask) {
+                const uint32_t kept = kept_at_cut<PX>(cuts + st.sid[t], n_cuts, &sm.ray[0][lane], 32, r3.w);
+                any_valid = false;
+#pragma unroll
+                for (int q = 0; q < PX; ++q) {
+                    valid[q] = valid[q] && ((kept >> q & 1u) || !(alpha[q] < r2.w));
+                    any_valid = any_valid || valid[q];
+                }
+                if (!__any_sync(0xffffffffu, any_valid)) continue;
+            }
+#pragma unroll
+            for (int q = 0; q < PX; ++q) {
+                if (!valid[q]) alpha[q] = 0.f;
+                // geometry and opacity only while alpha is not clamped at 0.999
+                if (!(valid[q] && ov[q] <= 0.999f)) vis[q] = 0.f;
+            }
+            const V al = P::make(alpha);
+            // 1 / (1 - alpha), 1 - alpha in [0.001, 1]: the hardware estimate and one Newton step (relative error below 2^-23)
+            const V na = add2(al, minus_one);
+            float y0[PX];
+            P::get(na, y0);
+#pragma unroll
+            for (int q = 0; q < PX; ++q) y0[q] = rcp_approx(-y0[q]);
+            const V y = P::make(y0), ra = fma2(y, fma2(na, y, one), y);
+            T = mul2(T, ra);
+            const V fac = mul2(al, T), nfac = mul2(fac, minus_one);
+            // minus colour . v_colour of this entry: the colours only ever meet the output gradient in this product
+            V ncv = fma2(P::all(r3.x), vcr, fma2(P::all(r3.y), vcg, mul2(P::all(r3.z), vcb)));
+            if (EXTRA) ncv = fma2(P::all(st.zw[t].y), vcx, ncv);
+            const V v_alpha = fma2(ra, behind, mul2(mul2(ncv, minus_one), T));
+            behind = fma2(ncv, fac, behind);
+            const V q = mul2(P::make(vis), v_alpha);
+            const V omega = mul2(f.w, rden), qo = mul2(q, omega);
+            const V th1 = mul2(qo, f.e1), th2 = mul2(qo, f.e2), t1 = mul2(th1, omega), t2 = mul2(th2, omega);
+            const uint32_t g = st.sid[t];
+                        auto put = [&](int k, V v) { sm.red[k * kRedStride + lane] = P::sum(v); };
+            put(0, th1); put(1, th2); put(2, mul2(th1, phi)); put(3, mul2(th2, phi));
+            put(4, mul2(t1, f.e1)); put(5, mul2(t1, f.e2)); put(6, mul2(t2, f.e2)); put(7, mul2(q, phi));
+            put(8, mul2(nfac, vcr)); put(9, mul2(nfac, vcg)); put(10, mul2(nfac, vcb)); put(11, q);
+            if (XGRAD) {
+                const float s = __reduce_add_sync_f32(P::sum(mul2(nfac, vcx)));
+                if (lane == 0) atomicAdd(accum_extra + g, s);
+            }
+            __syncwarp();
+            pending = g;
+        }
+    }
+    flush(pending);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1202,19 +1610,31 @@ int launch_raster_fwd(const RasterArgs& a, float* render, float* alphas, int32_t
     if (n_tiles == 0) return LFS_OK;
     if (a.channels != 1 && a.channels != 3 && a.channels != 4) { set_error("raster_fwd: channels must be 1, 3 or 4"); return LFS_EINVAL; }
     LFS_TIMED("raster_fwd", st);
-#define LFS_FWD3(MODEL, EXTRA, RS)                                                                                         \
-    raster_fwd_kernel<MODEL, EXTRA, RS><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets,   \
-                                                                    a.n_isects_dev, a.n_isects_host, a.overflow, a.background,  \
-                                                                    a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H,   \
-                                                                    a.tw, n_tiles, render, alphas, last_ids, extra_sum)
-#define LFS_FWD(MODEL, EXTRA) do { if (a.rolling) LFS_FWD3(MODEL, EXTRA, true); else LFS_FWD3(MODEL, EXTRA, false); } while (0)
+    // Two pixels per thread where the patches of twice the size still fill the GPU. fwd us with one and two, 1296x840-like scenes of 100 k Gaussians: 510
+    // tiles 91 and 117, 920 tiles 98 and 104, 1,400 tiles 122 and 107, 2,170 tiles 158 and 129. A wide-angle lens shows the scene on a tenth of its tiles or
+    // so: fisheye, 600 k, 4,096 tiles 239 and 344, 8,100 tiles 216 and 278, 14,400 tiles 309 and 271.
+    const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
+    const bool two = n_tiles >= (planar ? 8 : 80) * num_sms();
+#define LFS_FWD_RS(MODEL, EXTRA)                                                                                                    \
+    raster_fwd_rs_kernel<MODEL, EXTRA><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev,       \
+                                                                   a.n_isects_host, a.overflow, a.background, a.masks, a.tile_order, a.channels,   \
+                                                                   a.normalize, a.W, a.H, a.tw, n_tiles, render, alphas, last_ids, extra_sum)
+#define LFS_FWD_PATCH(MODEL, EXTRA, PX)                                                                                             \
+    raster_fwd_patch_kernel<MODEL, EXTRA, PX><<<n_tiles * (2 / PX), 128, 4 * sizeof(FwdPatchWarp<PX>), st>>>(                       \
+        a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background,  \
+        a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render, alphas, last_ids, extra_sum)
+#define LFS_FWD2(MODEL, EXTRA) do { if (two) LFS_FWD_PATCH(MODEL, EXTRA, 2); else LFS_FWD_PATCH(MODEL, EXTRA, 1); } while (0)
+#define LFS_FWD(MODEL) do { if (a.rolling) { if (extra) LFS_FWD_RS(MODEL, true); else LFS_FWD_RS(MODEL, false); }                   \
+                            else if (extra) LFS_FWD2(MODEL, true); else LFS_FWD2(MODEL, false); } while (0)
     const bool extra = a.channels != 3;
-    if (a.model == LFS_PINHOLE) { if (extra) LFS_FWD(LFS_PINHOLE, true); else LFS_FWD(LFS_PINHOLE, false); }
-    else if (a.model == LFS_PINHOLE_OPENCV) { if (extra) LFS_FWD(LFS_PINHOLE_OPENCV, true); else LFS_FWD(LFS_PINHOLE_OPENCV, false); }
-    else if (a.model == LFS_EQUIRECTANGULAR) { if (extra) LFS_FWD3(LFS_EQUIRECTANGULAR, true, false); else LFS_FWD3(LFS_EQUIRECTANGULAR, false, false); }
-    else { if (extra) LFS_FWD(LFS_FISHEYE, true); else LFS_FWD(LFS_FISHEYE, false); }
-#undef LFS_FWD3
+    if (a.model == LFS_PINHOLE) LFS_FWD(LFS_PINHOLE);
+    else if (a.model == LFS_PINHOLE_OPENCV) LFS_FWD(LFS_PINHOLE_OPENCV);
+    else if (a.model == LFS_EQUIRECTANGULAR) { if (extra) LFS_FWD2(LFS_EQUIRECTANGULAR, true); else LFS_FWD2(LFS_EQUIRECTANGULAR, false); }
+    else LFS_FWD(LFS_FISHEYE);
 #undef LFS_FWD
+#undef LFS_FWD2
+#undef LFS_FWD_PATCH
+#undef LFS_FWD_RS
     return check_launch("raster_fwd");
 }
 
@@ -1225,45 +1645,41 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     if (a.channels != 1 && a.channels != 3 && a.channels != 4) { set_error("raster_bwd: channels must be 1, 3 or 4"); return LFS_EINVAL; }
     if (a.normalize && !extra_sum) { set_error("raster_bwd: expected-depth modes need the forward's blended sum"); return LFS_EINVAL; }
     LFS_TIMED("raster_bwd", st);
-    // Two pixels per thread where the patches are filled and the CTAs of half the threads still fill the GPU: planar cameras and
-    // at least eight tiles per SM. 4,293 tiles (1 M Gaussians, 1296x840) 787 us against 992 with one pixel; 2,170 (120 k, 979x547) 241
-    // against 306; 1,080 (250 k, 640x427, the other side of the line, which could lie lower) 302 against 335; 256 (16 k, 256x256) 111
-    // against 88. A wide-angle camera shows Gaussians a few pixels across in the middle of its image, where the larger patch wastes lanes
-    // and few tiles carry the work (250 k Gaussians, 1024x1024 fisheye, the one such scene measured, with earlier kernels: 478 us against
-    // 392).
+    // Two pixels per thread where the patches of twice the size still fill the GPU (launch_raster_fwd). bwd us with one and two, planar, 100 k Gaussians: 256
+    // tiles 190 and 266, 510 tiles 176 and 174 (20 k: 100 and 111, 400 k: 234 and 246), 920 tiles 211 and 165, 2,170 tiles 361 and 255; fisheye, 600 k: 4,096 tiles
+    // 395 and 453, 8,100 tiles 418 and 379.
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
     const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
-    const bool wide = planar && !a.rolling && n_tiles >= 8 * num_sms();
-    constexpr int kBatch = 64;
-#define LFS_BWD6(MODEL, EXTRA, XGRAD, RS, PX)                                                                                  \
+    const bool two = n_tiles >= (planar ? 4 : 40) * num_sms();
+#define LFS_BWD_RS(MODEL, EXTRA, XGRAD)                                                                                        \
     do {                                                                                                                       \
-        constexpr int smem = (int)sizeof(BwdShared<kBatch, RS ? kSumsRs : kSums, PX, !RS>);                                \
-        raster_bwd_kernel<MODEL, kBatch, EXTRA, XGRAD, RS, PX><<<n_tiles, 256 / PX, smem, st>>>(                               \
+        constexpr int smem = (int)sizeof(BwdShared<64>);                                                                       \
+        raster_bwd_rs_kernel<MODEL, 64, EXTRA, XGRAD><<<n_tiles, kBlock, smem, st>>>(                                          \
+            a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background, \
+            a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
+            v_alphas, accum, accum_extra);                                                                                     \
+    } while (0)
+#define LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, PX)                                                                                 \
+    do {                                                                                                                       \
+        raster_bwd_patch_kernel<MODEL, EXTRA, XGRAD, PX><<<n_tiles * (2 / PX), 128, 4 * sizeof(BwdPatchWarp<PX>), st>>>(       \
             a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow,    \
             a.background,                                                                                                      \
             a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
             v_alphas, accum, accum_extra);                                                                                     \
     } while (0)
-#define LFS_BWD_PLANAR(MODEL, EXTRA, XGRAD)                                                                                    \
-    do {                                                                                                                       \
-        if (a.rolling) LFS_BWD6(MODEL, EXTRA, XGRAD, true, 1);                                                                 \
-        else if (wide) LFS_BWD6(MODEL, EXTRA, XGRAD, false, 2);                                                                \
-        else LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1);                                                                          \
-    } while (0)
-#define LFS_BWD_FISHEYE(MODEL, EXTRA, XGRAD)                                                                                   \
-    do { if (a.rolling) LFS_BWD6(MODEL, EXTRA, XGRAD, true, 1); else LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1); } while (0)
-#define LFS_BWD_EQUIRECT(MODEL, EXTRA, XGRAD) LFS_BWD6(MODEL, EXTRA, XGRAD, false, 1)
+#define LFS_BWD_ORIGIN(MODEL, EXTRA, XGRAD) do { if (two) LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, 2); else LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, 1); } while (0)
+#define LFS_BWD_ANY(MODEL, EXTRA, XGRAD) do { if (a.rolling) LFS_BWD_RS(MODEL, EXTRA, XGRAD); else LFS_BWD_ORIGIN(MODEL, EXTRA, XGRAD); } while (0)
 #define LFS_BWD(KIND, MODEL)                                                                                                   \
     do { if (!extra) KIND(MODEL, false, false); else if (!xgrad) KIND(MODEL, true, false); else KIND(MODEL, true, true); } while (0)
-    if (a.model == LFS_PINHOLE) LFS_BWD(LFS_BWD_PLANAR, LFS_PINHOLE);
-    else if (a.model == LFS_PINHOLE_OPENCV) LFS_BWD(LFS_BWD_PLANAR, LFS_PINHOLE_OPENCV);
-    else if (a.model == LFS_EQUIRECTANGULAR) LFS_BWD(LFS_BWD_EQUIRECT, LFS_EQUIRECTANGULAR);
-    else LFS_BWD(LFS_BWD_FISHEYE, LFS_FISHEYE);
+    if (a.model == LFS_PINHOLE) LFS_BWD(LFS_BWD_ANY, LFS_PINHOLE);
+    else if (a.model == LFS_PINHOLE_OPENCV) LFS_BWD(LFS_BWD_ANY, LFS_PINHOLE_OPENCV);
+    else if (a.model == LFS_EQUIRECTANGULAR) LFS_BWD(LFS_BWD_ORIGIN, LFS_EQUIRECTANGULAR);
+    else LFS_BWD(LFS_BWD_ANY, LFS_FISHEYE);
 #undef LFS_BWD
-#undef LFS_BWD_EQUIRECT
-#undef LFS_BWD_FISHEYE
-#undef LFS_BWD_PLANAR
-#undef LFS_BWD6
+#undef LFS_BWD_ANY
+#undef LFS_BWD_ORIGIN
+#undef LFS_BWD_PATCH
+#undef LFS_BWD_RS
     return check_launch("raster_bwd");
 }
 
