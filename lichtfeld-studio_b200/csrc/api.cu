@@ -82,7 +82,7 @@ RenderWs carve_render(const lfs_render_config& cfg, void* base) {
     w.tile_offsets = c.take<int32_t>((size_t)tw * th + 1);
     w.last_ids = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
     w.extra_sum = c.take<float>((size_t)cfg.image_width * cfg.image_height);  // blended depth before the division (ED modes)
-    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th));
+    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th, (int64_t)cap));
     w.tile_order = tile_list_order(w.list_state, (int64_t)tw * th);
     w.bytes = c.total();
     return w;
@@ -118,7 +118,7 @@ EwaWs carve_ewa(const lfs_ewa_config& cfg, void* base) {
     w.flatten_ids = c.take<int32_t>(cap);
     w.tile_offsets = c.take<int32_t>((size_t)tw * th + 1);
     w.n_contrib = c.take<int32_t>((size_t)cfg.image_width * cfg.image_height);
-    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th));
+    w.list_state = c.take<int32_t>(tile_list_state_words((int64_t)tw * th, (int64_t)cap));
     w.tile_order = tile_list_order(w.list_state, (int64_t)tw * th);
     w.bytes = c.total();
     return w;

@@ -223,7 +223,9 @@ static_assert(kBucketBelow<8> == kBucketBelow<10> + 8, "");
 
 // Words of the list state in front of the per-bin arrays.
 // lists of at least 2^10 and 2^8 entries, and of any
-constexpr int kMetaLists = 0, kMetaWords = 16, kKinds = 3;
+constexpr int kMetaLists = 0, kMetaParts = 8, kMetaWords = 16, kKinds = 3;
+// Lists longer than kRoomCta are sorted in parts of some kPart entries, by as many CTAs.
+constexpr int kRoomCta = 8192, kPart = 3072;
 
 // One cluster: counts -> offsets [n_bins + 1] and cursors, the total and the overflow flag (with it all offsets are 0: the list is not
 // built), the launch order, and how many lists each kind of sorting group has. Every CTA takes a run of bins, 1024 at a time; the CTAs
@@ -233,7 +235,7 @@ constexpr int kMetaLists = 0, kMetaWords = 16, kKinds = 3;
 constexpr int kScanCluster = 8;
 __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) tile_scan_kernel(
     int n_bins, TileCounters t, int64_t capacity, int64_t* carry, int32_t* __restrict__ n_out, int32_t* overflow, int32_t* __restrict__ offsets,
-    int32_t* __restrict__ order, int2* __restrict__ ranges, int32_t* __restrict__ meta) {
+    int32_t* __restrict__ order, int2* __restrict__ ranges, int4* __restrict__ parts, int32_t* __restrict__ meta) {
     __shared__ int64_t warp_sums[32], block_sum;
     __shared__ int hist[132], cursor[132], sm[33];
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -297,15 +299,16 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) til
         const int before = block_excl_scan(all, sum_all, sm);
         if (threadIdx.x < 132) cursor[threadIdx.x] = before + earlier;
     }
-    cluster.sync();   // nobody reads another CTA's memory, or the carry, from here on
+    __syncthreads();
+    if (rank == 0 && threadIdx.x < kMetaWords) {
+        // the first CTA's share of a bucket starts where the bucket does
+        const int k = threadIdx.x;
+        meta[k] = k == kKinds - 1 ? cursor[131] : k < kKinds - 1 ? cursor[kBucketBelow<10> + 8 * k] : 0;
+    }
+    cluster.sync();   // nobody reads another CTA's memory, or the carry, from here on; meta is set
     const bool dropped = overflow && total > capacity;
     const int32_t total32 = (int32_t)min(total, (int64_t)0x7fffffff);
     if (rank == 0) {
-        // the first CTA's share starts where the bucket does
-        if (threadIdx.x < kMetaWords) {
-            const int k = threadIdx.x;
-            meta[k] = k == kKinds - 1 ? cursor[131] : k < kKinds - 1 ? cursor[kBucketBelow<10> + 8 * k] : 0;
-        }
         if (threadIdx.x == 0) {
             if (n_out) *n_out = total32;
             if (dropped) *overflow = 1;
@@ -327,7 +330,12 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) til
         if (i < last) {
             order[slot] = i;
             int64_t pos = at + ex;
-            ranges[slot] = make_int2((int)min(pos, capacity), (int)min(pos + c, capacity) - (int)min(pos, capacity));
+            const int from = (int)min(pos, capacity), n = (int)min(pos + c, capacity) - from;
+            ranges[slot] = make_int2(from, n);
+            if (n > kRoomCta && !dropped) {
+                const int k = (n + kPart - 1) / kPart, base = atomicAdd(meta + kMetaParts, k);
+                for (int q = 0; q < k; ++q) parts[base + q] = make_int4(from, n, i, q);
+            }
             offsets[i] = dropped ? 0 : (int32_t)min(pos, (int64_t)0x7fffffff);
             for (int r0 = 0; r0 < t.replicas; r0 += 8) {
                 int v[8];
@@ -354,7 +362,8 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) til
 // barriers between the passes bound it: 45 us for 1 M Gaussians at 1296x840 (lists of 967), 157 for 3 M at 1600x1064 (lists of 2,136).
 // Up to eight entries per thread stay in registers between the passes; with sixteen (RELOAD) they are read again.
 constexpr int kSortThreads = 512, kHeavy = 96, kLongLog = 11;
-constexpr int kRoomCta = 16 * kSortThreads, kRoomGroup = 1024, kRoomWarp = 256;
+constexpr int kRoomGroup = 1024, kRoomWarp = 256;
+static_assert(kRoomCta == 16 * kSortThreads, "");
 struct SortShared {
     uint64_t entry[kRoomCta];
     uint32_t start[kRoomCta / 32 * 33 + 64];      // every group has its own run and four more words (bucket_slot)
@@ -490,69 +499,76 @@ __device__ __forceinline__ void sort_group(int tid, int group, int n, uint64_t* 
     else sort_group_k<G, 16, true>(tid, group, n, entry, start, red, load, out);
 }
 
-// A list of any length, by the whole CTA: a histogram over 2048 bins of the keys from `next` on (64 bits, which are all different), then
-// runs of bins that hold up to 4096 entries are gathered into shared memory and sorted. A bin that holds more by itself is cut into
-// 2048 again.
-template <class Out>
-__device__ void sort_long(int n, const uint64_t* __restrict__ list, SortShared& sm, Out out) {
-    constexpr int kBins = 1 << kLongLog, kRoom = 8 * kSortThreads;
+// The keys of a list between lo and hi (both included; `count` of them), sorted by the whole CTA: a histogram over 2048 bins of the keys from `next` on (64
+// bits, which are all different), then runs of bins that hold up to 4096 entries are gathered into shared memory and sorted. A bin that holds more by
+// itself is cut into 2048 again.
+template <class Visit>
+__device__ __forceinline__ void visit_list(int n, const uint64_t* __restrict__ list, Visit visit) {
+    int i = threadIdx.x;
+    for (; i + 7 * kSortThreads < n; i += 8 * kSortThreads) {   // eight loads in flight
+        uint64_t k[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) k[u] = list[i + u * kSortThreads];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) visit(k[u]);
+    }
+    for (; i < n; i += kSortThreads) visit(list[i]);
+}
+constexpr int kLongBins = 1 << kLongLog;
+// counts of the keys in [next, top] by (key - next) >> shift, as an exclusive prefix in sm.cum [kLongBins + 1]
+__device__ __forceinline__ void long_histogram(int n, const uint64_t* __restrict__ list, SortShared& sm, uint64_t next, uint64_t top, int shift) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint64_t lo = ~0ull, hi = 0;
-    for (int i = tid; i < n; i += kSortThreads) {
-        const uint64_t k = list[i];
-        lo = min(lo, k); hi = max(hi, k);
+    constexpr int kOwn = kLongBins / kSortThreads;
+    __syncthreads();
+    for (int i = tid; i < kLongBins; i += kSortThreads) sm.cum[i] = 0;
+    __syncthreads();
+    visit_list(n, list, [&](uint64_t k) {
+        if (k >= next && k <= top) atomicAdd(&sm.cum[(k - next) >> shift], 1u);
+    });
+    __syncthreads();
+    uint32_t c[kOwn], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) { c[j] = sm.cum[tid * kOwn + j]; sum += c[j]; }
+    uint32_t at = (uint32_t)warp_incl_scan((int)sum);
+    if (lane == 31) sm.red[1][warp][0] = at;
+    __syncthreads();
+    {
+        const uint32_t v = sm.red[1][lane & (kSortThreads / 32 - 1)][0];
+        at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u) - sum;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (lane == 0) { sm.red64[0][warp] = lo; sm.red64[1][warp] = hi; }
+    for (int j = 0; j < kOwn; ++j) { sm.cum[tid * kOwn + j] = at; at += c[j]; }
+    if (tid == kSortThreads - 1) sm.cum[kLongBins] = at;
     __syncthreads();
-    for (int w = 0; w < kSortThreads / 32; ++w) { lo = min(lo, sm.red64[0][w]); hi = max(hi, sm.red64[1][w]); }
+}
+__device__ __forceinline__ int long_shift(uint64_t range) { return max(0, 64 - __clzll((long long)range) - kLongLog); }
+
+template <class Out>
+__device__ void sort_long(int n, const uint64_t* __restrict__ list, uint64_t lo, uint64_t hi, int count, SortShared& sm, Out out) {
+    constexpr int kRoom = 8 * kSortThreads;
+    const int tid = threadIdx.x;
     uint64_t next = lo;   // every smaller key is out
     int done = 0;
-    while (done < n) {
+    while (done < count) {
         uint64_t top = hi;
         int shift;
         for (;;) {
-            shift = max(0, 64 - __clzll((long long)(top - next)) - kLongLog);
-            __syncthreads();
-            for (int i = tid; i < kBins; i += kSortThreads) sm.cum[i] = 0;
-            __syncthreads();
-            for (int i = tid; i < n; i += kSortThreads) {
-                const uint64_t k = list[i];
-                if (k >= next && k <= top) atomicAdd(&sm.cum[(k - next) >> shift], 1u);
-            }
-            __syncthreads();
-            uint32_t c[kBins / kSortThreads], sum = 0;
-#pragma unroll
-            for (int j = 0; j < kBins / kSortThreads; ++j) { c[j] = sm.cum[tid * (kBins / kSortThreads) + j]; sum += c[j]; }
-            uint32_t at = (uint32_t)warp_incl_scan((int)sum);
-            if (lane == 31) sm.red[1][warp][0] = at;
-            __syncthreads();
-            {
-                const uint32_t v = sm.red[1][lane & (kSortThreads / 32 - 1)][0];
-                at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u) - sum;
-            }
-#pragma unroll
-            for (int j = 0; j < kBins / kSortThreads; ++j) { sm.cum[tid * (kBins / kSortThreads) + j] = at; at += c[j]; }
-            if (tid == kSortThreads - 1) sm.cum[kBins] = at;
-            __syncthreads();
+            shift = long_shift(top - next);
+            long_histogram(n, list, sm, next, top, shift);
             // the first bin that holds anything: the last one that starts at 0
             int b = 0;
-            for (int step = kBins / 2; step > 0; step >>= 1)
+            for (int step = kLongBins / 2; step > 0; step >>= 1)
                 if (sm.cum[b + step] == 0) b += step;
             if (shift == 0 || sm.cum[b + 1] <= (uint32_t)kRoom) break;
             next += (uint64_t)b << shift;
             top = min(top, next + (((uint64_t)1 << shift) - 1));
         }
         int s = 0;
-        while (s < kBins && done < n) {
+        while (s < kLongBins && done < count) {
             const uint32_t have = sm.cum[s];
             int e = s;   // the last bin boundary within reach
-            for (int step = kBins; step > 0; step >>= 1)
-                if (e + step <= kBins && sm.cum[e + step] - have <= (uint32_t)kRoom) e += step;
+            for (int step = kLongBins; step > 0; step >>= 1)
+                if (e + step <= kLongBins && sm.cum[e + step] - have <= (uint32_t)kRoom) e += step;
             if (e == s) {
                 if (shift > 0) break;
                 // more than 4096 equal keys: not from this file's callers, but the loop has to end
@@ -566,24 +582,55 @@ __device__ void sort_long(int n, const uint64_t* __restrict__ list, SortShared& 
             if (m > 0) {
                 if (tid == 0) sm.cursor = 0;
                 __syncthreads();
-                for (int i = tid; i < n; i += kSortThreads) {
-                    const uint64_t k = list[i];
+                visit_list(n, list, [&](uint64_t k) {
                     if (k >= next && k <= top) {
                         const int b = (int)((k - next) >> shift);
                         if (b >= s && b < e) sm.entry[min(atomicAdd(&sm.cursor, 1u), (uint32_t)kRoom - 1u)] = k;
                     }
-                }
+                });
                 __syncthreads();
                 sort_group<kSortThreads, false>(tid, 0, m, sm.entry, sm.start, sm.red, [&](int i) { return sm.entry[i]; },
-                                         [&](int i, uint64_t k) { out(done + i, k); });
+                                                [&](int i, uint64_t k) { out(done + i, k); });
                 done += m;
             }
             s = e;
         }
-        if (s == kBins || (uint64_t)s > ((top - next) >> shift)) next = top + 1;   // top == hi: done == n
+        if (s == kLongBins || (uint64_t)s > ((top - next) >> shift)) next = top + 1;   // top == hi: done == count
         else next += (uint64_t)s << shift;
     }
     __syncthreads();
+}
+
+// Part q of a list of n entries, by the whole CTA. Every part counts the list's keys into the same bins and takes those that start in its own share of the
+// ranks, so the parts need nothing from one another.
+template <class Out>
+__device__ void sort_part(int q, int n, const uint64_t* __restrict__ list, SortShared& sm, Out out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, parts = (n + kPart - 1) / kPart;
+    uint64_t lo = ~0ull, hi = 0;
+    visit_list(n, list, [&](uint64_t k) { lo = min(lo, k); hi = max(hi, k); });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) { sm.red64[0][warp] = lo; sm.red64[1][warp] = hi; }
+    __syncthreads();
+    for (int w = 0; w < kSortThreads / 32; ++w) { lo = min(lo, sm.red64[0][w]); hi = max(hi, sm.red64[1][w]); }
+    const int shift = long_shift(hi - lo);
+    long_histogram(n, list, sm, lo, hi, shift);
+    // first bin that starts at or after the share's first rank
+    auto bound = [&](uint32_t rank) {
+        int b = 0;   // bins that start before it
+        for (int step = kLongBins; step > 0; step >>= 1)
+            if (b + step <= kLongBins && sm.cum[b + step - 1] < rank) b += step;
+        return b;
+    };
+    const int from = bound((uint32_t)((int64_t)n * q / parts)), to = q + 1 == parts ? kLongBins : bound((uint32_t)((int64_t)n * (q + 1) / parts));
+    const uint32_t first = sm.cum[from], count = sm.cum[to] - first;
+    __syncthreads();   // sm.cum is counted anew
+    if (count == 0) return;
+    const uint64_t key_lo = lo + ((uint64_t)from << shift), key_hi = to == kLongBins ? hi : lo + ((uint64_t)to << shift) - 1;
+    sort_long(n, list, key_lo, key_hi, (int)count, sm, [&](int i, uint64_t k) { out((int)first + i, k); });
 }
 
 // Groups of G threads share lists first .. last - 1 of the launch order: a round gives one list to every group, the longest to the first group of every
@@ -605,7 +652,8 @@ __device__ __forceinline__ void share_lists(int tid, int group, int first, int l
 
 // OP: operator level, with the 64-bit keys.
 template <bool OP>
-__global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_t* __restrict__ order, const int2* __restrict__ ranges, const int32_t* __restrict__ meta,
+__global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_t* __restrict__ order, const int2* __restrict__ ranges, const int4* __restrict__ parts,
+                                                                    const int32_t* __restrict__ meta,
                                                                     const uint64_t* __restrict__ entries, const int32_t* __restrict__ overflow,
                                                                     int64_t first_bin, uint32_t n_tiles, uint32_t tile_n_bits,
                                                                     int32_t* __restrict__ flatten_ids, int64_t* __restrict__ isect_ids) {
@@ -613,8 +661,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
     SortShared& sm = *reinterpret_cast<SortShared*>(smem_raw);
     if (overflow && *overflow) return;
     const int tid = threadIdx.x;
-    auto writer = [&](int idx, int from) {
-        const int64_t id = OP ? first_bin + order[idx] : 0;
+    auto writer = [&](int bin, int from) {
+        const int64_t id = OP ? first_bin + bin : 0;
         const int64_t tile_key = OP ? (id / n_tiles << tile_n_bits | id % n_tiles) << 32 : 0;
         return [=](int i, uint64_t k) {
             flatten_ids[from + i] = (int32_t)(uint32_t)k;
@@ -622,11 +670,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
         };
     };
     const int n_cta = meta[kMetaLists], n_group = meta[kMetaLists + 1], n_warp = meta[kMetaLists + 2];
+    for (int u = blockIdx.x, n_parts = meta[kMetaParts]; u < n_parts; u += gridDim.x) {
+        const int4 part = parts[u];
+        sort_part(part.w, part.y, entries + part.x, sm, writer(part.z, part.x));
+        __syncthreads();
+    }
     share_lists<kSortThreads>(tid, 0, 0, n_cta, ranges, [&](int idx, int from, int n) {
         if (n <= kRoomCta)
-            sort_group<kSortThreads, true>(tid, 0, n, sm.entry, sm.start, sm.red, [&](int i) { return entries[from + i]; }, writer(idx, from));
-        else
-            sort_long(n, entries + from, sm, writer(idx, from));
+            sort_group<kSortThreads, true>(tid, 0, n, sm.entry, sm.start, sm.red, [&](int i) { return entries[from + i]; }, writer(OP ? order[idx] : 0, from));
     });
     __syncthreads();
     {
@@ -634,7 +685,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
         uint32_t (*red)[kSortThreads / 32][2] = reinterpret_cast<uint32_t (*)[kSortThreads / 32][2]>(&sm.red[0][group * 4][0]);
         share_lists<128>(t, group, n_cta, n_group, ranges, [&](int idx, int from, int n) {
             sort_group<128, false>(t, group, n, sm.entry + group * kRoomGroup, sm.start + group * (kRoomGroup / 32 * 33 + 4), red,
-                                   [&](int i) { return entries[from + i]; }, writer(idx, from));
+                                   [&](int i) { return entries[from + i]; }, writer(OP ? order[idx] : 0, from));
         });
     }
     __syncthreads();
@@ -642,7 +693,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
         const int group = tid / 32, t = tid % 32;
         share_lists<32>(t, group, n_group, n_warp, ranges, [&](int idx, int from, int n) {
             sort_group<32, false>(t, group, n, sm.entry + group * kRoomWarp, sm.start + group * (kRoomWarp / 32 * 33 + 4), sm.red,
-                                  [&](int i) { return entries[from + i]; }, writer(idx, from));
+                                  [&](int i) { return entries[from + i]; }, writer(OP ? order[idx] : 0, from));
         });
     }
 }
@@ -706,7 +757,7 @@ static uint32_t bit_width_u32(uint32_t v) {
     return b;
 }
 
-// ---- list state: kMetaWords | carry (int64) | counts [replicas][stride] | cursors [replicas][stride] | order [bins] | ranges [bins] | offsets [bins + 1] --------
+// ---- list state: kMetaWords | carry (int64) | counts [replicas][stride] | cursors [replicas][stride] | order [bins] | ranges [bins] | offsets [bins + 1] | parts --------
 namespace {
 int64_t pad8(int64_t n) { return (n + 7) / 8 * 8; }
 // Counters of neighbouring tiles share a 32-byte sector, and the memory system applies one request to a sector at a time: some 12 cycles each.
@@ -722,6 +773,7 @@ struct ListState {
     int32_t *meta, *order, *offsets;
     int64_t* carry;
     int2* ranges;
+    int4* parts;   // [capacity / kPart + capacity / kRoomCta + 1]
     TileCounters t;
 };
 ListState list_state(int32_t* base, int64_t bins) {
@@ -735,12 +787,16 @@ ListState list_state(int32_t* base, int64_t bins) {
     s.order = s.t.cursors + (size_t)s.t.replicas * s.t.stride;
     s.ranges = reinterpret_cast<int2*>(s.order + pad8(bins));
     s.offsets = s.order + 3 * pad8(bins);
+    s.parts = reinterpret_cast<int4*>(s.offsets + pad8(bins + 1));
     return s;
 }
-size_t list_words(int64_t bins, int64_t counters) { return (size_t)(kMetaWords + 16 + 2 * counters + 3 * pad8(bins) + pad8(bins + 1)); }
+// a list of n > kRoomCta entries has at most n / kPart + 1 parts, and there are at most capacity / kRoomCta such lists
+size_t list_words(int64_t bins, int64_t counters, int64_t capacity) {
+    return (size_t)(kMetaWords + 16 + 2 * counters + 3 * pad8(bins) + pad8(bins + 1) + 4 * (capacity / kPart + capacity / kRoomCta + 1));
+}
 }  // namespace
 
-size_t tile_list_state_words(int64_t bins) { return list_words(bins, list_replicas(bins) * pad8(bins)); }
+size_t tile_list_state_words(int64_t bins, int64_t capacity) { return list_words(bins, list_replicas(bins) * pad8(bins), capacity); }
 TileCounters tile_list_counters(int32_t* state, int64_t bins) { return list_state(state, bins).t; }
 const int32_t* tile_list_order(const int32_t* state, int64_t bins) { return list_state(const_cast<int32_t*>(state), bins).order; }
 int clear_tile_counters(const TileCounters& t, cudaStream_t st) {
@@ -749,7 +805,7 @@ int clear_tile_counters(const TileCounters& t, cudaStream_t st) {
 
 static int launch_tile_scan(int bins, const ListState& s, int64_t capacity, int64_t* carry, int32_t* n_out, int32_t* overflow, int32_t* offsets, cudaStream_t st) {
     LFS_TIMED("tile_scan", st);
-    tile_scan_kernel<<<kScanCluster, 1024, 0, st>>>(bins, s.t, capacity, carry, n_out, overflow, offsets, s.order, s.ranges, s.meta);
+    tile_scan_kernel<<<kScanCluster, 1024, 0, st>>>(bins, s.t, capacity, carry, n_out, overflow, offsets, s.order, s.ranges, s.parts, s.meta);
     return check_launch("tile_scan");
 }
 
@@ -758,7 +814,7 @@ static int launch_tile_sort(int bins, const ListState& s, const uint64_t* entrie
                             uint32_t tile_n_bits, int32_t* flatten_ids, int64_t* isect_ids, cudaStream_t st) {
     LFS_TIMED("tile_sort", st);
     cudaFuncSetAttribute(tile_sort_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortShared));
-    tile_sort_kernel<OP><<<min(bins, 2 * num_sms()), kSortThreads, sizeof(SortShared), st>>>(s.order, s.ranges, s.meta, entries, overflow, first_bin, n_tiles,
+    tile_sort_kernel<OP><<<min(bins, 2 * num_sms()), kSortThreads, sizeof(SortShared), st>>>(s.order, s.ranges, s.parts, s.meta, entries, overflow, first_bin, n_tiles,
                                                                                              tile_n_bits, flatten_ids, isect_ids);
     return check_launch("tile_sort");
 }
@@ -798,7 +854,7 @@ size_t isect_lists_bytes(int64_t total, int64_t n_isects, IsectBuffers* b, void*
     };
     IsectBuffers x;
     // any number of bins up to kOperatorBins, each with its replicas: 65,536 counters and the padding of 16 sets, or one set
-    x.state = (int32_t*)take(list_words(kOperatorBins, kOperatorBins + 8 * 16) * sizeof(int32_t));
+    x.state = (int32_t*)take(list_words(kOperatorBins, kOperatorBins + 8 * 16, n_isects) * sizeof(int32_t));
     x.scratch.block_sums = (uint32_t*)take((kScanBlocks + 1) * sizeof(uint32_t));
     // sorted: the entries; unsorted: the prefix over the Gaussians
     const size_t entries = (size_t)n_isects * sizeof(uint64_t), prefix = (size_t)total * sizeof(int32_t);

@@ -18,7 +18,7 @@ struct TileListArgs {
     int32_t* flatten_ids;  // [capacity]
     int32_t* overflow;     // device flag set when an instance does not fit: no list is built, all offsets are 0
     int32_t* tile_offsets; // [tw*th + 1]
-    int32_t* state;        // [tile_list_state_words(tw*th)], 16-byte aligned
+    int32_t* state;        // [tile_list_state_words(tw*th, capacity)], 16-byte aligned
     // EWA path: when set, a Gaussian's instances are the tiles of its bounds rectangle that pass the exact
     // ellipse test (`tiles` holds that count); means2d / radii / depths are unused
     const ushort4* ewa_bounds = nullptr;        // [N] (x_min, x_max, y_min, y_max) in tiles
@@ -28,7 +28,7 @@ struct TileListArgs {
 };
 
 int build_tile_lists(const TileListArgs& a, cudaStream_t st);
-size_t tile_list_state_words(int64_t bins);
+size_t tile_list_state_words(int64_t bins, int64_t capacity);
 TileCounters tile_list_counters(int32_t* state, int64_t bins);
 int clear_tile_counters(const TileCounters& t, cudaStream_t st);
 const int32_t* tile_list_order(const int32_t* state, int64_t bins);   // [bins]: tile indices, longest lists first
