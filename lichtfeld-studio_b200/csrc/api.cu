@@ -751,8 +751,10 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
                                  cfg->thin_prism_coeffs, cfg->image_width, cfg->image_height, cfg->camera_model, w.cam, st);
     if (rc != LFS_OK) return rc;
     cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st);
-    const TileCounters counters = tile_list_counters(w.list_state, (int64_t)tw * th);
+    TileCounters counters = tile_list_counters(w.list_state, (int64_t)tw * th);
     clear_tile_counters(counters, st);
+    const bool apart = count_tiles_apart(cfg->N, (int64_t)tw * th);
+    if (apart) counters.counts = nullptr;
     const ProjParams pp = make_proj_params(cfg->eps2d, cfg->near_plane, cfg->far_plane, cfg->radius_clip, cfg->ut);
     PackOptions opt;
     opt.scaling_modifier = cfg_modifier(*cfg);
@@ -764,6 +766,7 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
     if (rc != LFS_OK) return rc;
     if (projected && cudaEventRecord(projected, st) != cudaSuccess) { set_error("cudaEventRecord failed"); return LFS_ECUDA; }
     TileListArgs a{};
+    a.count = apart;
     a.N = cfg->N; a.tw = tw; a.th = th; a.tile_size = cfg->tile_size;
     a.means2d = w.means2d; a.radii = w.radii; a.depths = w.depths; a.tiles = w.tiles;
     a.n_isects_dev = w.counters + 1; a.capacity = cfg->isect_capacity; a.overflow = w.counters + 0;

@@ -544,11 +544,12 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
 // The tiles of the 32 rectangles that the lanes of a warp hold (count tiles each, in row-major order from (x0, y0), `width` wide), 32 at a time:
 // every lane gets one tile and the lane that owns it, so that a rectangle of many tiles does not hold up 31 lanes. All lanes call;
 // f(on, owner, tile x, tile y, index in the rectangle) is called with on = false past the last tile. With U > 1 the results of U calls
-// are collected before then(owner, result) takes them, so that U requests to memory are in flight.
+// are collected before then(owner, result) takes them, so that U requests to memory are in flight. `parts` warps that hold the same rectangles share
+// their tiles, this one takes the share `part`.
 template <int U, class F, class Then>
-__device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y0, uint32_t width, F f, Then then) {
+__device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y0, uint32_t width, int part, int parts, F f, Then then) {
     const int incl = warp_incl_scan(count), total = __shfl_sync(0xffffffffu, incl, 31);
-    for (int base = 0; base < total; base += 32 * U) {
+    for (int base = 32 * U * part; base < total; base += 32 * U * parts) {
         int owners[U], got[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -566,9 +567,9 @@ __device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y
         for (int u = 0; u < U; ++u) then(owners[u], got[u]);
     }
 }
-template <class F>
+template <int U = 1, class F>
 __device__ __forceinline__ void for_each_tile(int count, uint32_t x0, uint32_t y0, uint32_t width, F f) {
-    for_each_tile<1>(count, x0, y0, width, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) { f(on, owner, tx, ty, local); return 0; },
+    for_each_tile<U>(count, x0, y0, width, 0, 1, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) { f(on, owner, tx, ty, local); return 0; },
                      [](int, int) {});
 }
 

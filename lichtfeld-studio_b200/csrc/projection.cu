@@ -687,9 +687,9 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE && RS ? 2 : 4) proje
             tiles[g] = nt;
             ++local_visible;
         }
-        // the lists' lengths, in the shadow of the SH rows
+        // the lists' lengths, in the shadow of the SH rows (unless tile_histogram_kernel counts them)
         int32_t* counts = tile_counters.counts + tile_counters.replica((int64_t)chunk * 32);
-        if (any_vis)
+        if (any_vis && tile_counters.counts)
             for_each_tile(nt, x0, y0, x1 - x0, [&](bool on, int, uint32_t tx, uint32_t ty, uint32_t) {
                 if (on && tx < tw && ty < th) atomicAdd(counts + (size_t)ty * tw + tx, 1);
             });

@@ -95,11 +95,13 @@ constexpr int kInFlight = 4;
 __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(int64_t total, int N, int tw, int th, float tile_size, const int32_t* __restrict__ tiles,
                                                                 const float* __restrict__ means2d, const int32_t* __restrict__ radii,
                                                                 const float* __restrict__ depths, int64_t first_bin, int64_t n_bins, int64_t capacity,
-                                                                const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries) {
+                                                                const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries, int parts) {
     if (overflow && *overflow) return;
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total; base += stride) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32), chunks = (total + 31) / 32;
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < chunks * parts; w += warps) {
+        const int64_t base = w % chunks * 32;
+        const int part = (int)(w / chunks);
         const int64_t i = base + lane;
         int32_t* cursors = t.cursors + t.replica(base);
         const int nt = i < total ? max(tiles[i], 0) : 0;
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(int64_t total, i
             tile_rect(means2d[i * 2], means2d[i * 2 + 1], radii[i * 2], radii[i * 2 + 1], tile_size, tw, th, x0, y0, x1, y1);
             key = __float_as_uint(depths[i]);
         }
-        for_each_tile<kInFlight>(nt, x0, y0, x1 - x0, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
+        for_each_tile<kInFlight>(nt, x0, y0, x1 - x0, part, parts, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
             const int64_t bin = (N == total ? 0 : (base + owner) / N * ((int64_t)tw * th)) + (int64_t)ty * tw + tx - first_bin;
             return on && bin >= 0 && bin < n_bins ? atomicAdd(cursors + bin, 1) : -1;
         }, [&](int owner, int pos) {
@@ -124,11 +126,13 @@ __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(int64_t total, i
 __global__ void __launch_bounds__(kThreads) ewa_scatter_kernel(int N, int tw, const int32_t* __restrict__ n_touched, const ushort4* __restrict__ bounds,
                                                                const uint64_t* __restrict__ masks, const float4* __restrict__ records,
                                                                const uint32_t* __restrict__ depth_bits, int64_t n_bins, int64_t capacity,
-                                                               const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries) {
+                                                               const int32_t* __restrict__ overflow, TileCounters t, uint64_t* __restrict__ entries, int parts) {
     if (*overflow) return;
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < N; base += stride) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32), chunks = (N + 31) / 32;
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < chunks * parts; w += warps) {
+        const int64_t base = w % chunks * 32;
+        const int part = (int)(w / chunks);
         const int64_t i = base + lane;
         int32_t* cursors = t.cursors + t.replica(base);
         const bool on_screen = i < N && n_touched[i] > 0;
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(kThreads) ewa_scatter_kernel(int N, int tw, co
         uint32_t key = 0;
         if (on_screen) { b = bounds[i]; mask = masks[i]; key = depth_bits[i]; }
         const int width = b.y - b.x, area = width * (b.w - b.z);
-        for_each_tile<kInFlight>(area, b.x, b.z, width, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) {
+        for_each_tile<kInFlight>(area, b.x, b.z, width, part, parts, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t local) {
             const uint64_t m = __shfl_sync(0xffffffffu, mask, owner);
             const int owner_area = __shfl_sync(0xffffffffu, area, owner);
             const int64_t g = base + owner, bin = (int64_t)ty * tw + tx;
@@ -159,19 +163,22 @@ __global__ void __launch_bounds__(kThreads) ewa_scatter_kernel(int N, int tw, co
 // Operator level: instances per tile.
 __global__ void __launch_bounds__(kThreads) tile_histogram_kernel(int64_t total, int N, int tw, int th, float tile_size, const int32_t* __restrict__ tiles,
                                                                   const float* __restrict__ means2d, const int32_t* __restrict__ radii, int64_t first_bin,
-                                                                  int64_t n_bins, TileCounters t) {
+                                                                  int64_t n_bins, TileCounters t, int parts) {
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total; base += stride) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32), chunks = (total + 31) / 32;
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; w < chunks * parts; w += warps) {
+        const int64_t base = w % chunks * 32;
+        const int part = (int)(w / chunks);
         const int64_t i = base + lane;
         int32_t* counts = t.counts + t.replica(base);
         const int nt = i < total ? max(tiles[i], 0) : 0;
         uint32_t x0 = 0, y0 = 0, x1 = 0, y1 = 0;
         if (nt > 0) tile_rect(means2d[i * 2], means2d[i * 2 + 1], radii[i * 2], radii[i * 2 + 1], tile_size, tw, th, x0, y0, x1, y1);
-        for_each_tile(nt, x0, y0, x1 - x0, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
+        for_each_tile<1>(nt, x0, y0, x1 - x0, part, parts, [&](bool on, int owner, uint32_t tx, uint32_t ty, uint32_t) {
             const int64_t bin = (N == total ? 0 : (base + owner) / N * ((int64_t)tw * th)) + (int64_t)ty * tw + tx - first_bin;
             if (on && bin >= 0 && bin < n_bins) atomicAdd(counts + bin, 1);
-        });
+            return 0;
+        }, [](int, int) {});
     }
 }
 
@@ -819,20 +826,36 @@ static int launch_tile_sort(int bins, const ListState& s, const uint64_t* entrie
     return check_launch("tile_sort");
 }
 
+// Warps per 32 Gaussians, where four or more of them still fit the GPU with eight CTAs per SM: of few Gaussians on a large image each has hundreds of tiles
+// (11 k at 2790x1646, 160 each: scatter 102 -> 24 us; 60 k, EWA, 777x519: 16.8 -> 12.9).
+static int scatter_parts(int64_t total) {
+    const int64_t parts = (int64_t)64 * num_sms() / max((total + 31) / 32, (int64_t)1);
+    return parts < 4 ? 1 : (int)min(parts, (int64_t)8);
+}
+// The per-Gaussian stage has one warp per 32 Gaussians, so where scatter_parts takes more and the image is large beside the Gaussians' number the
+// counting gets a launch of its own (the same scene: projection 77 us, of which 61 went into the counting; 77 -> 16 and 17 for the launch).
+bool count_tiles_apart(int64_t N, int64_t bins) { return scatter_parts(N) > 1 && 8 * bins >= N; }
+
 int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
+    const int parts = scatter_parts(a.N);
     const int bins = a.tw * a.th;
     const ListState s = list_state(a.state, bins);
+    if (a.count && a.N > 0) {
+        LFS_TIMED("tile_histogram", st);
+        tile_histogram_kernel<<<grid_for((int64_t)a.N * parts, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d,
+                                                                                            a.radii, 0, bins, s.t, parts);
+    }
     int rc = launch_tile_scan(bins, s, a.capacity, nullptr, a.n_isects_dev, a.overflow, a.tile_offsets, st);
     if (rc != LFS_OK) return rc;
     if (a.N > 0 && a.capacity > 0 && bins > 0) {
         {
             LFS_TIMED("tile_scatter", st);
             if (a.ewa_bounds)
-                ewa_scatter_kernel<<<grid_for(a.N, kThreads), kThreads, 0, st>>>(a.N, a.tw, a.tiles, a.ewa_bounds, a.ewa_masks, a.ewa_records, a.ewa_depth_bits,
-                                                                                 bins, a.capacity, a.overflow, s.t, a.entries);
+                ewa_scatter_kernel<<<grid_for((int64_t)a.N * parts, kThreads), kThreads, 0, st>>>(a.N, a.tw, a.tiles, a.ewa_bounds, a.ewa_masks, a.ewa_records, a.ewa_depth_bits,
+                                                                                 bins, a.capacity, a.overflow, s.t, a.entries, parts);
             else
-                tile_scatter_kernel<<<grid_for(a.N, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d, a.radii,
-                                                                                  a.depths, 0, bins, a.capacity, a.overflow, s.t, a.entries);
+                tile_scatter_kernel<<<grid_for((int64_t)a.N * parts, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d, a.radii,
+                                                                                  a.depths, 0, bins, a.capacity, a.overflow, s.t, a.entries, parts);
         }
         rc = launch_tile_sort<false>(bins, s, a.entries, a.overflow, 0, 1, 0, a.flatten_ids, nullptr, st);
         if (rc != LFS_OK) return rc;
@@ -873,7 +896,7 @@ int build_isect_lists(int C, int N, int tw, int th, int tile_size, int sort, con
         set_error("build_isect_lists: tile and camera ids need more than 32 bits");
         return LFS_EINVAL;
     }
-    const int grid = grid_for(total, kThreads);
+    const int parts = scatter_parts(total), grid = grid_for(total * parts, kThreads);
     if (!sort) {
         const int rc = exclusive_scan(tiles, total, b.prefix, nullptr, b.scratch, st);
         if (rc != LFS_OK) return rc;
@@ -889,14 +912,14 @@ int build_isect_lists(int C, int N, int tw, int th, int tile_size, int sort, con
         if (clear_tile_counters(s.t, st) != LFS_OK) { set_error("build_isect_lists: memset failed"); return LFS_ECUDA; }
         {
             LFS_TIMED("tile_histogram", st);
-            tile_histogram_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, first, bins, s.t);
+            tile_histogram_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, first, bins, s.t, parts);
         }
         int rc = launch_tile_scan(bins, s, n_isects, s.carry, nullptr, nullptr, s.offsets, st);
         if (rc != LFS_OK) return rc;
         {
             LFS_TIMED("tile_scatter", st);
             tile_scatter_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, depths, first, bins, n_isects, nullptr,
-                                                           s.t, b.entries);
+                                                           s.t, b.entries, parts);
         }
         rc = launch_tile_sort<true>(bins, s, b.entries, nullptr, first, n_tiles, tile_n_bits, flatten_ids, isect_ids, st);
         if (rc != LFS_OK) return rc;

@@ -7,6 +7,7 @@ namespace lfs {
 
 // Lists of one camera. The per-Gaussian stage has counted the instances of every tile into the counters (cleared before it).
 struct TileListArgs {
+    bool count;          // the instances have not been counted yet (see count_tiles_apart)
     int N, tw, th, tile_size;
     const float* means2d;
     const int32_t* radii;
@@ -28,6 +29,8 @@ struct TileListArgs {
 };
 
 int build_tile_lists(const TileListArgs& a, cudaStream_t st);
+// whether a kernel of its own counts the instances of N Gaussians in `bins` tiles, instead of the per-Gaussian stage
+bool count_tiles_apart(int64_t N, int64_t bins);
 size_t tile_list_state_words(int64_t bins, int64_t capacity);
 TileCounters tile_list_counters(int32_t* state, int64_t bins);
 int clear_tile_counters(const TileCounters& t, cudaStream_t st);
