@@ -515,7 +515,9 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         const float slope = phi_max >= 1.0f ? 1e30f : sqrtf(fmaxf(phi_max, 0.f) / (1.0f - phi_max));
         box.z = __float_as_uint(m2 > 0.f ? slope : INFINITY);
         rec[1] = make_float4(p2[0], p2[1], p2[2], phi_cut);
-        rec[2] = make_float4(p3[0], p3[1], p3[2], (1.0f / 255.0f) * __expf(fminf(band, 8.0f)));
+        // alpha below which kept_at_cut decides; infinity marks an infinite or NaN colour
+        const bool finite = fabsf(r) + fabsf(g) + fabsf(b) + fabsf(extra) < INFINITY;
+        rec[2] = make_float4(p3[0], p3[1], p3[2], finite ? (1.0f / 255.0f) * __expf(fminf(band, 8.0f)) : INFINITY);
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);

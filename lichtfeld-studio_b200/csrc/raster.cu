@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     }
     const CamDev& cam = cams[0];
     f3 d[PX];
-    bool takes_part[PX];
+    bool takes_part[PX], going[PX];
     float dc[3][PX];
     uint32_t cur_idx[PX];
 #pragma unroll
@@ -339,14 +339,12 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
         f3 wd;
         takes_part[q] = pixel_cam_dir<MODEL>(cam, (float)(j0 + q) + 0.5f, (float)i + 0.5f, d[q], wd) && i < H && j0 + q < W;
         sm.ray[q][lane] = wd;
-        dc[1][q] = d[q].y; dc[2][q] = d[q].z;
-        // a pixel that takes no part, or no longer, has no direction: every comparison with its distance is false
-        dc[0][q] = takes_part[q] ? d[q].x : CUDART_NAN_F;
+        dc[0][q] = d[q].x; dc[1][q] = d[q].y; dc[2][q] = d[q].z;
+        going[q] = takes_part[q];
         cur_idx[q] = 0;
     }
     const PatchRays rays = patch_rays<MODEL, PX>(d, takes_part);
-    V dx = P::make(dc[0]);
-    const V dy = P::make(dc[1]), dz = P::make(dc[2]), minus_one = P::all(-1.0f);
+    const V dx = P::make(dc[0]), dy = P::make(dc[1]), dz = P::make(dc[2]), minus_one = P::all(-1.0f);
     V T = P::all(1.0f), pr = P::all(0.f), pg = P::all(0.f), pb = P::all(0.f), px = P::all(0.f);
 
     const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
@@ -361,11 +359,9 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     }
     for (int b = 0; b < n_batches; ++b) {
         const int32_t batch_start = range_start + 32 * b;
-        float left[PX];
-        P::get(dx, left);
         bool any_left = false;
 #pragma unroll
-        for (int q = 0; q < PX; ++q) any_left = any_left || left[q] == left[q];
+        for (int q = 0; q < PX; ++q) any_left = any_left || going[q];
         // also: everybody has finished walking batch b - 1, whose buffer is filled next
         if (!__any_sync(0xffffffffu, any_left)) break;
         const uint32_t staged = feed.mask;
@@ -377,11 +373,17 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
             cp_async_wait<0>();
         }
         __syncwarp();
-        const WarpStage& st = sm.stage[b & 1];
+        WarpStage& st = sm.stage[b & 1];
         // entries whose forms miss this warp's patch are dropped up front
         bool reached = staged >> lane & 1u;
+        // an infinite or NaN colour (make_record marks it): zero times it is not zero, so it is added where a pair near the cut is decided
+        if (reached && st.rec[2][lane].w == CUDART_INF_F) {
+            st.rec[3][lane] = make_float4(0.f, 0.f, 0.f, st.rec[3][lane].w);
+            st.zw[lane].y = 0.f;
+        }
         if (reached) reached = patch_reached<MODEL>(st.rec[0][lane], st.rec[1][lane], st.rec[2][lane], st.zw[lane].x, rays);
         uint32_t bits = __ballot_sync(0xffffffffu, reached);
+        __syncwarp();
         while (bits) {
             const int t = __ffs(bits) - 1;
             bits &= bits - 1;
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
             bool valid[PX], any_valid = false;
 #pragma unroll
             for (int q = 0; q < PX; ++q) {
-                valid[q] = E[q] <= limit[q];
+                valid[q] = going[q] && !(E[q] > limit[q]);
                 any_valid = any_valid || valid[q];
             }
             if (kVote && !__any_sync(0xffffffffu, any_valid)) continue;
@@ -414,6 +416,19 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
                 const uint32_t kept = kept_at_cut<PX>(cuts + st.sid[t], n_cuts, &sm.ray[0][lane], 32, r3.w);
 #pragma unroll
                 for (int q = 0; q < PX; ++q) valid[q] = valid[q] && ((kept >> q & 1u) || !(alpha[q] < r2.w));
+                if (r2.w == CUDART_INF_F) {
+                    const float4 colour = records[(size_t)st.sid[t] * 4 + 3];
+                    float tq[PX], c0[PX], c1[PX], c2[PX], c3[PX];
+                    P::get(T, tq); P::get(pr, c0); P::get(pg, c1); P::get(pb, c2); P::get(px, c3);
+#pragma unroll
+                    for (int q = 0; q < PX; ++q) {
+                        if (!valid[q] || tq[q] * (1.0f - alpha[q]) <= 1e-4f) continue;
+                        const float w = tq[q] * alpha[q];
+                        c0[q] += w * colour.x; c1[q] += w * colour.y; c2[q] += w * colour.z;
+                        if (EXTRA) c3[q] += w * __uint_as_float(bounds[st.sid[t]].w);
+                    }
+                    pr = P::make(c0); pg = P::make(c1); pb = P::make(c2); px = P::make(c3);
+                }
             }
 #pragma unroll
             for (int q = 0; q < PX; ++q)
@@ -426,13 +441,11 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
 #pragma unroll
             for (int q = 0; q < PX; ++q) stops = stops || nt[q] <= 1e-4f;   // no pixel without alpha comes here: its T is above
             if (stops) {
-                float x[PX], t0[PX];
-                P::get(dx, x);
+                float t0[PX];
                 P::get(T, t0);
 #pragma unroll
                 for (int q = 0; q < PX; ++q)
-                    if (nt[q] <= 1e-4f) { valid[q] = false; alpha[q] = 0.f; nt[q] = t0[q]; x[q] = CUDART_NAN_F; }
-                dx = P::make(x);
+                    if (nt[q] <= 1e-4f) { valid[q] = going[q] = false; alpha[q] = 0.f; nt[q] = t0[q]; }
                 al = P::make(alpha);
                 next_T = P::make(nt);
             }
