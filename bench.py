@@ -42,14 +42,14 @@ if str(ROOT) not in sys.path:
 
 LRS = [1.6e-4, 2.5e-3, 1.25e-4, 5e-3, 1e-3, 5e-2]  # means, sh0, shN, scaling, rotation, opacity
 METRIC = "train steps/s (fwd+loss+bwd+Adam)"
-# Profiler counters of ONE raster_bwd_kernel launch on train_1m (ncu, --clock-control none): DRAM bytes read + written,
+# Profiler counters of ONE raster_bwd_patch_kernel launch on 1 M Gaussians at 1296x840 (ncu, --clock-control none): DRAM bytes read + written,
 # share of issue slots used, share of issued warp instructions on the FMA pipe relative to the FP32 peak rate. They are
-# reported next to the event-timed figures because a kernel's traffic and pipe utilisation cannot be read outside a profiler. Captured
-# before the pairs at the 1/255 cut got their own test, which adds a compare and a vote per walked entry.
-NCU_RASTER_BWD = {"dram_bytes": 182.6e6, "issue_slots_active": 0.78, "fma_pipe_of_fp32_peak": 0.42, "shared_pipe": 0.72,
-                  # 371e6 warp instructions on the FMA pipe x 32 lanes x 2 flop over the 4.24e8 pairs of the captured launch
+# reported next to the event-timed figures because a kernel's traffic and pipe utilisation cannot be read outside a profiler. The
+# kernel's arithmetic per pair is that of the scalar kernel before it, whose flops are counted here (packed instructions hide two in one).
+NCU_RASTER_BWD = {"dram_bytes": 132e6, "issue_slots_active": 0.71, "shared_pipe": 0.80,
+                  # 371e6 scalar warp instructions on the FMA pipe x 32 lanes x 2 flop over the 4.24e8 pairs of the captured launch
                   "executed_flop_per_pair": 56.1}
-NCU_RASTER_FWD_FLOP = 137e6 * 32 * 2   # FMA-pipe warp instructions of one raster_fwd_kernel launch on the same workload x lanes x 2
+NCU_RASTER_FWD_FLOP = 137e6 * 32 * 2   # FMA-pipe warp instructions of one launch of the scalar forward on the same workload x lanes x 2
 
 
 def load_peaks():
@@ -638,7 +638,7 @@ def run_ours(args):
         ncu = NCU_RASTER_BWD if workload == "train_1m" else None
         ach = ncu["executed_flop_per_pair"] * q_b / (t_bwd * 1e-3) / 1e12 if ncu else None
         ach_fwd = NCU_RASTER_FWD_FLOP / (t_fwd * 1e-3) / 1e12 if ncu else None
-        roofline = {"kernel": "raster_bwd_kernel", "bound": "fp32", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",
+        roofline = {"kernel": "raster_bwd_patch_kernel", "bound": "fp32", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",
                     "frac": ach / fp32_peak if ncu else None, "traffic": ncu["dram_bytes"] if ncu else None,
                     "pairs_per_s": q_b / (t_bwd * 1e-3),
                     # the reference's arithmetic per pair at this kernel's rate: a comparison of speeds, not a share of the peak
@@ -668,7 +668,7 @@ def run_ours(args):
         extra = {"roofline_adam": {"kernel": adam_kernel, "bound": "hbm", "achieved": adam_gbs,
                                    "peak": hbm_peak, "unit": "GB/s", "frac": adam_gbs / hbm_peak if adam_gbs else None,
                                    "traffic": None, "note": f"{adam_note}, of {peak_kind}"},
-                 "roofline_raster_fwd": {"kernel": "raster_fwd_kernel", "bound": "fp32",
+                 "roofline_raster_fwd": {"kernel": "raster_fwd_patch_kernel", "bound": "fp32",
                                          "achieved": ach_fwd, "peak": fp32_peak, "unit": "TFLOP/s",
                                          "frac": ach_fwd / fp32_peak if ncu else None,
                                          "reference_arithmetic": 70.0 * q_list / (t_fwd * 1e-3) / 1e12,
