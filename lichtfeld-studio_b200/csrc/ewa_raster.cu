@@ -7,7 +7,7 @@
 // Design: a warp owns a patch of pixels and walks its tile's depth-sorted list by itself, 32 entries at a time: packed 48-byte records come to its part of
 // shared memory by 16-byte asynchronous copies while the batch before is walked. It tests the 32 entries against its patch with the same
 // ellipse-versus-rectangle test that built the tile lists, and walks only those that can reach it. (With the warps of a tile on one staged batch, a barrier
-// apart: 1 M Gaussians, 1296x840, forward 350 us against 345, backward 617 against 546; 100 k at 256x256 142 against 89 and 200 against 125.) A thread owns
+// apart: 1 M Gaussians, 1296x840, forward 350 us against 330, backward 617 against 546; 100 k at 256x256 142 against 89 and 200 against 125.) A thread owns
 // one pixel or two horizontally adjacent ones, evaluated by the packed fp32 instructions. The backward walks the lists
 // from the warp's last contributor to the front (transmittance is recovered by division, so no per-bucket state
 // is stored by the forward, unlike the reference); an entry's nine gradient terms are summed over the warp by a transpose through shared memory and leave as
@@ -17,6 +17,7 @@
 #include "gsmath.cuh"
 #include "pixels.cuh"
 #include <math_constants.h>
+#include <type_traits>
 
 namespace lfs {
 namespace {
@@ -73,6 +74,15 @@ __device__ __forceinline__ typename Pixels<PX>::V ewa_sigma(const float4& r0, fl
     return fma2(P::all(0.5f), X, mul2(mul2(P::all(r0.w), dx), P::all(dy)));
 }
 constexpr float kNegLog2e = -1.4426950408889634f;
+template <int PX>
+__device__ __forceinline__ typename Pixels<PX>::V chosen(const bool* which, typename Pixels<PX>::V yes, typename Pixels<PX>::V no) {
+    float y[PX], n[PX];
+    Pixels<PX>::get(yes, y);
+    Pixels<PX>::get(no, n);
+#pragma unroll
+    for (int q = 0; q < PX; ++q) y[q] = which[q] ? y[q] : n[q];
+    return Pixels<PX>::make(y);
+}
 
 // A warp owns a patch of 8 x 4 PX pixels and stages its own entries: no barrier, and a warp whose pixels are finished stops by itself. Which pairs count is
 // decided on 8x4 pixels whatever PX is (ewa_rect_contributes says why that matters).
@@ -133,20 +143,15 @@ __global__ void __launch_bounds__(128, PX == 2 ? 8 : 10) ewa_blend_fwd_kernel(
             kept = lane < 16 ? bits : lower;
             bits |= lower;
         }
-        // entries whose colour is infinite or NaN: zero times such a colour is not zero, so they are added apart, where they count
+        // entries of infinite colour: zero times it is not zero, so its pixels are chosen one by one
         bool odd_colour = false;
         if (bits >> lane & 1u) odd_colour = !(fabsf(st.r1[lane].z) + fabsf(st.r1[lane].w) + fabsf(st.r2[lane].x) < CUDART_INF_F);
-        const uint32_t odd = __ballot_sync(0xffffffffu, odd_colour);
+        uint32_t odd = __ballot_sync(0xffffffffu, odd_colour);
         uint32_t mine[PX];   // the entries that a pixel still asks
 #pragma unroll
         for (int q = 0; q < PX; ++q) mine[q] = going[q] ? kept : 0u;
-        while (bits) {
-            const int t = __ffs(bits) - 1;
-            const uint32_t lowest = bits & (0u - bits);
-            bits &= bits - 1;
-            const float4 r0 = st.r0[t];
-            float4 r1 = st.r1[t];
-            float blue = st.r2[t].x;
+        auto blend = [&](int t, uint32_t lowest, auto finite) {
+            const float4 r0 = st.r0[t], r1 = st.r1[t];
             const V dx = add2(P::all(r0.x), npx), sigma = ewa_sigma<PX>(r0, r1.x, dx, r0.y - py);
             float s[PX], e[PX], a[PX];
             P::get(sigma, s);
@@ -165,10 +170,10 @@ __global__ void __launch_bounds__(128, PX == 2 ? 8 : 10) ewa_blend_fwd_kernel(
             V next_T = mul2(T, mul2(add2(al, minus_one), minus_one));
             float nt[PX];
             P::get(next_T, nt);
-            bool rare = (odd & lowest) != 0u;
+            bool stops = false;
 #pragma unroll
-            for (int q = 0; q < PX; ++q) rare = rare || nt[q] < kEwaMinTransmittance;   // no pixel without alpha stops: its T is not below
-            if (rare) {
+            for (int q = 0; q < PX; ++q) stops = stops || nt[q] < kEwaMinTransmittance;   // no pixel without alpha comes here: its T is not below
+            if (stops) {
                 float t0[PX];
                 P::get(T, t0);
 #pragma unroll
@@ -176,21 +181,33 @@ __global__ void __launch_bounds__(128, PX == 2 ? 8 : 10) ewa_blend_fwd_kernel(
                     if (nt[q] < kEwaMinTransmittance) { valid[q] = going[q] = false; mine[q] = 0u; a[q] = 0.f; nt[q] = t0[q]; }
                 al = P::make(a);
                 next_T = P::make(nt);
-                if ((odd & lowest) != 0u) {
-                    float r[PX], g[PX], bl[PX];
-                    P::get(cr, r); P::get(cg, g); P::get(cb, bl);
-#pragma unroll
-                    for (int q = 0; q < PX; ++q)
-                        if (valid[q]) { r[q] += t0[q] * a[q] * r1.z; g[q] += t0[q] * a[q] * r1.w; bl[q] += t0[q] * a[q] * blue; }
-                    cr = P::make(r); cg = P::make(g); cb = P::make(bl);
-                    r1.z = r1.w = blue = 0.f;
-                }
             }
             const V w = mul2(T, al);
-            cr = fma2(w, P::all(r1.z), cr); cg = fma2(w, P::all(r1.w), cg); cb = fma2(w, P::all(blue), cb);
+            const V red = fma2(w, P::all(r1.z), cr), green = fma2(w, P::all(r1.w), cg), blue = fma2(w, P::all(st.r2[t].x), cb);
+            if constexpr (decltype(finite)::value) {
+                cr = red; cg = green; cb = blue;
+            } else {
+                cr = chosen<PX>(valid, red, cr); cg = chosen<PX>(valid, green, cg); cb = chosen<PX>(valid, blue, cb);
+            }
             T = next_T;
 #pragma unroll
             for (int q = 0; q < PX; ++q) last[q] = valid[q] ? 32 * b + t + 1 : last[q];
+        };
+        while (bits) {
+            // up to the next odd one, or all
+            uint32_t run = bits & ((odd & (0u - odd)) - 1u);
+            bits &= ~run;
+            while (run) {
+                const uint32_t lowest = run & (0u - run);
+                blend(__ffs(run) - 1, lowest, std::true_type{});
+                run &= run - 1;
+            }
+            if (odd) {
+                const uint32_t lowest = odd & (0u - odd);
+                blend(__ffs(odd) - 1, lowest, std::false_type{});
+                odd &= odd - 1;
+                bits &= ~lowest;
+            }
         }
     }
     cp_async_wait<0>();

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     }
     const CamDev& cam = cams[0];
     f3 d[PX];
-    bool takes_part[PX], going[PX];
+    bool takes_part[PX];
     float dc[3][PX];
     uint32_t cur_idx[PX];
 #pragma unroll
@@ -339,12 +339,14 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
         f3 wd;
         takes_part[q] = pixel_cam_dir<MODEL>(cam, (float)(j0 + q) + 0.5f, (float)i + 0.5f, d[q], wd) && i < H && j0 + q < W;
         sm.ray[q][lane] = wd;
-        dc[0][q] = d[q].x; dc[1][q] = d[q].y; dc[2][q] = d[q].z;
-        going[q] = takes_part[q];
+        dc[1][q] = d[q].y; dc[2][q] = d[q].z;
+        // a pixel that takes no part, or no longer, has no direction: every comparison with its distance is false
+        dc[0][q] = takes_part[q] ? d[q].x : CUDART_NAN_F;
         cur_idx[q] = 0;
     }
     const PatchRays rays = patch_rays<MODEL, PX>(d, takes_part);
-    const V dx = P::make(dc[0]), dy = P::make(dc[1]), dz = P::make(dc[2]), minus_one = P::all(-1.0f);
+    V dx = P::make(dc[0]);
+    const V dy = P::make(dc[1]), dz = P::make(dc[2]), minus_one = P::all(-1.0f);
     V T = P::all(1.0f), pr = P::all(0.f), pg = P::all(0.f), pb = P::all(0.f), px = P::all(0.f);
 
     const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
@@ -359,9 +361,11 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     }
     for (int b = 0; b < n_batches; ++b) {
         const int32_t batch_start = range_start + 32 * b;
+        float left[PX];
+        P::get(dx, left);
         bool any_left = false;
 #pragma unroll
-        for (int q = 0; q < PX; ++q) any_left = any_left || going[q];
+        for (int q = 0; q < PX; ++q) any_left = any_left || left[q] == left[q];
         // also: everybody has finished walking batch b - 1, whose buffer is filled next
         if (!__any_sync(0xffffffffu, any_left)) break;
         const uint32_t staged = feed.mask;
@@ -396,7 +400,7 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
             bool valid[PX], any_valid = false;
 #pragma unroll
             for (int q = 0; q < PX; ++q) {
-                valid[q] = going[q] && !(E[q] > limit[q]);
+                valid[q] = E[q] <= limit[q];
                 any_valid = any_valid || valid[q];
             }
             if (kVote && !__any_sync(0xffffffffu, any_valid)) continue;
@@ -441,11 +445,13 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
 #pragma unroll
             for (int q = 0; q < PX; ++q) stops = stops || nt[q] <= 1e-4f;   // no pixel without alpha comes here: its T is above
             if (stops) {
-                float t0[PX];
+                float x[PX], t0[PX];
+                P::get(dx, x);
                 P::get(T, t0);
 #pragma unroll
                 for (int q = 0; q < PX; ++q)
-                    if (nt[q] <= 1e-4f) { valid[q] = going[q] = false; alpha[q] = 0.f; nt[q] = t0[q]; }
+                    if (nt[q] <= 1e-4f) { valid[q] = false; alpha[q] = 0.f; nt[q] = t0[q]; x[q] = CUDART_NAN_F; }
+                dx = P::make(x);
                 al = P::make(alpha);
                 next_T = P::make(nt);
             }
