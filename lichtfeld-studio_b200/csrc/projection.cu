@@ -518,6 +518,16 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         // alpha below which kept_at_cut decides; infinity marks an infinite or NaN colour
         const bool finite = fabsf(r) + fabsf(g) + fabsf(b) + fabsf(extra) < INFINITY;
         rec[2] = make_float4(p3[0], p3[1], p3[2], finite ? (1.0f / 255.0f) * __expf(fminf(band, 8.0f)) : INFINITY);
+        // A scale without a reciprocal makes the forms infinite or NaN, or the limit NaN, and NaN is the response along every ray; min(0.999, NaN) blends it with 0.999
+        // into every pixel of its tiles. Forms that every pixel accepts, no box and an exponent of NaN say so without a test per pair.
+        const float forms = fabsf(p1[0]) + fabsf(p1[1]) + fabsf(p1[2]) + fabsf(p2[0]) + fabsf(p2[1]) + fabsf(p2[2]) + fabsf(p3[0]) + fabsf(p3[1]) + fabsf(p3[2]);
+        if (!(forms < INFINITY) || isnan(phi_cut)) {
+            rec[0] = make_float4(0.f, 0.f, 0.f, NAN);
+            rec[1] = make_float4(0.f, 0.f, 0.f, 1.0f);
+            rec[2] = make_float4(0.f, 0.f, 1.0f, rec[2].w);
+            box.z = __float_as_uint(INFINITY);
+            return;
+        }
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);

@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
             bool valid[PX], any_valid = false, near_cut = false;
 #pragma unroll
             for (int q = 0; q < PX; ++q) {
-                valid[q] = batch_end - t <= bin_final[q] && !(E[q] > limit[q]);
+                valid[q] = batch_end - t <= bin_final[q] && E[q] <= limit[q];   // the forward's comparison: it decides for NaN too
                 any_valid = any_valid || valid[q];
                 den[q] = rcp_approx(den[q]);
             }
