@@ -832,7 +832,7 @@ int lfs_render_forward_shade(const lfs_render_config* cfg, const lfs_splats* par
     cudaStream_t st = S(stream);
     const int tw = (cfg->image_width + 15) / 16, th = (cfg->image_height + 15) / 16;
     if (mode_channels(cfg->render_mode) != 1) {
-        rc = launch_sh_color(cfg->N, cfg->sh_coeffs, cfg->sh_degree, *params, w.cam, w.radii, w.records, st);
+        rc = launch_sh_color(cfg->N, cfg->sh_coeffs, cfg->sh_degree, *params, w.cam, w.radii, cfg_rolling(*cfg), w.records, st);
         if (rc != LFS_OK) return rc;
     }
     rc = render_forward_blend(cfg, background, render, alpha, status_dev, w, st);

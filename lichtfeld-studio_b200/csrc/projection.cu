@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(256, MODEL == LFS_FISHEYE && RS ? 2 : 4) proje
 __global__ void __launch_bounds__(256) sh_color_kernel(int N, int K, int sh_degree, const float* __restrict__ means,
                                                        const float* __restrict__ sh0, const float* __restrict__ shN,
                                                        const CamDev* __restrict__ cams, const int32_t* __restrict__ radii,
-                                                       float4* __restrict__ records) {
+                                                       int rolling, float4* __restrict__ records) {
     extern __shared__ __align__(16) float s_rows[];
     const float cx = cams[0].campos[0], cy = cams[0].campos[1], cz = cams[0].campos[2];
     const int rest = (K - 1) * 3;
@@ -791,19 +791,21 @@ __global__ void __launch_bounds__(256) sh_color_kernel(int N, int K, int sh_degr
             float* out = reinterpret_cast<float*>(records + (size_t)g * 4 + 3);
 #pragma unroll
             for (int c = 0; c < 3; ++c) out[c] = fmaxf(rgb[c] + 0.5f, 0.0f);
+            // make_record's mark of an infinite colour; it was given none. (Under a rolling shutter the word belongs to the ray origin.)
+            if (!rolling && !(out[0] + out[1] + out[2] < INFINITY)) records[(size_t)g * 4 + 2].w = INFINITY;
         }
         __syncwarp();
     }
 }
 
-int launch_sh_color(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const int32_t* radii, float4* records,
+int launch_sh_color(int N, int K, int sh_degree, const lfs_splats& p, const CamDev* cam, const int32_t* radii, int rolling, float4* records,
                     cudaStream_t st) {
     if (N == 0) return LFS_OK;
     const size_t smem = (size_t)8 * 32 * (K - 1) * 3 * sizeof(float);
     if (smem > 200 * 1024) { set_error("sh_color: too many SH coefficients"); return LFS_EINVAL; }
     if (smem > 48 * 1024) cudaFuncSetAttribute(sh_color_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     LFS_TIMED("sh_color", st);
-    sh_color_kernel<<<grid_for(N, 256), 256, smem, st>>>(N, K, sh_degree, p.means, p.sh0, p.shN, cam, radii, records);
+    sh_color_kernel<<<grid_for(N, 256), 256, smem, st>>>(N, K, sh_degree, p.means, p.sh0, p.shN, cam, radii, rolling, records);
     return check_launch("sh_color");
 }
 

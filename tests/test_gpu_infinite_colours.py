@@ -43,3 +43,23 @@ def test_only_blended_pixels_are_infinite(pkg, synth, W, H, lens, ewa):
     assert 0 < blended.sum() < blended.size
     assert np.array_equal(~np.isfinite(infinite).all(0), blended)
     assert np.array_equal(infinite[:, ~blended], dark[:, ~blended])
+
+
+# the colours in a call of their own after the lists (the form of the data-parallel step)
+@pytest.mark.parametrize("W,H,mode", [(41, 23, 0), (1024, 600, 0), (137, 90, 4)])
+@pytest.mark.parametrize("value", [np.inf, 1e9])
+def test_split_forward_is_the_whole_one(pkg, synth, W, H, mode, value):
+    n = 40
+    rng = np.random.default_rng(W)
+    P = dict(means=0.3 * rng.standard_normal((n, 3)), sh0=0.5 * rng.standard_normal((n, 1, 3)), shN=0.1 * rng.standard_normal((n, 3, 3)),
+             scaling_raw=-2.0 + 0.3 * rng.standard_normal((n, 3)), rotation_raw=rng.standard_normal((n, 4)), opacity_raw=rng.standard_normal((n, 1)))
+    P["sh0"][17] = value
+    tr = pkg.trainer
+    model = tr.SplatData(n, 4, DEV).load({k: np.ascontiguousarray(v, np.float32) for k, v in P.items()})
+    rast = tr.Rasterizer(model, W, H, 1, render_mode=mode)
+    cam = tr.Camera(T(synth.hemisphere_poses(1, 4.0)[0]), T(synth.intrinsics(1.2 * W, 1.2 * W, W / 2.0, H / 2.0)), W, H)
+    whole = rast.forward(cam, None).render.cpu().numpy()
+    assert np.isfinite(whole).any() and not (np.isfinite(whole).all() and np.isinf(value))
+    rast.forward_lists(cam)
+    split = rast.forward_shade(None).render.cpu().numpy()
+    assert np.array_equal(whole, split, equal_nan=True)
