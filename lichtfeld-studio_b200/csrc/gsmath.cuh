@@ -135,7 +135,8 @@ __device__ __forceinline__ double angle_near(const AxisAngle& a, float n, float 
     y = fma(y, fma(-dot, y, 1.0), y);
     double t = cross * y;
     t = fma(fma(-t, dot, cross), y, t);
-    if (!(fabs(t) < 0.03125)) return atan2(nd, zd);   // far apart, or out of the range of the float reciprocal
+    // far apart, or a product whose float reciprocal is infinite (t is NaN) or flushed towards 0 (t would be 0)
+    if (!(fabs(t) < 0.03125 && dot < 8e37)) return atan2(nd, zd);
     const double s = t * t;
     double p = fma(s, -1.0 / 11.0, 1.0 / 9.0);
     p = fma(s, p, -1.0 / 7.0);
