@@ -366,9 +366,10 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
         bool any_left = false;
 #pragma unroll
         for (int q = 0; q < PX; ++q) any_left = any_left || left[q] == left[q];
-        // also: everybody has finished walking batch b - 1, whose buffer is filled next
         if (!__any_sync(0xffffffffu, any_left)) break;
         const uint32_t staged = feed.mask;
+        // everybody has read batch b - 1, whose buffer is filled next: a vote would not order memory
+        __syncwarp();
         if (b + 1 < n_batches) {
             feed.stage(sm.stage[(b + 1) & 1], total - 32 * (b + 1), patch_x, patch_y, records, bounds, batch_ids(b + 3), lane);
             if (!staged) continue;
