@@ -391,7 +391,7 @@ __device__ __forceinline__ void group_sync(int group) {
 __device__ __forceinline__ uint32_t bucket_slot(uint32_t b) { return b + (b >> 5); }
 
 template <int G, int K, bool RELOAD, class Load, class Out>
-__device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t* __restrict__ entry, uint32_t* __restrict__ start,
+__device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t* entry, uint32_t* __restrict__ start,
                                              uint32_t (*red)[kSortThreads / 32][2], Load load, Out out) {
     constexpr int kWarps = G / 32;
     const int lane = tid & 31, warp = tid >> 5;
@@ -497,9 +497,9 @@ __device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t
     }
     group_sync<G>(group);
 }
-// n <= 8 G, or 16 G where the entries can be read again
+// n <= 8 G, or 16 G where the entries can be read again. `load` may read `entry` itself unless LONG: every entry is in a register before the first is written.
 template <int G, bool LONG, class Load, class Out>
-__device__ __forceinline__ void sort_group(int tid, int group, int n, uint64_t* __restrict__ entry, uint32_t* __restrict__ start,
+__device__ __forceinline__ void sort_group(int tid, int group, int n, uint64_t* entry, uint32_t* __restrict__ start,
                                            uint32_t (*red)[kSortThreads / 32][2], Load load, Out out) {
     if (n <= 4 * G) sort_group_k<G, 4, false>(tid, group, n, entry, start, red, load, out);
     else if (!LONG || n <= 8 * G) sort_group_k<G, 8, false>(tid, group, n, entry, start, red, load, out);
