@@ -637,8 +637,10 @@ int lfs_ewa_forward(const lfs_ewa_config* cfg, const lfs_splats* params, const f
     const EwaCamera cam = ewa_camera(*cfg, w2c, cam_position);
     const size_t bins = (size_t)cam.tw * cam.th;
     const TileCounters counters = tile_list_counters(w.list_state, (int64_t)bins);
-    cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st);
-    clear_tile_counters(counters, st);
+    if (cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st) != cudaSuccess || clear_tile_counters(counters, st) != LFS_OK) {
+        set_error("lfs_ewa_forward: memset failed");
+        return LFS_ECUDA;
+    }
     rc = launch_ewa_preprocess(cfg->N, *params, cam, w.n_touched, w.bounds, w.records, w.depth_bits, w.masks, counters,
                                reinterpret_cast<float4*>(w.accum), w.counters + 2, st);
     if (rc != LFS_OK) return rc;
@@ -750,9 +752,11 @@ static int render_forward_lists(const lfs_render_config* cfg, const lfs_splats* 
     int rc = launch_camera_setup(1, viewmat, cfg->viewmat_end, cfg_rs_type(*cfg), K, cfg->radial_coeffs, cfg->tangential_coeffs,
                                  cfg->thin_prism_coeffs, cfg->image_width, cfg->image_height, cfg->camera_model, w.cam, st);
     if (rc != LFS_OK) return rc;
-    cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st);
     TileCounters counters = tile_list_counters(w.list_state, (int64_t)tw * th);
-    clear_tile_counters(counters, st);
+    if (cudaMemsetAsync(w.counters, 0, 16 * sizeof(int32_t), st) != cudaSuccess || clear_tile_counters(counters, st) != LFS_OK) {
+        set_error("lfs_render_forward: memset failed");
+        return LFS_ECUDA;
+    }
     const bool apart = count_tiles_apart(cfg->N, (int64_t)tw * th);
     if (apart) counters.counts = nullptr;
     const ProjParams pp = make_proj_params(cfg->eps2d, cfg->near_plane, cfg->far_plane, cfg->radius_clip, cfg->ut);
