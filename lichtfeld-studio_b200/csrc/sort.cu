@@ -229,10 +229,11 @@ constexpr int kBucketBelow = (32 - K) * 4;
 static_assert(kBucketBelow<8> == kBucketBelow<10> + 8, "");
 
 // Words of the list state in front of the per-bin arrays.
-// lists of at least 2^10 and 2^8 entries, and of any
-constexpr int kMetaLists = 0, kMetaParts = 8, kMetaWords = 16, kKinds = 3;
-// Lists longer than kRoomCta are sorted in parts of some kPart entries, by as many CTAs.
-constexpr int kRoomCta = 8192, kPart = 3072;
+// lists of at least 2^10 and 2^8 entries, and of any; of at least 2^kFarLog
+constexpr int kMetaLists = 0, kMetaFar = 3, kMetaParts = 8, kMetaWords = 16, kKinds = 3;
+// Lists longer than kRoomCta are sorted in parts of some kPart entries, by as many CTAs. Each part reads the whole list, so lists of 2^kFarLog and
+// more are cut into bins first, where there may be such lists (tile_far_kernel).
+constexpr int kRoomCta = 8192, kPart = 3072, kFarLog = 16;
 
 // One cluster: counts -> offsets [n_bins + 1] and cursors, the total and the overflow flag (with it all offsets are 0: the list is not
 // built), the launch order, and how many lists each kind of sorting group has. Every CTA takes a run of bins, 1024 at a time; the CTAs
@@ -242,7 +243,7 @@ constexpr int kRoomCta = 8192, kPart = 3072;
 constexpr int kScanCluster = 8;
 __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) tile_scan_kernel(
     int n_bins, TileCounters t, int64_t capacity, int64_t* carry, int32_t* __restrict__ n_out, int32_t* overflow, int32_t* __restrict__ offsets,
-    int32_t* __restrict__ order, int2* __restrict__ ranges, int4* __restrict__ parts, int32_t* __restrict__ meta) {
+    int32_t* __restrict__ order, int2* __restrict__ ranges, int4* __restrict__ parts, int32_t* __restrict__ meta, bool far_lists) {
     __shared__ int64_t warp_sums[32], block_sum;
     __shared__ int hist[132], cursor[132], sm[33];
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -310,7 +311,7 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) til
     if (rank == 0 && threadIdx.x < kMetaWords) {
         // the first CTA's share of a bucket starts where the bucket does
         const int k = threadIdx.x;
-        meta[k] = k == kKinds - 1 ? cursor[131] : k < kKinds - 1 ? cursor[kBucketBelow<10> + 8 * k] : 0;
+        meta[k] = k == kKinds - 1 ? cursor[131] : k < kKinds - 1 ? cursor[kBucketBelow<10> + 8 * k] : k == kMetaFar && far_lists ? cursor[kBucketBelow<kFarLog>] : 0;
     }
     cluster.sync();   // nobody reads another CTA's memory, or the carry, from here on; meta is set
     const bool dropped = overflow && total > capacity;
@@ -339,7 +340,7 @@ __global__ void __cluster_dims__(kScanCluster, 1, 1) __launch_bounds__(1024) til
             int64_t pos = at + ex;
             const int from = (int)min(pos, capacity), n = (int)min(pos + c, capacity) - from;
             ranges[slot] = make_int2(from, n);
-            if (n > kRoomCta && !dropped) {
+            if (n > kRoomCta && !dropped && !(far_lists && c >> kFarLog)) {
                 const int k = (n + kPart - 1) / kPart, base = atomicAdd(meta + kMetaParts, k);
                 for (int q = 0; q < k; ++q) parts[base + q] = make_int4(from, n, i, q);
             }
@@ -390,9 +391,8 @@ __device__ __forceinline__ void group_sync(int group) {
 // Where a bucket's word lies: one word is left out after every 32, so that threads that own runs of 2 to 16 buckets read different banks.
 __device__ __forceinline__ uint32_t bucket_slot(uint32_t b) { return b + (b >> 5); }
 
-template <int G, int K, bool RELOAD, class Load, class Out>
-__device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t* entry, uint32_t* __restrict__ start,
-                                             uint32_t (*red)[kSortThreads / 32][2], Load load, Out out) {
+template <int G, int K, bool RELOAD, class Red, class Load, class Out>
+__device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t* entry, uint32_t* __restrict__ start, Red red, Load load, Out out) {
     constexpr int kWarps = G / 32;
     const int lane = tid & 31, warp = tid >> 5;
     uint64_t key[RELOAD ? 1 : K];
@@ -446,7 +446,7 @@ __device__ __forceinline__ void sort_group_k(int tid, int group, int n, uint64_t
         group_sync<G>(group);
         const uint32_t v = red[1][lane & (kWarps - 1)][0];
         most = __reduce_max_sync(0xffffffffu, red[1][lane & (kWarps - 1)][1]);
-        at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u);   // warp < kWarps <= 16 lanes
+        at += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0u);   // warp < kWarps <= 32 lanes
     }
     at -= sum;
 #pragma unroll
@@ -506,24 +506,23 @@ __device__ __forceinline__ void sort_group(int tid, int group, int n, uint64_t* 
     else sort_group_k<G, 16, true>(tid, group, n, entry, start, red, load, out);
 }
 
-// The keys of a list between lo and hi (both included; `count` of them), sorted by the whole CTA: a histogram over 2048 bins of the keys from `next` on (64
-// bits, which are all different), then runs of bins that hold up to 4096 entries are gathered into shared memory and sorted. A bin that holds more by
-// itself is cut into 2048 again.
-template <class Visit>
-__device__ __forceinline__ void visit_list(int n, const uint64_t* __restrict__ list, Visit visit) {
-    int i = threadIdx.x;
-    for (; i + 7 * kSortThreads < n; i += 8 * kSortThreads) {   // eight loads in flight
+// visit(k) for the entries k of a list, by the whole CTA, eight loads in flight.
+template <class List, class Visit>
+__device__ __forceinline__ void visit_list(int n, List list, Visit visit) {
+    int i = (int)threadIdx.x;
+    for (; i + 7 * kSortThreads < n; i += 8 * kSortThreads) {
         uint64_t k[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) k[u] = list[i + u * kSortThreads];
+        for (int u = 0; u < 8; ++u) k[u] = list(i + u * kSortThreads);
 #pragma unroll
         for (int u = 0; u < 8; ++u) visit(k[u]);
     }
-    for (; i < n; i += kSortThreads) visit(list[i]);
+    for (; i < n; i += kSortThreads) visit(list(i));
 }
 constexpr int kLongBins = 1 << kLongLog;
 // counts of the keys in [next, top] by (key - next) >> shift, as an exclusive prefix in sm.cum [kLongBins + 1]
-__device__ __forceinline__ void long_histogram(int n, const uint64_t* __restrict__ list, SortShared& sm, uint64_t next, uint64_t top, int shift) {
+template <class List>
+__device__ __forceinline__ void long_histogram(int n, List list, SortShared& sm, uint64_t next, uint64_t top, int shift) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int kOwn = kLongBins / kSortThreads;
     __syncthreads();
@@ -550,8 +549,11 @@ __device__ __forceinline__ void long_histogram(int n, const uint64_t* __restrict
 }
 __device__ __forceinline__ int long_shift(uint64_t range) { return max(0, 64 - __clzll((long long)range) - kLongLog); }
 
-template <class Out>
-__device__ void sort_long(int n, const uint64_t* __restrict__ list, uint64_t lo, uint64_t hi, int count, SortShared& sm, Out out) {
+// The keys of a list between lo and hi (both included; `count` of them), sorted by the whole CTA: a histogram over 2048 bins of the keys from `next` on (64
+// bits, which are all different), then runs of bins that hold up to 4096 entries are gathered into shared memory and sorted. A bin that holds more by
+// itself is cut into 2048 again.
+template <class List, class Out>
+__device__ void sort_long(int n, List list, uint64_t lo, uint64_t hi, int count, SortShared& sm, Out out) {
     constexpr int kRoom = 8 * kSortThreads;
     const int tid = threadIdx.x;
     uint64_t next = lo;   // every smaller key is out
@@ -608,12 +610,12 @@ __device__ void sort_long(int n, const uint64_t* __restrict__ list, uint64_t lo,
     __syncthreads();
 }
 
-// Part q of a list of n entries, by the whole CTA. Every part counts the list's keys into the same bins and takes those that start in its own share of the
-// ranks, so the parts need nothing from one another.
-template <class Out>
-__device__ void sort_part(int q, int n, const uint64_t* __restrict__ list, SortShared& sm, Out out) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, parts = (n + kPart - 1) / kPart;
-    uint64_t lo = ~0ull, hi = 0;
+// smallest and largest key of a list, to all threads of the CTA
+template <class List>
+__device__ __forceinline__ void list_bounds(int n, List list, SortShared& sm, uint64_t& lo, uint64_t& hi) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    lo = ~0ull;
+    hi = 0;
     visit_list(n, list, [&](uint64_t k) { lo = min(lo, k); hi = max(hi, k); });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -623,6 +625,15 @@ __device__ void sort_part(int q, int n, const uint64_t* __restrict__ list, SortS
     if (lane == 0) { sm.red64[0][warp] = lo; sm.red64[1][warp] = hi; }
     __syncthreads();
     for (int w = 0; w < kSortThreads / 32; ++w) { lo = min(lo, sm.red64[0][w]); hi = max(hi, sm.red64[1][w]); }
+}
+
+// Part q of a list of n entries, by the whole CTA. Every part counts the list's keys into the same bins and takes those that start in its own share of the
+// ranks, so the parts need nothing from one another.
+template <class List, class Out>
+__device__ void sort_part(int q, int n, List list, SortShared& sm, Out out) {
+    const int parts = (n + kPart - 1) / kPart;
+    uint64_t lo, hi;
+    list_bounds(n, list, sm, lo, hi);
     const int shift = long_shift(hi - lo);
     long_histogram(n, list, sm, lo, hi, shift);
     // first bin that starts at or after the share's first rank
@@ -638,6 +649,159 @@ __device__ void sort_part(int q, int n, const uint64_t* __restrict__ list, SortS
     if (count == 0) return;
     const uint64_t key_lo = lo + ((uint64_t)from << shift), key_hi = to == kLongBins ? hi : lo + ((uint64_t)to << shift) - 1;
     sort_long(n, list, key_lo, key_hi, (int)count, sm, [&](int i, uint64_t k) { out((int)first + i, k); });
+}
+
+// ---- far lists ------------------------------------------------------------------------------------------
+// A list of 65,536 entries and more: 8,192 keys drawn from it and sorted give the limits of 4,096 bins. A cluster counts the list into them, an eighth by
+// every CTA, and with the counts of all eight drops the Gaussians into their bins in flatten_ids. Where there are fewer lists than clusters, several share a list:
+// each reads all of it, counts what lies below its own share of the bins and places what lies in it. A cluster with a list to itself leaves the bins of the
+// keys in the list, so that it searches once. The parts that follow are runs of bins: a sort CTA
+// reads its own part only, with the depths fetched by index. Drawn limits, since a key range cut evenly puts most of a distant object between two of them as
+// soon as one Gaussian floats near the camera. A bin holds n / 4096 entries, some five times that at the worst.
+// Bound by the shared-memory pipe: the search for a key's bin (12 conflicting loads) and the atomics. Sorting, this kernel included, in us, with lists of every
+// length read four times by each of their parts and now: 1 M Gaussians, two lists of 632 k 1102 and 338; 1 M at 64x64, four lists of 419 k 4669 and 632; 4 M,
+// two of 2.5 M 14654 and 1198; 4 M at 64x64 63446 and 2257. Two lists of 190 k (300 k Gaussians) 183 and 179, which is where the line lies.
+constexpr int kFarThreads = 1024, kFarCluster = 8, kFarClusters = 16, kFarBins = 4096;
+struct FarShared {
+    uint64_t entry[2 * kFarBins];
+    uint32_t start[2 * kFarBins / 32 * 33 + 64];
+    uint32_t red[2][kFarThreads / 32][2];
+    uint64_t limit[kFarBins];        // the first key of bin b + 1
+    uint32_t count[kFarBins];        // read by the other CTAs of the cluster
+    uint32_t cursor[kFarBins];
+    uint32_t first[kFarBins + 1];    // of every bin, from the start of the list
+    int scan[33];
+    int below;                       // keys before the share, in this CTA's eighth of the list
+    int part0;
+};
+__global__ void __cluster_dims__(kFarCluster, 1, 1) __launch_bounds__(kFarThreads) tile_far_kernel(
+    const int32_t* __restrict__ order, const int2* __restrict__ ranges, int4* __restrict__ parts, int32_t* meta,
+    uint64_t* entries, const int32_t* __restrict__ overflow, int32_t* __restrict__ flatten_ids) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FarShared& sm = *reinterpret_cast<FarShared*>(smem_raw);
+    if (overflow && *overflow) return;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, rank = (int)cluster.block_rank();
+    constexpr int kOwn = kFarBins / kFarThreads, kDrawn = 2 * kFarBins, kAhead = 8;
+    const int n_far = meta[kMetaFar], clusters = gridDim.x / kFarCluster, shares = max(1, clusters / max(n_far, 1));
+    for (int job = blockIdx.x / kFarCluster; job < n_far * shares; job += clusters) {
+        const int idx = job / shares, from = ranges[idx].x, n = ranges[idx].y;
+        if (n <= kRoomCta) continue;   // cut off by the capacity: sorted like any short list
+        uint64_t* list = entries + from;
+        // every CTA draws the same keys: one from each of as many stretches of the list
+        sort_group_k<kFarThreads, kDrawn / kFarThreads, false>(tid, 0, kDrawn, sm.entry, sm.start, sm.red, [&](int i) {
+            const int64_t a = (int64_t)n * i / kDrawn, b = (int64_t)n * (i + 1) / kDrawn;
+            return list[a + (int64_t)(((uint64_t)((uint32_t)i * 2654435769u) * (uint64_t)(b - a)) >> 32)];
+        }, [&](int i, uint64_t k) { if (i & 1) sm.limit[i >> 1] = k; });
+        for (int b = tid; b < kFarBins; b += kFarThreads) sm.count[b] = 0;
+        if (tid == 0) sm.below = 0;
+        cluster.sync();   // nobody overwrites a key that another CTA still draws
+        const int bin0 = kFarBins * (job % shares) / shares, bin1 = kFarBins * (job % shares + 1) / shares;
+        const uint64_t key0 = bin0 ? sm.limit[bin0 - 1] : 0, key1 = bin1 < kFarBins ? sm.limit[bin1 - 1] : ~0ull;   // no key has all bits set
+        const int lo = (int)((int64_t)n * rank / kFarCluster), hi = (int)((int64_t)n * (rank + 1) / kFarCluster);
+        auto bins = [&](int i0, uint64_t (&k)[kAhead], int (&b)[kAhead]) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) { k[u] = i0 + u * kFarThreads < hi ? list[i0 + u * kFarThreads] : ~0ull; b[u] = 0; }
+#pragma unroll
+            for (int step = kFarBins / 2; step > 0; step >>= 1)
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u)
+                    if (k[u] >= key0 && k[u] < key1 && sm.limit[b[u] + step - 1] <= k[u]) b[u] += step;
+        };
+        int below = 0;
+        for (int i0 = lo + tid; i0 < hi; i0 += kAhead * kFarThreads) {
+            uint64_t k[kAhead];
+            int b[kAhead];
+            bins(i0, k, b);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                below += k[u] < key0 ? 1 : 0;
+                if (k[u] >= key0 && k[u] < key1) {
+                    atomicAdd(&sm.count[b[u]], 1u);
+                    if (shares == 1) list[i0 + u * kFarThreads] = (uint64_t)b[u] << 32 | (uint32_t)k[u];   // for this thread, below
+                }
+            }
+        }
+        below = __reduce_add_sync(0xffffffffu, below);
+        if ((tid & 31) == 0) atomicAdd(&sm.below, below);
+        cluster.sync();
+        uint32_t all[kOwn], earlier[kOwn], sum = 0;
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j) {
+            all[j] = earlier[j] = 0;
+#pragma unroll
+            for (int r = 0; r < kFarCluster; ++r) {
+                const uint32_t c = cluster.map_shared_rank(sm.count, r)[tid * kOwn + j];
+                all[j] += c;
+                if (r < rank) earlier[j] += c;
+            }
+            sum += all[j];
+        }
+        int base = 0;
+#pragma unroll
+        for (int r = 0; r < kFarCluster; ++r) base += *cluster.map_shared_rank(&sm.below, r);
+        int total;
+        uint32_t at = (uint32_t)(base + block_excl_scan((int)sum, total, sm.scan));
+#pragma unroll
+        for (int j = 0; j < kOwn; ++j) {
+            sm.first[tid * kOwn + j] = at;
+            sm.cursor[tid * kOwn + j] = at + earlier[j];
+            at += all[j];
+        }
+        const int n_parts = (total + kPart - 1) / kPart;
+        if (tid == 0) {
+            sm.first[kFarBins] = (uint32_t)(base + total);
+            if (rank == 0) sm.part0 = atomicAdd(meta + kMetaParts, n_parts);
+        }
+        cluster.sync();   // the counts of the other CTAs have been read
+        for (int i0 = lo + tid; i0 < hi; i0 += kAhead * kFarThreads) {
+            uint64_t k[kAhead];
+            int b[kAhead];
+            if (shares == 1) {
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) { k[u] = i0 + u * kFarThreads < hi ? list[i0 + u * kFarThreads] : ~0ull; b[u] = (int)(k[u] >> 32); }
+            } else {
+                bins(i0, k, b);
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (k[u] >= key0 && k[u] < key1) flatten_ids[from + (int)atomicAdd(&sm.cursor[b[u]], 1u)] = (int32_t)(uint32_t)k[u];
+        }
+        if (rank == 0) {
+            // first bin that starts at or after a rank of the share
+            auto bound = [&](int64_t r) {
+                int b = 0;
+                for (int step = kFarBins; step > 0; step >>= 1)
+                    if (b + step <= kFarBins && (int64_t)sm.first[b + step - 1] - base < r) b += step;
+                return b;
+            };
+            for (int q = tid; q < n_parts; q += kFarThreads) {
+                const int b0 = bound((int64_t)total * q / n_parts), b1 = q + 1 == n_parts ? kFarBins : bound((int64_t)total * (q + 1) / n_parts);
+                parts[sm.part0 + q] = make_int4(from + (int)sm.first[b0], (int)(sm.first[b1] - sm.first[b0]), order[idx], -1);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// n Gaussians of a far list, by the whole CTA, sorted where they lie. `room`: n entries that nobody needs any more.
+template <class Out>
+__device__ __forceinline__ void sort_far_part(int n, const int32_t* ids, const uint32_t* __restrict__ keys, uint64_t* room, SortShared& sm, Out out) {
+    auto load = [&](int i) {
+        const uint32_t id = (uint32_t)ids[i];
+        return (uint64_t)keys[id] << 32 | id;
+    };
+    if (n <= kRoomCta) {
+        if (n > 0) sort_group<kSortThreads, true>(threadIdx.x, 0, n, sm.entry, sm.start, sm.red, load, out);
+        return;
+    }
+    // bins of a list of ten million and more
+    for (int i = threadIdx.x; i < n; i += kSortThreads) __stcg(reinterpret_cast<unsigned long long*>(room + i), (unsigned long long)load(i));
+    __syncthreads();
+    auto list = [&](int i) { return (uint64_t)__ldcg(reinterpret_cast<const unsigned long long*>(room + i)); };
+    uint64_t lo, hi;
+    list_bounds(n, list, sm, lo, hi);
+    sort_long(n, list, lo, hi, n, sm, out);
 }
 
 // Groups of G threads share lists first .. last - 1 of the launch order: a round gives one list to every group, the longest to the first group of every
@@ -657,11 +821,11 @@ __device__ __forceinline__ void share_lists(int tid, int group, int first, int l
     }
 }
 
-// OP: operator level, with the 64-bit keys.
+// OP: operator level, with the 64-bit keys. keys: depth bits by flattened Gaussian index.
 template <bool OP>
 __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_t* __restrict__ order, const int2* __restrict__ ranges, const int4* __restrict__ parts,
-                                                                    const int32_t* __restrict__ meta,
-                                                                    const uint64_t* __restrict__ entries, const int32_t* __restrict__ overflow,
+                                                                    const int32_t* __restrict__ meta, const uint32_t* __restrict__ keys,
+                                                                    uint64_t* entries, const int32_t* __restrict__ overflow,
                                                                     int64_t first_bin, uint32_t n_tiles, uint32_t tile_n_bits,
                                                                     int32_t* __restrict__ flatten_ids, int64_t* __restrict__ isect_ids) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -679,7 +843,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
     const int n_cta = meta[kMetaLists], n_group = meta[kMetaLists + 1], n_warp = meta[kMetaLists + 2];
     for (int u = blockIdx.x, n_parts = meta[kMetaParts]; u < n_parts; u += gridDim.x) {
         const int4 part = parts[u];
-        sort_part(part.w, part.y, entries + part.x, sm, writer(part.z, part.x));
+        if (part.w < 0) sort_far_part(part.y, flatten_ids + part.x, keys, entries + part.x, sm, writer(part.z, part.x));
+        else sort_part(part.w, part.y, [&](int i) { return entries[part.x + i]; }, sm, writer(part.z, part.x));
         __syncthreads();
     }
     share_lists<kSortThreads>(tid, 0, 0, n_cta, ranges, [&](int idx, int from, int n) {
@@ -780,7 +945,7 @@ struct ListState {
     int32_t *meta, *order, *offsets;
     int64_t* carry;
     int2* ranges;
-    int4* parts;   // [capacity / kPart + capacity / kRoomCta + 1]
+    int4* parts;   // [capacity / kPart + capacity / kRoomCta + 1 + kFarClusters]
     TileCounters t;
 };
 ListState list_state(int32_t* base, int64_t bins) {
@@ -797,9 +962,10 @@ ListState list_state(int32_t* base, int64_t bins) {
     s.parts = reinterpret_cast<int4*>(s.offsets + pad8(bins + 1));
     return s;
 }
-// a list of n > kRoomCta entries has at most n / kPart + 1 parts, and there are at most capacity / kRoomCta such lists
+// a list of n > kRoomCta entries has at most n / kPart + 1 parts, one more for every further cluster that shares it, and there are at most capacity / kRoomCta such
+// lists
 size_t list_words(int64_t bins, int64_t counters, int64_t capacity) {
-    return (size_t)(kMetaWords + 16 + 2 * counters + 3 * pad8(bins) + pad8(bins + 1) + 4 * (capacity / kPart + capacity / kRoomCta + 1));
+    return (size_t)(kMetaWords + 16 + 2 * counters + 3 * pad8(bins) + pad8(bins + 1) + 4 * (capacity / kPart + capacity / kRoomCta + 1 + kFarClusters));
 }
 }  // namespace
 
@@ -810,19 +976,28 @@ int clear_tile_counters(const TileCounters& t, cudaStream_t st) {
     return cudaMemsetAsync(t.counts, 0, (size_t)t.replicas * t.stride * sizeof(int32_t), st) == cudaSuccess ? LFS_OK : LFS_ECUDA;
 }
 
-static int launch_tile_scan(int bins, const ListState& s, int64_t capacity, int64_t* carry, int32_t* n_out, int32_t* overflow, int32_t* offsets, cudaStream_t st) {
+static int launch_tile_scan(int bins, const ListState& s, int64_t capacity, int64_t* carry, int32_t* n_out, int32_t* overflow, int32_t* offsets, bool far_lists,
+                            cudaStream_t st) {
     LFS_TIMED("tile_scan", st);
-    tile_scan_kernel<<<kScanCluster, 1024, 0, st>>>(bins, s.t, capacity, carry, n_out, overflow, offsets, s.order, s.ranges, s.parts, s.meta);
+    tile_scan_kernel<<<kScanCluster, 1024, 0, st>>>(bins, s.t, capacity, carry, n_out, overflow, offsets, s.order, s.ranges, s.parts, s.meta, far_lists);
     return check_launch("tile_scan");
 }
 
+// A list holds a Gaussian once, so only many Gaussians make a list long enough for tile_far_kernel to pay; where there is none it costs a launch of 2 us.
+static bool far_lists_possible(int64_t N) { return N > 262144; }
+
 template <bool OP>
-static int launch_tile_sort(int bins, const ListState& s, const uint64_t* entries, const int32_t* overflow, int64_t first_bin, uint32_t n_tiles,
-                            uint32_t tile_n_bits, int32_t* flatten_ids, int64_t* isect_ids, cudaStream_t st) {
+static int launch_tile_sort(int bins, const ListState& s, const uint32_t* keys, uint64_t* entries, const int32_t* overflow, int64_t first_bin, uint32_t n_tiles,
+                            uint32_t tile_n_bits, int32_t* flatten_ids, int64_t* isect_ids, bool far_lists, cudaStream_t st) {
+    if (far_lists) {
+        LFS_TIMED("tile_far", st);
+        cudaFuncSetAttribute(tile_far_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FarShared));
+        tile_far_kernel<<<kFarClusters * kFarCluster, kFarThreads, sizeof(FarShared), st>>>(s.order, s.ranges, s.parts, s.meta, entries, overflow, flatten_ids);
+    }
     LFS_TIMED("tile_sort", st);
     cudaFuncSetAttribute(tile_sort_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortShared));
-    tile_sort_kernel<OP><<<min(bins, 2 * num_sms()), kSortThreads, sizeof(SortShared), st>>>(s.order, s.ranges, s.parts, s.meta, entries, overflow, first_bin, n_tiles,
-                                                                                             tile_n_bits, flatten_ids, isect_ids);
+    tile_sort_kernel<OP><<<min(bins, 2 * num_sms()), kSortThreads, sizeof(SortShared), st>>>(s.order, s.ranges, s.parts, s.meta, keys, entries, overflow, first_bin,
+                                                                                             n_tiles, tile_n_bits, flatten_ids, isect_ids);
     return check_launch("tile_sort");
 }
 
@@ -845,7 +1020,8 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
         tile_histogram_kernel<<<grid_for((int64_t)a.N * parts, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d,
                                                                                             a.radii, 0, bins, s.t, parts);
     }
-    int rc = launch_tile_scan(bins, s, a.capacity, nullptr, a.n_isects_dev, a.overflow, a.tile_offsets, st);
+    const bool far_lists = far_lists_possible(a.N);
+    int rc = launch_tile_scan(bins, s, a.capacity, nullptr, a.n_isects_dev, a.overflow, a.tile_offsets, far_lists, st);
     if (rc != LFS_OK) return rc;
     if (a.N > 0 && a.capacity > 0 && bins > 0) {
         {
@@ -857,7 +1033,8 @@ int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
                 tile_scatter_kernel<<<grid_for((int64_t)a.N * parts, kThreads), kThreads, 0, st>>>(a.N, a.N, a.tw, a.th, (float)a.tile_size, a.tiles, a.means2d, a.radii,
                                                                                   a.depths, 0, bins, a.capacity, a.overflow, s.t, a.entries, parts);
         }
-        rc = launch_tile_sort<false>(bins, s, a.entries, a.overflow, 0, 1, 0, a.flatten_ids, nullptr, st);
+        const uint32_t* keys = a.ewa_bounds ? a.ewa_depth_bits : reinterpret_cast<const uint32_t*>(a.depths);
+        rc = launch_tile_sort<false>(bins, s, keys, a.entries, a.overflow, 0, 1, 0, a.flatten_ids, nullptr, far_lists, st);
         if (rc != LFS_OK) return rc;
     }
     return check_launch("build_tile_lists");
@@ -905,6 +1082,7 @@ int build_isect_lists(int C, int N, int tw, int th, int tile_size, int sort, con
                                                         isect_ids, flatten_ids);
         return check_launch("emit_unsorted");
     }
+    const bool far_lists = far_lists_possible(N);
     cudaMemsetAsync(list_state(b.state, 1).carry, 0, sizeof(int64_t), st);
     for (int64_t first = 0; first < n_ids; first += kOperatorBins) {
         const int bins = (int)min(kOperatorBins, n_ids - first);
@@ -914,14 +1092,15 @@ int build_isect_lists(int C, int N, int tw, int th, int tile_size, int sort, con
             LFS_TIMED("tile_histogram", st);
             tile_histogram_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, first, bins, s.t, parts);
         }
-        int rc = launch_tile_scan(bins, s, n_isects, s.carry, nullptr, nullptr, s.offsets, st);
+        int rc = launch_tile_scan(bins, s, n_isects, s.carry, nullptr, nullptr, s.offsets, far_lists, st);
         if (rc != LFS_OK) return rc;
         {
             LFS_TIMED("tile_scatter", st);
             tile_scatter_kernel<<<grid, kThreads, 0, st>>>(total, N, tw, th, (float)tile_size, tiles, means2d, radii, depths, first, bins, n_isects, nullptr,
                                                            s.t, b.entries, parts);
         }
-        rc = launch_tile_sort<true>(bins, s, b.entries, nullptr, first, n_tiles, tile_n_bits, flatten_ids, isect_ids, st);
+        rc = launch_tile_sort<true>(bins, s, reinterpret_cast<const uint32_t*>(depths), b.entries, nullptr, first, n_tiles, tile_n_bits, flatten_ids, isect_ids,
+                                    far_lists, st);
         if (rc != LFS_OK) return rc;
     }
     return check_launch("build_isect_lists");

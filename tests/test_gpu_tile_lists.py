@@ -64,3 +64,37 @@ def test_many_lists(pkg, C, N, tw, th, ts, radius):
     rng = np.random.default_rng(N)
     m = rng.random((C, N, 2)) * [tw * ts, th * ts]
     _check(pkg, m, rng.integers(0, radius, (C, N, 2)), np.exp(rng.standard_normal((C, N))), tw, th, ts)
+
+
+# Lists of 65,536 entries and more among more than 262,144 Gaussians are cut into bins by drawn limits first. Twelve million: bins beyond the sorting room.
+@pytest.mark.parametrize("n,depths,tiles", [(262_144, "spread", 1), (262_145, "spread", 1), (262_145, "equal", 1), (262_145, "few", 1), (262_145, "far", 1),
+                                            (262_145, "negative", 1), (300_007, "far", 3), (500_000, "spread", 7), (1_200_000, "far", 9), (1_000_003, "far", 1), (12_000_000, "spread", 1)])
+def test_far_lists(pkg, n, depths, tiles):
+    rng = np.random.default_rng(n)
+    d = torch.from_numpy(DEPTHS[depths](rng, n).astype(F)).cuda()
+    tile = torch.arange(n, device="cuda") % (n if tiles == 1 else 9) % tiles      # of seven tiles two hold twice as much as the others
+    m = torch.stack([16.0 * tile + 8.0, torch.full((n,), 8.0, device="cuda")], -1)[None].float().contiguous()
+    r = torch.ones((1, n, 2), dtype=torch.int32, device="cuda")
+    _, k, i = pkg.ops.intersect_tile(m, r, d[None].contiguous(), None, None, 1, 16, tiles, 1, True)
+    key = (tile << 32) | (d.view(torch.int32).long() & 0xFFFFFFFF)
+    order = torch.sort(key, stable=True).indices
+    assert torch.equal(k, key[order]) and torch.equal(i.long(), order)
+
+
+# A Gaussian behind the camera makes far lists possible; it must not make a difference. Some 330,000 entries in a tile among the 262,144 or 262,145.
+@pytest.mark.parametrize("ewa", [False, True])
+def test_far_lists_of_a_render(pkg, synth, ewa):
+    n, W, H = 262_144, 96, 64
+    P = synth.make_gaussians(n + 1, 5, "cube", 0)
+    P["means"][n] = [0.0, -400.0, 0.0]
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a, F)).cuda()
+    tr = pkg.trainer
+    cam = tr.Camera(T(synth.look_at_origin([0.3, -40.0, 0.4])), T(synth.intrinsics(200.0, 200.0, 40.0, 24.0)), W, H)
+    images = []
+    for count in (n, n + 1):
+        model = tr.SplatData(count, 1, "cuda:0").load({k: v[:count] for k, v in P.items()})
+        rast = (tr.FastRasterizer if ewa else tr.Rasterizer)(model, W, H, 0)
+        images.append(rast.forward(cam, None).image.clone())
+        if not ewa:
+            assert (torch.diff(rast.state()["tile_offsets"]) >= 65_536).any()
+    assert images[0].abs().max() > 0.1 and torch.equal(*images)
