@@ -131,12 +131,13 @@ struct AxisAngle { double n, z, theta; };
 __device__ __forceinline__ double angle_near(const AxisAngle& a, float n, float z) {
     const double nd = n, zd = z;
     const double cross = fma(nd, a.z, -(zd * a.n)), dot = fma(zd, a.z, nd * a.n);
-    double y = (double)(1.0f / (float)dot);
+    const float start = 1.0f / (float)dot;
+    double y = (double)start;
     y = fma(y, fma(-dot, y, 1.0), y);
     double t = cross * y;
     t = fma(fma(-t, dot, cross), y, t);
-    // far apart, or a product whose float reciprocal is infinite (t is NaN) or flushed towards 0 (t would be 0)
-    if (!(fabs(t) < 0.03125 && dot < 8e37)) return atan2(nd, zd);
+    // far apart, or a product whose float reciprocal is infinite (t is NaN) or below the normal numbers (t would be 0 or lose bits)
+    if (!(fabs(t) < 0.03125 && start >= FLT_MIN)) return atan2(nd, zd);
     const double s = t * t;
     double p = fma(s, -1.0 / 11.0, 1.0 / 9.0);
     p = fma(s, p, -1.0 / 7.0);

@@ -453,7 +453,7 @@ __device__ __forceinline__ bool fisheye_box(const CamDev& cam, const float* mc, 
 
 // Only the lists are pinned to unfused arithmetic (file header); everything here spells its products and sums as fma.
 template <int MODEL, bool RS>
-__device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
+__device__ __forceinline__ void make_forms(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz,
                                             f3 scale, float r, float g, float b, float opacity, float extra, float4* rec,
                                             float4* __restrict__ cut, int64_t n, const float4& tiles, uint4& box) {
     float R[9], inv_norm, qn[4];
@@ -518,16 +518,6 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         // alpha below which kept_at_cut decides; infinity marks an infinite or NaN colour
         const bool finite = fabsf(r) + fabsf(g) + fabsf(b) + fabsf(extra) < INFINITY;
         rec[2] = make_float4(p3[0], p3[1], p3[2], finite ? (1.0f / 255.0f) * __expf(fminf(band, 8.0f)) : INFINITY);
-        // A scale without a reciprocal makes the forms infinite or NaN, or the limit NaN, and NaN is the response along every ray; min(0.999, NaN) blends it with 0.999
-        // into every pixel of its tiles. Forms that every pixel accepts, no box and an exponent of NaN say so without a test per pair.
-        const float forms = fabsf(p1[0]) + fabsf(p1[1]) + fabsf(p1[2]) + fabsf(p2[0]) + fabsf(p2[1]) + fabsf(p2[2]) + fabsf(p3[0]) + fabsf(p3[1]) + fabsf(p3[2]);
-        if (!(forms < INFINITY) || isnan(phi_cut)) {
-            rec[0] = make_float4(0.f, 0.f, 0.f, NAN);
-            rec[1] = make_float4(0.f, 0.f, 0.f, 1.0f);
-            rec[2] = make_float4(0.f, 0.f, 1.0f, rec[2].w);
-            box.z = __float_as_uint(INFINITY);
-            return;
-        }
     }
     if (MODEL == LFS_EQUIRECTANGULAR) return;
     const float rho2 = 2.0f * (fmaxf(-0.02f - thr, 0.f) + 0.03f);
@@ -563,6 +553,25 @@ __device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw
         }
         box.x = packed[0];
         box.y = packed[1];
+    }
+}
+
+// The record of a Gaussian. A scale without a reciprocal makes the forms infinite or NaN, or the limit NaN, and NaN is the response along every ray;
+// min(0.999, NaN) blends it with 0.999 into every pixel of its tiles. Forms that every pixel accepts, no box and an exponent of NaN say so without a test per pair.
+// Tested on the finished record: tested where the forms are made it cost the fisheye kernel registers (6 M Gaussians 1262 -> 1325 us, here 1266).
+template <int MODEL, bool RS>
+__device__ __forceinline__ void make_record(const CamDev& cam, f3 mean, float qw, float qx, float qy, float qz, f3 scale, float r, float g, float b,
+                                            float opacity, float extra, float4* rec, float4* __restrict__ cut, int64_t n, const float4& tiles, uint4& box) {
+    make_forms<MODEL, RS>(cam, mean, qw, qx, qy, qz, scale, r, g, b, opacity, extra, rec, cut, n, tiles, box);
+    if (RS) return;
+    const float forms = fabsf(rec[0].x) + fabsf(rec[0].y) + fabsf(rec[0].z) + fabsf(rec[1].x) + fabsf(rec[1].y) + fabsf(rec[1].z) + fabsf(rec[2].x) +
+                        fabsf(rec[2].y) + fabsf(rec[2].z);
+    if (!(forms < INFINITY) || isnan(rec[1].w)) {
+        rec[0] = make_float4(0.f, 0.f, 0.f, NAN);
+        rec[1] = make_float4(0.f, 0.f, 0.f, 1.0f);
+        rec[2] = make_float4(0.f, 0.f, 1.0f, rec[2].w);
+        box.x = box.y = 0xFFFF0000u;
+        box.z = __float_as_uint(INFINITY);
     }
 }
 
