@@ -628,9 +628,11 @@ __device__ __forceinline__ void list_bounds(int n, List list, SortShared& sm, ui
 }
 
 // Part q of a list of n entries, by the whole CTA. Every part counts the list's keys into the same bins and takes those that start in its own share of the
-// ranks, so the parts need nothing from one another.
+// ranks, so the parts need nothing from one another. A call, as sort_far_part: long lists are rare, and inlined they cost the others registers.
 template <class List, class Out>
-__device__ void sort_part(int q, int n, List list, SortShared& sm, Out out) {
+__device__ __noinline__ void sort_part(int q, int n, List list, Out out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SortShared& sm = *reinterpret_cast<SortShared*>(smem_raw);
     const int parts = (n + kPart - 1) / kPart;
     uint64_t lo, hi;
     list_bounds(n, list, sm, lo, hi);
@@ -786,7 +788,9 @@ __global__ void __cluster_dims__(kFarCluster, 1, 1) __launch_bounds__(kFarThread
 
 // n Gaussians of a far list, by the whole CTA, sorted where they lie. `room`: n entries that nobody needs any more.
 template <class Out>
-__device__ __forceinline__ void sort_far_part(int n, const int32_t* ids, const uint32_t* __restrict__ keys, uint64_t* room, SortShared& sm, Out out) {
+__device__ __noinline__ void sort_far_part(int n, const int32_t* ids, const uint32_t* __restrict__ keys, uint64_t* room, Out out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SortShared& sm = *reinterpret_cast<SortShared*>(smem_raw);
     auto load = [&](int i) {
         const uint32_t id = (uint32_t)ids[i];
         return (uint64_t)keys[id] << 32 | id;
@@ -843,8 +847,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) tile_sort_kernel(const int32_
     const int n_cta = meta[kMetaLists], n_group = meta[kMetaLists + 1], n_warp = meta[kMetaLists + 2];
     for (int u = blockIdx.x, n_parts = meta[kMetaParts]; u < n_parts; u += gridDim.x) {
         const int4 part = parts[u];
-        if (part.w < 0) sort_far_part(part.y, flatten_ids + part.x, keys, entries + part.x, sm, writer(part.z, part.x));
-        else sort_part(part.w, part.y, [&](int i) { return entries[part.x + i]; }, sm, writer(part.z, part.x));
+        if (part.w < 0) sort_far_part(part.y, flatten_ids + part.x, keys, entries + part.x, writer(part.z, part.x));
+        else sort_part(part.w, part.y, [list = entries + part.x](int i) { return list[i]; }, writer(part.z, part.x));
         __syncthreads();
     }
     share_lists<kSortThreads>(tid, 0, 0, n_cta, ranges, [&](int idx, int from, int n) {
