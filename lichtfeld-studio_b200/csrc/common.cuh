@@ -48,6 +48,23 @@ inline int grid_for(int64_t n, int block, int max_blocks_per_sm = 8) {
     return (int)g;
 }
 
+template <class... P, class... A>
+void launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) { kernel<<<grid, block, smem, st>>>(args...); }
+// A launch that starts as soon as every CTA of the launch before it has called let_next_start() or has ended. That launch has to have started behind everything
+// the new one reads, and one thread of the new one calls wait_for_previous(), so that what comes after it comes after both.
+template <class... P, class... A>
+void launch_beside(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute beside;
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = &beside; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // Per-camera constants derived once per call by camera_setup_kernel from the row-major
 // world-to-camera matrix and the intrinsics (global shutter).

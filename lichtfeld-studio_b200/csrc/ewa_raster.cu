@@ -90,13 +90,15 @@ template <int PX>
 __global__ void __launch_bounds__(128, PX == 2 ? 8 : 10) ewa_blend_fwd_kernel(
     const float4* __restrict__ records, const uint32_t* __restrict__ ids, const int32_t* __restrict__ tile_offsets,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const int32_t* __restrict__ tile_order,
-    int W, int H, int tw, float* __restrict__ image, float* __restrict__ alpha_map, int32_t* __restrict__ n_contrib) {
+    int W, int H, int tw, int n_tiles, Outsized out, float* __restrict__ image, float* __restrict__ alpha_map, int32_t* __restrict__ n_contrib) {
     using P = Pixels<PX>;
     using V = typename P::V;
     __shared__ EwaStage stages[4][2];
     EwaStage* stage = stages[threadIdx.x >> 5];
+    side_by_side<PX>(out);
     const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
     const int tile = tile_order ? tile_order[slot] : slot;
+    if ((PX == 1 ? out.share > 0 : slot < out.slots) && is_outsized(tile_offsets[tile + 1] - tile_offsets[tile], tile_offsets[n_tiles], out) != (PX == 1)) return;
     const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
     const int patch_j = (tile % tw) * 16 + (warp & 1) * 8, patch_i = (tile / tw) * 16 + (warp >> 1) * 4 * PX;
     const int i = patch_i + (PX == 2 ? lane >> 2 : lane >> 3), j0 = patch_j + (PX == 2 ? 2 * (lane & 3) : lane & 7);
@@ -241,16 +243,18 @@ template <int PX>
 __global__ void __launch_bounds__(128, PX == 2 ? 6 : 8) ewa_blend_bwd_kernel(
     const float4* __restrict__ records, const uint32_t* __restrict__ ids, const int32_t* __restrict__ tile_offsets,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const int32_t* __restrict__ tile_order,
-    int W, int H, int tw, const float* __restrict__ alpha_map, const int32_t* __restrict__ n_contrib,
+    int W, int H, int tw, int n_tiles, Outsized out, const float* __restrict__ alpha_map, const int32_t* __restrict__ n_contrib,
     const float* __restrict__ grad_image,
     const float* __restrict__ grad_alpha, float* __restrict__ accum) {
     using P = Pixels<PX>;
     using V = typename P::V;
     __shared__ EwaBwdWarp warps[4];
     EwaBwdWarp& sm = warps[threadIdx.x >> 5];
+    side_by_side<PX>(out);
     if (overflow && *overflow) return;
     const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
     const int tile = tile_order ? tile_order[slot] : slot;
+    if ((PX == 1 ? out.share > 0 : slot < out.slots) && is_outsized(tile_offsets[tile + 1] - tile_offsets[tile], tile_offsets[n_tiles], out) != (PX == 1)) return;
     const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
     // warps tile the 16x16 block as patches of 8 x 4 PX pixels: one or two of the forward's 8x4 patches, one above the other
     const int patch_j = (tile % tw) * 16 + (warp & 1) * 8, patch_i = (tile / tw) * 16 + (warp >> 1) * 4 * PX;
@@ -656,12 +660,14 @@ int launch_ewa_blend_fwd(const EwaBlendArgs& a, float* image, float* alpha, int3
     const int n_tiles = a.tw * a.th;
     if (n_tiles == 0) return LFS_OK;
     LFS_TIMED("ewa_blend_fwd", st);
-#define LFS_EWA_FWD(PX)                                                                                                             \
-    ewa_blend_fwd_kernel<PX><<<n_tiles * (2 / PX), 128, 0, st>>>(a.records, a.instance_ids, a.tile_offsets, a.overflow, a.background,  \
-                                                                 a.tile_order, a.W, a.H, a.tw, image, alpha, n_contrib)
+    const Outsized out = outsized_lists(a.tile_order, n_tiles);   // the forward always leaves a launch order
+#define LFS_EWA_FWD(LAUNCH, PX, TILES, OUT)                                                                                         \
+    LAUNCH(ewa_blend_fwd_kernel<PX>, (TILES) * (2 / PX), 128, 0, st, a.records, a.instance_ids, a.tile_offsets, a.overflow, a.background,  \
+                                                                 a.tile_order, a.W, a.H, a.tw, n_tiles, OUT, image, alpha, n_contrib)
     // Two pixels per thread where the patches of twice the size still fill the GPU. us with one and two, 100 k Gaussians: 920 tiles 81 and 95, 2,170 tiles 125
     // and 121 (400 k: 160 and 166), 4,293 tiles 201 and 183.
-    if (n_tiles >= 16 * num_sms()) LFS_EWA_FWD(2); else LFS_EWA_FWD(1);
+    if (n_tiles >= 16 * num_sms()) { LFS_EWA_FWD(launch, 1, out.slots, out); LFS_EWA_FWD(launch_beside, 2, n_tiles, out); }
+    else LFS_EWA_FWD(launch, 1, n_tiles, Outsized{});
 #undef LFS_EWA_FWD
     return check_launch("ewa_blend_fwd");
 }
@@ -671,13 +677,15 @@ int launch_ewa_blend_bwd(const EwaBlendArgs& a, const float* alpha, const int32_
     const int n_tiles = a.tw * a.th;
     if (n_tiles == 0) return LFS_OK;
     LFS_TIMED("ewa_blend_bwd", st);
-#define LFS_EWA_BWD(PX)                                                                                                             \
-    ewa_blend_bwd_kernel<PX><<<n_tiles * (2 / PX), 128, 0, st>>>(a.records, a.instance_ids, a.tile_offsets, a.overflow, a.background,      \
-                                                           a.tile_order, a.W, a.H, a.tw, alpha, n_contrib, grad_image, grad_alpha,   \
+    const Outsized out = outsized_lists(a.tile_order, n_tiles);
+#define LFS_EWA_BWD(LAUNCH, PX, TILES, OUT)                                                                                         \
+    LAUNCH(ewa_blend_bwd_kernel<PX>, (TILES) * (2 / PX), 128, 0, st, a.records, a.instance_ids, a.tile_offsets, a.overflow, a.background,      \
+                                                           a.tile_order, a.W, a.H, a.tw, n_tiles, OUT, alpha, n_contrib, grad_image, grad_alpha,   \
                                                            accum)
     // Two pixels per thread as in the forward; the sums of an entry are then formed half as often. us with one and two, 100 k Gaussians: 256 tiles 125 and 205, 510
     // tiles 134 and 147, 920 tiles 164 and 144, 4,293 tiles 473 and 310.
-    if (n_tiles >= 4 * num_sms()) LFS_EWA_BWD(2); else LFS_EWA_BWD(1);
+    if (n_tiles >= 4 * num_sms()) { LFS_EWA_BWD(launch, 1, out.slots, out); LFS_EWA_BWD(launch_beside, 2, n_tiles, out); }
+    else LFS_EWA_BWD(launch, 1, n_tiles, Outsized{});
 #undef LFS_EWA_BWD
     return check_launch("ewa_blend_bwd");
 }

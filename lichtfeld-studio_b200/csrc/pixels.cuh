@@ -1,7 +1,7 @@
 // The pixels of a thread of the blend kernels: one, or two in the halves of a 64-bit register.
 #pragma once
 
-#include <cuda_runtime.h>
+#include "common.cuh"
 
 namespace lfs {
 
@@ -55,5 +55,29 @@ struct Pixels<1> {
     static __device__ __forceinline__ void get(V v, float* a) { a[0] = v; }
     static __device__ __forceinline__ float sum(V v) { return v; }
 };
+
+// Few tiles can carry a large image (a distant object, the inset of a lens), and then the walk of the longest lists is what a kernel with two pixels per thread takes.
+// Lists that hold more than one in `share` of all instances are left to a launch with one pixel per thread, twice the warps, beside the other one. Forward +
+// backward of 200 k and 1.5 M Gaussians in us at 1920x1080, with two pixels everywhere and now: seen on some 64 tiles 318 + 322 and 142 + 218, 1014 + 970 and 752 + 688,
+// on 30 tiles 752 + 700 and 412 + 341, 3239 + 3056 and 1469 + 989; EWA, 30 tiles 705 + 725 and 458 + 437, 2896 + 3598 and 1817 + 1850. Where no list is that
+// long the second launch costs 1 to 2 us. On an image of few tiles lists of several times the mean are common, and the launch with two pixels has the cheaper
+// sums: there a list counts from one in half an SM on (EWA backward of 1.2 M on 858 tiles, 299 us: 333 with one in 107).
+struct Outsized { int share, slots; };   // slots: tiles that may have an outsized list, from the start of the launch order
+inline Outsized outsized_lists(const int32_t* tile_order, int n_tiles) {
+    const bool few = n_tiles < 16 * num_sms();
+    if (few && !tile_order) return Outsized{};   // the second launch would look at all the tiles: 10 us beside 260 (operators, 1,080 tiles)
+    const int share = few ? num_sms() / 2 : 3 * num_sms();
+    // fewer than `share` lists are outsized, and at most a quarter as many others come before the last of them, since the order tells lengths apart by quarters
+    // of a power of two; without an order any tile may have one
+    const int slots = share + share / 4 + 1;
+    return Outsized{share, !tile_order || n_tiles < slots ? n_tiles : slots};
+}
+__device__ __forceinline__ bool is_outsized(int32_t n, int32_t n_isects, const Outsized& o) { return (int64_t)n * o.share > n_isects; }
+// First thing in both kernels of such a pair; either also runs alone, with share = 0.
+template <int PX>
+__device__ __forceinline__ void side_by_side(const Outsized& o) {
+    if (PX == 1) { if (o.share) let_next_start(); }
+    else if (blockIdx.x == gridDim.x - 1) wait_for_previous();
+}
 
 }  // namespace lfs

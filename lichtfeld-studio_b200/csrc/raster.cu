@@ -290,26 +290,31 @@ struct FwdPatchWarp {
 // RGB_ED of gsplat/Rasterization.cpp:373-393); `normalize` divides it by max(alpha, 1e-10) on output (the
 // expected-depth modes of src/training/rasterization/rasterizer.cpp:186-198) and keeps the undivided value
 // in extra_sum for the backward.
-// Pixels whose pair is rejected go on with alpha = 0. A wide-angle camera's warps have many entries that reach no pixel, where leaving early pays
-// (6 M fisheye 1300 -> 1164 us); a planar camera's have few (1 M, 1296x840: 352 us against 361 with the vote).
+// Pixels whose pair is rejected go on with alpha = 0. VOTE: the warp leaves an entry that reaches no pixel. A wide-angle camera's warps have many of those
+// (6 M fisheye 1300 -> 1164 us), and so have the outsized lists (pixels.cuh), whose Gaussians are small beside a patch (two of 632 k entries 82 -> 55 ms); a planar
+// camera's others have few (1 M, 1296x840: 352 us against 361 with the vote; 16 k at 256x256 52 against 56).
 // Eight CTAs of 64 registers per SM; seven 378 us, nine the same.
-template <int MODEL, bool EXTRA, int PX>
+template <int MODEL, bool EXTRA, int PX, bool VOTE>
 __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,
     const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
-    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
+    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles, Outsized out,
     float* __restrict__ render, float* __restrict__ alphas, int32_t* __restrict__ last_ids, float* __restrict__ extra_sum) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using P = Pixels<PX>;
     using V = typename P::V;
-    constexpr bool kVote = MODEL != LFS_PINHOLE && MODEL != LFS_PINHOLE_OPENCV;
     FwdPatchWarp<PX>& sm = reinterpret_cast<FwdPatchWarp<PX>*>(smem_raw)[threadIdx.x >> 5];
 
+    side_by_side<PX>(out);
     if (overflow && *overflow) return;
     const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
     const int tile = tile_order ? tile_order[slot] : slot;
+    if (PX == 1 ? out.share > 0 : slot < out.slots) {
+        const int32_t all = load_count(n_isects_dev, n_isects_host), n = (tile == n_tiles - 1 ? all : tile_offsets[tile + 1]) - tile_offsets[tile];
+        if (is_outsized(n, all, out) != (PX == 1)) return;
+    }
     const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
     // warps tile the 16x16 block as patches of 8 x 4 PX pixels
     const int patch_x0 = (tile % tw) * 16 + (warp & 1) * 8, patch_y0 = (tile / tw) * 16 + (warp >> 1) * 4 * PX;
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
                 valid[q] = E[q] <= limit[q];
                 any_valid = any_valid || valid[q];
             }
-            if (kVote && !__any_sync(0xffffffffu, any_valid)) continue;
+            if (VOTE && !__any_sync(0xffffffffu, any_valid)) continue;
 #pragma unroll
             for (int q = 0; q < PX; ++q) den[q] = rcp_approx(den[q]);
             P::get(mul2(P::all(r0.w), mul2(f.E, P::make(den))), ex);
@@ -877,7 +882,7 @@ __global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
     const uint4* __restrict__ bounds, const uint32_t* __restrict__ flatten_ids,
     const int32_t* __restrict__ tile_offsets, const int32_t* __restrict__ n_isects_dev, int64_t n_isects_host,
     const int32_t* __restrict__ overflow, const float* __restrict__ background, const uint8_t* __restrict__ masks,
-    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles,
+    const int32_t* __restrict__ tile_order, int channels, int normalize, int W, int H, int tw, int n_tiles, Outsized out,
     const float* __restrict__ render_alphas, const int32_t* __restrict__ last_ids, const float* __restrict__ extra_sum,
     const float* __restrict__ v_render, const float* __restrict__ v_alphas, float* __restrict__ accum,
     float* __restrict__ accum_extra) {
@@ -886,9 +891,14 @@ __global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
     using V = typename P::V;
     BwdPatchWarp<PX>& sm = reinterpret_cast<BwdPatchWarp<PX>*>(smem_raw)[threadIdx.x >> 5];
 
+    side_by_side<PX>(out);
     if (overflow && *overflow) return;
     const int slot = PX == 2 ? blockIdx.x : blockIdx.x >> 1;
     const int tile = tile_order ? tile_order[slot] : slot;
+    const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
+    const int32_t range_start = tile_offsets[tile];
+    const int32_t range_end = (tile == n_tiles - 1) ? n_isects : tile_offsets[tile + 1];
+    if ((PX == 1 ? out.share > 0 : slot < out.slots) && is_outsized(range_end - range_start, n_isects, out) != (PX == 1)) return;
     if (masks && !masks[tile]) return;  // gsplat/RasterizeToPixelsFromWorld3DGSBwd.cu:84
     const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + (PX == 2 ? 0 : (blockIdx.x & 1) * 4);
     const CamDev& cam = cams[0];
@@ -950,9 +960,6 @@ __global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
     warp_bin_final = __reduce_max_sync(0xffffffffu, warp_bin_final);
     const PatchRays rays = patch_rays<MODEL, PX>(d, takes_part);
 
-    const int32_t n_isects = load_count(n_isects_dev, n_isects_host);
-    const int32_t range_start = tile_offsets[tile];
-    const int32_t range_end = (tile == n_tiles - 1) ? n_isects : tile_offsets[tile + 1];
     // back to front from the patch's last contributor: slot e of batch b holds list position top - 32 b - e
     const int32_t top = min(range_end - 1, warp_bin_final);
     const int total = top - range_start + 1, n_batches = (total + 31) / 32;
@@ -1061,7 +1068,7 @@ __global__ void __launch_bounds__(128, PX == 2 ? 5 : 6) raster_bwd_patch_kernel(
             const V omega = mul2(f.w, rden), qo = mul2(q, omega);
             const V th1 = mul2(qo, f.e1), th2 = mul2(qo, f.e2), t1 = mul2(th1, omega), t2 = mul2(th2, omega);
             const uint32_t g = st.sid[t];
-                        auto put = [&](int k, V v) { sm.red[k * kRedStride + lane] = P::sum(v); };
+            auto put = [&](int k, V v) { sm.red[k * kRedStride + lane] = P::sum(v); };
             put(0, th1); put(1, th2); put(2, mul2(th1, phi)); put(3, mul2(th2, phi));
             put(4, mul2(t1, f.e1)); put(5, mul2(t1, f.e2)); put(6, mul2(t2, f.e2)); put(7, mul2(q, phi));
             put(8, mul2(nfac, vcr)); put(9, mul2(nfac, vcg)); put(10, mul2(nfac, vcb)); put(11, q);
@@ -1586,15 +1593,23 @@ int launch_raster_fwd(const RasterArgs& a, float* render, float* alphas, int32_t
     // so: fisheye, 600 k, 4,096 tiles 239 and 344, 8,100 tiles 216 and 278, 14,400 tiles 309 and 271.
     const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
     const bool two = n_tiles >= (planar ? 8 : 80) * num_sms();
+    const Outsized out = outsized_lists(a.tile_order, n_tiles);
 #define LFS_FWD_RS(MODEL, EXTRA)                                                                                                    \
     raster_fwd_rs_kernel<MODEL, EXTRA><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev,       \
                                                                    a.n_isects_host, a.overflow, a.background, a.masks, a.tile_order, a.channels,   \
                                                                    a.normalize, a.W, a.H, a.tw, n_tiles, render, alphas, last_ids, extra_sum)
-#define LFS_FWD_PATCH(MODEL, EXTRA, PX)                                                                                             \
-    raster_fwd_patch_kernel<MODEL, EXTRA, PX><<<n_tiles * (2 / PX), 128, 4 * sizeof(FwdPatchWarp<PX>), st>>>(                       \
+#define LFS_FWD_PATCH(LAUNCH, MODEL, EXTRA, PX, VOTE, TILES, OUT)                                                                   \
+    LAUNCH(raster_fwd_patch_kernel<MODEL, EXTRA, PX, VOTE>, (TILES) * (2 / PX), 128, 4 * sizeof(FwdPatchWarp<PX>), st,              \
         a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow, a.background,  \
-        a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render, alphas, last_ids, extra_sum)
-#define LFS_FWD2(MODEL, EXTRA) do { if (two) LFS_FWD_PATCH(MODEL, EXTRA, 2); else LFS_FWD_PATCH(MODEL, EXTRA, 1); } while (0)
+        a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, OUT, render, alphas, last_ids, extra_sum)
+#define LFS_FWD2(MODEL, EXTRA)                                                                                                      \
+    do {                                                                                                                            \
+        constexpr bool kWide = MODEL != LFS_PINHOLE && MODEL != LFS_PINHOLE_OPENCV;                                                 \
+        if (!two) { LFS_FWD_PATCH(launch, MODEL, EXTRA, 1, kWide, n_tiles, Outsized{}); break; }                                    \
+        if (!out.share) { LFS_FWD_PATCH(launch, MODEL, EXTRA, 2, kWide, n_tiles, out); break; }                                     \
+        LFS_FWD_PATCH(launch, MODEL, EXTRA, 1, true, out.slots, out);                                                               \
+        LFS_FWD_PATCH(launch_beside, MODEL, EXTRA, 2, kWide, n_tiles, out);                                                         \
+    } while (0)
 #define LFS_FWD(MODEL) do { if (a.rolling) { if (extra) LFS_FWD_RS(MODEL, true); else LFS_FWD_RS(MODEL, false); }                   \
                             else if (extra) LFS_FWD2(MODEL, true); else LFS_FWD2(MODEL, false); } while (0)
     const bool extra = a.channels != 3;
@@ -1622,6 +1637,7 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
     const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
     const bool two = n_tiles >= (planar ? 4 : 40) * num_sms();
+    const Outsized out = outsized_lists(a.tile_order, n_tiles);
 #define LFS_BWD_RS(MODEL, EXTRA, XGRAD)                                                                                        \
     do {                                                                                                                       \
         constexpr int smem = (int)sizeof(BwdShared<64>);                                                                       \
@@ -1630,15 +1646,21 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
             a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
             v_alphas, accum, accum_extra);                                                                                     \
     } while (0)
-#define LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, PX)                                                                                 \
+#define LFS_BWD_PATCH(LAUNCH, MODEL, EXTRA, XGRAD, PX, TILES, OUT)                                                             \
     do {                                                                                                                       \
-        raster_bwd_patch_kernel<MODEL, EXTRA, XGRAD, PX><<<n_tiles * (2 / PX), 128, 4 * sizeof(BwdPatchWarp<PX>), st>>>(       \
+        LAUNCH(raster_bwd_patch_kernel<MODEL, EXTRA, XGRAD, PX>, (TILES) * (2 / PX), 128, 4 * sizeof(BwdPatchWarp<PX>), st,    \
             a.cam, a.records, a.cuts, a.n_cuts, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev, a.n_isects_host, a.overflow,    \
             a.background,                                                                                                      \
-            a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, render_alphas, last_ids, extra_sum, v_render, \
+            a.masks, a.tile_order, a.channels, a.normalize, a.W, a.H, a.tw, n_tiles, OUT, render_alphas, last_ids, extra_sum, v_render, \
             v_alphas, accum, accum_extra);                                                                                     \
     } while (0)
-#define LFS_BWD_ORIGIN(MODEL, EXTRA, XGRAD) do { if (two) LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, 2); else LFS_BWD_PATCH(MODEL, EXTRA, XGRAD, 1); } while (0)
+#define LFS_BWD_ORIGIN(MODEL, EXTRA, XGRAD)                                                                                    \
+    do {                                                                                                                       \
+        if (!two) { LFS_BWD_PATCH(launch, MODEL, EXTRA, XGRAD, 1, n_tiles, Outsized{}); break; }                               \
+        if (!out.share) { LFS_BWD_PATCH(launch, MODEL, EXTRA, XGRAD, 2, n_tiles, out); break; }                                \
+        LFS_BWD_PATCH(launch, MODEL, EXTRA, XGRAD, 1, out.slots, out);                                                         \
+        LFS_BWD_PATCH(launch_beside, MODEL, EXTRA, XGRAD, 2, n_tiles, out);                                                    \
+    } while (0)
 #define LFS_BWD_ANY(MODEL, EXTRA, XGRAD) do { if (a.rolling) LFS_BWD_RS(MODEL, EXTRA, XGRAD); else LFS_BWD_ORIGIN(MODEL, EXTRA, XGRAD); } while (0)
 #define LFS_BWD(KIND, MODEL)                                                                                                   \
     do { if (!extra) KIND(MODEL, false, false); else if (!xgrad) KIND(MODEL, true, false); else KIND(MODEL, true, true); } while (0)
