@@ -1589,10 +1589,10 @@ int launch_raster_fwd(const RasterArgs& a, float* render, float* alphas, int32_t
     if (a.channels != 1 && a.channels != 3 && a.channels != 4) { set_error("raster_fwd: channels must be 1, 3 or 4"); return LFS_EINVAL; }
     LFS_TIMED("raster_fwd", st);
     // Two pixels per thread where the patches of twice the size still fill the GPU. fwd us with one and two, 1296x840-like scenes of 100 k Gaussians: 510
-    // tiles 91 and 117, 920 tiles 98 and 104, 1,400 tiles 122 and 107, 2,170 tiles 158 and 129. A wide-angle lens shows the scene on a tenth of its tiles or
-    // so: fisheye, 600 k, 4,096 tiles 239 and 344, 8,100 tiles 216 and 278, 14,400 tiles 309 and 271.
-    const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
-    const bool two = n_tiles >= (planar ? 8 : 80) * num_sms();
+    // tiles 91 and 117, 920 tiles 98 and 104, 1,400 tiles 122 and 107, 2,170 tiles 158 and 129. A fisheye shows the scene on a tenth of its tiles or
+    // so: 600 k, 4,096 tiles 239 and 344, 8,100 tiles 216 and 278, 14,400 tiles 309 and 271. An equirectangular camera sees all around: 100 k and 600 k, 512
+    // tiles 68 and 81, 91 and 100, 2,048 tiles 131 and 110, 125 and 106, 8,192 tiles 416 and 303, 381 and 276.
+    const bool two = n_tiles >= (a.model == LFS_FISHEYE ? 80 : 8) * num_sms();
     const Outsized out = outsized_lists(a.tile_order, n_tiles);
 #define LFS_FWD_RS(MODEL, EXTRA)                                                                                                    \
     raster_fwd_rs_kernel<MODEL, EXTRA><<<n_tiles, kBlock, 0, st>>>(a.cam, a.records, a.bounds, a.flatten_ids, a.tile_offsets, a.n_isects_dev,       \
@@ -1633,10 +1633,10 @@ int launch_raster_bwd(const RasterArgs& a, const float* render_alphas, const int
     LFS_TIMED("raster_bwd", st);
     // Two pixels per thread where the patches of twice the size still fill the GPU (launch_raster_fwd). bwd us with one and two, planar, 100 k Gaussians: 256
     // tiles 190 and 266, 510 tiles 176 and 174 (20 k: 100 and 111, 400 k: 234 and 246), 920 tiles 211 and 165, 2,170 tiles 361 and 255; fisheye, 600 k: 4,096 tiles
-    // 395 and 453, 8,100 tiles 418 and 379.
+    // 395 and 453, 8,100 tiles 418 and 379; equirectangular, 100 k and 600 k: 512 tiles 103 and 108, 102 and 116, 2,048 tiles 239 and 179, 204 and 155, 8,192 tiles
+    // 756 and 519, 649 and 447.
     const bool extra = a.channels != 3, xgrad = extra && accum_extra != nullptr;
-    const bool planar = a.model == LFS_PINHOLE || a.model == LFS_PINHOLE_OPENCV;
-    const bool two = n_tiles >= (planar ? 4 : 40) * num_sms();
+    const bool two = n_tiles >= (a.model == LFS_FISHEYE ? 40 : 4) * num_sms();
     const Outsized out = outsized_lists(a.tile_order, n_tiles);
 #define LFS_BWD_RS(MODEL, EXTRA, XGRAD)                                                                                        \
     do {                                                                                                                       \

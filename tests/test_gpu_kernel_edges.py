@@ -160,3 +160,28 @@ def test_fewer_gaussians_than_the_workspace_was_made_for(pkg, synth, ewa):
 def test_offsets_of_a_list_that_was_given_up(pkg, n, C, tw, th):
     ids = torch.full((n,), torch.iinfo(torch.int64).max, dtype=torch.int64, device=DEV)
     assert (pkg.ops.intersect_offset(ids, C, tw, th) == 0).all()
+
+
+# An equirectangular camera inside the scene, on both sides of the tile counts at which a thread owns two pixels (4 per SM backward, 8 forward): 512, 1,250
+# and 2,048 tiles.
+@pytest.mark.parametrize("W,H", [(512, 256), (800, 400), (1024, 512)])
+def test_equirectangular_on_both_sides_of_the_two_pixel_rules(pkg, orc, synth, W, H):
+    tr, capi = pkg.trainer, pkg._capi
+    n, deg = 4000, 1
+    P = synth.make_gaussians(n, 6, "cube", deg)
+    P["scaling_raw"] = (P["scaling_raw"] + np.float32(0.7)).astype(np.float32)
+    vm = np.eye(4, dtype=np.float32)
+    vm[:3, 3] = [0.05, -0.02, 0.1]
+    K, bg = synth.intrinsics(100.0, 100.0, W / 2, H / 2), np.array([0.2, 0.4, 0.1], np.float32)
+    fwd = orc.render_fwd(P, vm, K, W, H, deg, background=bg, camera_model=orc.EQUIRECTANGULAR)
+    model = tr.SplatData(n, (deg + 1) ** 2, DEV).load(P)
+    grads, rast = model.like(), tr.Rasterizer(model, W, H, deg, camera_model=capi.EQUIRECTANGULAR)
+    out = rast.forward(tr.Camera(T(vm), T(K), W, H, capi.EQUIRECTANGULAR), T(bg))
+    # azimuths and elevations come from single-precision arc functions on both sides: a projection that rounds differently moves a tile of a faint rim
+    diff = np.abs(out.image.cpu().numpy() - fwd["render"]).max(-1)
+    assert diff.max() < 1e-2 and (diff > 1e-4).sum() <= W * H // 500, (diff.max(), (diff > 1e-4).sum())
+    v = np.random.default_rng(1).normal(size=(H, W, 3)).astype(np.float32) * 1e-3
+    bwd = orc.render_bwd(P, fwd, vm, K, W, H, deg, v, background=bg, camera_model=orc.EQUIRECTANGULAR)
+    rast.backward(T(v), grads, T(bg))
+    for name in NAMES:
+        assert rel_l2(grads.tensor(name).cpu().numpy(), bwd[name]) < 2e-3, name
