@@ -1,9 +1,31 @@
-// The pixels of a thread of the blend kernels: one, or two in the halves of a 64-bit register.
+// What the blend kernels of both paths share: copies and approximations, the pixels of a thread (one, or two in the halves of a 64-bit register), and how the
+// tiles are dealt to kernels with one pixel per thread and with two.
 #pragma once
 
 #include "common.cuh"
 
 namespace lfs {
+
+// 16-byte asynchronous copies to shared memory.
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// One special-function instruction (relative error 2^-23); __fdividef spends four more on denominators above 2^126.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float exp2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 
 // Two pixels of one thread as one operand of the packed fp32 instructions (one issue slot for both, each half rounded like the
 // scalar instruction). A factor that both pixels share costs nothing to replicate: in a loop of nothing else, four packed fmas with

@@ -75,17 +75,6 @@ __device__ __forceinline__ RayForms ray_forms(const float4& r0, const float4& r1
     f.den = f.w * f.w + f.E;
     return f;
 }
-// One special-function instruction (relative error 2^-23); __fdividef spends four more on denominators above 2^126.
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float exp2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 // The directions of a warp's patch as an axis-aligned box around a centre (camera space; depth 0 for the planar models), over
 // the pixels that take part.
@@ -174,14 +163,6 @@ struct Stage {
     float4 rec[BATCH * 4];  // packed records
     uint4 box[BATCH];       // rows of RasterArgs::bounds
 };
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // Each thread owns kParts quarter-record slots q = k * BLOCK + tid of a batch: entry q >> 2, part q & 3.
 template <int BATCH, int BLOCK>

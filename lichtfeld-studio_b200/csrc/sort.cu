@@ -5,7 +5,7 @@
 //
 // The reference sorts n_isects 12-byte (int64 key, int32 value) pairs over 32 + tile_bits + cam_bits bits. The order that comes out
 // (camera, tile, depth bits, ties by ascending flattened Gaussian index) is a total one inside each tile, so nothing has to be stable:
-// the per-Gaussian stage counts the instances of every tile (one reduction to memory per instance), one CTA turns the counts into
+// the per-Gaussian stage counts the instances of every tile (one reduction to memory per instance), one cluster turns the counts into
 // offsets, the instances drop into their tile's range in any order (8 bytes each, one returning atomic), and every range is sorted by
 // (depth bits, index) where it fits into shared memory. Against two global radix sorts (depth of N, then tile of the instances) the
 // instances are written twice instead of six times and there are three launches instead of eleven. All of the list build, projection's
@@ -1012,7 +1012,9 @@ static int scatter_parts(int64_t total) {
     return parts < 4 ? 1 : (int)min(parts, (int64_t)8);
 }
 // The per-Gaussian stage has one warp per 32 Gaussians, so where scatter_parts takes more and the image is large beside the Gaussians' number the
-// counting gets a launch of its own (the same scene: projection 77 us, of which 61 went into the counting; 77 -> 16 and 17 for the launch).
+// counting gets a launch of its own (the same scene: projection 77 us, of which 61 went into the counting; 77 -> 16 and 17 for the launch). Render of 3 k, 10 k and 60 k
+// Gaussians, counted in the projection and apart, us: 4,293 tiles, 10 and 40 tiles a Gaussian: 84 and 86, 110 and 112, 199 and 205; 244 and 190, 288 and 234, 535 and 503;
+// 18,025 tiles: 180 and 173, 267 and 259, 556 and 554; 824 and 565, 1002 and 746, 428 and 264. It costs 7 us at most and saves up to 260.
 bool count_tiles_apart(int64_t N, int64_t bins) { return scatter_parts(N) > 1 && 8 * bins >= N; }
 
 int build_tile_lists(const TileListArgs& a, cudaStream_t st) {
