@@ -1,6 +1,5 @@
-"""Sizes at which the kernels change path or leave a remainder: list sorts on both sides of the look-back limit, tiles of the
-sort and of the emission, grids on both sides of the two-pixel backward, camera boxes under strong distortion, and the row
-stores of tensors that are not 16-byte aligned."""
+"""Sizes at which the kernels change path or leave a remainder: lists counted and filled by one or by several warps per 32 Gaussians, grids on both sides
+of the two-pixel rules, camera boxes under strong distortion, and the row stores of tensors that are not 16-byte aligned."""
 import numpy as np
 import pytest
 import torch
@@ -16,11 +15,11 @@ def T(a):
     return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
 
 
-# n: one below / at / above the 256 and 1024 Gaussians of an emission tile, the 2048 keys of a sort tile, the 2,097,152 keys of a
-# look-back depth sort; radius (in tiles): 2.4 M x 1 and 45 k x 15 x 15 instances lie on either side of the 6,291,456 of the tile sort
+# n: a part of a warp, of a CTA of 256, and more; at and above the 75,776 Gaussians up to which several warps share 32 of them (148 SMs); millions of
+# them; radius: rectangles of one tile to 15 x 15
 @pytest.mark.parametrize("n,tw,th,rad", [(1, 3, 2, 8.0), (255, 5, 4, 20.0), (256, 5, 4, 20.0), (1025, 40, 3, 40.0), (2047, 9, 7, 24.0),
                                          (2049, 9, 7, 24.0), (70_001, 60, 40, 30.0), (2_097_152, 200, 150, 4.0),
-                                         (2_097_153, 200, 150, 4.0), (45_001, 60, 50, 120.0)])
+                                         (2_097_153, 200, 150, 4.0), (45_001, 60, 50, 120.0), (75_776, 60, 40, 30.0), (75_777, 60, 40, 30.0)])
 def test_tile_lists_against_a_stable_sort(pkg, n, tw, th, rad):
     gen = torch.Generator(device=DEV).manual_seed(n)
     u = lambda *s: torch.rand(s, generator=gen, device=DEV)
@@ -48,8 +47,10 @@ def test_tile_lists_against_a_stable_sort(pkg, n, tw, th, rad):
     assert torch.equal(ids, key[order]) and torch.equal(flat.long(), g[order])
 
 
-# 37 x 32 = 1184 tiles = eight per SM of a 148-SM GPU: the first size of the two-pixel backward; one column fewer stays below
-@pytest.mark.parametrize("W,H,lens,mode", [(592, 512, False, 0), (576, 512, False, 0), (601, 523, True, 0), (601, 523, False, 4)])
+# On a 148-SM GPU 37 x 16 tiles are four per SM, the first size of the two-pixel backward, 37 x 32 eight, the first of the two-pixel forward; one column
+# fewer stays below
+@pytest.mark.parametrize("W,H,lens,mode", [(592, 512, False, 0), (576, 512, False, 0), (601, 523, True, 0), (601, 523, False, 4), (592, 256, False, 0),
+                                           (576, 256, False, 0), (592, 256, True, 4), (576, 256, True, 4)])
 def test_backward_on_both_sides_of_the_two_pixel_rule(pkg, orc, synth, W, H, lens, mode):
     tr = pkg.trainer
     n, deg = 6000, 1
@@ -63,7 +64,10 @@ def test_backward_on_both_sides_of_the_two_pixel_rule(pkg, orc, synth, W, H, len
     grads = model.like()
     rast = tr.Rasterizer(model, W, H, deg, render_mode=mode)
     cam = tr.Camera(T(vm), T(K), W, H, **(dict(radial=T(radial), tangential=T(tangential)) if lens else {}))
-    rast.forward(cam, T(bg))
+    out = rast.forward(cam, T(bg))
+    # a pair at the 1/255 cut moves its pixel by 4e-3 of a colour at most
+    diff = np.abs(out.render.cpu().numpy() - fwd["render"])[..., :3].max(-1)
+    assert diff.max() < 1e-2 and (diff > 1e-4).sum() <= W * H // 500, (diff.max(), (diff > 1e-4).sum())
     rng = np.random.default_rng(1)
     v_r = rng.normal(size=(H, W, CH)).astype(np.float32) * 1e-3
     if CH == 4:
@@ -77,7 +81,8 @@ def test_backward_on_both_sides_of_the_two_pixel_rule(pkg, orc, synth, W, H, len
         assert rel_l2(grads.tensor(name).cpu().numpy(), bwd[name]) < 2e-3, name
 
 
-@pytest.mark.parametrize("W,H", [(592, 512), (576, 512)])
+# four tiles per SM backward, sixteen (37 x 64) forward
+@pytest.mark.parametrize("W,H", [(592, 512), (576, 512), (592, 256), (576, 256), (592, 1024), (576, 1024)])
 def test_ewa_backward_on_both_sides_of_the_two_pixel_rule(pkg, orc, synth, W, H):
     tr = pkg.trainer
     n, deg = 6000, 1
@@ -87,7 +92,9 @@ def test_ewa_backward_on_both_sides_of_the_two_pixel_rule(pkg, orc, synth, W, H)
     fwd = orc.ewa_forward(P, vm, campos, W, H, K[0, 0], K[1, 1], K[0, 2], K[1, 2], 4, background=bg)
     model = tr.SplatData(n, 4, DEV).load(P)
     rast, grads = tr.FastRasterizer(model, W, H, deg), model.like()
-    rast.forward(tr.Camera(T(vm), T(K), W, H), T(bg), cam_position=T(np.asarray(campos, np.float32)))
+    out = rast.forward(tr.Camera(T(vm), T(K), W, H), T(bg), cam_position=T(np.asarray(campos, np.float32)))
+    diff = np.abs(out.image.cpu().numpy() - fwd["image"]).max(0)
+    assert diff.max() < 1e-2 and (diff > 1e-4).sum() <= W * H // 500, (diff.max(), (diff > 1e-4).sum())
     gi = np.random.default_rng(2).normal(size=(3, H, W)).astype(np.float32) * 1e-3
     bwd = orc.ewa_backward(P, fwd, gi)
     rast.backward(T(gi), grads, T(bg))
@@ -133,8 +140,7 @@ def test_ssim_tile_edges(pkg, orc, H, W):
     assert rel_l2(g.cpu().numpy(), orc.fusedssim_backward(a[0], b[0], dl[0], *ref[1:])) < 1e-4
 
 
-# A model with room for 2,100,000 Gaussians that holds 2,090,000: the workspace is made for the former, whose depth sort is of the
-# other kind than the latter's
+# A model with room for 2,100,000 Gaussians that holds 2,090,000: the workspace is sized for the former and laid out for the latter
 @pytest.mark.parametrize("ewa", [False, True])
 def test_fewer_gaussians_than_the_workspace_was_made_for(pkg, synth, ewa):
     tr = pkg.trainer
@@ -155,7 +161,7 @@ def test_fewer_gaussians_than_the_workspace_was_made_for(pkg, synth, ewa):
     assert torch.equal(image, make(exact).forward(cam, bg).image)
 
 
-# What the list build leaves when it gives up: the largest key throughout. Its offsets are empty lists for every tile.
+# Keys that belong to no tile, the largest there are: every tile's list is empty
 @pytest.mark.parametrize("n,C,tw,th", [(1, 1, 3, 2), (5000, 1, 81, 53), (300, 3, 7, 5)])
 def test_offsets_of_a_list_that_was_given_up(pkg, n, C, tw, th):
     ids = torch.full((n,), torch.iinfo(torch.int64).max, dtype=torch.int64, device=DEV)

@@ -98,3 +98,20 @@ def test_far_lists_of_a_render(pkg, synth, ewa):
         if not ewa:
             assert (torch.diff(rast.state()["tile_offsets"]) >= 65_536).any()
     assert images[0].abs().max() > 0.1 and torch.equal(*images)
+
+
+# The fused path counts the instances in the projection, or, where few Gaussians face many tiles (eight tiles a Gaussian or more while several warps share
+# 32 of them, up to 75,776 on 148 SMs), in a launch of its own: 192 and 9,600 tiles, a Gaussian on either side of each limit.
+@pytest.mark.parametrize("n,W,H", [(1535, 256, 192), (1536, 256, 192), (1537, 256, 192), (75_776, 1920, 1280), (75_777, 1920, 1280)])
+def test_lists_of_a_render(pkg, synth, n, W, H):
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a, F)).cuda()
+    tr = pkg.trainer
+    model = tr.SplatData(n, 1, "cuda:0").load(synth.make_gaussians(n, 2, "cube", 0))
+    rast = tr.Rasterizer(model, W, H, 0, isect_capacity=1 << 22)
+    rast.forward(tr.Camera(T(synth.look_at_origin([0.3, -4.0, 0.4])), T(synth.intrinsics(1.1 * W, 1.1 * W, W / 2, H / 2)), W, H), None)
+    st = {k: v.cpu().numpy() for k, v in rast.state().items() if torch.is_tensor(v)}
+    tw, th = W // 16, H // 16
+    keys, ids = _instances(st["means2d"][None], st["radii"][None], st["depths"][None], 16, tw, th)
+    order = np.argsort(keys, kind="stable")
+    assert ids.size > 2 * n and np.array_equal(st["flatten_ids"], ids[order])
+    assert np.array_equal(st["tile_offsets"], np.searchsorted(keys[order] >> 32, np.arange(tw * th + 1)))
