@@ -86,13 +86,13 @@ struct Pixels<1> {
 // sums: there a list counts from one in half an SM on (EWA backward of 1.2 M on 858 tiles, 299 us: 333 with one in 107).
 struct Outsized { int share, slots; };   // slots: tiles that may have an outsized list, from the start of the launch order
 inline Outsized outsized_lists(const int32_t* tile_order, int n_tiles) {
-    const bool few = n_tiles < 16 * num_sms();
-    if (few && !tile_order) return Outsized{};   // the second launch would look at all the tiles: 10 us beside 260 (operators, 1,080 tiles)
-    const int share = few ? num_sms() / 2 : 3 * num_sms();
+    // without an order (operators) the second launch would have to look at every tile: 10 us beside 350, 1.0 M on 5,922 tiles 14 beside 445 and 17 beside 895
+    if (!tile_order) return Outsized{};
+    const int share = n_tiles >= 16 * num_sms() ? 3 * num_sms() : num_sms() / 2;
     // fewer than `share` lists are outsized, and at most a quarter as many others come before the last of them, since the order tells lengths apart by quarters
-    // of a power of two; without an order any tile may have one
+    // of a power of two
     const int slots = share + share / 4 + 1;
-    return Outsized{share, !tile_order || n_tiles < slots ? n_tiles : slots};
+    return Outsized{share, n_tiles < slots ? n_tiles : slots};
 }
 __device__ __forceinline__ bool is_outsized(int32_t n, int32_t n_isects, const Outsized& o) { return (int64_t)n * o.share > n_isects; }
 // First thing in both kernels of such a pair; either also runs alone, with share = 0.

@@ -274,7 +274,8 @@ struct FwdPatchWarp {
 // Pixels whose pair is rejected go on with alpha = 0. VOTE: the warp leaves an entry that reaches no pixel. A wide-angle camera's warps have many of those
 // (6 M fisheye 1300 -> 1164 us), and so have the outsized lists (pixels.cuh), whose Gaussians are small beside a patch (two of 632 k entries 82 -> 55 ms); a planar
 // camera's others have few (1 M, 1296x840: 352 us against 361 with the vote; 16 k at 256x256 52 against 56).
-// Eight CTAs of 64 registers per SM; seven 378 us, nine the same.
+// Eight CTAs of 64 registers per SM; seven 378 us, nine the same. The other cameras' two-pixel kernels spill 16 to 36 bytes and still want eight: opencv
+// 400 k 326 us against 340 with seven, 6 M fisheye 1143 against 1209.
 template <int MODEL, bool EXTRA, int PX, bool VOTE>
 __global__ void __launch_bounds__(128, 8) raster_fwd_patch_kernel(
     const CamDev* __restrict__ cams, const float4* __restrict__ records, const float4* __restrict__ cuts, int64_t n_cuts,

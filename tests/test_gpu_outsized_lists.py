@@ -55,7 +55,7 @@ def test_three_linear_forms(pkg, orc, synth, W, H, behind):
     for name in NAMES:
         # random output gradients cancel over the pixels of a Gaussian: a pair on the other side of the cut weighs a thousandth
         assert rel_l2(grads.tensor(name).cpu().numpy(), bwd[name]) < 2e-3, name
-    # the operators have no launch order: every tile is looked at
+    # the operators have no launch order and walk all lists alike
     quats, scales, opac = orc.act_quat(P["rotation_raw"])[0], orc.act_scale(P["scaling_raw"]), orc.act_opacity(P["opacity_raw"])
     render, _, _ = pkg.ops.rasterize_to_pixels_from_world_3dgs_fwd(
         T(P["means"]), T(quats), T(scales), T(fwd["colors"][None]), T(opac[None]), T(bg[None]), None, W, H, 16, T(vm[None]), None, T(K[None]), 0,
