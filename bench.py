@@ -42,14 +42,12 @@ if str(ROOT) not in sys.path:
 
 LRS = [1.6e-4, 2.5e-3, 1.25e-4, 5e-3, 1e-3, 5e-2]  # means, sh0, shN, scaling, rotation, opacity
 METRIC = "train steps/s (fwd+loss+bwd+Adam)"
-# Profiler counters of ONE raster_bwd_patch_kernel launch on 1 M Gaussians at 1296x840 (ncu, --clock-control none): DRAM bytes read + written,
-# share of issue slots used, share of issued warp instructions on the FMA pipe relative to the FP32 peak rate. They are
-# reported next to the event-timed figures because a kernel's traffic and pipe utilisation cannot be read outside a profiler. The
-# kernel's arithmetic per pair is that of the scalar kernel before it, whose flops are counted here (packed instructions hide two in one).
-NCU_RASTER_BWD = {"dram_bytes": 132e6, "issue_slots_active": 0.71, "shared_pipe": 0.80,
-                  # 371e6 scalar warp instructions on the FMA pipe x 32 lanes x 2 flop over the 4.24e8 pairs of the captured launch
-                  "executed_flop_per_pair": 56.1}
-NCU_RASTER_FWD_FLOP = 137e6 * 32 * 2   # FMA-pipe warp instructions of one launch of the scalar forward on the same workload x lanes x 2
+# Profiler counters of ONE raster_bwd_patch_kernel launch of this benchmark's step, 1 M Gaussians at 1296x840 (ncu, --clock-control none): DRAM bytes read +
+# written, share of issue slots used, share of the shared-memory data pipe. They are reported next to the event-timed figures because a kernel's traffic and pipe
+# utilisation cannot be read outside a profiler. Flops: thread instructions fadd + fmul + 2 ffma + 2 (fadd2 + fmul2) + 4 ffma2, the packed ones holding two pixels.
+NCU_RASTER_BWD = {"dram_bytes": 121e6, "issue_slots_active": 0.68, "shared_pipe": 0.79,
+                  "executed_flop_per_pair": 14.78e9 / 4.244e8}   # over the pairs at positions up to the pixels' last contributors
+NCU_RASTER_FWD_FLOP = 7.6e9   # one raster_fwd_patch_kernel launch, counted alike
 
 
 def load_peaks():
@@ -613,8 +611,10 @@ def run_ours(args):
         small = dp_self_check(pkg, dev, rank, world, args.dp_mode, dp_split, dp_rank1, args.dp_ordering, args.dp_multicast, args.dp_color_after_projection)
         dp_check = {"ok": bool(same_params and small["ok"]), "bench_parameters_identical_on_all_ranks": bool(same_params), **small}
     if rank == 0:
-        # every bracket holds one launch; camera set-up and the loss' last kernel have none
-        gpu_launches_step = sum(len(vs) / n_prof for vs in kernels.values()) + 2
+        # every bracket holds one launch, those of the blend kernels two where a thread owns two pixels (8 tiles per SM forward, 4 backward); camera set-up
+        # and the loss' last kernel have none
+        tiles_per_sm = ((W + 15) // 16) * ((H + 15) // 16) / torch.cuda.get_device_properties(dev).multi_processor_count
+        gpu_launches_step = sum(len(vs) / n_prof for vs in kernels.values()) + 2 + cams_per_rank * ((tiles_per_sm >= 8) + (tiles_per_sm >= 4))
         st = rast.state()
         last, offs = st["last_ids"].long(), st["tile_offsets"].long()
         tw = (W + 15) // 16
@@ -658,7 +658,7 @@ def run_ours(args):
             adam_kernel = "adam_sh_rank1_kernel"
             adam_note = f"(24 B x {rest} shN floats + 24 B) x {n} Gaussians"
         adam_gbs = adam_bytes / (t_adam * 1e-3) / 1e9 if np.isfinite(t_adam) else None   # N > 1: Adam runs inside the exchange
-        list_keys = ("tile_scan", "tile_scatter", "tile_sort")
+        list_keys = ("tile_scan", "tile_scatter", "tile_far", "tile_sort")
         t_lists = sum(float(np.sum(kernels[k])) / calls for k in list_keys if k in kernels)
         V, I = float(status[2]), float(status[1])
         tiles = ((W + 15) // 16) * ((H + 15) // 16)
@@ -673,7 +673,7 @@ def run_ours(args):
                                          "frac": ach_fwd / fp32_peak if ncu else None,
                                          "reference_arithmetic": 70.0 * q_list / (t_fwd * 1e-3) / 1e12,
                                          "note": f"executed flops from the profiler capture; reference_arithmetic: 70 flop x {q_list} list entries x pixels (upper bound of pairs visited), may exceed the peak"},
-                 "roofline_tile_lists": {"kernel": "tile_scan + tile_scatter + tile_sort", "bound": "hbm",
+                 "roofline_tile_lists": {"kernel": "tile_scan + tile_scatter + tile_far + tile_sort", "bound": "hbm",
                                          "achieved": list_bytes / (t_lists * 1e-3) / 1e9 if t_lists else None, "peak": hbm_peak, "unit": "GB/s",
                                          "frac": list_bytes / (t_lists * 1e-3) / 1e9 / hbm_peak if t_lists else None, "ms": t_lists,
                                          "note": f"20 V + 36 I + 4 tiles bytes, of {peak_kind}"},
@@ -838,7 +838,7 @@ def run_forward_only(args):
     torch.cuda.synchronize()
     km = {k: float(np.mean(v)) for k, v in _kernel_means(capi.profile_collect()).items()}
     capi.profile_enable(False)
-    sort_ms = sum(km.get(k, 0.0) for k in ("tile_scan", "tile_scatter", "tile_sort"))
+    sort_ms = sum(km.get(k, 0.0) for k in ("tile_scan", "tile_scatter", "tile_far", "tile_sort"))
     hbm_peak, kind = load_peaks()
     V, I = float(np.mean(n_vis)), float(np.mean(n_isects))
     tiles = ((W + 15) // 16) * ((H + 15) // 16)
@@ -848,11 +848,11 @@ def run_forward_only(args):
            "data": "synthetic", "config": {"workload": args.workload, "gaussians": n, "image": [W, H], "poses": len(cams),
                                            "camera": "fisheye" if cfg["model"] == 2 else "pinhole"},
            "clocks": clocks, "n_isects_mean": I, "n_isects_max": int(np.max(n_isects)), "n_visible_mean": V, "tile_list_ms": sort_ms,
-           "kernel_ms": km, "gpu_launches": int(reps * len(cams) * 6),
+           "kernel_ms": km, "gpu_launches": int(reps * len(cams) * 8),   # camera, projection, scan, scatter, far, sort, two blends
            "roofline": {"kernel": "tile-list stage (scan + scatter + sort)", "bound": "hbm",
                         "achieved": sort_bytes / (sort_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                         "frac": sort_bytes / (sort_ms * 1e-3) / 1e9 / hbm_peak, "traffic": None,
-                        "note": f"20 V + 36 I + 4 tiles bytes, of {kind}; three launches"}}
+                        "note": f"20 V + 36 I + 4 tiles bytes, of {kind}; four launches"}}
     print(json.dumps(_finite(out)), flush=True)
 
 
@@ -921,7 +921,7 @@ def run_ewa(args):
            "dtype": "f32", "data": "synthetic",
            "config": {"workload": "ewa_1m", "gaussians": n, "image": [W, H], "sh_degree": deg, "path": "default (non --gut) EWA rasterizer",
                       "l2": "inputs larger than L2 (parameters, moments and gradients streamed per step)"},
-           "clocks": clocks, "n_instances": int(st[1]), "n_visible": int(st[2]), "kernel_ms": km, "gpu_launches": int(args.steps * 12),
+           "clocks": clocks, "n_instances": int(st[1]), "n_visible": int(st[2]), "kernel_ms": km, "gpu_launches": int(args.steps * 15),
            "roofline": {"kernel": "adam_groups_kernel", "bound": "hbm", "achieved": adam_bytes / (t_adam * 1e-3) / 1e9, "peak": hbm_peak,
                         "unit": "GB/s", "frac": adam_bytes / (t_adam * 1e-3) / 1e9 / hbm_peak, "traffic": None,
                         "note": f"the blend kernels are instruction-issue bound; the streaming kernel shown is Adam, of {kind}"}}
